@@ -674,13 +674,16 @@ struct Rec {
     void run(int pass, uint32_t level = 0, uint32_t cycle = 0) {
         timed(pass, [&] { wig::launch_pass(ln.Bt, ln.S, b->hw[0].D, pass, level, cycle, s); });
     }
-    // cgStart + cgJoin as the fast forms run them (profiled as the two passes)
+    // cgStart + cgJoin as a step runs them (profiled as the two passes)
     void labels() {
         timed(WIG_PASS_CG_START, [&] { wig::launch_labels(ln.Bt, ln.S, s, 0); });
         timed(WIG_PASS_CG_JOIN, [&] { wig::launch_labels(ln.Bt, ln.S, s, 1); });
     }
-    void norm(int which, uint32_t cycle) {
-        timed(WIG_SLOT_NORM, [&] { wig::launch_norm(b->hw[0].D, which, cycle, s); });
+    void norm() {
+        timed(WIG_SLOT_NORM, [&] { wig::launch_norm(b->hw[0].D, s); });
+    }
+    void cycle_end() {
+        timed(WIG_SLOT_NORM, [&] { wig::launch_cycle_end(ln.Bt, b->hw[0].D, s); });
     }
     void sched(int phase) {
         cudaEvent_t a = nullptr, e = nullptr;
@@ -786,57 +789,117 @@ uint32_t record_book(Rec& R) {
     return R.launches;
 }
 
-// Records the plain form's step of world 0 (one kernel per reference pass,
-// every iteration encoded) on stream s; returns the kernels launched.
-uint32_t record_step(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags, bool shifted, cudaStream_t s, Prof* prof) {
+// Captures a WHILE node at the capture point of stream `outer`, its body
+// from the launches fn(stream, handle) makes on stream `inner`.  The
+// condition starts true; a kernel of the body sets it each time round.
+template <class Fn>
+int capture_while(cudaStream_t outer, cudaStream_t inner, Fn fn) {
+    cudaStreamCaptureStatus cs;
+    cudaGraph_t g = nullptr;
+    const cudaGraphNode_t* deps = nullptr;
+    size_t nd = 0;
+    CUDA_TRY(cudaStreamGetCaptureInfo(outer, &cs, nullptr, &g, &deps, &nd));
+    cudaGraphConditionalHandle handle;
+    CUDA_TRY(cudaGraphConditionalHandleCreate(&handle, g, 1, cudaGraphCondAssignDefault));
+    cudaGraphNodeParams cp = {};
+    cp.type = cudaGraphNodeTypeConditional;
+    cp.conditional.handle = handle;
+    cp.conditional.type = cudaGraphCondTypeWhile;
+    cp.conditional.size = 1;
+    cudaGraphNode_t cnode;
+    CUDA_TRY(cudaGraphAddNode(&cnode, g, deps, nd, &cp));
+    CUDA_TRY(cudaStreamUpdateCaptureDependencies(outer, &cnode, 1, cudaStreamSetCaptureDependencies));
+    cudaGraph_t body = cp.conditional.phGraph_out[0];
+    CUDA_TRY(cudaStreamBeginCaptureToGraph(inner, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
+    fn((unsigned long long)handle);
+    cudaGraph_t captured = nullptr;
+    CUDA_TRY(cudaStreamEndCapture(inner, &captured));
+    return WIG_OK;
+}
+
+// One iteration of the plain form's solve of world 0 (js/sim.js:2551-2591),
+// the passes taking the iteration from the world's StepState; `sh`: the
+// tiling of its first relaxation (its second is on the other, so every
+// iteration starts on the same one).
+void record_cycle(Rec& R, bool sh) {
+    const uint32_t deepest = R.b->L[0].levels, cycle = wig::CYCLE_LOOP;
+    R.run(WIG_PASS_RELAX_RIMS, 0, cycle);
+    R.run(sh ? WIG_PASS_RELAX_SHIFTED : WIG_PASS_RELAX, 0, cycle);
+    for (uint32_t l = 1; l <= deepest; l++) {
+        R.run(WIG_PASS_RESTRICT, l, cycle);
+        if (l < deepest) {
+            R.run(WIG_PASS_SMOOTH_RED, l, cycle);
+            R.run(WIG_PASS_SMOOTH_BLACK, l, cycle);
+        }
+    }
+    R.run(WIG_PASS_SOLVE, deepest, cycle);
+    for (uint32_t l = deepest - 1; l >= 1; l--) {
+        R.run(WIG_PASS_PROLONG, l, cycle);
+        R.run(WIG_PASS_SMOOTH_RED, l, cycle);
+        R.run(WIG_PASS_SMOOTH_BLACK, l, cycle);
+    }
+    R.run(WIG_PASS_PROLONG_FINE, 0, cycle);
+    R.run(WIG_PASS_RELAX_RIMS, 0, cycle);
+    R.run(sh ? WIG_PASS_RELAX : WIG_PASS_RELAX_SHIFTED, 0, cycle);
+    R.run(WIG_PASS_CG_RHO, 0, cycle);
+    R.run(WIG_PASS_CG_BETA, 0, cycle);
+    R.run(WIG_PASS_CG_DIRECTION, 0, cycle);
+    if (has_bodies(R.b)) R.run(WIG_PASS_CG_BODY_P, 0, cycle);
+    R.run(WIG_PASS_CG_APPLY, 0, cycle);
+    R.run(WIG_PASS_CG_ALPHA, 0, cycle);
+    R.run(WIG_PASS_CG_UPDATE, 0, cycle);
+    R.cycle_end();
+}
+
+// Records the plain form's step of world 0 (one kernel per reference pass)
+// on stream s.  With `capture`, s is capturing into a graph and the
+// iterations are a WHILE node's body captured on the lane's second stream:
+// a step launches the iterations it needs, where encoding all max_cycles of
+// them, each kernel returning at once past convergence, took 5.9 ms a step
+// of the 256x256 body tank (64 encoded, 8-11 needed; 18 ms its first step).
+// Else they are launched from the host, each decided by reading back the
+// device's verdict.  *outside and *body as in record_step_fast.
+int record_step(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags, bool shifted, cudaStream_t s, Prof* prof,
+                bool capture, uint32_t* outside, uint32_t* body) {
     Rec R{b, ln, s, prof};
-    const bool tol = (flags & WIG_STEP_TOLERANCE) != 0u;
-    if (flags & WIG_STEP_BOOKKEEPING_ONLY) return record_book(R);
+    *body = 0;
+    if (flags & WIG_STEP_BOOKKEEPING_ONLY) {
+        *outside = record_book(R);
+        return WIG_OK;
+    }
     record_pre(R, (flags & WIG_STEP_VISCOUS) != 0u);
-    const uint32_t deepest = b->L[0].levels;
-    R.run(WIG_PASS_CG_START);
-    R.run(WIG_PASS_CG_JOIN);
+    R.labels();
     R.run(WIG_PASS_CG_ANCHOR);
     const bool bodies = has_bodies(b);
     if (bodies) R.run(WIG_PASS_CG_BODY_X);
     R.run(WIG_PASS_CG_RESIDUAL);
-    if (tol) R.norm(0, 0);
+    if (flags & WIG_STEP_TOLERANCE) R.norm();
     R.run(WIG_PASS_CG_PREPARE);
-    bool sh = shifted;
-    for (uint32_t cycle = 0; cycle < max_cycles; cycle++) {
-        R.run(WIG_PASS_RELAX_RIMS, 0, cycle);
-        R.run(sh ? WIG_PASS_RELAX_SHIFTED : WIG_PASS_RELAX, 0, cycle);
-        sh = !sh;
-        for (uint32_t l = 1; l <= deepest; l++) {
-            R.run(WIG_PASS_RESTRICT, l, cycle);
-            if (l < deepest) {
-                R.run(WIG_PASS_SMOOTH_RED, l, cycle);
-                R.run(WIG_PASS_SMOOTH_BLACK, l, cycle);
-            }
+    ln.Bt.max_cycles = max_cycles;
+    ln.Bt.cond = 0;
+    if (capture) {
+        int rc = capture_while(s, ln.cap2, [&](unsigned long long cond) {
+            ln.Bt.cond = cond;
+            Rec C{b, ln, ln.cap2, nullptr};
+            record_cycle(C, shifted);
+            *body = C.launches;
+            ln.Bt.cond = 0;
+        });
+        if (rc) return rc;
+    } else {
+        uint32_t* cont = reinterpret_cast<uint32_t*>(ln.h_rsub);  // a word of pinned scratch
+        for (uint32_t c = 0; c < max_cycles; c++) {
+            record_cycle(R, shifted);
+            CUDA_TRY(cudaMemcpyAsync(cont, ln.d_loop, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+            CUDA_TRY(cudaStreamSynchronize(s));
+            if (!*cont) break;
         }
-        R.run(WIG_PASS_SOLVE, deepest, cycle);
-        for (uint32_t l = deepest - 1; l >= 1; l--) {
-            R.run(WIG_PASS_PROLONG, l, cycle);
-            R.run(WIG_PASS_SMOOTH_RED, l, cycle);
-            R.run(WIG_PASS_SMOOTH_BLACK, l, cycle);
-        }
-        R.run(WIG_PASS_PROLONG_FINE, 0, cycle);
-        R.run(WIG_PASS_RELAX_RIMS, 0, cycle);
-        R.run(sh ? WIG_PASS_RELAX_SHIFTED : WIG_PASS_RELAX, 0, cycle);
-        sh = !sh;
-        R.run(WIG_PASS_CG_RHO, 0, cycle);
-        R.run(WIG_PASS_CG_BETA, 0, cycle);
-        R.run(WIG_PASS_CG_DIRECTION, 0, cycle);
-        if (bodies) R.run(WIG_PASS_CG_BODY_P, 0, cycle);
-        R.run(WIG_PASS_CG_APPLY, 0, cycle);
-        R.run(WIG_PASS_CG_ALPHA, 0, cycle);
-        R.run(WIG_PASS_CG_UPDATE, 0, cycle);
-        if (tol) R.norm(1, cycle);
     }
     R.run(WIG_PASS_CG_FINISH);
     if (bodies) R.run(WIG_PASS_CG_BODY_F);
     record_post(R);
-    return R.launches;
+    *outside = R.launches;
+    return WIG_OK;
 }
 
 // Records the fast form's step of the lane's worlds.  With `capture`, s is
@@ -881,29 +944,13 @@ int record_step_fast(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags
         R.launches++;
         *body = 0;
     } else if (capture) {
-        cudaStreamCaptureStatus cs;
-        cudaGraph_t g = nullptr;
-        const cudaGraphNode_t* deps = nullptr;
-        size_t nd = 0;
-        CUDA_TRY(cudaStreamGetCaptureInfo(s, &cs, nullptr, &g, &deps, &nd));
-        cudaGraphConditionalHandle handle;
-        CUDA_TRY(cudaGraphConditionalHandleCreate(&handle, g, 1, cudaGraphCondAssignDefault));
-        cudaGraphNodeParams cp = {};
-        cp.type = cudaGraphNodeTypeConditional;
-        cp.conditional.handle = handle;
-        cp.conditional.type = cudaGraphCondTypeWhile;
-        cp.conditional.size = 1;
-        cudaGraphNode_t cnode;
-        CUDA_TRY(cudaGraphAddNode(&cnode, g, deps, nd, &cp));
-        CUDA_TRY(cudaStreamUpdateCaptureDependencies(s, &cnode, 1, cudaStreamSetCaptureDependencies));
-        cudaGraph_t bodyGraph = cp.conditional.phGraph_out[0];
-        CUDA_TRY(cudaStreamBeginCaptureToGraph(ln.cap2, bodyGraph, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
-        wig::Batch Bc = ln.Bt;
-        Bc.cond = (unsigned long long)handle;
         wig::NestCapture nest{ln.cap3, cudaSuccess};
-        *body = wig::fast_cycle(Bc, ln.S, one, ln.cap2, nullptr, &nest);
-        cudaGraph_t captured = nullptr;
-        CUDA_TRY(cudaStreamEndCapture(ln.cap2, &captured));
+        int rc = capture_while(s, ln.cap2, [&](unsigned long long cond) {
+            wig::Batch Bc = ln.Bt;
+            Bc.cond = cond;
+            *body = wig::fast_cycle(Bc, ln.S, one, ln.cap2, nullptr, &nest);
+        });
+        if (rc) return rc;
         CUDA_TRY(nest.err);
     } else {
         uint32_t* cont = reinterpret_cast<uint32_t*>(ln.h_rsub);  // a word of pinned scratch
@@ -1087,17 +1134,14 @@ int batch_step(wig_batch* b, const StepArgs& a) {
         Graph G;
         CUDA_TRY(cudaStreamBeginCapture(ln.cap, cudaStreamCaptureModeThreadLocal));
         uint32_t n = 0, nb = 0;
-        if (plain) {
-            n = record_step(b, ln, a.max_cycles, shape, sh, ln.cap, nullptr);
-        } else {
-            int rc2 = record_step_fast(b, ln, a.max_cycles, shape, sh, ln.cap, nullptr, true, &n, &nb);
-            if (rc2) {
-                std::string m = g_last_error;
-                cudaGraph_t junk = nullptr;
-                cudaStreamEndCapture(ln.cap, &junk);
-                if (junk) cudaGraphDestroy(junk);
-                return fail(rc2, m);
-            }
+        const int rc2 = plain ? record_step(b, ln, a.max_cycles, shape, sh, ln.cap, nullptr, true, &n, &nb)
+                              : record_step_fast(b, ln, a.max_cycles, shape, sh, ln.cap, nullptr, true, &n, &nb);
+        if (rc2) {
+            std::string m = g_last_error;
+            cudaGraph_t junk = nullptr;
+            cudaStreamEndCapture(ln.cap, &junk);
+            if (junk) cudaGraphDestroy(junk);
+            return fail(rc2, m);
         }
         cudaError_t e = cudaStreamEndCapture(ln.cap, &G.g);
         if (e != cudaSuccess) return fail(WIG_E_CUDA, std::string("stream capture: ") + cudaGetErrorString(e));
@@ -1140,15 +1184,15 @@ int batch_step_profile(wig_batch* b, const StepArgs& a, float* ms_out, uint32_t*
     ln.last_body = 0;
     uint32_t bucket = 0;
     ln.S = step_shape(b, a, &bucket);
+    uint32_t n = 0, nb = 0;
     if (plain) {
-        ln.last_launches = record_step(b, ln, a.max_cycles, shape, sh, a.s, &prof);
+        rc = record_step(b, ln, a.max_cycles, shape, sh, a.s, &prof, false, &n, &nb);
     } else {
         zero_dirty(b, a);
-        uint32_t n = 0, nb = 0;
         rc = record_step_fast(b, ln, a.max_cycles, shape, sh, a.s, &prof, false, &n, &nb);
-        if (rc) return rc;
-        ln.last_launches = n;
     }
+    if (rc) return rc;
+    ln.last_launches = n;
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaStreamSynchronize(a.s));
     for (int k = 0; k < WIG_PROFILE_SLOTS; k++) { ms_out[k] = 0.0f; calls_out[k] = 0u; }

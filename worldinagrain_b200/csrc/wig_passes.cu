@@ -34,6 +34,17 @@ __device__ __forceinline__ I2 lidCell(const W& w, uint32_t wid) {
 
 __device__ __forceinline__ uint32_t vload(const uint32_t* p) { return *(const volatile uint32_t*)p; }
 
+// A solve pass's iteration: the one given, which does nothing once the solve
+// has converged (fluid.wgsl:2223-2226), or (CYCLE_LOOP) the one the step's
+// loop is in, which the loop starts only when it has not.
+__device__ __forceinline__ bool skips(const W& w, uint32_t& cycle) {
+    if (cycle == CYCLE_LOOP) {
+        cycle = w.D.st->cycle;
+        return false;
+    }
+    return w.converged(cycle);
+}
+
 // union-find over G_REGION words (label.wgsl:27-55), lock-free by atomicMin.
 __device__ uint32_t ufFind(const W& w, uint32_t i) {
     uint32_t x = i;
@@ -1407,8 +1418,8 @@ __global__ void k_cgJoin(Batch Bt) {
         }
     }
 }
-// cgStart with the block's own part of cgJoin's labelling, for the fast
-// forms' steps (the per-pass dispatch and the plain form keep k_cgStart and
+// cgStart with the block's own part of cgJoin's labelling, for the
+// steps (the per-pass dispatch keeps k_cgStart and
 // k_cgJoin): each liquid cell's region link goes straight to the smallest
 // index of the liquid cells its block joins it to (min-label propagation
 // over the block's 4-neighbour liquid edges in shared memory, at most 63
@@ -1563,20 +1574,36 @@ __device__ double sumBlocks64(const W& w, const double* buf, int comp, double* s
     return r;
 }
 
-// ||b||^2 of the tolerance form (after cgResidual), and ||r||/||b|| (after
-// cgUpdate): one CTA of 256.
-__global__ void __launch_bounds__(256) k_norm(Dev D, int which, uint32_t cycle) {
+// ||b||^2 of the tolerance form, after cgResidual: one CTA of 256.
+__global__ void __launch_bounds__(256) k_norm(Dev D) {
     W w(D);
     __shared__ double s[256];
-    if (which == 1 && w.converged(cycle)) return;
     double v = sumBlocks64(w, D.norm64, 0, s);
     if (threadIdx.x == 0) {
-        if (which == 0) {
-            D.st->bnorm2 = v;
-            D.st->rel = 1.0;
-        } else {
-            D.st->rel = D.st->bnorm2 > 0.0 ? sqrt(v / D.st->bnorm2) : 0.0;
-        }
+        D.st->bnorm2 = v;
+        D.st->rel = 1.0;
+    }
+}
+
+// An iteration's end, after cgUpdate: the tolerance form's ||r||/||b||, and
+// whether the step's loop runs the next one: not once the solve has
+// converged (fluid.wgsl:2223-2226), nor past max_cycles.  The iterations the
+// reference still dispatches then only clear their next residual slots
+// (cgUpdate's first lines): cleared here.  One CTA of 256.
+__global__ void __launch_bounds__(256) k_cycleEnd(Dev D, uint32_t max_cycles, unsigned long long cond, uint32_t* loop) {
+    W w(D);
+    __shared__ double s[256];
+    double v = 0.0;
+    if (D.st->tol_mode) v = sumBlocks64(w, D.norm64, 0, s);
+    if (threadIdx.x == 0) {
+        if (D.st->tol_mode) D.st->rel = D.st->bnorm2 > 0.0 ? sqrt(v / D.st->bnorm2) : 0.0;
+        const uint32_t next = D.st->cycle + 1u;
+        const bool more = next < max_cycles && !w.converged(next);
+        D.st->cycle = next;
+        *loop = more ? 1u : 0u;
+        if (cond) cudaGraphSetConditional(cond, more ? 1u : 0u);
+        if (!more)
+            for (uint32_t c = next; c < max_cycles; c++) D.blocks[w.countSlot(COUNT_RESIDUAL + (c + 1u) % 3u)] = 0u;
     }
 }
 
@@ -1585,7 +1612,7 @@ __global__ void __launch_bounds__(256) k_norm(Dev D, int which, uint32_t cycle) 
 // relaxRims (fluid.wgsl:2096-2107)
 __global__ void k_relaxRims(Dev D, uint32_t cycle) {
     W w(D);
-    if (w.converged(cycle)) return;
+    if (skips(w, cycle)) return;
     FOR_ACTIVE(D, w, wid) {
         I2 c = lidCell(w, wid);
         if (!w.inWorld(c)) continue;
@@ -1616,7 +1643,7 @@ __global__ void __launch_bounds__(64) k_relax(Dev D, int shift, uint32_t cycle) 
     W w(D);
     __shared__ float tpx[RIM * RIM], tpy[RIM * RIM], trho[RIM * RIM], tshare[RIM * RIM];
     __shared__ int s_live, s_ox, s_oy;
-    if (w.converged(cycle)) return;
+    if (skips(w, cycle)) return;
     const uint32_t na = w.activeCount();
     const uint32_t total = na + (shift ? D.edge_tiles : 0u);
     for (uint32_t j = blockIdx.x; j < total; j += gridDim.x) {
@@ -1701,7 +1728,7 @@ __global__ void __launch_bounds__(64) k_relax(Dev D, int shift, uint32_t cycle) 
 __global__ void k_restrict(Dev D, uint32_t l, uint32_t cycle) {
     W w(D);
     I2 c{(int)(blockIdx.x * blockDim.x + threadIdx.x), (int)(blockIdx.y * blockDim.y + threadIdx.y)};
-    if (!inLevel(D, l, c) || w.activeCount() == 0u || w.converged(cycle)) return;
+    if (!inLevel(D, l, c) || w.activeCount() == 0u || skips(w, cycle)) return;
     uint32_t at = levelSlot(D, l, c);
     float4* F4 = reinterpret_cast<float4*>(D.field);
     int span = 1 << l;
@@ -1737,7 +1764,7 @@ __global__ void k_restrict(Dev D, uint32_t l, uint32_t cycle) {
 __global__ void k_smooth(Dev D, uint32_t l, int color, uint32_t cycle) {
     W w(D);
     I2 c{(int)(blockIdx.x * blockDim.x + threadIdx.x), (int)(blockIdx.y * blockDim.y + threadIdx.y)};
-    if (!inLevel(D, l, c) || ((c.x + c.y) & 1) != color || w.activeCount() == 0u || w.converged(cycle)) return;
+    if (!inLevel(D, l, c) || ((c.x + c.y) & 1) != color || w.activeCount() == 0u || skips(w, cycle)) return;
     uint32_t at = levelSlot(D, l, c);
     float rho = w.fv(at + 1u)[0];
     if (rho <= 0.0f) return;
@@ -1757,7 +1784,7 @@ __global__ void k_smooth(Dev D, uint32_t l, int color, uint32_t cycle) {
 __global__ void __launch_bounds__(512) k_solve(Dev D, uint32_t l, uint32_t cycle) {
     W w(D);
     __shared__ float px[WIG_MG_COARSEST], py[WIG_MG_COARSEST], rx[WIG_MG_COARSEST], ry[WIG_MG_COARSEST], rh[WIG_MG_COARSEST];
-    if (w.converged(cycle)) return;
+    if (skips(w, cycle)) return;
     const int sx = (int)D.level_w[l], sy = (int)D.level_h[l];
     const uint32_t n = min((uint32_t)(sx * sy), WIG_MG_COARSEST);
     const uint32_t j = threadIdx.x;
@@ -1802,7 +1829,7 @@ __global__ void __launch_bounds__(512) k_solve(Dev D, uint32_t l, uint32_t cycle
 __global__ void k_prolong(Dev D, uint32_t l, uint32_t cycle) {
     W w(D);
     I2 c{(int)(blockIdx.x * blockDim.x + threadIdx.x), (int)(blockIdx.y * blockDim.y + threadIdx.y)};
-    if (!inLevel(D, l, c) || w.activeCount() == 0u || w.converged(cycle)) return;
+    if (!inLevel(D, l, c) || w.activeCount() == 0u || skips(w, cycle)) return;
     uint32_t at = levelSlot(D, l, c);
     if (w.fv(at + 1u)[0] > 0.0f) {
         V2 e = prolonged(w, l, c);
@@ -1815,7 +1842,7 @@ __global__ void k_prolong(Dev D, uint32_t l, uint32_t cycle) {
 // prolongFine (fluid.wgsl:2500-2512)
 __global__ void k_prolongFine(Dev D, uint32_t cycle) {
     W w(D);
-    if (w.converged(cycle)) return;
+    if (skips(w, cycle)) return;
     FOR_ACTIVE(D, w, wid) {
         I2 c = lidCell(w, wid);
         if (!w.inWorld(c)) continue;
@@ -1890,7 +1917,7 @@ __global__ void __launch_bounds__(64) k_cgRho(Dev D, uint32_t cycle) {
     W w(D);
     __shared__ float sx[64], sy[64];
     __shared__ double dx[64], dy[64];
-    if (w.converged(cycle)) return;
+    if (skips(w, cycle)) return;
     const bool f64 = D.st->f64 != 0u;
     FOR_ACTIVE(D, w, wid) {
         I2 c = lidCell(w, wid);
@@ -1926,7 +1953,7 @@ __global__ void __launch_bounds__(256) k_cgBeta(Dev D, uint32_t cycle) {
     W w(D);
     __shared__ float sx[256], sy[256];
     __shared__ double s64[256];
-    if (w.converged(cycle) || w.activeCount() == 0u) return;
+    if (skips(w, cycle) || w.activeCount() == 0u) return;
     float* at = D.cg + 4u * (size_t)(D.C + D.B);
     if (D.st->f64) {
         double rz = sumBlocks64(w, D.part64, 0, s64);
@@ -1954,7 +1981,7 @@ __global__ void __launch_bounds__(256) k_cgBeta(Dev D, uint32_t cycle) {
 // cgDirection (fluid.wgsl:2767-2776)
 __global__ void k_cgDirection(Dev D, uint32_t cycle) {
     W w(D);
-    if (w.converged(cycle)) return;
+    if (skips(w, cycle)) return;
     const float beta = D.cg[4u * (size_t)(D.C + D.B) + 2u];
     const bool f64 = D.st->f64 != 0u;
     const double beta64 = D.st->beta;
@@ -1991,7 +2018,7 @@ __global__ void __launch_bounds__(64) k_cgApply(Dev D, uint32_t cycle) {
     W w(D);
     __shared__ float sx[64], sy[64];
     __shared__ double dx[64];
-    if (w.converged(cycle)) return;
+    if (skips(w, cycle)) return;
     const bool f64 = D.st->f64 != 0u;
     FOR_ACTIVE(D, w, wid) {
         I2 c = lidCell(w, wid);
@@ -2025,7 +2052,7 @@ __global__ void __launch_bounds__(256) k_cgAlpha(Dev D, uint32_t cycle) {
     W w(D);
     __shared__ float sx[256], sy[256];
     __shared__ double s64[256];
-    if (w.converged(cycle) || w.activeCount() == 0u) return;
+    if (skips(w, cycle) || w.activeCount() == 0u) return;
     // the bodies' sums of this iteration's direction, done with, emptied for
     // the iteration after next (fluid.wgsl:2808-2813)
     if (D.pushes) {
@@ -2060,11 +2087,12 @@ __global__ void __launch_bounds__(64) k_cgUpdate(Dev D, uint32_t cycle) {
     W w(D);
     __shared__ uint32_t most;
     __shared__ double sb[64];
+    const bool skip = skips(w, cycle);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         D.blocks[w.countSlot(COUNT_RESIDUAL + (cycle + 1u) % 3u)] = 0u;
-        if (!w.converged(cycle)) D.blocks[w.countSlot(COUNT_CYCLES)] += 1u;
+        if (!skip) D.blocks[w.countSlot(COUNT_CYCLES)] += 1u;
     }
-    if (w.converged(cycle)) return;
+    if (skip) return;
     const float alpha = D.cg[4u * (size_t)(D.C + D.B) + 1u];
     const bool f64 = D.st->f64 != 0u, tol = D.st->tol_mode != 0u;
     const double alpha64 = D.st->alpha;
@@ -2788,7 +2816,7 @@ __global__ void __launch_bounds__(64) k_bodyFaces(Dev D) {
 // the pressure it ends with.
 __global__ void __launch_bounds__(64) k_cgBody(Dev D, int which, uint32_t cycle) {
     W w(D);
-    if (which == 1 && w.converged(cycle)) return;
+    if (which == 1 && skips(w, cycle)) return;
     FOR_ACTIVE(D, w, wid) {
         const I2 c = lidCell(w, wid);
         if (!w.inWorld(c) || w.gridAt(c).z <= 0.0f) continue;
@@ -2945,9 +2973,10 @@ void launch_labels(const Batch& Bt, const BatchShape& S, cudaStream_t s, int par
     else k_cgJoinAcross<<<A, 64, 0, s>>>(Bt);
 }
 
-int launch_norm(const Dev& D, int which, uint32_t cycle, cudaStream_t s) {
-    k_norm<<<1, 256, 0, s>>>(D, which, cycle);
-    return WIG_OK;
+void launch_norm(const Dev& D, cudaStream_t s) { k_norm<<<1, 256, 0, s>>>(D); }
+
+void launch_cycle_end(const Batch& Bt, const Dev& D, cudaStream_t s) {
+    k_cycleEnd<<<1, 256, 0, s>>>(D, Bt.max_cycles, Bt.cond, Bt.loop);
 }
 
 }  // namespace wig

@@ -21,16 +21,23 @@ struct BatchShape {
 // CTAs for a kernel over list `list` with `per_sm` CTAs a multiprocessor.
 unsigned list_grid(const BatchShape& S, uint32_t list, unsigned per_sm);
 
+// A solve pass's `cycle` in a step's loop: the iteration the world's
+// StepState says (a pass of that iteration, not converged before it).
+constexpr uint32_t CYCLE_LOOP = 0xffffffffu;
+
 // One reference pass (enum wig_pass) at Level (level, cycle), on stream s:
 // over the batch's work lists, or (the plain form's solve passes) over
 // world 0, whose descriptor D0 is.
 int launch_pass(const Batch& Bt, const BatchShape& S, const Dev& D0, int pass, uint32_t level, uint32_t cycle,
                 cudaStream_t s);
-// The fast forms' cgStart + cgJoin: part 0 cgStart with each block's own
+// A step's cgStart + cgJoin: part 0 cgStart with each block's own
 // labelling (k_cgStartLocal), part 1 the joins between blocks; the same
 // regions and roots as the two passes.
 void launch_labels(const Batch& Bt, const BatchShape& S, cudaStream_t s, int part);
-// The plain form's tolerance norms on world 0: which 0 = ||b||^2 after
-// cgResidual, 1 = ||r||/||b|| after cgUpdate.
-int launch_norm(const Dev& D, int which, uint32_t cycle, cudaStream_t s);
+// The plain form's ||b||^2 of world 0 after cgResidual (the tolerance form).
+void launch_norm(const Dev& D, cudaStream_t s);
+// The end of an iteration of the plain form's loop on world 0, after
+// cgUpdate: the tolerance form's ||r||/||b||, and the loop's verdict into
+// Bt.loop and the WHILE node's condition Bt.cond (0: none).
+void launch_cycle_end(const Batch& Bt, const Dev& D, cudaStream_t s);
 }  // namespace wig
