@@ -1085,7 +1085,7 @@ void zero_dirty(wig_batch* b, const StepArgs& a) {
     for (uint32_t i = 0; i < a.count; i++) {
         const uint32_t k = a.worlds[i];
         if (!b->dirty[k]) continue;
-        wig::fast_zero_level0(b->hw[k].S, b->hw[k].D.C, a.s);
+        wig::fast_zero_level0(b->hw[k], a.s);
         b->dirty[k] = 0;
     }
 }

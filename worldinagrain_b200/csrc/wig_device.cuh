@@ -136,8 +136,8 @@ struct Dev {
     const wig_elem* elems;
     uint32_t n_elems;
     StepState* st;
-    double* part64;   // 2 doubles per block: FP64 partial sums
-    double* norm64;   // 2 doubles per block: FP64 norms' partials
+    double* part64;   // FP64 partial sums: component c of block b at c * B + b
+    double* norm64;   // FP64 norms' partials, likewise
     uint32_t* motion; // binding 12, the free bodies' table (null: no free bodies)
     uint32_t* pushes; // binding 16, the solve's exact sums of what it does to each body
     uint32_t* stamps; // binding 14, the bodies' buffer, read for its swept stamps (null: no seams or cups)
@@ -416,8 +416,8 @@ struct FastW {
     float *rimx, *rimy;        // level 0: the relaxation's rim snapshot
     float *X, *R, *P, *Q;      // level 0: CG's x, r, p, A p
     float* P2;                 // level 0: p of the fast form's odd iterations (p of the even ones in P)
-    float* part32;             // 2 per block
-    double* part64;            // 2 per block
+    float* part32;             // partial sums: component c of block b at c * B + b
+    double* part64;            // the same in FP64
     uint32_t lc;               // first level the one-CTA coarse kernel solves
     uint32_t lp;               // first level CTA 0 of the persistent solve holds
 };
@@ -428,6 +428,15 @@ struct alignas(16) World {
     FastW S;
 };
 static_assert(sizeof(World) % 16 == 0, "World copies in 16-byte words");
+
+// Block n's partial sums back to +0 (a block not worked on).
+__device__ __forceinline__ void zeroPartials(const Dev& D, const FastW& F, uint32_t n) {
+    for (uint32_t c = 0; c < 2u; c++) {
+        F.part32[c * D.B + n] = 0.0f;
+        F.part64[c * D.B + n] = 0.0;
+        D.norm64[c * D.B + n] = 0.0;
+    }
+}
 
 // Work lists.  A kernel's CTAs take the items of one list in turn (grid
 // stride); an item is a world of the batch (its index in the world table, the

@@ -16,9 +16,10 @@
 //     threadfence reduction: the same fixed tree order, one launch fewer);
 //   * the iterations are the body of a CUDA-graph WHILE node: a step runs as
 //     many as it needs, with no launches for the converged ones.
-// The scratch keeps one invariant: level-0 arrays are zero outside the
-// blocks worked on (zeroed at allocation, when a world is uploaded, and as
-// blocks retire), where the reference's field is zero too.
+// The scratch keeps one invariant: level-0 arrays and the blocks' partial
+// sums are zero outside the blocks worked on (zeroed at allocation, when a
+// world is uploaded, and as blocks retire), where the reference's field is
+// zero too.
 
 #include <algorithm>
 
@@ -114,7 +115,7 @@ __device__ T sumBlocks256(const W& w, const T* part, int comp, T* s) {
         for (int u = 0; u < 16; u++) {
             const uint32_t k = k0 + 256u * (uint32_t)u;
             st[u] = k < B ? __ldcg(&state[k]) : 0u;
-            v[u] = k < B ? __ldcg(&part[2u * k + (uint32_t)comp]) : T(0);
+            v[u] = k < B ? __ldcg(&part[(uint32_t)comp * B + k]) : T(0);
         }
 #pragma unroll
         for (int u = 0; u < 16; u++)
@@ -153,8 +154,8 @@ __device__ void sumBlocks256x2(const W& w, const T* part, T* s0, T* s1, T* out0,
         for (int u = 0; u < 16; u++) {
             const uint32_t k = k0 + 256u * (uint32_t)u;
             st[u] = k < B ? __ldcg(&state[k]) : 0u;
-            v0[u] = k < B ? __ldcg(&part[2u * k]) : T(0);
-            v1[u] = k < B ? __ldcg(&part[2u * k + 1u]) : T(0);
+            v0[u] = k < B ? __ldcg(&part[k]) : T(0);
+            v1[u] = k < B ? __ldcg(&part[B + k]) : T(0);
         }
 #pragma unroll
         for (int u = 0; u < 16; u++)
@@ -352,7 +353,7 @@ __global__ void __launch_bounds__(256) k_fSetup(Batch Bt, const __grid_constant_
         if (tol) {
             double v = tree64x4(s64, b2);
             if (valid && (threadIdx.x & 63u) == 0u) {
-                D.norm64[2u * w.blockIndex(w.activeBlock(wid))] = v;
+                D.norm64[w.blockIndex(w.activeBlock(wid))] = v;
             }
             pend_ += min(4u, na - g * 4u);
             if (flushTiles(Bt, g_it, e_it, it, pend_, &D.st->fdone[0], na)) {
@@ -382,13 +383,14 @@ __global__ void __launch_bounds__(256) k_fSetup(Batch Bt, const __grid_constant_
     }
 }
 
-// The level-0 arrays neighbours read, zeroed in the blocks not worked on
-// (the invariant), for worlds whose scratch is lent by a pool for the step:
+// The level-0 arrays neighbours read and the block partials, zeroed in the
+// blocks not worked on (the invariant), for worlds whose scratch is lent by a pool for the step:
 // a CTA per block of the world.
 __global__ void k_fZeroIdle(Batch Bt) {
     FOR_ITEMS(Bt, L_WB, it) {
         FAST_ITEM_G(Bt, it, D, F, w, n);
         if (D.st->book != 0u || (D.blocks[w.stateSlot(n)] & ACTIVE) != 0u) continue;
+        if (threadIdx.x == 0) zeroPartials(D, F, n);
         for (uint32_t t = threadIdx.x; t < 64u; t += blockDim.x) {
             const I2 bq_ = w.blockAt(n);
             I2 c{bq_.x * BLOCK + (int)(t & 7u), bq_.y * BLOCK + (int)(t >> 3)};
@@ -400,8 +402,11 @@ __global__ void k_fZeroIdle(Batch Bt) {
     }
 }
 
-// Zeroes the level-0 arrays the neighbours read (after an upload).
-__global__ void k_fZero(FastW F, uint32_t C) {
+// Zeroes the level-0 arrays the neighbours read and the block partials
+// (after an upload).
+__global__ void k_fZero(Dev D, FastW F) {
+    const uint32_t C = D.C;
+    for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < D.B; n += gridDim.x * blockDim.x) zeroPartials(D, F, n);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < C; i += gridDim.x * blockDim.x) {
         F.L[0].px[i] = 0.0f; F.L[0].py[i] = 0.0f; F.L[0].rho[i] = 0.0f;
         F.rimx[i] = 0.0f; F.rimy[i] = 0.0f; F.P[i] = 0.0f;
@@ -1773,115 +1778,244 @@ __global__ void k_fProlongFine(Batch Bt, const __grid_constant__ WorldSrc<ONE> s
 
 // ================================================================ conjugate gradients
 
-// cgRho + cgBeta (fluid.wgsl:2736-2764): four tiles a 256-thread CTA; the CTA
-// that counts a world's last tile sums its blocks' partials (sumBlocks' order).
-template <bool ONE>
-__global__ void __launch_bounds__(256) k_fRhoBeta(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
-    __shared__ WorldCopy wc_;
-    if (!ONE) worldCopyInit(wc_);
-    __shared__ float sx[256], sy[256];
-    __shared__ double s64[256], s64b[256];
-    __shared__ float ux[2][128], uy[2][128];
-    __shared__ double ex64[2][128], ey64[2][128];
-    uint32_t pend_ = 0;  // tiles finished of the current world, not yet counted
-    uint32_t par = 0;    // the tree buffers of this item
-    FOR_ITEMS(Bt, L_ACT4, it) {
-        FAST_ITEM(Bt, it, D, F, w, g);
-        if (D.st->cont == 0u) continue;
-        const bool f64 = D.st->f64 != 0u;
-        const uint32_t cycle = D.st->cycle;
-        const Lvl& L0 = F.L[0];
-        const uint32_t na = w.activeCount();
-        const uint32_t wid = g * 4u + (threadIdx.x >> 6);
-        const bool valid = wid < na;
-        float vx = 0.0f, vy = 0.0f;
-        double ex = 0.0, ey = 0.0;
-        if (valid) {
-            I2 c = tileCell(w, wid);
-            if (w.inWorld(c)) {
-                uint32_t i = w.cellIndex(c);
-                // loaded beside the density, not after it: one dependent
-                // load fewer on the item's path
-                const float rho = L0.rho[i], z = L0.px[i], r = F.R[i], q = F.Q[i];
-                if (rho > 0.0f) {
-                    vx = r * z;
-                    vy = q * z;
-                    ex = (double)r * (double)z;
-                    ey = (double)q * (double)z;
-                }
-            }
-        }
-        // the f32 trees only without FP64 dots, which read none of them
-        if (f64) {
-            tilePut(ex64[par], ex);
-            tilePut(ey64[par], ey);
-        } else {
-            tilePut(ux[par], vx);
-            tilePut(uy[par], vy);
-        }
-        __syncthreads();
-        float tx = 0.0f, ty = 0.0f;
-        double dx = 0.0, dy = 0.0;
-        if (f64) {
-            dx = tileSum(ex64[par], ex);
-            dy = tileSum(ey64[par], ey);
-        } else {
-            tx = tileSum(ux[par], vx);
-            ty = tileSum(uy[par], vy);
-        }
-        par ^= 1u;
-        if (valid && (threadIdx.x & 63u) == 0u) {
-            const uint32_t b = w.blockIndex(w.activeBlock(wid));
-            if (f64) {
-                F.part64[2u * b] = dx;
-                F.part64[2u * b + 1u] = dy;
-            } else {
-                F.part32[2u * b] = tx;
-                F.part32[2u * b + 1u] = ty;
-            }
-        }
-        pend_ += min(4u, na - g * 4u);
-        if (flushTiles(Bt, g_it, e_it, it, pend_, &D.st->fdone[1], na)) {
-            if (f64) {
-                double rz, zq;
-                sumBlocks256x2(w, F.part64, s64, s64b, &rz, &zq);
-                if (threadIdx.x == 0) {
-                    double beta = (cycle == 0u || D.st->pq <= 0.0) ? 0.0 : -zq / D.st->pq;
-                    D.st->rz = rz;
-                    D.st->beta = beta;
-                }
-            } else {
-                float rz, zq;
-                sumBlocks256x2(w, F.part32, sx, sy, &rz, &zq);
-                if (threadIdx.x == 0) {
-                    float beta = (cycle == 0u || D.st->pq32 <= 0.0f) ? 0.0f : -zq / D.st->pq32;
-                    D.st->rz32 = rz;
-                    D.st->beta32 = beta;
-                }
-            }
-        }
+// The CG kernels: a warp a tile of 8x8 cells, lane l the cells l and l + 32
+// of the tile (rows l / 8 and l / 8 + 4), so a tile's tree of 64 (its first
+// step adds l + 32 to l, the rest are shuffles) needs no barrier and no
+// shared memory; a warp has two tiles' loads in flight.  A CTA takes a
+// contiguous run of the active blocks, world by world, and counts each
+// world's tiles once.  What bounds them is latency: per launch the chain
+// state -> block index -> cells -> partial -> count -> the last CTA's sum
+// of all the partials, against 2-5 us for their bytes on the 1024x1024
+// world.  As four 64-thread tiles a 256-thread CTA under a barrier an item
+// they took 15-18 us a launch there (83-95 us on the 2048x2048 column).
+constexpr int CG_THREADS = 512, CG_WARPS = CG_THREADS / 32;
+
+// The CTA's run over the active blocks, a world's part of it at a time:
+// body(world, its active count, the part's first tile, its tiles).
+template <bool ONE, class Body>
+__device__ __forceinline__ void forTileRuns(const Batch& Bt, const WorldSrc<ONE>& src, WorldCopy& wc, Body body) {
+    const uint32_t n = Bt.n(L_ACT), per = (n + gridDim.x - 1u) / gridDim.x;
+    uint32_t g = blockIdx.x * per;
+    const uint32_t e = min(g + per, n);
+    while (g < e) {
+        const uint32_t it = Bt.item(L_ACT, g), j0 = Bt.unit(it);
+        const World& Wd = src.get(Bt, it, wc);
+        const uint32_t na = W(Wd.D).activeCount();
+        // (a world's items are its units 0 .. na - 1 in order)
+        const uint32_t m = max(min(e - g, na - j0), 1u);
+        body(Wd, na, j0, m);
+        g += m;
     }
 }
 
-// cgDirection + cgApply + cgAlpha (fluid.wgsl:2767-2814): the direction p =
-// z + beta p_old of the cell and of its liquid neighbours (worked again from
-// their z and p_old, the same arithmetic), q = A p, and the tile trees of
-// p q.  p_old is read from one of the two p arrays and p written to the
-// other (by the iteration's parity), so no CTA reads a p that another
-// writes in the launch.
+// A lane's two cells of tile wid: their indices and whether they are in the
+// world (a ragged world's last blocks), and the tile's block.
+struct TileLane {
+    uint32_t n, i[2];
+    int x, y[2];
+    bool in[2];
+};
+__device__ __forceinline__ TileLane tileLane(const W& w, uint32_t wid, bool live) {
+    TileLane t;
+    const int lane = (int)(threadIdx.x & 31u);
+    t.n = live ? w.D.blocks[w.activeSlot(wid)] : 0u;
+    const I2 b = w.blockAt(t.n);
+    t.x = b.x * BLOCK + (lane & 7);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        t.y[h] = b.y * BLOCK + (lane >> 3) + 4 * h;
+        t.in[h] = live && w.inWorld(I2{t.x, t.y[h]});
+        t.i[h] = t.in[h] ? w.cellIndex(I2{t.x, t.y[h]}) : 0u;
+    }
+    return t;
+}
+
+// A tile's tree of 64 (sumBlock, fluid.wgsl:2628-2641) from a lane's two
+// values; the sum in lane 0.
+template <class T>
+__device__ __forceinline__ T warpTree(T lo, T hi) {
+    T v = lo + hi;
+#pragma unroll
+    for (int h = 16; h > 0; h >>= 1) v = v + __shfl_down_sync(0xffffffffu, v, h);
+    return v;
+}
+
+// sumBlocks (fluid.wgsl:2645-2661) of the first NC components of a world's
+// B block partials by a CTA of CG_THREADS: column li (of 256) adds blocks
+// li, li + 256, ... in that order, 16 rows' loads in flight a thread.  Two
+// components: a half of the CTA each.  One: the halves take 16 rows each of
+// a column in turn and pass its sum on, so the order of the adds stays.
+// A block not worked on has partials of +0, and a sum that starts from +0 is
+// never -0, so adding them changes no bit: its state is not read.  The sums
+// in thread 0.
+template <class T, int NC>
+__device__ __noinline__ void sumBlocksCg(uint32_t B, const T* part, T* s, T* out) {
+    constexpr uint32_t ROWS = 16u, HALF = 256u * ROWS;
+    const uint32_t li = threadIdx.x & 255u, half = threadIdx.x >> 8;
+    T* own = s + (NC == 2 ? 256u * half : 0u) + li;
+    const T* at = part + (NC == 2 ? (size_t)B * half : 0u);
+    T acc = T(0);
+    for (uint32_t r0 = 0; r0 < B; r0 += NC == 2 ? HALF : 2u * HALF) {
+        T v[ROWS];
+        const uint32_t k0 = r0 + (NC == 2 ? 0u : half * HALF) + li;
+#pragma unroll
+        for (uint32_t u = 0; u < ROWS; u++) v[u] = k0 + 256u * u < B ? __ldcg(at + k0 + 256u * u) : T(0);
+        if (NC == 2 || half == 0u) {
+#pragma unroll
+            for (uint32_t u = 0; u < ROWS; u++) acc = acc + v[u];
+        }
+        if (NC == 2 || r0 + HALF >= B) continue;  // (uniform: the second half has no row)
+        if (half == 0u) *own = acc;
+        __syncthreads();
+        if (half == 1u) {
+            acc = *own;
+#pragma unroll
+            for (uint32_t u = 0; u < ROWS; u++) acc = acc + v[u];
+            *own = acc;
+        }
+        __syncthreads();
+        if (half == 0u) acc = *own;
+    }
+    const bool adds = NC == 2 || half == 0u;
+    if (adds) *own = acc;
+    __syncthreads();
+#pragma unroll
+    for (uint32_t h = 128u; h > 32u; h >>= 1) {
+        if (adds && li < h) *own = *own + own[h];
+        __syncthreads();
+    }
+    if (adds && li < 32u) {
+        T v = *own + own[32];
+#pragma unroll
+        for (int h = 16; h > 0; h >>= 1) v = v + __shfl_down_sync(0xffffffffu, v, h);
+        if (li == 0u) *own = v;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0u) {
+#pragma unroll
+        for (int c = 0; c < NC; c++) out[c] = s[256 * c];
+    }
+}
+
+// Counts the CTA's m tiles of a world whose partials its warps' first lanes
+// have written; true in the CTA that counted the world's last tile (a
+// threadfence reduction's test).  first(): thread 0's, before the count.
+template <class First>
+__device__ __forceinline__ bool countTiles(uint32_t* counter, uint32_t m, uint32_t total, First first) {
+    __shared__ int last;
+    if ((threadIdx.x & 31u) == 0u) __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        first();
+        const uint32_t old = atomicAdd(counter, m);
+        last = old + m == total ? 1 : 0;
+        if (last) {
+            *counter = 0u;
+            __threadfence();
+        }
+    }
+    __syncthreads();
+    return last != 0;
+}
+
+// cgRho + cgBeta (fluid.wgsl:2736-2764).
 template <bool ONE>
-__global__ void __launch_bounds__(256) k_fApplyAlpha(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
+__global__ void __launch_bounds__(CG_THREADS, 2) k_fRhoBeta(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
     if (!ONE) worldCopyInit(wc_);
-    __shared__ float sx[256];
+    __shared__ double s64[512];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    forTileRuns<ONE>(Bt, src, wc_, [&](const World& Wd, uint32_t na, uint32_t j0, uint32_t m) {
+        const Dev& D = Wd.D;
+        const FastW& F = Wd.S;
+        const W w(D);
+        if (D.st->cont == 0u) return;
+        const bool f64 = D.st->f64 != 0u;
+        const uint32_t cycle = D.st->cycle;
+        const Lvl& L0 = F.L[0];
+        for (uint32_t t0 = warp; t0 < m; t0 += 2u * CG_WARPS) {
+            TileLane t[2];
+            float rho[2][2], z[2][2], r[2][2], q[2][2];
+#pragma unroll
+            for (int u = 0; u < 2; u++) t[u] = tileLane(w, j0 + t0 + (uint32_t)u * CG_WARPS, t0 + (uint32_t)u * CG_WARPS < m);
+#pragma unroll
+            for (int u = 0; u < 2; u++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const uint32_t i = t[u].i[h];
+                    rho[u][h] = L0.rho[i];
+                    z[u][h] = L0.px[i];
+                    r[u][h] = F.R[i];
+                    q[u][h] = F.Q[i];
+                }
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                if (t0 + (uint32_t)u * CG_WARPS >= m) break;  // (warp-uniform)
+                const bool f0 = t[u].in[0] && rho[u][0] > 0.0f, f1 = t[u].in[1] && rho[u][1] > 0.0f;
+                // the f32 trees only without FP64 dots, which read none of them
+                if (f64) {
+                    const double x = warpTree(f0 ? (double)r[u][0] * (double)z[u][0] : 0.0,
+                                              f1 ? (double)r[u][1] * (double)z[u][1] : 0.0);
+                    const double y = warpTree(f0 ? (double)q[u][0] * (double)z[u][0] : 0.0,
+                                              f1 ? (double)q[u][1] * (double)z[u][1] : 0.0);
+                    if (lane == 0u) {
+                        F.part64[t[u].n] = x;
+                        F.part64[D.B + t[u].n] = y;
+                    }
+                } else {
+                    const float x = warpTree(f0 ? r[u][0] * z[u][0] : 0.0f, f1 ? r[u][1] * z[u][1] : 0.0f);
+                    const float y = warpTree(f0 ? q[u][0] * z[u][0] : 0.0f, f1 ? q[u][1] * z[u][1] : 0.0f);
+                    if (lane == 0u) {
+                        F.part32[t[u].n] = x;
+                        F.part32[D.B + t[u].n] = y;
+                    }
+                }
+            }
+        }
+        if (!countTiles(&D.st->fdone[1], m, na, [] {})) return;
+        if (f64) {
+            double v[2];
+            sumBlocksCg<double, 2>(D.B, F.part64, s64, v);
+            if (threadIdx.x == 0) {
+                D.st->rz = v[0];
+                D.st->beta = (cycle == 0u || D.st->pq <= 0.0) ? 0.0 : -v[1] / D.st->pq;
+            }
+        } else {
+            float v[2];
+            sumBlocksCg<float, 2>(D.B, F.part32, reinterpret_cast<float*>(s64), v);
+            if (threadIdx.x == 0) {
+                D.st->rz32 = v[0];
+                D.st->beta32 = (cycle == 0u || D.st->pq32 <= 0.0f) ? 0.0f : -v[1] / D.st->pq32;
+            }
+        }
+    });
+}
+
+// cgDirection + cgApply + cgAlpha (fluid.wgsl:2767-2814): the direction p =
+// z + beta p_old of the tile's cells and of the 32 cells around it, a cell
+// of these a lane (worked again from their z and p_old, the same
+// arithmetic), in the warp's 10x10 of shared memory; q = A p, and the tile
+// trees of p q.  p_old is read from one of the two p arrays and p written
+// to the other (by the iteration's parity), so no warp reads a p that
+// another writes in the launch.
+template <bool ONE>
+__global__ void __launch_bounds__(CG_THREADS, 2) k_fApplyAlpha(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
+    __shared__ WorldCopy wc_;
+    if (!ONE) worldCopyInit(wc_);
     __shared__ double s64[256];
-    __shared__ float ux[2][128];
-    __shared__ double ex64[2][128];
-    uint32_t pend_ = 0;  // tiles finished of the current world, not yet counted
-    uint32_t par = 0;    // the tree buffers of this item
-    FOR_ITEMS(Bt, L_ACT4, it) {
-        FAST_ITEM(Bt, it, D, F, w, g);
-        if (D.st->cont == 0u) continue;
+    __shared__ float tp[CG_WARPS][RIM * RIM];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    float* sp = tp[warp];
+    // the lane's cell around the tile: left and right columns, rows above
+    // and below, 8 lanes each
+    const int side = (int)(lane >> 3), at = (int)(lane & 7u);
+    const int ox = side == 0 ? -1 : side == 1 ? BLOCK : at, oy = side == 2 ? -1 : side == 3 ? BLOCK : at;
+    const int so = (oy + 1) * RIM + ox + 1;
+    forTileRuns<ONE>(Bt, src, wc_, [&](const World& Wd, uint32_t na, uint32_t j0, uint32_t m) {
+        const Dev& D = Wd.D;
+        const FastW& F = Wd.S;
+        const W w(D);
+        if (D.st->cont == 0u) return;
         const bool f64 = D.st->f64 != 0u;
         const float beta = D.st->beta32;
         const double beta64 = D.st->beta;
@@ -1889,80 +2023,84 @@ __global__ void __launch_bounds__(256) k_fApplyAlpha(Batch Bt, const __grid_cons
         const float* Pold = odd ? F.P2 : F.P;
         float* Pnew = odd ? F.P : F.P2;
         const Lvl& L0 = F.L[0];
-        const uint32_t na = w.activeCount();
-        const uint32_t wid = g * 4u + (threadIdx.x >> 6);
-        const bool valid = wid < na;
-        // cgDirection's p of liquid cell k
-        auto dir = [&](uint32_t k) {
-            const float z = L0.px[k];
-            return f64 ? (float)((double)z + beta64 * (double)Pold[k]) : z + beta * Pold[k];
-        };
-        float vx = 0.0f;
-        double ex = 0.0;
-        if (valid) {
-            I2 c = tileCell(w, wid);
-            if (w.inWorld(c)) {
-                uint32_t i = w.cellIndex(c);
-                float p = 0.0f, q = 0.0f;
-                // the cell's and its neighbours' words loaded beside the
-                // density (neighbour indices clamp onto the cell), not after
-                const float rho = L0.rho[i];
-                const uint8_t m = F.fmask[i];
-                const float b[4] = {L0.b0[i], L0.b1[i], L0.b2[i], L0.b3[i]};
-                const float dgp = L0.diag[i] + F.pin[i];
-                const float pi = dir(i);
-                float pn[4];
+        auto dir = [&](float z, float p) { return f64 ? (float)((double)z + beta64 * (double)p) : z + beta * p; };
+        for (uint32_t t0 = warp; t0 < m; t0 += CG_WARPS) {
+            const TileLane t = tileLane(w, j0 + t0, true);
+            const I2 b = w.blockAt(t.n);
+            const I2 oc{b.x * BLOCK + ox, b.y * BLOCK + oy};
+            const bool oin = w.inWorld(oc);
+            const uint32_t oi = oin ? w.cellIndex(oc) : 0u;
+            const float oz = L0.px[oi], op = Pold[oi];
+            float rho[2], bl[2], br[2], bu[2], bd[2], dgp[2], z[2], po[2];
+            uint8_t mk[2];
 #pragma unroll
-                for (int d = 0; d < 4; d++) pn[d] = dir(nbr(i, c.x, c.y, D.W, D.H, d));
-                if (rho > 0.0f) {
-                    p = pi;
+            for (int h = 0; h < 2; h++) {
+                const uint32_t i = t.i[h];
+                rho[h] = L0.rho[i];
+                mk[h] = F.fmask[i];
+                bl[h] = L0.b0[i];
+                br[h] = L0.b1[i];
+                bu[h] = L0.b2[i];
+                bd[h] = L0.b3[i];
+                dgp[h] = L0.diag[i] + F.pin[i];
+                z[h] = L0.px[i];
+                po[h] = Pold[i];
+            }
+            float p[2];
+            const int c0 = ((int)(lane >> 3) + 1) * RIM + (int)(lane & 7u) + 1;
+            sp[so] = dir(oz, op);
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                p[h] = dir(z[h], po[h]);
+                sp[c0 + 4 * RIM * h] = p[h];
+            }
+            __syncwarp();
+            float q[2];
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int c = c0 + 4 * RIM * h;
+                q[h] = 0.0f;
+                if (t.in[h] && rho[h] > 0.0f) {
                     float sum = 0.0f;
-#pragma unroll
-                    for (int d = 0; d < 4; d++)
-                        if (m & (1u << d)) sum = sum + b[d] * pn[d];
-                    q = dgp * p - sum + 0.0f;
+                    if (mk[h] & 1u) sum = sum + bl[h] * sp[c - 1];
+                    if (mk[h] & 2u) sum = sum + br[h] * sp[c + 1];
+                    if (mk[h] & 4u) sum = sum + bu[h] * sp[c - RIM];
+                    if (mk[h] & 8u) sum = sum + bd[h] * sp[c + RIM];
+                    q[h] = dgp[h] * p[h] - sum + 0.0f;
+                } else {
+                    p[h] = 0.0f;
                 }
-                Pnew[i] = p;
-                F.Q[i] = q;
-                vx = p * q;
-                ex = (double)p * (double)q;
+                if (t.in[h]) {
+                    Pnew[t.i[h]] = p[h];
+                    F.Q[t.i[h]] = q[h];
+                }
             }
-        }
-        if (f64) tilePut(ex64[par], ex);
-        else tilePut(ux[par], vx);
-        __syncthreads();
-        float tx = 0.0f;
-        double dx = 0.0;
-        if (f64) dx = tileSum(ex64[par], ex);
-        else tx = tileSum(ux[par], vx);
-        par ^= 1u;
-        if (valid && (threadIdx.x & 63u) == 0u) {
-            const uint32_t b = w.blockIndex(w.activeBlock(wid));
             if (f64) {
-                F.part64[2u * b] = dx;
-                F.part64[2u * b + 1u] = 0.0;
+                const double x = warpTree((double)p[0] * (double)q[0], (double)p[1] * (double)q[1]);
+                if (lane == 0u) F.part64[t.n] = x;
             } else {
-                F.part32[2u * b] = tx;
-                F.part32[2u * b + 1u] = 0.0f;
+                const float x = warpTree(p[0] * q[0], p[1] * q[1]);
+                if (lane == 0u) F.part32[t.n] = x;
+            }
+            __syncwarp();  // the warp's p is free for its next tile
+        }
+        if (!countTiles(&D.st->fdone[2], m, na, [] {})) return;
+        if (f64) {
+            double v[1];
+            sumBlocksCg<double, 1>(D.B, F.part64, s64, v);
+            if (threadIdx.x == 0) {
+                D.st->pq = v[0];
+                D.st->alpha = v[0] <= 0.0 ? 0.0 : D.st->rz / v[0];
+            }
+        } else {
+            float v[1];
+            sumBlocksCg<float, 1>(D.B, F.part32, reinterpret_cast<float*>(s64), v);
+            if (threadIdx.x == 0) {
+                D.st->pq32 = v[0];
+                D.st->alpha32 = v[0] <= 0.0f ? 0.0f : D.st->rz32 / v[0];
             }
         }
-        pend_ += min(4u, na - g * 4u);
-        if (flushTiles(Bt, g_it, e_it, it, pend_, &D.st->fdone[2], na)) {
-            if (f64) {
-                double pq = sumBlocks256(w, F.part64, 0, s64);
-                if (threadIdx.x == 0) {
-                    D.st->pq = pq;
-                    D.st->alpha = pq <= 0.0 ? 0.0 : D.st->rz / pq;
-                }
-            } else {
-                float pq = sumBlocks256(w, F.part32, 0, sx);
-                if (threadIdx.x == 0) {
-                    D.st->pq32 = pq;
-                    D.st->alpha32 = pq <= 0.0f ? 0.0f : D.st->rz32 / pq;
-                }
-            }
-        }
-    }
+    });
 }
 
 // cgUpdate (fluid.wgsl:2852-2880), the tolerance form's norm, and the loop's
@@ -1970,106 +2108,110 @@ __global__ void __launch_bounds__(256) k_fApplyAlpha(Batch Bt, const __grid_cons
 // (converged, fluid.wgsl:2223-2226) or max_cycles are done; the loop runs on
 // while any world does.
 template <bool ONE>
-__global__ void __launch_bounds__(256) k_fUpdate(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
+__global__ void __launch_bounds__(CG_THREADS, 2) k_fUpdate(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
     if (!ONE) worldCopyInit(wc_);
-    __shared__ uint32_t umost[2][4];  // the upper warps' largest |r| (bits of a non-negative float)
-    __shared__ uint32_t runMost;      // the largest |r| of the current world's run
+    __shared__ uint32_t runMost;  // the largest |r| of the current world's run (bits of a non-negative float)
     __shared__ double s64[256];
-    __shared__ double ur2[2][128];
     if (threadIdx.x == 0) runMost = 0u;
-    uint32_t pend_ = 0;  // tiles finished of the current world, not yet counted
-    uint32_t par = 0;    // the tree buffers of this item
-    FOR_ITEMS(Bt, L_ACT4, it) {
-        FAST_ITEM(Bt, it, D, F, w, g);
-        if (D.st->cont == 0u) continue;
+    __syncthreads();
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    forTileRuns<ONE>(Bt, src, wc_, [&](const World& Wd, uint32_t na, uint32_t j0, uint32_t m) {
+        const Dev& D = Wd.D;
+        const FastW& F = Wd.S;
+        const W w(D);
+        if (D.st->cont == 0u) return;
         const uint32_t cycle = D.st->cycle;
         const bool f64 = D.st->f64 != 0u, tol = D.st->tol_mode != 0u;
         const float alpha = D.st->alpha32;
         const double alpha64 = D.st->alpha;
         const Lvl& L0 = F.L[0];
-        const uint32_t na = w.activeCount();
-        const uint32_t wid = g * 4u + (threadIdx.x >> 6);
-        const bool valid = wid < na;
-        uint32_t m = 0u;
-        double r2 = 0.0;
-        if (valid) {
-            I2 c = tileCell(w, wid);
-            if (w.inWorld(c)) {
-                uint32_t i = w.cellIndex(c);
-                // loaded beside the density, not after it
-                const float rho = L0.rho[i], vx = F.X[i], vy = F.R[i], vz = ((cycle & 1u) ? F.P : F.P2)[i];
-                const float vw = F.Q[i], py = L0.py[i];
-                if (rho > 0.0f) {
+        const float* P = (cycle & 1u) ? F.P : F.P2;
+        uint32_t most = 0u;
+        for (uint32_t t0 = warp; t0 < m; t0 += 2u * CG_WARPS) {
+            TileLane t[2];
+            float rho[2][2], vx[2][2], vy[2][2], vz[2][2], vw[2][2], py[2][2];
+#pragma unroll
+            for (int u = 0; u < 2; u++) t[u] = tileLane(w, j0 + t0 + (uint32_t)u * CG_WARPS, t0 + (uint32_t)u * CG_WARPS < m);
+#pragma unroll
+            for (int u = 0; u < 2; u++)
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const uint32_t i = t[u].i[h];
+                    rho[u][h] = L0.rho[i];
+                    vx[u][h] = F.X[i];
+                    vy[u][h] = F.R[i];
+                    vz[u][h] = P[i];
+                    vw[u][h] = F.Q[i];
+                    py[u][h] = L0.py[i];
+                }
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                if (t0 + (uint32_t)u * CG_WARPS >= m) break;  // (warp-uniform)
+                double r2[2] = {0.0, 0.0};
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    if (!t[u].in[h] || !(rho[u][h] > 0.0f)) continue;
+                    const uint32_t i = t[u].i[h];
                     float r, x;
                     if (f64) {
-                        r = (float)((double)vy - alpha64 * (double)vw);
-                        x = (float)((double)vx + alpha64 * (double)vz);
+                        r = (float)((double)vy[u][h] - alpha64 * (double)vw[u][h]);
+                        x = (float)((double)vx[u][h] + alpha64 * (double)vz[u][h]);
                     } else {
-                        r = vy - alpha * vw;
-                        x = vx + alpha * vz;
+                        r = vy[u][h] - alpha * vw[u][h];
+                        x = vx[u][h] + alpha * vz[u][h];
                     }
                     F.X[i] = x;
                     F.R[i] = r;
                     L0.px[i] = 0.0f;
                     L0.rx[i] = -r;
                     F.rimx[i] = 0.0f;
-                    F.rimy[i] = py;
-                    m = __float_as_uint(fabsf(r));
-                    r2 = (double)r * (double)r;
+                    F.rimy[i] = py[u][h];
+                    most = max(most, __float_as_uint(fabsf(r)));
+                    r2[h] = (double)r * (double)r;
+                }
+                if (tol) {
+                    const double v = warpTree(r2[0], r2[1]);
+                    if (lane == 0u) D.norm64[t[u].n] = v;
                 }
             }
         }
-        // the tile's largest |r| (a max: any order) and its tree of r^2
-        m = __reduce_max_sync(0xffffffffu, m);
-        if ((threadIdx.x & 63u) == 32u) umost[par][threadIdx.x >> 6] = m;
-        if (tol) tilePut(ur2[par], r2);
-        __syncthreads();
-        double t2 = 0.0;
-        if (tol) t2 = tileSum(ur2[par], r2);
-        if (valid && (threadIdx.x & 63u) == 0u) {
-            if (tol) D.norm64[2u * w.blockIndex(w.activeBlock(wid))] = t2;
-            atomicMax(&runMost, max(m, umost[par][threadIdx.x >> 6]));
-        }
-        par ^= 1u;
-        pend_ += min(4u, na - g * 4u);
-        if (worldRunEnds(Bt, L_ACT4, g_it, e_it, it)) {
-            // the run's largest |r| into the world's residual slot (a max of
-            // maxima: the same word), before its tiles are counted
-            __syncthreads();
-            if (threadIdx.x == 0) {
+        // the run's largest |r| into the world's residual slot (a max of
+        // maxima: the same word), before its tiles are counted
+        most = __reduce_max_sync(0xffffffffu, most);
+        if (lane == 0u && most) atomicMax(&runMost, most);
+        if (!countTiles(&D.st->fdone[3], m, na, [&] {
                 atomicMax(&D.blocks[w.countSlot(COUNT_RESIDUAL + cycle % 3u)], runMost);
                 runMost = 0u;
                 __threadfence();
-            }
-        }
-        if (flushTiles(Bt, g_it, e_it, it, pend_, &D.st->fdone[3], na)) {
+            }))
+            return;
+        double rr[1] = {0.0};
+        if (tol) sumBlocksCg<double, 1>(D.B, D.norm64, s64, rr);
+        if (threadIdx.x == 0) {
             bool conv;
             if (tol) {
-                double rr = sumBlocks256(w, D.norm64, 0, s64);
-                double rel = D.st->bnorm2 > 0.0 ? sqrt(rr / D.st->bnorm2) : 0.0;
-                if (threadIdx.x == 0) D.st->rel = rel;
+                const double rel = D.st->bnorm2 > 0.0 ? sqrt(rr[0] / D.st->bnorm2) : 0.0;
+                D.st->rel = rel;
                 conv = rel <= D.st->tol;
             } else {
                 conv = __uint_as_float(__ldcg(&D.blocks[w.countSlot(COUNT_RESIDUAL + cycle % 3u)])) < LIQUID_TOLERANCE;
             }
-            if (threadIdx.x == 0) {
-                const uint32_t next = cycle + 1u;
-                // the mixed form checks the true residual every 8th iteration
-                // and before it stops (k_fTrueCheck may then go on)
-                const bool check = Bt.mixed != 0u && tol && (conv || (next % 8u) == 0u || next >= Bt.max_cycles);
-                const uint32_t cont = (!conv && next < Bt.max_cycles) ? 1u : 0u;
-                D.st->cycle = next;
-                D.st->cont = cont;
-                D.st->check = check ? 1u : 0u;
-                if (check && Bt.cond_check) cudaGraphSetConditional(Bt.cond_check, 1u);
-                if (cont) {
-                    *Bt.loop = 1u;
-                    if (Bt.cond) cudaGraphSetConditional(Bt.cond, 1u);
-                }
+            const uint32_t next = cycle + 1u;
+            // the mixed form checks the true residual every 8th iteration
+            // and before it stops (k_fTrueCheck may then go on)
+            const bool check = Bt.mixed != 0u && tol && (conv || (next % 8u) == 0u || next >= Bt.max_cycles);
+            const uint32_t cont = (!conv && next < Bt.max_cycles) ? 1u : 0u;
+            D.st->cycle = next;
+            D.st->cont = cont;
+            D.st->check = check ? 1u : 0u;
+            if (check && Bt.cond_check) cudaGraphSetConditional(Bt.cond_check, 1u);
+            if (cont) {
+                *Bt.loop = 1u;
+                if (Bt.cond) cudaGraphSetConditional(Bt.cond, 1u);
             }
         }
-    }
+    });
 }
 
 // The true residual -(b + A x) of liquid cell i at c, worked in FP64 from the
@@ -2128,8 +2270,8 @@ __global__ void __launch_bounds__(256) k_fTrueCheck(Batch Bt, const __grid_const
         const double u2 = tree64x4(s64, f2);
         if (valid && (threadIdx.x & 63u) == 0u) {
             const uint32_t b = w.blockIndex(w.activeBlock(wid));
-            D.norm64[2u * b] = t2;
-            D.norm64[2u * b + 1u] = u2;
+            D.norm64[b] = t2;
+            D.norm64[D.B + b] = u2;
         }
         pend_ += min(4u, na - g * 4u);
         if (flushTiles(Bt, g_it, e_it, it, pend_, &D.st->fdone[4], na)) {
@@ -2479,11 +2621,11 @@ __global__ void __launch_bounds__(256, 4) k_fSolve(Fast F, int shifted) {
             }
             if (valid && (threadIdx.x & 63u) == 0u) {
                 const uint32_t b = w.blockIndex(w.activeBlock(wid));
-                F.part32[2u * b] = tx;
-                F.part32[2u * b + 1u] = ty;
+                F.part32[b] = tx;
+                F.part32[D.B + b] = ty;
                 if (f64) {
-                    F.part64[2u * b] = dx;
-                    F.part64[2u * b + 1u] = dy;
+                    F.part64[b] = dx;
+                    F.part64[D.B + b] = dy;
                 }
             }
         }
@@ -2560,11 +2702,11 @@ __global__ void __launch_bounds__(256, 4) k_fSolve(Fast F, int shifted) {
             if (f64) dx = tree64x4(s64, ex);
             if (valid && (threadIdx.x & 63u) == 0u) {
                 const uint32_t b = w.blockIndex(w.activeBlock(wid));
-                F.part32[2u * b] = tx;
-                F.part32[2u * b + 1u] = 0.0f;
+                F.part32[b] = tx;
+                F.part32[D.B + b] = 0.0f;
                 if (f64) {
-                    F.part64[2u * b] = dx;
-                    F.part64[2u * b + 1u] = 0.0;
+                    F.part64[b] = dx;
+                    F.part64[D.B + b] = 0.0;
                 }
             }
         }
@@ -2629,7 +2771,7 @@ __global__ void __launch_bounds__(256, 4) k_fSolve(Fast F, int shifted) {
                 if (tol) t2 = tree64x4(s64, r2);
                 __syncthreads();
                 if (valid && (threadIdx.x & 63u) == 0u) {
-                    if (tol) D.norm64[2u * w.blockIndex(w.activeBlock(wid))] = t2;
+                    if (tol) D.norm64[w.blockIndex(w.activeBlock(wid))] = t2;
                     atomicMax(&D.blocks[w.countSlot(COUNT_RESIDUAL + cycle % 3u)], most[threadIdx.x >> 6]);
                 }
                 __syncthreads();
@@ -2670,7 +2812,7 @@ size_t fast_cluster_smem(const Dev& D, uint32_t lc) {
     return clusterFloats(D.level_w, D.level_h, lc, D.levels, nullptr) * sizeof(float);
 }
 
-void fast_zero_level0(const FastW& F, uint32_t cells, cudaStream_t s) { k_fZero<<<148 * 4, 256, 0, s>>>(F, cells); }
+void fast_zero_level0(const World& Wd, cudaStream_t s) { k_fZero<<<148 * 4, 256, 0, s>>>(Wd.D, Wd.S); }
 
 void fast_zero_idle(const Batch& Bt, const BatchShape& S, cudaStream_t s) {
     k_fZeroIdle<<<list_grid(S, L_WB, 32), 64, 0, s>>>(Bt);
@@ -2749,6 +2891,8 @@ uint32_t fast_cycle_t(const Batch& Bt0, const BatchShape& S, const World* one, c
         Bt.cond_drift = (unsigned long long)hd;
     }
     const unsigned G = list_grid(S, L_ACT, 32), G4 = list_grid(S, L_ACT4, S.cg_per_sm);
+    // the CG kernels: at most a tile a warp
+    const unsigned GC = std::max(std::min((S.max_items[L_ACT] + CG_WARPS - 1u) / CG_WARPS, 148u * S.cg_per_sm), 1u);
     const unsigned GR = std::max(std::min((S.max_items[L_RELAX] + 3u) / 4u, 148u * S.relax_per_sm), 1u);
     uint32_t launches = 0;
     auto mark = [&](int slot, int phase) {
@@ -2813,13 +2957,13 @@ uint32_t fast_cycle_t(const Batch& Bt0, const BatchShape& S, const World* one, c
     LAUNCH_T(k_fRelax, T, GR, 128, 0, 1);
     mark(WIG_SLOT_F_RELAX, 1);
     mark(WIG_SLOT_F_RHO_BETA, 0);
-    LAUNCH(k_fRhoBeta, G4, 256, 0);
+    LAUNCH(k_fRhoBeta, GC, CG_THREADS, 0);
     mark(WIG_SLOT_F_RHO_BETA, 1);
     mark(WIG_SLOT_F_APPLY_ALPHA, 0);
-    LAUNCH(k_fApplyAlpha, G4, 256, 0);
+    LAUNCH(k_fApplyAlpha, GC, CG_THREADS, 0);
     mark(WIG_SLOT_F_APPLY_ALPHA, 1);
     mark(WIG_SLOT_F_UPDATE, 0);
-    LAUNCH(k_fUpdate, G4, 256, 0);
+    LAUNCH(k_fUpdate, GC, CG_THREADS, 0);
     mark(WIG_SLOT_F_UPDATE, 1);
     if (Bt.mixed && hc && hd) {
         // captured: launched only on the iterations that check (not counted

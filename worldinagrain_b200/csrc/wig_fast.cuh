@@ -58,8 +58,8 @@ uint32_t fast_cycle(const Batch& Bt, const BatchShape& S, const World* one, cuda
                     NestCapture* nest = nullptr);
 // cgFinish; `two_p`: the fast form's p is in P or P2 by the iterations' parity.
 void fast_finish(const Batch& Bt, const BatchShape& S, const World* one, bool two_p, cudaStream_t s, const Marker* m);
-// Level 0's arrays of one world zeroed (after its buffers are written by the host).
-void fast_zero_level0(const FastW& F, uint32_t cells, cudaStream_t s);
+// Level 0's arrays and the block partials of one world zeroed (after its buffers are written by the host).
+void fast_zero_level0(const World& Wd, cudaStream_t s);
 // The same for the blocks not worked on, of every world of the step whose
 // scratch a pool lends (after compact).
 void fast_zero_idle(const Batch& Bt, const BatchShape& S, cudaStream_t s);

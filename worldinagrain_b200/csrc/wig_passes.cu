@@ -797,6 +797,8 @@ __global__ void k_retire(Batch Bt) {
     FOR_ITEMS(Bt, L_RET, it) {
         ITEM_WORLD_C(Bt, it, D, w, wid);
         uint32_t n = D.blocks[w.retiredSlot(wid)];
+        // the solve's sums over the world's blocks take its partials for +0
+        if (threadIdx.x == 0) zeroPartials(D, wc_.w.S, n);
         const I2 bq_ = w.blockAt(n);
         I2 c{bq_.x * BLOCK + (int)(threadIdx.x & 7u), bq_.y * BLOCK + (int)(threadIdx.x >> 3)};
         if (!w.inWorld(c)) continue;
@@ -1527,7 +1529,7 @@ __global__ void k_cgResidual(Dev D) {
         if (tol) {
             sb[threadIdx.x] = b2;
             tree64(sb);
-            if (threadIdx.x == 0) D.norm64[2u * w.blockIndex(w.activeBlock(wid))] = sb[0];
+            if (threadIdx.x == 0) D.norm64[w.blockIndex(w.activeBlock(wid))] = sb[0];
             __syncthreads();
         }
     }
@@ -1557,7 +1559,7 @@ __device__ double sumBlocks64(const W& w, const double* buf, int comp, double* s
         for (int u = 0; u < 16; u++) {
             const uint32_t k = k0 + 256u * (uint32_t)u;
             st[u] = k < B ? w.D.blocks[w.stateSlot(k)] : 0u;
-            v[u] = k < B ? buf[2u * k + (uint32_t)comp] : 0.0;
+            v[u] = k < B ? buf[(uint32_t)comp * B + k] : 0.0;
         }
 #pragma unroll
         for (int u = 0; u < 16; u++)
@@ -1940,8 +1942,8 @@ __global__ void __launch_bounds__(64) k_cgRho(Dev D, uint32_t cycle) {
             tree64(dy);
             if (threadIdx.x == 0) {
                 uint32_t b = w.blockIndex(w.activeBlock(wid));
-                D.part64[2u * b] = dx[0];
-                D.part64[2u * b + 1u] = dy[0];
+                D.part64[b] = dx[0];
+                D.part64[D.B + b] = dy[0];
             }
             __syncthreads();
         }
@@ -2039,8 +2041,8 @@ __global__ void __launch_bounds__(64) k_cgApply(Dev D, uint32_t cycle) {
             tree64(dx);
             if (threadIdx.x == 0) {
                 uint32_t b = w.blockIndex(w.activeBlock(wid));
-                D.part64[2u * b] = dx[0];
-                D.part64[2u * b + 1u] = 0.0;
+                D.part64[b] = dx[0];
+                D.part64[D.B + b] = 0.0;
             }
             __syncthreads();
         }
@@ -2121,7 +2123,7 @@ __global__ void __launch_bounds__(64) k_cgUpdate(Dev D, uint32_t cycle) {
         if (tol) {
             sb[threadIdx.x] = r2;
             tree64(sb);
-            if (threadIdx.x == 0) D.norm64[2u * w.blockIndex(w.activeBlock(wid))] = sb[0];
+            if (threadIdx.x == 0) D.norm64[w.blockIndex(w.activeBlock(wid))] = sb[0];
         }
         __syncthreads();
         if (threadIdx.x == 0) atomicMax(&D.blocks[w.countSlot(COUNT_RESIDUAL + cycle % 3u)], most);
