@@ -260,9 +260,10 @@ void dev_shape(wig::Dev& D, const wig_world_layout& L) {
 // Bytes of a world's fast scratch and FP64 partials.
 size_t scratch_bytes(const wig::Dev& D) {
     const size_t C = D.C;
-    size_t bytes = align256(C) + 18u * align256(C * 4u) + align256(4u * C * 2u);  // + level 0's binary16 copies
+    // level 0: mask; pot, rim and the binary16 coefficients; b; rho, ry, X, R, P, Q, P2
+    size_t bytes = align256(C) + 3u * align256(C * 8u) + align256(C * 16u) + 7u * align256(C * 4u);
     for (uint32_t l = 1; l <= D.levels; l++) {
-        bytes += 12u * align256((size_t)D.level_w[l] * D.level_h[l] * 4u);
+        bytes += 11u * align256((size_t)D.level_w[l] * D.level_h[l] * 4u);
         bytes += align256(5u * (size_t)D.level_w[l] * D.level_h[l] * 2u);  // the binary16 operator
     }
     bytes += align256(2u * (size_t)D.B * 4u) + 3u * align256(2u * (size_t)D.B * 8u);
@@ -277,21 +278,23 @@ void scratch_take(wig::World& Wd, char* p, uint32_t coarse_cells) {
     auto take = [&](size_t n) { char* q = p; p += align256(n); return q; };
     auto fl = [&](size_t n) { return reinterpret_cast<float*>(take(n * 4u)); };
     const size_t C = D.C;
-    F.fmask = reinterpret_cast<uint8_t*>(take(C));
-    for (uint32_t l = 0; l <= D.levels; l++) {
-        const size_t n = l == 0 ? C : (size_t)D.level_w[l] * D.level_h[l];
+    F.Z.mask = reinterpret_cast<uint8_t*>(take(C));
+    F.Z.pot = reinterpret_cast<float2*>(take(C * 8u));
+    F.Z.rim = reinterpret_cast<float2*>(take(C * 8u));
+    F.Z.b = reinterpret_cast<float4*>(take(C * 16u));
+    F.Z.rho = fl(C); F.Z.ry = fl(C);
+    for (uint32_t l = 1; l <= D.levels; l++) {
+        const size_t n = (size_t)D.level_w[l] * D.level_h[l];
         wig::Lvl& V = F.L[l];
         V.px = fl(n); V.py = fl(n); V.rx = fl(n); V.ry = fl(n); V.rho = fl(n);
-        V.b0 = fl(n); V.b1 = fl(n); V.b2 = fl(n); V.b3 = fl(n); V.diag = fl(n);
-        V.ux = l == 0 ? nullptr : fl(n);
-        V.uy = l == 0 ? nullptr : fl(n);
+        V.b0 = fl(n); V.b1 = fl(n); V.b2 = fl(n); V.b3 = fl(n);
+        V.ux = fl(n); V.uy = fl(n);
     }
     F.H[0] = wig::LvlH{reinterpret_cast<__half*>(take(4u * C * 2u)), (uint32_t)C, 0u};
     for (uint32_t l = 1; l <= D.levels; l++) {
         const size_t n = (size_t)D.level_w[l] * D.level_h[l];
         F.H[l] = wig::LvlH{reinterpret_cast<__half*>(take(5u * n * 2u)), (uint32_t)n, 0u};
     }
-    F.pin = fl(C); F.rimx = fl(C); F.rimy = fl(C);
     F.X = fl(C); F.R = fl(C); F.P = fl(C); F.Q = fl(C); F.P2 = fl(C);
     F.part32 = fl(2u * (size_t)D.B);
     F.part64 = reinterpret_cast<double*>(take(2u * (size_t)D.B * 8u));

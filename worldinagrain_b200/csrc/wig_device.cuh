@@ -385,22 +385,35 @@ __device__ __forceinline__ float fineBeta(float a, float b, float da, float db) 
 
 // ---------------------------------------------------------------- batches
 
-// One multigrid level's arrays in the fast form's scratch, a float per cell
-// (row-major, the level's width): potentials and right-hand sides (pressure
-// x, drift y), density, and the stencil's coefficients to the left, right,
-// upper and lower neighbours (0 past an obstacle or the edge) with their sum.
+// One coarse multigrid level's arrays in the fast form's scratch, a float per
+// cell (row-major, the level's width): potentials and right-hand sides
+// (pressure x, drift y), density, and the stencil's coefficients to the
+// left, right, upper and lower neighbours (0 past an obstacle or the edge;
+// the diagonal is their sum in this order).
 struct Lvl {
     float *px, *py, *rx, *ry, *rho;
-    float *b0, *b1, *b2, *b3, *diag;
-    float *ux, *uy;  // levels >= 1: the potentials after the V-cycle's way up (the way down's stay in px, py)
+    float *b0, *b1, *b2, *b3;
+    float *ux, *uy;  // the potentials after the V-cycle's way up (the way down's stay in px, py)
 };
+
+// Level 0, the cells (row-major).  What its kernels read of one cell lies
+// together: both potentials in 8 bytes, the four coefficients in 16, the
+// flags in one.  Its right-hand sides are -R (CG's residual) and ry.
+struct Fine {
+    float2* pot;    // potentials (pressure, drift)
+    float2* rim;    // the potentials before the next relaxation (relaxRims' snapshot; the potentials where not liquid)
+    float4* b;      // the stencil's coefficients, as Lvl's
+    float *rho, *ry;
+    uint8_t* mask;  // FM_*; bit d < 4 set when neighbour d is liquid
+};
+constexpr uint32_t FM_PIN = 16u, FM_LIQUID = 32u;  // held at PIN; liquid
 
 // A level's operator in binary16 (the mixed-precision form), n values an
 // array from base: on a coarse level its density and four stencil
 // coefficients (rho, b0, b1, b2, b3), whose potentials and right-hand sides
 // are stored as bf16 in the first half of Lvl's f32 arrays; on level 0 the
-// four coefficients alone, the copies the smoother reads (the CG's A p reads
-// Lvl's f32 ones).
+// four coefficients alone, a cell's together, the copies the smoother reads
+// (the CG's A p reads Fine's f32 ones).
 struct LvlH {
     __half* base;
     uint32_t n;
@@ -409,11 +422,9 @@ struct LvlH {
 
 // A world's fast-form scratch.
 struct FastW {
-    Lvl L[WIG_MG_LEVELS + 1];  // level 0 (the cells) .. levels
+    Fine Z;                    // level 0
+    Lvl L[WIG_MG_LEVELS + 1];  // levels 1 .. levels
     LvlH H[WIG_MG_LEVELS + 1]; // the operator in binary16 (the mixed form): level 0's coefficients, levels 1 ..
-    float* pin;                // level 0: PIN at a pinned root, else 0
-    uint8_t* fmask;            // level 0: bit d set when neighbour d is liquid
-    float *rimx, *rimy;        // level 0: the relaxation's rim snapshot
     float *X, *R, *P, *Q;      // level 0: CG's x, r, p, A p
     float* P2;                 // level 0: p of the fast form's odd iterations (p of the even ones in P)
     float* part32;             // partial sums: component c of block b at c * B + b

@@ -275,6 +275,14 @@ struct WorldSrc<false> {
 
 // ================================================================ set-up
 
+// The level-0 words of cell i that neighbours read, zeroed.
+__device__ __forceinline__ void zeroFine(const FastW& F, uint32_t i) {
+    F.Z.pot[i] = make_float2(0.0f, 0.0f);
+    F.Z.rim[i] = make_float2(0.0f, 0.0f);
+    F.Z.rho[i] = 0.0f;
+    F.P[i] = 0.0f;
+}
+
 // cgStart, cgResidual, cgPrepare (fluid.wgsl:2665-2732) into the scratch,
 // the cells' coefficients worked out (four tiles a 256-thread CTA, a world's
 // group of four active blocks an item; the CTA that counts a world's last
@@ -290,7 +298,7 @@ __global__ void __launch_bounds__(256) k_fSetup(Batch Bt, const __grid_constant_
         FAST_ITEM(Bt, it, D, F, w, g);
         const uint32_t na = w.activeCount();
         const bool tol = D.st->tol_mode != 0u;
-        const Lvl& L0 = F.L[0];
+        const Fine& Z = F.Z;
         const uint32_t wid = g * 4u + (threadIdx.x >> 6);
         const bool valid = wid < na;
         double b2 = 0.0;
@@ -300,19 +308,18 @@ __global__ void __launch_bounds__(256) k_fSetup(Batch Bt, const __grid_constant_
             const uint32_t i = w.cellIndex(c);
             const float4 gc = w.f4(2u * i), dr = w.f4(2u * i + 1u);
             const float rho = gc.z;
-            L0.rho[i] = rho;
+            Z.rho[i] = rho;
             F.X[i] = gc.x;
             F.P[i] = 0.0f;
             F.Q[i] = 0.0f;
-            L0.px[i] = 0.0f;
-            L0.py[i] = dr.x;
-            L0.ry[i] = dr.y;
-            F.rimx[i] = 0.0f;
-            F.rimy[i] = dr.x;
+            Z.pot[i] = make_float2(0.0f, dr.x);
+            Z.rim[i] = make_float2(0.0f, dr.x);
+            Z.ry[i] = dr.y;
             float bb[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-            float R = 0.0f, pinv = 0.0f;
-            uint8_t mask = 0;
+            float R = 0.0f;
+            uint32_t mask = 0;
             if (rho > 0.0f) {
+                mask = FM_LIQUID;
                 const float share = w.densityAt(c);
                 float sx = 0.0f, dg = 0.0f;
                 for (int d = 0; d < 4; d++) {
@@ -323,32 +330,27 @@ __global__ void __launch_bounds__(256) k_fSetup(Batch Bt, const __grid_constant_
                     if (r < 0.0f) continue;
                     float beta = fineBeta(rho, r, share, w.densityAt(n));
                     bb[d] = beta;
-                    if (r > 0.0f) mask |= (uint8_t)(1u << d);
+                    if (r > 0.0f) mask |= 1u << d;
                     // the stencil over the warm pressure (cgResidual runs before cgPrepare)
                     sx = sx + beta * gn.x;
                     dg = dg + beta;
                 }
-                pinv = (vld(w.gwp(i, G_REGION)) == i) ? PIN : 0.0f;
+                const float pinv = (vld(w.gwp(i, G_REGION)) == i) ? PIN : 0.0f;
+                if (pinv > 0.0f) mask |= FM_PIN;
                 float res = gc.y - (sx - (dg + pinv) * gc.x) / 1.0f;
                 R = -res - 0.0f;
                 double bd = (double)gc.y;
                 b2 = bd * bd;
             }
-            L0.b0[i] = bb[0]; L0.b1[i] = bb[1]; L0.b2[i] = bb[2]; L0.b3[i] = bb[3];
-            L0.diag[i] = bb[0] + bb[1] + bb[2] + bb[3];
+            Z.b[i] = make_float4(bb[0], bb[1], bb[2], bb[3]);
             if (Bt.mixed) {
                 // the smoother's copies of the coefficients (the mixed form)
-                __half* h = F.H[0].base;
-                const uint32_t n = F.H[0].n;
-                h[i] = __float2half_rn(bb[0]);
-                h[n + i] = __float2half_rn(bb[1]);
-                h[2u * n + i] = __float2half_rn(bb[2]);
-                h[3u * n + i] = __float2half_rn(bb[3]);
+                __half2* h = reinterpret_cast<__half2*>(F.H[0].base) + 2u * (size_t)i;
+                h[0] = __floats2half2_rn(bb[0], bb[1]);
+                h[1] = __floats2half2_rn(bb[2], bb[3]);
             }
-            F.pin[i] = pinv;
-            F.fmask[i] = mask;
+            Z.mask[i] = (uint8_t)mask;
             F.R[i] = R;
-            L0.rx[i] = rho > 0.0f ? -R : 0.0f;
         }
         if (tol) {
             double v = tree64x4(s64, b2);
@@ -376,9 +378,7 @@ __global__ void __launch_bounds__(256) k_fSetup(Batch Bt, const __grid_constant_
         I2 c{bq_.x * BLOCK + (int)(threadIdx.x & 7u), bq_.y * BLOCK + (int)((threadIdx.x >> 3) & 7u)};
         if (w.inWorld(c)) {
             uint32_t i = w.cellIndex(c);
-            const Lvl& L0 = F.L[0];
-            L0.px[i] = 0.0f; L0.py[i] = 0.0f; L0.rho[i] = 0.0f;
-            F.rimx[i] = 0.0f; F.rimy[i] = 0.0f; F.P[i] = 0.0f;
+            zeroFine(F, i);
         }
     }
 }
@@ -396,8 +396,7 @@ __global__ void k_fZeroIdle(Batch Bt) {
             I2 c{bq_.x * BLOCK + (int)(t & 7u), bq_.y * BLOCK + (int)(t >> 3)};
             if (!w.inWorld(c)) continue;
             const uint32_t i = w.cellIndex(c);
-            F.L[0].px[i] = 0.0f; F.L[0].py[i] = 0.0f; F.L[0].rho[i] = 0.0f;
-            F.rimx[i] = 0.0f; F.rimy[i] = 0.0f; F.P[i] = 0.0f;
+            zeroFine(F, i);
         }
     }
 }
@@ -408,20 +407,20 @@ __global__ void k_fZero(Dev D, FastW F) {
     const uint32_t C = D.C;
     for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < D.B; n += gridDim.x * blockDim.x) zeroPartials(D, F, n);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < C; i += gridDim.x * blockDim.x) {
-        F.L[0].px[i] = 0.0f; F.L[0].py[i] = 0.0f; F.L[0].rho[i] = 0.0f;
-        F.rimx[i] = 0.0f; F.rimy[i] = 0.0f; F.P[i] = 0.0f;
+        zeroFine(F, i);
     }
 }
 
 // ================================================================ level storage
 
-// A level's arrays as stored, the operator (density, stencil coefficients,
-// diagonal) in T: f32 (the plain precision) or binary16 (the mixed form);
-// values are read into and worked in f32.  The potentials, right-hand sides and way-up potentials of a level whose
-// operator is stored as T: f32 with an f32 operator; bf16 (8 bits of
-// mantissa, f32's range, so no scaling as a residual shrinks) with the mixed
-// form's binary16 operator.  Both are stored in the level's f32 arrays (a
-// bf16 array fills the first half of one).
+// A coarse level's arrays as stored, the operator (density, stencil
+// coefficients) in T: f32 (the plain precision) or binary16 (the mixed
+// form); values are read into and worked in f32.  The potentials,
+// right-hand sides and way-up potentials of a level whose operator is stored
+// as T: f32 with an f32 operator; bf16 (8 bits of mantissa, f32's range, so
+// no scaling as a residual shrinks) with the mixed form's binary16 operator.
+// Both are stored in the level's f32 arrays (a bf16 array fills the first
+// half of one).
 template <class T>
 struct PotOf {
     using type = float;
@@ -430,22 +429,6 @@ template <>
 struct PotOf<__half> {
     using type = __nv_bfloat16;
 };
-// A level's arrays: potentials and right-hand sides of P, densities of R,
-// the stencil's coefficients (and, when B is f32, their stored sum) of B.
-template <class P, class R, class B>
-struct LRefX {
-    P *px, *py, *rx, *ry;
-    R* rho;
-    B *b0, *b1, *b2, *b3, *diag;
-};
-// Levels 1 down as the form stores them (operator T).
-template <class T>
-using LRef = LRefX<typename PotOf<T>::type, T, T>;
-// Level 0 as the form's smoother reads it: all f32, or (the mixed form) its
-// coefficients from their binary16 copies, the potentials, right-hand sides
-// and densities f32 (the CG's A p keeps the f32 coefficients).
-template <class T>
-using L0Ref = LRefX<float, float, T>;
 __device__ __forceinline__ float ld(const float* p) { return *p; }
 __device__ __forceinline__ float ld(const __half* p) { return __half2float(*p); }
 __device__ __forceinline__ float ld(const __nv_bfloat16* p) { return __bfloat162float(*p); }
@@ -453,12 +436,33 @@ __device__ __forceinline__ void st(float* p, float v) { *p = v; }
 __device__ __forceinline__ void st(__half* p, float v) { *p = __float2half_rn(v); }
 __device__ __forceinline__ void st(__nv_bfloat16* p, float v) { *p = __float2bfloat16_rn(v); }
 
+// A cell's coefficients' sum, its diagonal.  In binary16 of the rounded
+// coefficients, so the rounded operator keeps its diagonal equal to the sum
+// of its off-diagonals (a separately rounded diagonal could fall below it
+// and make a region with no free surface indefinite).
+__device__ __forceinline__ float diagOf(float4 b) { return ((b.x + b.y) + b.z) + b.w; }
+
+// Levels 1 down as the form stores them: potentials and right-hand sides of
+// PotOf<T>, densities and coefficients of T.
+template <class T>
+struct LRef {
+    using P = typename PotOf<T>::type;
+    P *px, *py, *rx, *ry;
+    T *rho, *b0, *b1, *b2, *b3;
+    __device__ __forceinline__ float2 pot(uint32_t k) const { return make_float2(ld(px + k), ld(py + k)); }
+    __device__ __forceinline__ float2 rhs(uint32_t k) const { return make_float2(ld(rx + k), ld(ry + k)); }
+    __device__ __forceinline__ float4 coef(uint32_t k) const {
+        return make_float4(ld(b0 + k), ld(b1 + k), ld(b2 + k), ld(b3 + k));
+    }
+    __device__ __forceinline__ float dens(uint32_t k) const { return ld(rho + k); }
+    __device__ __forceinline__ float pin(uint32_t) const { return 0.0f; }
+};
 template <class T>
 __device__ __forceinline__ LRef<T> lref(const FastW& F, uint32_t l);
 template <>
 __device__ __forceinline__ LRef<float> lref<float>(const FastW& F, uint32_t l) {
     const Lvl& V = F.L[l];
-    return LRef<float>{V.px, V.py, V.rx, V.ry, V.rho, V.b0, V.b1, V.b2, V.b3, V.diag};
+    return LRef<float>{V.px, V.py, V.rx, V.ry, V.rho, V.b0, V.b1, V.b2, V.b3};
 }
 template <>
 __device__ __forceinline__ LRef<__half> lref<__half>(const FastW& F, uint32_t l) {
@@ -467,21 +471,26 @@ __device__ __forceinline__ LRef<__half> lref<__half>(const FastW& F, uint32_t l)
     const uint32_t n = F.H[l].n;
     using P = __nv_bfloat16;
     return LRef<__half>{reinterpret_cast<P*>(V.px), reinterpret_cast<P*>(V.py), reinterpret_cast<P*>(V.rx),
-                        reinterpret_cast<P*>(V.ry), b, b + n, b + 2u * n, b + 3u * n, b + 4u * n, nullptr};
+                        reinterpret_cast<P*>(V.ry), b, b + n, b + 2u * n, b + 3u * n, b + 4u * n};
+}
+// Level 0 as the form's smoother reads it: all f32, or (the mixed form) its
+// coefficients from their binary16 copies (the CG's A p keeps the f32 ones).
+__device__ __forceinline__ float4 fineCoef(const FastW& F, uint32_t i, float) { return F.Z.b[i]; }
+__device__ __forceinline__ float4 fineCoef(const FastW& F, uint32_t i, __half) {
+    const uint2 q = reinterpret_cast<const uint2*>(F.H[0].base)[i];
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&q.x));
+    const float2 c = __half22float2(*reinterpret_cast<const __half2*>(&q.y));
+    return make_float4(a.x, a.y, c.x, c.y);
 }
 template <class T>
-__device__ __forceinline__ L0Ref<T> lref0(const FastW& F);
-template <>
-__device__ __forceinline__ L0Ref<float> lref0<float>(const FastW& F) {
-    return lref<float>(F, 0u);
-}
-template <>
-__device__ __forceinline__ L0Ref<__half> lref0<__half>(const FastW& F) {
-    const Lvl& V = F.L[0];
-    __half* b = F.H[0].base;
-    const uint32_t n = F.H[0].n;
-    return L0Ref<__half>{V.px, V.py, V.rx, V.ry, V.rho, b, b + n, b + 2u * n, b + 3u * n, nullptr};
-}
+struct LRef0 {
+    const FastW& F;
+    __device__ __forceinline__ float2 pot(uint32_t k) const { return F.Z.pot[k]; }
+    __device__ __forceinline__ float2 rhs(uint32_t k) const { return make_float2(-F.R[k], F.Z.ry[k]); }
+    __device__ __forceinline__ float4 coef(uint32_t k) const { return fineCoef(F, k, T()); }
+    __device__ __forceinline__ float dens(uint32_t k) const { return F.Z.rho[k]; }
+    __device__ __forceinline__ float pin(uint32_t k) const { return (F.Z.mask[k] & FM_PIN) != 0u ? PIN : 0.0f; }
+};
 // Level l's way-up potentials (l >= 1) as a level of operator T stores them.
 template <class T>
 __device__ __forceinline__ typename PotOf<T>::type* upx(const FastW& F, uint32_t l) {
@@ -490,18 +499,6 @@ __device__ __forceinline__ typename PotOf<T>::type* upx(const FastW& F, uint32_t
 template <class T>
 __device__ __forceinline__ typename PotOf<T>::type* upy(const FastW& F, uint32_t l) {
     return reinterpret_cast<typename PotOf<T>::type*>(F.L[l].uy);
-}
-
-// A cell's diagonal: stored in f32 (the sum of its four coefficients, in
-// that order); in binary16 not stored but the sum of the rounded
-// coefficients, so the rounded operator keeps its diagonal equal to the sum
-// of its off-diagonals (a separately rounded diagonal could fall below it
-// and make a region with no free surface indefinite).
-template <class P, class R>
-__device__ __forceinline__ float diagAt(const LRefX<P, R, float>& V, uint32_t k) { return V.diag[k]; }
-template <class P, class R>
-__device__ __forceinline__ float diagAt(const LRefX<P, R, __half>& V, uint32_t k) {
-    return ((ld(V.b0 + k) + ld(V.b1 + k)) + ld(V.b2 + k)) + ld(V.b3 + k);
 }
 
 // ================================================================ relaxation
@@ -514,23 +511,40 @@ __device__ I2 tileBlockF(const W& w, uint32_t wid, int shift) {
     return j <= high ? I2{wide, j} : I2{j - high - 1, high};
 }
 
-// relaxTile (fluid.wgsl:2109-2182) over the scratch: the rim snapshot's
-// values for liquid cells, the potentials (zero) elsewhere.  A warp a tile
-// (four a CTA, each warp its own run of the list): lane l holds the red and
-// the black cell of quarter l % 4 of row l / 4, so every lane works in every
-// sweep and a sweep ends at a warp barrier.  Within a colour the cells are
-// independent, so each keeps the reference's arithmetic and order.
+// mixf(a, b, 1): a 0 + b, its product exact, so one fused operation rounds
+// as the two do.
+__device__ __forceinline__ float mixed1(float a, float b) {
+    static_assert(SMOOTH_OMEGA == 1.0f, "the smoother's relaxation factor");
+    return __fmaf_rn(a, 0.0f, b);
+}
+
+// relaxTile (fluid.wgsl:2109-2182) over the scratch, from the rim snapshot.
+// A warp a tile (four a CTA, each warp its own run of the list): lane l
+// holds the red and the black cell of quarter l % 4 of row l / 4, so every
+// lane works in every sweep and a sweep ends at a warp barrier; and it loads
+// one of the 32 cells around the tile (the stencil reads no corner).  Within
+// a colour the cells are independent, so each keeps the reference's
+// arithmetic and order.  Bound by its instructions: 11 loads a lane and 8
+// sweeps of two divisions each; the tile's potentials lie in pairs, rows 12
+// pairs apart, so a half-warp's reads of a sweep touch each bank once.  With
+// a float an array (38 loads a lane, the sweeps reading x and y apart) it
+// took 17 us on the 1024x1024 world and 84 us on the 2048x2048 column.
 // `second`: the iteration's relaxation after the V-cycle, on the other
 // tiling from the first (each world's first tiling is its step's).
+constexpr int RXS = RIM + 2;
 template <bool ONE, class T>
 __global__ void __launch_bounds__(128) k_fRelax(Batch Bt, const __grid_constant__ WorldSrc<ONE> src, int second) {
-    __shared__ float tpx[4][RIM * RIM], tpy[4][RIM * RIM];
+    __shared__ float2 tp[4][RIM * RXS];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    float* sx_ = tpx[warp];
-    float* sy_ = tpy[warp];
+    float2* sp = tp[warp];
     const uint32_t n = Bt.n(L_RELAX);
     const uint32_t warps = gridDim.x * 4u, per = (n + warps - 1u) / warps;
     const uint32_t first = (blockIdx.x * 4u + warp) * per, last = min(first + per, n);
+    const int ly = (int)(lane >> 2), q = (int)(lane & 3u);
+    // the lane's cell around the tile: the left and right columns, the rows
+    // above and below, 8 lanes each
+    const int side = (int)(lane >> 3), along = (int)(lane & 7u);
+    const int rx_ = side == 0 ? -1 : side == 1 ? BLOCK : along, ry_ = side == 2 ? -1 : side == 3 ? BLOCK : along;
     for (uint32_t g = first; g < last; g++) {
         const uint32_t it = Bt.item(L_RELAX, g);
         const World& Wd = src.getG(Bt, it);
@@ -540,141 +554,97 @@ __global__ void __launch_bounds__(128) k_fRelax(Batch Bt, const __grid_constant_
         const uint32_t j = Bt.unit(it);
         if (D.st->cont == 0u) continue;
         const int shift = ((D.st->shift_first ^ (uint32_t)second) & 1u) ? BLOCK / 2 : 0;
-        const Lvl& L0 = F.L[0];
+        const Fine& Z = F.Z;
         const uint32_t na = w.activeCount();
         const uint32_t wid = j < na ? j : D.B + (j - na);
         const I2 b = tileBlockF(w, wid, shift);
         const int ox = b.x * BLOCK - shift, oy = b.y * BLOCK - shift;
         if (b.x < 0 || ox >= D.W || oy >= D.H) continue;
-        if ((w.statesOf(I2{ox / BLOCK, oy / BLOCK}, I2{(ox + BLOCK - 1) / BLOCK, (oy + BLOCK - 1) / BLOCK}) & HAS_FLUID) == 0u)
-            continue;
-        // the lane's two cells first (independent of the tile's loads)
-        const int ly = (int)(lane >> 2), q = (int)(lane & 3u);
+        const uint32_t states = w.statesOf(I2{ox / BLOCK, oy / BLOCK}, I2{(ox + BLOCK - 1) / BLOCK, (oy + BLOCK - 1) / BLOCK});
+        // the lane's two cells and its cell around the tile, all loads
+        // issued together (and before the tile's state is known)
         const int p0 = (ox + oy + ly) & 1;
         int t[2];
-        uint32_t idx[2];
-        bool solving[2], visc[2];
-        float rx[2], ry[2], bx[2], by[2], bz[2], bw[2], dxx[2], dyy[2];
+        uint32_t idx[2], mk[2];
+        float R[2], ry[2];
+        float4 bb[2];
+        float2 v[2];
 #pragma unroll
         for (int c = 0; c < 2; c++) {
             const int lx = 2 * q + (c == 0 ? p0 : 1 - p0);
             const I2 me{ox + lx, oy + ly};
-            t[c] = (ly + 1) * RIM + lx + 1;
-            float r_x = 0.0f, r_y = 0.0f, b0 = 0.0f, b1 = 0.0f, b2 = 0.0f, b3 = 0.0f, dg = 0.0f, pv = 0.0f;
-            uint32_t id = 0;
-            bool fluid = false;
-            if (w.inWorld(me)) {
-                id = w.cellIndex(me);
-                const L0Ref<T> S0 = lref0<T>(F);
-                fluid = L0.rho[id] > 0.0f;
-                r_x = L0.rx[id];
-                r_y = L0.ry[id];
-                b0 = ld(S0.b0 + id);
-                b1 = ld(S0.b1 + id);
-                b2 = ld(S0.b2 + id);
-                b3 = ld(S0.b3 + id);
-                dg = diagAt(S0, id);
-                pv = F.pin[id];
-            }
-            if (!fluid) {
-                r_x = 0.0f; r_y = 0.0f; b0 = 0.0f; b1 = 0.0f; b2 = 0.0f; b3 = 0.0f; dg = 0.0f; pv = 0.0f;
-            }
-            idx[c] = id;
-            rx[c] = r_x; ry[c] = r_y; bx[c] = b0; by[c] = b1; bz[c] = b2; bw[c] = b3;
-            dxx[c] = dg + pv;
-            dyy[c] = fmaxf(dg, 1e-30f);
-            solving[c] = fluid && dxx[c] > 0.0f;
+            const bool in = w.inWorld(me);
+            t[c] = (ly + 1) * RXS + lx + 1;
+            idx[c] = in ? w.cellIndex(me) : 0u;
+            mk[c] = in ? Z.mask[idx[c]] : 0u;
+            R[c] = F.R[idx[c]];
+            ry[c] = Z.ry[idx[c]];
+            bb[c] = fineCoef(F, idx[c], T());
+            v[c] = in ? Z.rim[idx[c]] : make_float2(0.0f, 0.0f);
+        }
+        const I2 rc{ox + rx_, oy + ry_};
+        const float2 around = w.inWorld(rc) ? Z.rim[w.cellIndex(rc)] : make_float2(0.0f, 0.0f);
+        if ((states & HAS_FLUID) == 0u) continue;
+        float dx[2], dy[2];
+        bool solving[2], visc[2];
+#pragma unroll
+        for (int c = 0; c < 2; c++) {
+            const float dg = diagOf(bb[c]);
+            dx[c] = dg + ((mk[c] & FM_PIN) != 0u ? PIN : 0.0f);
+            dy[c] = fmaxf(dg, 1e-30f);
+            solving[c] = (mk[c] & FM_LIQUID) != 0u && dx[c] > 0.0f;
             visc[c] = dg > 0.0f;
+            sp[t[c]] = v[c];
         }
-        // the tile and its rim: the snapshot's values for liquid cells, the
-        // potentials elsewhere
-        // (the four rounds of the lane's loads issued together)
-        {
-            constexpr int NR = (RIM * RIM + 31) / 32;
-            float rr[NR], ax[NR], ay[NR], qx[NR], qy[NR];
-            bool inw[NR];
-#pragma unroll
-            for (int u = 0; u < NR; u++) {
-                const int k = (int)lane + 32 * u;
-                const I2 c{ox - 1 + k % RIM, oy - 1 + k / RIM};
-                inw[u] = k < RIM * RIM && w.inWorld(c);
-                const uint32_t i = inw[u] ? w.cellIndex(c) : 0u;
-                rr[u] = L0.rho[i];
-                ax[u] = F.rimx[i];
-                ay[u] = F.rimy[i];
-                qx[u] = L0.px[i];
-                qy[u] = L0.py[i];
-            }
-#pragma unroll
-            for (int u = 0; u < NR; u++) {
-                const int k = (int)lane + 32 * u;
-                if (k >= RIM * RIM) continue;
-                float px = 0.0f, py = 0.0f;
-                if (inw[u]) {
-                    px = rr[u] > 0.0f ? ax[u] : qx[u];
-                    py = rr[u] > 0.0f ? ay[u] : qy[u];
-                }
-                sx_[k] = px;
-                sy_[k] = py;
-            }
-        }
+        sp[(ry_ + 1) * RXS + rx_ + 1] = around;
         __syncwarp();
+#pragma unroll
         for (int sw = 0; sw < 2 * SWEEPS; sw++) {
             const int c = sw & 1;
             if (solving[c]) {
-                const int tc = t[c];
-                float sx = bx[c] * sx_[tc - 1] + by[c] * sx_[tc + 1] + bz[c] * sx_[tc - RIM] + bw[c] * sx_[tc + RIM];
-                float sy = bx[c] * sy_[tc - 1] + by[c] * sy_[tc + 1] + bz[c] * sy_[tc - RIM] + bw[c] * sy_[tc + RIM];
-                float nx = mixf(sx_[tc], (sx - rx[c]) / dxx[c], SMOOTH_OMEGA);
-                float ny = mixf(sy_[tc], (sy - ry[c]) / dyy[c], SMOOTH_OMEGA);
-                sx_[tc] = nx;
-                if (visc[c]) sy_[tc] = ny;
+                const float2* s = sp + t[c];
+                const float2 l = s[-1], r = s[1], u = s[-RXS], d = s[RXS];
+                const float sx = bb[c].x * l.x + bb[c].y * r.x + bb[c].z * u.x + bb[c].w * d.x;
+                const float sy = bb[c].x * l.y + bb[c].y * r.y + bb[c].z * u.y + bb[c].w * d.y;
+                // the right-hand side is -R
+                v[c].x = mixed1(v[c].x, (sx + R[c]) / dx[c]);
+                const float ny = mixed1(v[c].y, (sy - ry[c]) / dy[c]);
+                if (visc[c]) v[c].y = ny;
+                sp[t[c]] = v[c];
             }
             __syncwarp();
         }
 #pragma unroll
         for (int c = 0; c < 2; c++)
-            if (solving[c]) {
-                L0.px[idx[c]] = sx_[t[c]];
-                L0.py[idx[c]] = sy_[t[c]];
-            }
-        __syncwarp();
+            if (solving[c]) Z.pot[idx[c]] = v[c];
     }
 }
 
 // ================================================================ the levels
 
-// residualAt (fluid.wgsl:2306-2315) of cell k on a level held in arrays with
-// stored coefficients (level 0's pinned roots held at PIN).  The division by
-// h2, a power of two, is the multiplication by its exact inverse: the same
-// real number rounded once either way, so the same bits.
-template <class VT>
-__device__ __forceinline__ V2 residualStored(const VT& V, const float* pin, uint32_t k, int x, int y, int lw, int lh,
-                                             float inv_h2) {
-    float sx = 0.0f, sy = 0.0f;
-    const float b[4] = {ld(V.b0 + k), ld(V.b1 + k), ld(V.b2 + k), ld(V.b3 + k)};
-#pragma unroll
-    for (int d = 0; d < 4; d++) {
-        uint32_t n = nbr(k, x, y, lw, lh, d);
-        sx = sx + b[d] * ld(V.px + n);
-        sy = sy + b[d] * ld(V.py + n);
-    }
-    const float dg = diagAt(V, k);
-    const float pinx = pin ? pin[k] : 0.0f;
-    return V2{ld(V.rx + k) - (sx - (dg + pinx) * ld(V.px + k)) * inv_h2,
-              ld(V.ry + k) - (sy - (dg + 0.0f) * ld(V.py + k)) * inv_h2};
+// residualAt (fluid.wgsl:2306-2315) of a cell from its coefficients, its
+// potentials p, its neighbours' l, r, u, d, its right-hand side and pin.  The
+// division by h2, a power of two, is the multiplication by its exact
+// inverse: the same real number rounded once either way, so the same bits.
+__device__ __forceinline__ V2 residualOf(float4 b, float2 p, float2 l, float2 r, float2 u, float2 d, float2 rhs, float pin,
+                                         float inv_h2) {
+    const float sx = (((0.0f + b.x * l.x) + b.y * r.x) + b.z * u.x) + b.w * d.x;
+    const float sy = (((0.0f + b.x * l.y) + b.y * r.y) + b.z * u.y) + b.w * d.y;
+    const float dg = diagOf(b);
+    return V2{rhs.x - (sx - (dg + pin) * p.x) * inv_h2, rhs.y - (sy - (dg + 0.0f) * p.y) * inv_h2};
 }
 
 // restrictLevel's values of level-l cell (cx, cy) from level l - 1, stored
-// as TU (fluid.wgsl:2342-2377): the density and, with `res`, the restricted
-// residuals; all 0 in a block not worked on.  The four finer cells' words
-// are all loaded before any is used (a cell past the level's edge reads
-// the level's first cell and is then left out; a cell not liquid has its
-// residual worked and dropped), so their loads are in flight together; the
-// sums then take the liquid cells in the reference's order.
+// as VT reads it (fluid.wgsl:2342-2377): the density and, with `res`, the
+// restricted residuals; all 0 in a block not worked on.  The four finer
+// cells' words and the 12 potentials their stencils share are all loaded
+// before any is used (coordinates clamped onto the level, as the stencil's
+// neighbours are onto their cell; a cell not liquid has its residual worked
+// and dropped), so their loads are in flight together; the sums then take
+// the liquid cells in the reference's order.
 template <class VT>
-__device__ __forceinline__ void restrictedFrom(const Dev& D, const FastW& F, const W& w, uint32_t l, const VT& U, int cx,
-                                               int cy, bool res, float& rho_o, float& rx_o, float& ry_o) {
+__device__ __forceinline__ void restrictedFrom(const Dev& D, const W& w, uint32_t l, const VT& U, int cx, int cy, bool res,
+                                               float& rho_o, float& rx_o, float& ry_o) {
     const int span = 1 << l;
     if (span <= BLOCK) {
         I2 b{cx * span / BLOCK, cy * span / BLOCK};
@@ -686,25 +656,44 @@ __device__ __forceinline__ void restrictedFrom(const Dev& D, const FastW& F, con
         }
     }
     const int uw = (int)D.level_w[l - 1], uh = (int)D.level_h[l - 1];
-    const float inv_h2 = 1.0f / (float)(1u << (2u * (l - 1u)));
-    const float* pin = l == 1u ? F.pin : nullptr;
+    const int x0 = 2 * cx, y0 = 2 * cy;
+    const bool in_x = x0 + 1 < uw, in_y = y0 + 1 < uh;  // rhoAt outside the level: -1
+    const uint32_t xs[4] = {(uint32_t)max(x0 - 1, 0), (uint32_t)x0, (uint32_t)min(x0 + 1, uw - 1), (uint32_t)min(x0 + 2, uw - 1)};
+    const uint32_t ys[4] = {(uint32_t)max(y0 - 1, 0) * (uint32_t)uw, (uint32_t)y0 * (uint32_t)uw,
+                            (uint32_t)min(y0 + 1, uh - 1) * (uint32_t)uw, (uint32_t)min(y0 + 2, uh - 1) * (uint32_t)uw};
     float rq[4];
     V2 eq[4];
-    bool inq[4];
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-        const int kx = 2 * cx + (q & 1), ky = 2 * cy + (q >> 1);
-        inq[q] = kx < uw && ky < uh;  // rhoAt outside the level: -1
-        const int sx = inq[q] ? kx : 0, sy = inq[q] ? ky : 0;
-        const uint32_t k = (uint32_t)sy * (uint32_t)uw + (uint32_t)sx;
-        rq[q] = ld(U.rho + k);
-        eq[q] = res ? residualStored(U, pin, k, sx, sy, uw, uh, inv_h2) : V2{0.0f, 0.0f};
+    for (int q = 0; q < 4; q++) rq[q] = U.dens(ys[1 + (q >> 1)] + xs[1 + (q & 1)]);
+    if (res) {
+        const float inv_h2 = 1.0f / (float)(1u << (2u * (l - 1u)));
+        float2 p[4][4];  // [row][column], corners not read
+        float4 bq[4];
+        float2 hq[4];
+        float pq[4];
+#pragma unroll
+        for (int y = 0; y < 4; y++)
+#pragma unroll
+            for (int x = 0; x < 4; x++)
+                if ((x == 1 || x == 2) || (y == 1 || y == 2)) p[y][x] = U.pot(ys[y] + xs[x]);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const uint32_t k = ys[1 + (q >> 1)] + xs[1 + (q & 1)];
+            bq[q] = U.coef(k);
+            hq[q] = U.rhs(k);
+            pq[q] = U.pin(k);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int x = 1 + (q & 1), y = 1 + (q >> 1);
+            eq[q] = residualOf(bq[q], p[y][x], p[y][x - 1], p[y][x + 1], p[y - 1][x], p[y + 1][x], hq[q], pq[q], inv_h2);
+        }
     }
     float fluid = 0.0f, sum = 0.0f, rx = 0.0f, ry = 0.0f;
     bool air = false;
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-        if (!inq[q]) continue;
+        if ((!in_x && (q & 1)) || (!in_y && (q >> 1))) continue;
         const float rho = rq[q];
         if (rho == 0.0f) air = true;
         else if (rho > 0.0f) {
@@ -723,32 +712,28 @@ __device__ __forceinline__ void restrictedFrom(const Dev& D, const FastW& F, con
 }
 
 // restrictedFrom for level l of a form whose levels store operator T: from
-// level 0 as its smoother reads it, or from level l - 1.
-template <class T>
+// level 0 as its smoother reads it (FINE: l is 1), or from level l - 1.
+template <class T, bool FINE>
 __device__ __forceinline__ void restrictedAt(const Dev& D, const FastW& F, const W& w, uint32_t l, int cx, int cy,
                                              bool res, float& rho_o, float& rx_o, float& ry_o) {
-    if (l == 1u) restrictedFrom(D, F, w, l, lref0<T>(F), cx, cy, res, rho_o, rx_o, ry_o);
-    else restrictedFrom(D, F, w, l, lref<T>(F, l - 1u), cx, cy, res, rho_o, rx_o, ry_o);
+    if (FINE) restrictedFrom(D, w, l, LRef0<T>{F}, cx, cy, res, rho_o, rx_o, ry_o);
+    else restrictedFrom(D, w, l, lref<T>(F, l - 1u), cx, cy, res, rho_o, rx_o, ry_o);
 }
 
-// One coarse cell of restrictLevel, level l (stored as TV) from l - 1
-// (stored as TU): the cell's values, its potentials zeroed.
-template <class T>
-__device__ void restrictCellT(const Dev& D, const FastW& F, const W& w, uint32_t l, uint32_t j) {
+// One coarse cell of restrictLevel, level l from l - 1 (FINE: level 1 from
+// level 0) with the levels stored as T: the cell's values, its potentials
+// zeroed.
+template <class T, bool FINE>
+__device__ void restrictCell(const Dev& D, const FastW& F, const W& w, uint32_t l, uint32_t j) {
     const int lw = (int)D.level_w[l];
     const LRef<T> V = lref<T>(F, l);
     float rho, rx, ry;
-    restrictedAt<T>(D, F, w, l, (int)(j % (uint32_t)lw), (int)(j / (uint32_t)lw), true, rho, rx, ry);
+    restrictedAt<T, FINE>(D, F, w, l, (int)(j % (uint32_t)lw), (int)(j / (uint32_t)lw), true, rho, rx, ry);
     st(V.px + j, 0.0f);
     st(V.py + j, 0.0f);
     st(V.rx + j, rx);
     st(V.ry + j, ry);
     st(V.rho + j, rho);
-}
-// Level l from l - 1 with the levels stored as T (level 0 always f32).
-template <class T = float>
-__device__ __forceinline__ void restrictCell(const Dev& D, const FastW& F, const W& w, uint32_t l, uint32_t j) {
-    restrictCellT<T>(D, F, w, l, j);
 }
 
 // One cell of smoothAt (fluid.wgsl:2318-2334) on level l >= 1, the
@@ -764,24 +749,19 @@ __device__ void smoothCell(const Dev& D, const FastW& F, uint32_t l, int color, 
     float b[4];
     float dg;
     if (first) {
-        dg = 0.0f;
         for (int d = 0; d < 4; d++) {
             b[d] = 0.0f;
             if (!nbrIn(cx, cy, lw, lh, d)) continue;
             float r = ld(V.rho + nbr(j, cx, cy, lw, lh, d));
             if (r < 0.0f) continue;
             b[d] = faceBeta(rho, r);
-            dg = dg + b[d];
         }
         st(V.b0 + j, b[0]); st(V.b1 + j, b[1]); st(V.b2 + j, b[2]); st(V.b3 + j, b[3]);
-        if (V.diag) st(V.diag + j, dg);
-        // worked in what is stored, as later iterations read it
-        b[0] = ld(V.b0 + j); b[1] = ld(V.b1 + j); b[2] = ld(V.b2 + j); b[3] = ld(V.b3 + j);
-        dg = diagAt(V, j);
-    } else {
-        b[0] = ld(V.b0 + j); b[1] = ld(V.b1 + j); b[2] = ld(V.b2 + j); b[3] = ld(V.b3 + j);
-        dg = diagAt(V, j);
     }
+    // worked in what is stored, as later iterations read it
+    const float4 bs = V.coef(j);
+    b[0] = bs.x; b[1] = bs.y; b[2] = bs.z; b[3] = bs.w;
+    dg = diagOf(bs);
     if (dg <= 0.0f) return;
     float sx = 0.0f, sy = 0.0f;
 #pragma unroll
@@ -918,7 +898,7 @@ __device__ __forceinline__ void tileSmooth(LevelTile& t, int x0, int y0, int lw,
 // from the densities (as the step's first iteration works and stores them,
 // and later ones read them back), stored by the tile's own cells on the
 // first iteration.
-template <bool ONE, class T, int NT = 256>
+template <bool ONE, class T, int NT, bool FINE>
 __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 2) k_fDown(Batch Bt, const __grid_constant__ WorldSrc<ONE> src, uint32_t l) {
     __shared__ WorldCopy wc_;
     if (!ONE) worldCopyInit(wc_);
@@ -931,7 +911,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 2) k_fDown(Batch Bt, const
         if (l >= F.lc) {
             const int cx = x0 + (int)threadIdx.x % LT, cy = y0 + (int)threadIdx.x / LT;
             if (threadIdx.x < (unsigned)(LT * LT) && cx < lw && cy < lh)
-                restrictCell<T>(D, F, w, l, (uint32_t)(cy * lw + cx));
+                restrictCell<T, FINE>(D, F, w, l, (uint32_t)(cy * lw + cx));
             continue;
         }
         const LRef<T> V = lref<T>(F, l);
@@ -941,7 +921,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 2) k_fDown(Batch Bt, const
             float rho = -1.0f, rx = 0.0f, ry = 0.0f;
             if (cx >= 0 && cy >= 0 && cx < lw && cy < lh) {
                 const bool res = ix >= -1 && iy >= -1 && ix <= LT && iy <= LT;
-                restrictedAt<T>(D, F, w, l, cx, cy, res, rho, rx, ry);
+                restrictedAt<T, FINE>(D, F, w, l, cx, cy, res, rho, rx, ry);
             }
             t.rho[k] = asStored(rho, T());
             t.rx[k] = rx;
@@ -957,7 +937,6 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 2) k_fDown(Batch Bt, const
             const float rho = t.rho[i];
             if (rho <= 0.0f) continue;
             float b[4];
-            float dg = 0.0f;
 #pragma unroll
             for (int d = 0; d < 4; d++) {
                 b[d] = 0.0f;
@@ -965,19 +944,15 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 2) k_fDown(Batch Bt, const
                 const float r = t.rho[lsn(ix, iy, cx, cy, lw, lh, d)];
                 if (r < 0.0f) continue;
                 b[d] = faceBeta(rho, r);
-                dg = dg + b[d];
             }
             const bool own = ix >= 0 && iy >= 0 && ix < LT && iy < LT;
             if (first && own) {
                 const uint32_t j = (uint32_t)(cy * lw + cx);
                 st(V.b0 + j, b[0]); st(V.b1 + j, b[1]); st(V.b2 + j, b[2]); st(V.b3 + j, b[3]);
-                if (V.diag) st(V.diag + j, dg);
             }
 #pragma unroll
             for (int d = 0; d < 4; d++) t.b[d][i] = asStored(b[d], T());
-            // the diagonal as diagAt reads it: stored in f32, the rounded
-            // coefficients' sum in binary16
-            t.dg[i] = V.diag ? dg : ((t.b[0][i] + t.b[1][i]) + t.b[2][i]) + t.b[3][i];
+            t.dg[i] = ((t.b[0][i] + t.b[1][i]) + t.b[2][i]) + t.b[3][i];
         }
         __syncthreads();
         tileSmooth(t, x0, y0, lw, lh, (float)(1u << (2u * l)));
@@ -1029,7 +1004,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 2) k_fUp(Batch Bt, const _
                 px = ld(V.px + j);
                 py = ld(V.py + j);
                 const V2 e = prolongedFrom(urho, lux, luy, uw, uh, cx, cy);
-                float rx = 0.0f, ry = 0.0f, b0 = 0.0f, b1 = 0.0f, b2 = 0.0f, b3 = 0.0f, dg = 0.0f;
+                float rx = 0.0f, ry = 0.0f, b0 = 0.0f, b1 = 0.0f, b2 = 0.0f, b3 = 0.0f;
                 if (ring1) {
                     rx = ld(V.rx + j);
                     ry = ld(V.ry + j);
@@ -1037,7 +1012,6 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 2) k_fUp(Batch Bt, const _
                     b1 = ld(V.b1 + j);
                     b2 = ld(V.b2 + j);
                     b3 = ld(V.b3 + j);
-                    dg = diagAt(V, j);
                 }
                 if (rho > 0.0f) {
                     px = px + e.x;
@@ -1049,7 +1023,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 2) k_fUp(Batch Bt, const _
                         t.b[1][k] = b1;
                         t.b[2][k] = b2;
                         t.b[3][k] = b3;
-                        t.dg[k] = dg;
+                        t.dg[k] = ((b0 + b1) + b2) + b3;
                     }
                 }
             }
@@ -1757,21 +1731,19 @@ __global__ void k_fProlongFine(Batch Bt, const __grid_constant__ WorldSrc<ONE> s
     FOR_ITEMS(Bt, L_ACT, it) {
         FAST_ITEM(Bt, it, D, F, w, wid);
         if (D.st->cont == 0u) continue;
-        const Lvl& L0 = F.L[0];
         const T* urho = lref<T>(F, 1u).rho;
         I2 c = lidCell(w, wid);
         if (!w.inWorld(c)) continue;
         uint32_t i = w.cellIndex(c);
         // the cell's words and the prolongation's loaded together, then used
         // for a liquid cell only
-        const float rho = L0.rho[i], px0 = L0.px[i], py0 = L0.py[i];
+        const uint32_t mk = F.Z.mask[i];
+        const float2 p = F.Z.pot[i];
         const V2 e = prolongedFrom(urho, upx<T>(F, 1u), upy<T>(F, 1u), (int)D.level_w[1], (int)D.level_h[1], c.x, c.y);
-        if (rho > 0.0f) {
-            float px = px0 + e.x, py = py0 + e.y;
-            L0.px[i] = px;
-            L0.py[i] = py;
-            F.rimx[i] = px;
-            F.rimy[i] = py;
+        if ((mk & FM_LIQUID) != 0u) {
+            const float2 v = make_float2(p.x + e.x, p.y + e.y);
+            F.Z.pot[i] = v;
+            F.Z.rim[i] = v;
         }
     }
 }
@@ -1932,10 +1904,11 @@ __global__ void __launch_bounds__(CG_THREADS, 2) k_fRhoBeta(Batch Bt, const __gr
         if (D.st->cont == 0u) return;
         const bool f64 = D.st->f64 != 0u;
         const uint32_t cycle = D.st->cycle;
-        const Lvl& L0 = F.L[0];
+        const Fine& Z = F.Z;
         for (uint32_t t0 = warp; t0 < m; t0 += 2u * CG_WARPS) {
             TileLane t[2];
-            float rho[2][2], z[2][2], r[2][2], q[2][2];
+            uint32_t mk[2][2];
+            float z[2][2], r[2][2], q[2][2];
 #pragma unroll
             for (int u = 0; u < 2; u++) t[u] = tileLane(w, j0 + t0 + (uint32_t)u * CG_WARPS, t0 + (uint32_t)u * CG_WARPS < m);
 #pragma unroll
@@ -1943,15 +1916,15 @@ __global__ void __launch_bounds__(CG_THREADS, 2) k_fRhoBeta(Batch Bt, const __gr
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     const uint32_t i = t[u].i[h];
-                    rho[u][h] = L0.rho[i];
-                    z[u][h] = L0.px[i];
+                    mk[u][h] = Z.mask[i];
+                    z[u][h] = Z.pot[i].x;
                     r[u][h] = F.R[i];
                     q[u][h] = F.Q[i];
                 }
 #pragma unroll
             for (int u = 0; u < 2; u++) {
                 if (t0 + (uint32_t)u * CG_WARPS >= m) break;  // (warp-uniform)
-                const bool f0 = t[u].in[0] && rho[u][0] > 0.0f, f1 = t[u].in[1] && rho[u][1] > 0.0f;
+                const bool f0 = t[u].in[0] && (mk[u][0] & FM_LIQUID) != 0u, f1 = t[u].in[1] && (mk[u][1] & FM_LIQUID) != 0u;
                 // the f32 trees only without FP64 dots, which read none of them
                 if (f64) {
                     const double x = warpTree(f0 ? (double)r[u][0] * (double)z[u][0] : 0.0,
@@ -2022,7 +1995,7 @@ __global__ void __launch_bounds__(CG_THREADS, 2) k_fApplyAlpha(Batch Bt, const _
         const bool odd = (D.st->cycle & 1u) != 0u;
         const float* Pold = odd ? F.P2 : F.P;
         float* Pnew = odd ? F.P : F.P2;
-        const Lvl& L0 = F.L[0];
+        const Fine& Z = F.Z;
         auto dir = [&](float z, float p) { return f64 ? (float)((double)z + beta64 * (double)p) : z + beta * p; };
         for (uint32_t t0 = warp; t0 < m; t0 += CG_WARPS) {
             const TileLane t = tileLane(w, j0 + t0, true);
@@ -2030,20 +2003,16 @@ __global__ void __launch_bounds__(CG_THREADS, 2) k_fApplyAlpha(Batch Bt, const _
             const I2 oc{b.x * BLOCK + ox, b.y * BLOCK + oy};
             const bool oin = w.inWorld(oc);
             const uint32_t oi = oin ? w.cellIndex(oc) : 0u;
-            const float oz = L0.px[oi], op = Pold[oi];
-            float rho[2], bl[2], br[2], bu[2], bd[2], dgp[2], z[2], po[2];
-            uint8_t mk[2];
+            const float oz = Z.pot[oi].x, op = Pold[oi];
+            float4 bb[2];
+            float z[2], po[2];
+            uint32_t mk[2];
 #pragma unroll
             for (int h = 0; h < 2; h++) {
                 const uint32_t i = t.i[h];
-                rho[h] = L0.rho[i];
-                mk[h] = F.fmask[i];
-                bl[h] = L0.b0[i];
-                br[h] = L0.b1[i];
-                bu[h] = L0.b2[i];
-                bd[h] = L0.b3[i];
-                dgp[h] = L0.diag[i] + F.pin[i];
-                z[h] = L0.px[i];
+                mk[h] = Z.mask[i];
+                bb[h] = Z.b[i];
+                z[h] = Z.pot[i].x;
                 po[h] = Pold[i];
             }
             float p[2];
@@ -2060,13 +2029,14 @@ __global__ void __launch_bounds__(CG_THREADS, 2) k_fApplyAlpha(Batch Bt, const _
             for (int h = 0; h < 2; h++) {
                 const int c = c0 + 4 * RIM * h;
                 q[h] = 0.0f;
-                if (t.in[h] && rho[h] > 0.0f) {
+                if (t.in[h] && (mk[h] & FM_LIQUID) != 0u) {
                     float sum = 0.0f;
-                    if (mk[h] & 1u) sum = sum + bl[h] * sp[c - 1];
-                    if (mk[h] & 2u) sum = sum + br[h] * sp[c + 1];
-                    if (mk[h] & 4u) sum = sum + bu[h] * sp[c - RIM];
-                    if (mk[h] & 8u) sum = sum + bd[h] * sp[c + RIM];
-                    q[h] = dgp[h] * p[h] - sum + 0.0f;
+                    if (mk[h] & 1u) sum = sum + bb[h].x * sp[c - 1];
+                    if (mk[h] & 2u) sum = sum + bb[h].y * sp[c + 1];
+                    if (mk[h] & 4u) sum = sum + bb[h].z * sp[c - RIM];
+                    if (mk[h] & 8u) sum = sum + bb[h].w * sp[c + RIM];
+                    const float dgp = diagOf(bb[h]) + ((mk[h] & FM_PIN) != 0u ? PIN : 0.0f);
+                    q[h] = dgp * p[h] - sum + 0.0f;
                 } else {
                     p[h] = 0.0f;
                 }
@@ -2125,12 +2095,13 @@ __global__ void __launch_bounds__(CG_THREADS, 2) k_fUpdate(Batch Bt, const __gri
         const bool f64 = D.st->f64 != 0u, tol = D.st->tol_mode != 0u;
         const float alpha = D.st->alpha32;
         const double alpha64 = D.st->alpha;
-        const Lvl& L0 = F.L[0];
+        const Fine& Z = F.Z;
         const float* P = (cycle & 1u) ? F.P : F.P2;
         uint32_t most = 0u;
         for (uint32_t t0 = warp; t0 < m; t0 += 2u * CG_WARPS) {
             TileLane t[2];
-            float rho[2][2], vx[2][2], vy[2][2], vz[2][2], vw[2][2], py[2][2];
+            uint32_t mk[2][2];
+            float vx[2][2], vy[2][2], vz[2][2], vw[2][2], py[2][2];
 #pragma unroll
             for (int u = 0; u < 2; u++) t[u] = tileLane(w, j0 + t0 + (uint32_t)u * CG_WARPS, t0 + (uint32_t)u * CG_WARPS < m);
 #pragma unroll
@@ -2138,12 +2109,12 @@ __global__ void __launch_bounds__(CG_THREADS, 2) k_fUpdate(Batch Bt, const __gri
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     const uint32_t i = t[u].i[h];
-                    rho[u][h] = L0.rho[i];
+                    mk[u][h] = Z.mask[i];
                     vx[u][h] = F.X[i];
                     vy[u][h] = F.R[i];
                     vz[u][h] = P[i];
                     vw[u][h] = F.Q[i];
-                    py[u][h] = L0.py[i];
+                    py[u][h] = Z.pot[i].y;
                 }
 #pragma unroll
             for (int u = 0; u < 2; u++) {
@@ -2151,7 +2122,7 @@ __global__ void __launch_bounds__(CG_THREADS, 2) k_fUpdate(Batch Bt, const __gri
                 double r2[2] = {0.0, 0.0};
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
-                    if (!t[u].in[h] || !(rho[u][h] > 0.0f)) continue;
+                    if (!t[u].in[h] || (mk[u][h] & FM_LIQUID) == 0u) continue;
                     const uint32_t i = t[u].i[h];
                     float r, x;
                     if (f64) {
@@ -2163,10 +2134,8 @@ __global__ void __launch_bounds__(CG_THREADS, 2) k_fUpdate(Batch Bt, const __gri
                     }
                     F.X[i] = x;
                     F.R[i] = r;
-                    L0.px[i] = 0.0f;
-                    L0.rx[i] = -r;
-                    F.rimx[i] = 0.0f;
-                    F.rimy[i] = py[u][h];
+                    Z.pot[i].x = 0.0f;
+                    Z.rim[i] = make_float2(0.0f, py[u][h]);
                     most = max(most, __float_as_uint(fabsf(r)));
                     r2[h] = (double)r * (double)r;
                 }
@@ -2219,10 +2188,11 @@ __global__ void __launch_bounds__(CG_THREADS, 2) k_fUpdate(Batch Bt, const __gri
 // u (|d x| + sum |beta x_n|), u = 2^-24 (the CG's own residual cannot stay
 // below that floor's norm).
 __device__ __forceinline__ double trueResidualAt(const Dev& D, const FastW& F, I2 c, uint32_t i, double* floor2) {
-    const Lvl& L0 = F.L[0];
-    const uint8_t m = F.fmask[i];
-    const float bb[4] = {L0.b0[i], L0.b1[i], L0.b2[i], L0.b3[i]};
-    const double dx = (double)(L0.diag[i] + F.pin[i]) * (double)F.X[i];
+    const Fine& Z = F.Z;
+    const uint32_t m = Z.mask[i];
+    const float4 b4 = Z.b[i];
+    const float bb[4] = {b4.x, b4.y, b4.z, b4.w};
+    const double dx = (double)(diagOf(b4) + ((m & FM_PIN) != 0u ? PIN : 0.0f)) * (double)F.X[i];
     double ax = dx, mag = fabs(dx);
 #pragma unroll
     for (int d = 0; d < 4; d++)
@@ -2251,7 +2221,7 @@ __global__ void __launch_bounds__(256) k_fTrueCheck(Batch Bt, const __grid_const
     FOR_ITEMS(Bt, L_ACT4, it) {
         FAST_ITEM(Bt, it, D, F, w, g);
         if (D.st->check == 0u) continue;
-        const Lvl& L0 = F.L[0];
+        const Fine& Z = F.Z;
         const uint32_t na = w.activeCount();
         const uint32_t wid = g * 4u + (threadIdx.x >> 6);
         const bool valid = wid < na;
@@ -2260,7 +2230,7 @@ __global__ void __launch_bounds__(256) k_fTrueCheck(Batch Bt, const __grid_const
             I2 c = tileCell(w, wid);
             if (w.inWorld(c)) {
                 const uint32_t i = w.cellIndex(c);
-                if (L0.rho[i] > 0.0f) {
+                if ((Z.mask[i] & FM_LIQUID) != 0u) {
                     const double r = trueResidualAt(D, F, c, i, &f2);
                     r2 = r * r;
                 }
@@ -2297,8 +2267,7 @@ __global__ void __launch_bounds__(256) k_fTrueCheck(Batch Bt, const __grid_const
     }
 }
 
-// The true residual put in for the recursive one (CG's r and the
-// smoother's -r), for the worlds k_fTrueCheck found drifted.
+// The true residual put in for the recursive one, for the worlds k_fTrueCheck found drifted.
 template <bool ONE>
 __global__ void k_fTrueFix(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
@@ -2306,15 +2275,13 @@ __global__ void k_fTrueFix(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) 
     FOR_ITEMS(Bt, L_ACT, it) {
         FAST_ITEM(Bt, it, D, F, w, wid);
         if (D.st->drift == 0u) continue;
-        const Lvl& L0 = F.L[0];
+        const Fine& Z = F.Z;
         I2 c = lidCell(w, wid);
         if (!w.inWorld(c)) continue;
         const uint32_t i = w.cellIndex(c);
-        if (L0.rho[i] <= 0.0f) continue;
+        if ((Z.mask[i] & FM_LIQUID) == 0u) continue;
         double f2;
-        const float rf = (float)trueResidualAt(D, F, c, i, &f2);
-        F.R[i] = rf;
-        L0.rx[i] = -rf;
+        F.R[i] = (float)trueResidualAt(D, F, c, i, &f2);
     }
 }
 
@@ -2367,14 +2334,14 @@ __global__ void k_fFinish(Batch Bt, const __grid_constant__ WorldSrc<ONE> src, i
     }
     FOR_ITEMS(Bt, L_ACT, it) {
         FAST_ITEM(Bt, it, D, F, w, wid);
-        const Lvl& L0 = F.L[0];
+        const Fine& Z = F.Z;
         I2 c = lidCell(w, wid);
         if (!w.inWorld(c)) continue;
         uint32_t i = w.cellIndex(c);
         float* f = w.fv(2u * i);
         f[0] = F.X[i];
-        if (L0.rho[i] > 0.0f) f[1] = L0.rx[i];
-        w.fv(2u * i + 1u)[0] = L0.py[i];
+        if ((Z.mask[i] & FM_LIQUID) != 0u) f[1] = -F.R[i];
+        w.fv(2u * i + 1u)[0] = Z.pot[i].y;
         // the last iteration's p: P2 after an odd number of iterations
         const float* P = (two_p && (D.st->cycle & 1u)) ? F.P2 : F.P;
         reinterpret_cast<float4*>(D.cg)[i] = make_float4(F.X[i], F.R[i], P[i], F.Q[i]);
@@ -2432,7 +2399,7 @@ __device__ bool gridBarrier(StepState* st, uint32_t nblocks) {
 __device__ void relaxGroups(const Fast& F, const W& w, int shift, float (*tpx)[RIM * RIM], float (*tpy)[RIM * RIM],
                             int* s_live, int* s_ox, int* s_oy) {
     const Dev& D = F.D;
-    const Lvl& L0 = F.L[0];
+    const Fine& Z = F.Z;
     const uint32_t na = w.activeCount();
     const uint32_t total = na + (shift ? D.edge_tiles : 0u);
     const int q = (int)(threadIdx.x >> 6), lane = (int)(threadIdx.x & 63u);
@@ -2461,13 +2428,9 @@ __device__ void relaxGroups(const Fast& F, const W& w, int shift, float (*tpx)[R
                 float px = 0.0f, py = 0.0f;
                 if (w.inWorld(c)) {
                     uint32_t i = w.cellIndex(c);
-                    if (__ldcg(&L0.rho[i]) > 0.0f) {
-                        px = __ldcg(&F.rimx[i]);
-                        py = __ldcg(&F.rimy[i]);
-                    } else {
-                        px = __ldcg(&L0.px[i]);
-                        py = __ldcg(&L0.py[i]);
-                    }
+                    const float2 v = __ldcg(&Z.rim[i]);
+                    px = v.x;
+                    py = v.y;
                 }
                 tpx[q][k] = px;
                 tpy[q][k] = py;
@@ -2482,17 +2445,18 @@ __device__ void relaxGroups(const Fast& F, const W& w, int shift, float (*tpx)[R
         bool fluid = false;
         if (live && w.inWorld(me)) {
             idx = w.cellIndex(me);
-            fluid = __ldcg(&L0.rho[idx]) > 0.0f;
+            fluid = (Z.mask[idx] & FM_LIQUID) != 0u;
         }
         if (fluid) {
-            rx = __ldcg(&L0.rx[idx]);
-            ry = __ldcg(&L0.ry[idx]);
-            bx = L0.b0[idx];
-            by = L0.b1[idx];
-            bz = L0.b2[idx];
-            bw = L0.b3[idx];
-            diag = L0.diag[idx];
-            pinv = F.pin[idx];
+            rx = -__ldcg(&F.R[idx]);
+            ry = Z.ry[idx];
+            const float4 b4 = Z.b[idx];
+            bx = b4.x;
+            by = b4.y;
+            bz = b4.z;
+            bw = b4.w;
+            diag = diagOf(b4);
+            pinv = (Z.mask[idx] & FM_PIN) != 0u ? PIN : 0.0f;
         }
         const float dx = diag + pinv, dy = fmaxf(diag, 1e-30f);
         const bool solving = fluid && dx > 0.0f;
@@ -2509,8 +2473,7 @@ __device__ void relaxGroups(const Fast& F, const W& w, int shift, float (*tpx)[R
             __syncthreads();
         }
         if (solving) {
-            L0.px[idx] = tpx[q][t];
-            L0.py[idx] = tpy[q][t];
+            Z.pot[idx] = make_float2(tpx[q][t], tpy[q][t]);
         }
         __syncthreads();
     }
@@ -2532,7 +2495,7 @@ __global__ void __launch_bounds__(256, 4) k_fSolve(Fast F, int shifted) {
     const bool f64 = st->f64 != 0u, tol = st->tol_mode != 0u;
     const uint32_t na = w.activeCount();
     const uint32_t lp = F.lp;
-    const Lvl& L0 = F.L[0];
+    const Fine& Z = F.Z;
     if (na == 0u) {
         // nothing to solve: the first iteration counted, as cgUpdate counts it
         if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -2549,7 +2512,10 @@ __global__ void __launch_bounds__(256, 4) k_fSolve(Fast F, int shifted) {
         if (!gridBarrier(st, nb)) return;
         for (uint32_t l = 1; l < lp; l++) {
             const uint32_t n = D.level_w[l] * D.level_h[l];
-            for (uint32_t j = gt; j < n; j += gn) restrictCell(F.D, F, w, l, j);
+            for (uint32_t j = gt; j < n; j += gn) {
+                if (l == 1u) restrictCell<float, true>(F.D, F, w, l, j);
+                else restrictCell<float, false>(F.D, F, w, l, j);
+            }
             if (!gridBarrier(st, nb)) return;
             for (int color = 0; color < 2; color++) {
                 for (uint32_t j = gt; j < n; j += gn) smoothCell(F.D, F, l, color, cycle == 0u, j);
@@ -2558,7 +2524,10 @@ __global__ void __launch_bounds__(256, 4) k_fSolve(Fast F, int shifted) {
         }
         {
             const uint32_t n = D.level_w[lp] * D.level_h[lp];
-            for (uint32_t j = gt; j < n; j += gn) restrictCell(F.D, F, w, lp, j);
+            for (uint32_t j = gt; j < n; j += gn) {
+                if (lp == 1u) restrictCell<float, true>(F.D, F, w, lp, j);
+                else restrictCell<float, false>(F.D, F, w, lp, j);
+            }
             if (!gridBarrier(st, nb)) return;
         }
         if (blockIdx.x == 0) coarseLevels(F.D, F, w, lp, sm_coarse, s_off, false);
@@ -2579,14 +2548,12 @@ __global__ void __launch_bounds__(256, 4) k_fSolve(Fast F, int shifted) {
             I2 c{b.x * BLOCK + (int)(lane & 7u), b.y * BLOCK + (int)(lane >> 3)};
             if (!w.inWorld(c)) continue;
             uint32_t i = w.cellIndex(c);
-            if (L0.rho[i] > 0.0f) {
+            if ((Z.mask[i] & FM_LIQUID) != 0u) {
                 const Lvl& U = F.L[1];
                 V2 e = prolongedFrom(U.rho, U.px, U.py, (int)D.level_w[1], (int)D.level_h[1], c.x, c.y);
-                float px = L0.px[i] + e.x, py = L0.py[i] + e.y;
-                L0.px[i] = px;
-                L0.py[i] = py;
-                F.rimx[i] = px;
-                F.rimy[i] = py;
+                const float2 p = Z.pot[i], v = make_float2(p.x + e.x, p.y + e.y);
+                Z.pot[i] = v;
+                Z.rim[i] = v;
             }
         }
         if (!gridBarrier(st, nb)) return;
@@ -2602,8 +2569,8 @@ __global__ void __launch_bounds__(256, 4) k_fSolve(Fast F, int shifted) {
                 I2 c = tileCell(w, wid);
                 if (w.inWorld(c)) {
                     uint32_t i = w.cellIndex(c);
-                    if (L0.rho[i] > 0.0f) {
-                        float z = L0.px[i];
+                    if ((Z.mask[i] & FM_LIQUID) != 0u) {
+                        float z = Z.pot[i].x;
                         float r = F.R[i], q = F.Q[i];
                         vx = r * z;
                         vy = q * z;
@@ -2662,8 +2629,8 @@ __global__ void __launch_bounds__(256, 4) k_fSolve(Fast F, int shifted) {
                 if (!w.inWorld(c)) continue;
                 uint32_t i = w.cellIndex(c);
                 float p = 0.0f;
-                if (L0.rho[i] > 0.0f) {
-                    float z = L0.px[i];
+                if ((Z.mask[i] & FM_LIQUID) != 0u) {
+                    float z = Z.pot[i].x;
                     p = f64 ? (float)((double)z + beta64 * (double)F.P[i]) : z + beta * F.P[i];
                 }
                 F.P[i] = p;
@@ -2682,14 +2649,15 @@ __global__ void __launch_bounds__(256, 4) k_fSolve(Fast F, int shifted) {
                     uint32_t i = w.cellIndex(c);
                     float q = 0.0f;
                     const float p = __ldcg(&F.P[i]);
-                    if (L0.rho[i] > 0.0f) {
-                        const uint8_t m = F.fmask[i];
-                        const float bb[4] = {L0.b0[i], L0.b1[i], L0.b2[i], L0.b3[i]};
+                    if ((Z.mask[i] & FM_LIQUID) != 0u) {
+                        const uint32_t m = Z.mask[i];
+                        const float4 b4 = Z.b[i];
+                        const float bb[4] = {b4.x, b4.y, b4.z, b4.w};
                         float sum = 0.0f;
 #pragma unroll
                         for (int d = 0; d < 4; d++)
                             if (m & (1u << d)) sum = sum + bb[d] * __ldcg(&F.P[nbr(i, c.x, c.y, D.W, D.H, d)]);
-                        float dg = L0.diag[i] + F.pin[i];
+                        float dg = diagOf(b4) + ((m & FM_PIN) != 0u ? PIN : 0.0f);
                         q = dg * p - sum + 0.0f;
                     }
                     F.Q[i] = q;
@@ -2746,7 +2714,7 @@ __global__ void __launch_bounds__(256, 4) k_fSolve(Fast F, int shifted) {
                     I2 c = tileCell(w, wid);
                     if (w.inWorld(c)) {
                         uint32_t i = w.cellIndex(c);
-                        if (L0.rho[i] > 0.0f) {
+                        if ((Z.mask[i] & FM_LIQUID) != 0u) {
                             float vx = F.X[i], vy = F.R[i], vz = __ldcg(&F.P[i]), vw = __ldcg(&F.Q[i]);
                             float r, x;
                             if (f64) {
@@ -2758,10 +2726,9 @@ __global__ void __launch_bounds__(256, 4) k_fSolve(Fast F, int shifted) {
                             }
                             F.X[i] = x;
                             F.R[i] = r;
-                            L0.px[i] = 0.0f;
-                            L0.rx[i] = -r;
-                            F.rimx[i] = 0.0f;
-                            F.rimy[i] = __ldcg(&L0.py[i]);
+                            const float py = __ldcg(&Z.pot[i]).y;
+                            Z.pot[i].x = 0.0f;
+                            Z.rim[i] = make_float2(0.0f, py);
                             atomicMax(&most[threadIdx.x >> 6], __float_as_uint(fabsf(r)));
                             r2 = (double)r * (double)r;
                         }
@@ -2830,6 +2797,12 @@ void fast_zero_idle(const Batch& Bt, const BatchShape& S, cudaStream_t s) {
     do {                                                                                               \
         if (one) K<true, T, N><<<(grid), (N), (smem), s>>>(Bt, WorldSrc<true>{*one}, ##__VA_ARGS__);    \
         else K<false, T, N><<<(grid), (N), (smem), s>>>(Bt, WorldSrc<false>{}, ##__VA_ARGS__);          \
+    } while (0)
+// The down kernel with N threads a CTA, from level 0 (FINE) or a coarse level.
+#define LAUNCH_DOWN(T, N, FINE, grid, l)                                                      \
+    do {                                                                                      \
+        if (one) k_fDown<true, T, N, FINE><<<(grid), (N), 0, s>>>(Bt, WorldSrc<true>{*one}, l); \
+        else k_fDown<false, T, N, FINE><<<(grid), (N), 0, s>>>(Bt, WorldSrc<false>{}, l);       \
     } while (0)
 // The same for a kernel over levels stored as T.
 #define LAUNCH_T(K, T, grid, block, smem, ...)                                                        \
@@ -2914,10 +2887,14 @@ uint32_t fast_cycle_t(const Batch& Bt0, const BatchShape& S, const World* one, c
     for (uint32_t l = 1; l <= S.lc_max; l++) {
         mark(WIG_SLOT_F_RESTRICT, 0);
         const uint32_t list = L_RES + l - 1u;
-        if (wide(list))
-            LAUNCH_TN(k_fDown, T, 512, list_grid(S, list, S.level_per_sm), 0, l);
-        else
-            LAUNCH_T(k_fDown, T, list_grid(S, list, S.level_per_sm), 256, 0, l);
+        const unsigned grid = list_grid(S, list, S.level_per_sm);
+        if (l == 1u) {
+            if (wide(list)) LAUNCH_DOWN(T, 512, true, grid, l);
+            else LAUNCH_DOWN(T, 256, true, grid, l);
+        } else {
+            if (wide(list)) LAUNCH_DOWN(T, 512, false, grid, l);
+            else LAUNCH_DOWN(T, 256, false, grid, l);
+        }
         mark(WIG_SLOT_F_RESTRICT, 1);
     }
     mark(WIG_SLOT_F_COARSE, 0);
