@@ -651,6 +651,10 @@ struct Prof {
     std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> marks;
 };
 
+// The batch's only world (whose memory stays where it is: a batch of one is
+// never deferred), for the kernels to take as a parameter.
+const wig::World* one_world(const wig_batch* b) { return b->K == 1 ? &b->hw[0] : nullptr; }
+
 // Launch recording with optional per-launch events (Prof).
 struct Rec {
     wig_batch* b;
@@ -675,12 +679,12 @@ struct Rec {
         }
     }
     void run(int pass, uint32_t level = 0, uint32_t cycle = 0) {
-        timed(pass, [&] { wig::launch_pass(ln.Bt, ln.S, b->hw[0].D, pass, level, cycle, s); });
+        timed(pass, [&] { wig::launch_pass(ln.Bt, ln.S, one_world(b), b->hw[0].D, pass, level, cycle, s); });
     }
     // cgStart + cgJoin as a step runs them (profiled as the two passes)
     void labels() {
-        timed(WIG_PASS_CG_START, [&] { wig::launch_labels(ln.Bt, ln.S, s, 0); });
-        timed(WIG_PASS_CG_JOIN, [&] { wig::launch_labels(ln.Bt, ln.S, s, 1); });
+        timed(WIG_PASS_CG_START, [&] { wig::launch_labels(ln.Bt, ln.S, one_world(b), s, 0); });
+        timed(WIG_PASS_CG_JOIN, [&] { wig::launch_labels(ln.Bt, ln.S, one_world(b), s, 1); });
     }
     void norm() {
         timed(WIG_SLOT_NORM, [&] { wig::launch_norm(b->hw[0].D, s); });
@@ -696,7 +700,7 @@ struct Rec {
             cudaEventRecord(a, s);
         }
         wig::sched_lists(ln.Bt, ln.ctl, ln.S, phase, s);
-        launches += 2;
+        launches += ln.Bt.single ? 1u : 2u;
         if (prof) {
             cudaEventRecord(e, s);
             prof->marks.push_back({WIG_SLOT_SCHED, {a, e}});
@@ -929,7 +933,7 @@ int record_step_fast(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags
     ln.Bt.cond_check = 0;
     ln.Bt.cond_drift = 0;
     ln.Bt.mixed = (flags & WIG_STEP_MIXED) ? 1u : 0u;
-    const wig::World* one = b->K == 1 ? &b->hw[0] : nullptr;
+    const wig::World* one = one_world(b);
     if (b->pooled) {
         wig::fast_zero_idle(ln.Bt, ln.S, s);
         R.launches++;
@@ -1440,7 +1444,7 @@ int wig_fluid_dispatch(wig_fluid* h, const wig_params* P, int pass, uint32_t lev
     c.heads = nullptr;
     wig::sched_lists(ln.Bt, c, b->S, 0, s);
     wig::sched_lists(ln.Bt, c, b->S, 1, s);
-    int rc = wig::launch_pass(ln.Bt, b->S, b->hw[0].D, pass, level, cycle, s);
+    int rc = wig::launch_pass(ln.Bt, b->S, one_world(b), b->hw[0].D, pass, level, cycle, s);
     if (rc) return fail(rc, "launch");
     CUDA_TRY(cudaGetLastError());
     ln.last_stream = s;

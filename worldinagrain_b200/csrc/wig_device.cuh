@@ -528,16 +528,38 @@ __device__ __forceinline__ const World& worldOf(const Batch& Bt, uint32_t it, Wo
     return c.w;
 }
 
+// Where a kernel finds its items' world: in a batch of one, the world
+// itself, a kernel parameter (read as constants, with no load at a CTA's
+// start); else the CTA's shared copy of the world-table entry.
+template <bool ONE>
+struct WorldSrc;
+template <>
+struct WorldSrc<true> {
+    World w;
+    __device__ __forceinline__ const World& get(const Batch&, uint32_t, WorldCopy&) const { return w; }
+    __device__ __forceinline__ const World& getG(const Batch&, uint32_t) const { return w; }
+};
+template <>
+struct WorldSrc<false> {
+    __device__ __forceinline__ const World& get(const Batch& Bt, uint32_t it, WorldCopy& c) const {
+        return worldOf(Bt, it, c);
+    }
+    // without the CTA's copy (a warp's own item)
+    __device__ __forceinline__ const World& getG(const Batch& Bt, uint32_t it) const { return Bt.world(it); }
+};
+
 // An item's world D (with its accessors w) and unit j, read from the world
 // table (any thread, any loop).
 #define ITEM_WORLD(Bt, it, D, w, j)              \
     const Dev& D = (Bt).world(it).D;             \
     const W w(D);                                \
     const uint32_t j = (Bt).unit(it)
-// The same from the CTA's copy (every thread of the CTA, each item in turn;
-// the kernel declares `__shared__ WorldCopy wc_;` and calls worldCopyInit).
-#define ITEM_WORLD_C(Bt, it, D, w, j)            \
-    const Dev& D = worldOf((Bt), (it), wc_).D;   \
+// The same from a kernel's WorldSrc `src` (every thread of the CTA, each
+// item in turn; the kernel declares `__shared__ WorldCopy wc_;` and, but for
+// one world, calls worldCopyInit).
+#define ITEM_WORLD_S(Bt, it, D, w, j)            \
+    const World& Wd_##it = src.get((Bt), (it), wc_); \
+    const Dev& D = Wd_##it.D;                    \
     const W w(D);                                \
     const uint32_t j = (Bt).unit(it)
 

@@ -236,26 +236,6 @@ __device__ __forceinline__ I2 tileCell(const W& w, uint32_t wid) {
     return I2{b.x * BLOCK + (int)(threadIdx.x & 7u), b.y * BLOCK + (int)((threadIdx.x >> 3) & 7u)};
 }
 
-// Where a kernel finds its items' world: in a batch of one, the world
-// itself, a kernel parameter (read as constants, with no load at a CTA's
-// start); else the CTA's shared copy of the world-table entry.
-template <bool ONE>
-struct WorldSrc;
-template <>
-struct WorldSrc<true> {
-    World w;
-    __device__ __forceinline__ const World& get(const Batch&, uint32_t, WorldCopy&) const { return w; }
-    __device__ __forceinline__ const World& getG(const Batch&, uint32_t) const { return w; }
-};
-template <>
-struct WorldSrc<false> {
-    __device__ __forceinline__ const World& get(const Batch& Bt, uint32_t it, WorldCopy& c) const {
-        return worldOf(Bt, it, c);
-    }
-    // without the CTA's copy (a warp's own item)
-    __device__ __forceinline__ const World& getG(const Batch& Bt, uint32_t it) const { return Bt.world(it); }
-};
-
 // An item's world: its descriptor D, fast scratch F, accessors w, unit j,
 // from the CTA's copy of the world (every thread of the CTA, each item in
 // turn; the kernel declares `__shared__ WorldCopy wc_;`) or (FAST_ITEM_G)

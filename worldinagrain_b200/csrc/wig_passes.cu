@@ -460,11 +460,12 @@ __device__ void heldPush(const W& w, I2 c, uint32_t h, int32_t out[3]) {
 
 // sync / syncMarks (fluid.wgsl:608-659): a CTA per block of the world
 // (syncMarks: no claims, as a world's bookkeeping-only step takes it).
-__global__ void k_sync(Batch Bt, int sync_claims) {
+template <bool ONE>
+__global__ void k_sync(Batch Bt, const __grid_constant__ WorldSrc<ONE> src, int sync_claims) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
   FOR_ITEMS(Bt, L_WB, it) {
-    ITEM_WORLD_C(Bt, it, D, w, n);
+    ITEM_WORLD_S(Bt, it, D, w, n);
     const bool claims = sync_claims && D.st->book == 0u;
     const I2 b = w.blockAt(n);
     I2 c{b.x * BLOCK + (int)(threadIdx.x & 7u), b.y * BLOCK + (int)(threadIdx.x >> 3)};
@@ -585,11 +586,12 @@ __device__ __forceinline__ void storeParticle(const W& w, uint32_t m, V2 pos, V2
 }
 
 // syncParticles (fluid.wgsl:767-831): a thread per particle of `sorted`.
-__global__ void k_syncParticles(Batch Bt) {
+template <bool ONE>
+__global__ void k_syncParticles(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
   FOR_ITEMS(Bt, L_PS, qi) {
-    ITEM_WORLD_C(Bt, qi, D, w, chunk);
+    ITEM_WORLD_S(Bt, qi, D, w, chunk);
     uint32_t live = min(D.sorted[0], D.cap);
     uint32_t k0 = chunk * blockDim.x;
     if (k0 >= live) continue;  // whole CTA past the particles (uniform)
@@ -658,11 +660,12 @@ __device__ uint32_t seedId(const Dev& D, I2 c, uint32_t j) {
 }
 
 // syncSeed (fluid.wgsl:863-890): a CTA per block of the world.
-__global__ void k_syncSeed(Batch Bt) {
+template <bool ONE>
+__global__ void k_syncSeed(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
   FOR_ITEMS(Bt, L_WB, qi) {
-    ITEM_WORLD_C(Bt, qi, D, w, blk);
+    ITEM_WORLD_S(Bt, qi, D, w, blk);
     if (D.st->book) continue;
     const I2 bq_ = w.blockAt(blk);
     I2 c{bq_.x * BLOCK + (int)(threadIdx.x & 7u), bq_.y * BLOCK + (int)(threadIdx.x >> 3)};
@@ -727,12 +730,13 @@ __device__ __forceinline__ uint32_t marksAround(const W& w, I2 b) {
 // a block, for the second (runs of up to 64 blocks; a longer run reads them
 // again), which writes the states and the lists in block order after the
 // scan of the runs' counts.
-__global__ void __launch_bounds__(1024) k_compact(Batch Bt) {
+template <bool ONE>
+__global__ void __launch_bounds__(1024) k_compact(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     __shared__ uint32_t sa[1024], sr[1024];
     FOR_ITEMS(Bt, L_ONE_ALL, it) {
-        ITEM_WORLD_C(Bt, it, D, w, unused_);
+        ITEM_WORLD_S(Bt, it, D, w, unused_);
         (void)unused_;
         const uint32_t per = (D.B + 1023u) / 1024u;
         const uint32_t lo = min(threadIdx.x * per, D.B), hi = min(lo + per, D.B);
@@ -791,14 +795,15 @@ __global__ void __launch_bounds__(1024) k_compact(Batch Bt) {
 }
 
 // retire (fluid.wgsl:924-951)
-__global__ void k_retire(Batch Bt) {
+template <bool ONE>
+__global__ void k_retire(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_RET, it) {
-        ITEM_WORLD_C(Bt, it, D, w, wid);
+        ITEM_WORLD_S(Bt, it, D, w, wid);
         uint32_t n = D.blocks[w.retiredSlot(wid)];
         // the solve's sums over the world's blocks take its partials for +0
-        if (threadIdx.x == 0) zeroPartials(D, wc_.w.S, n);
+        if (threadIdx.x == 0) zeroPartials(D, Wd_it.S, n);
         const I2 bq_ = w.blockAt(n);
         I2 c{bq_.x * BLOCK + (int)(threadIdx.x & 7u), bq_.y * BLOCK + (int)(threadIdx.x >> 3)};
         if (!w.inWorld(c)) continue;
@@ -821,11 +826,12 @@ __global__ void k_retire(Batch Bt) {
 }
 
 // clear (fluid.wgsl:962-985)
-__global__ void k_clear(Batch Bt) {
+template <bool ONE>
+__global__ void k_clear(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_ACT, it) {
-        ITEM_WORLD_C(Bt, it, D, w, wid);
+        ITEM_WORLD_S(Bt, it, D, w, wid);
         I2 b = w.activeBlock(wid);
         if (threadIdx.x == 0) D.blocks[w.blockIndex(b)] = 0u;
         I2 c = lidCell(w, wid);
@@ -1014,10 +1020,11 @@ __device__ __forceinline__ void gatherWarp(const Dev& D, const W& w, uint32_t k,
     }
     __syncwarp();
 }
-__global__ void __launch_bounds__(256) k_gather(Batch Bt) {
+template <bool ONE>
+__global__ void __launch_bounds__(256) k_gather(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
     __shared__ GatherWin win_[8];
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     GatherWin& win = win_[threadIdx.x >> 5];
     {
         uint32_t* z = &win.u[0][0];
@@ -1025,7 +1032,7 @@ __global__ void __launch_bounds__(256) k_gather(Batch Bt) {
         __syncwarp();
     }
     FOR_ITEMS(Bt, L_PP, qi) {
-        ITEM_WORLD_C(Bt, qi, D, w, chunk);
+        ITEM_WORLD_S(Bt, qi, D, w, chunk);
         gatherWarp(D, w, chunk * blockDim.x + threadIdx.x, win);
     }
 }
@@ -1044,11 +1051,12 @@ __device__ bool wasOpen(const W& w, I2 q) {
 }
 
 // sealJoin (fluid.wgsl:1531-1543)
-__global__ void k_sealJoin(Batch Bt) {
+template <bool ONE>
+__global__ void k_sealJoin(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_ACT, it) {
-        ITEM_WORLD_C(Bt, it, D, w, wid);
+        ITEM_WORLD_S(Bt, it, D, w, wid);
         I2 c = lidCell(w, wid);
         if (!w.inWorld(c) || !mayBeSealed(w, c)) continue;
         for (int d = 0; d < 2; d++) {
@@ -1058,11 +1066,12 @@ __global__ void k_sealJoin(Batch Bt) {
     }
 }
 // sealAnchor (fluid.wgsl:1545-1554)
-__global__ void k_sealAnchor(Batch Bt) {
+template <bool ONE>
+__global__ void k_sealAnchor(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_ACT, it) {
-        ITEM_WORLD_C(Bt, it, D, w, wid);
+        ITEM_WORLD_S(Bt, it, D, w, wid);
         I2 c = lidCell(w, wid);
         if (!w.inWorld(c) || !mayBeSealed(w, c)) continue;
         if (wasOpen(w, beside(c, 0)) || wasOpen(w, beside(c, 1)) || wasOpen(w, beside(c, 2)) || wasOpen(w, beside(c, 3)))
@@ -1109,12 +1118,13 @@ __device__ float columnWeight(const W& w, I2 p, float density) {
 }
 
 // classify (fluid.wgsl:1578-1696), no bodies.
-__global__ void k_classify(Batch Bt) {
+template <bool ONE>
+__global__ void k_classify(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     __shared__ uint32_t blockBits;
     FOR_ITEMS(Bt, L_ACT, it) {
-        ITEM_WORLD_C(Bt, it, D, w, wid);
+        ITEM_WORLD_S(Bt, it, D, w, wid);
         const uint32_t frame = D.st->P.frame;
         const uint32_t mine = 1u << (frame & 1u), fall0 = 4u << (frame & 1u);
         if (threadIdx.x == 0) blockBits = 0u;
@@ -1282,11 +1292,12 @@ __device__ void setFace(const W& w, I2 at, bool isU) {
 }
 
 // setFaces (fluid.wgsl:1982-1994)
-__global__ void k_setFaces(Batch Bt) {
+template <bool ONE>
+__global__ void k_setFaces(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_ACT, it) {
-        ITEM_WORLD_C(Bt, it, D, w, wid);
+        ITEM_WORLD_S(Bt, it, D, w, wid);
         I2 c = lidCell(w, wid);
         if (!w.inWorld(c)) continue;
         int fs[4][3];
@@ -1329,11 +1340,12 @@ __device__ void viscousFace(const W& w, I2 at, bool isU, int color) {
 }
 
 // viscosityRed / viscosityBlack / unpress (fluid.wgsl:3409-3466)
-__global__ void k_viscosity(Batch Bt, int color) {
+template <bool ONE>
+__global__ void k_viscosity(Batch Bt, const __grid_constant__ WorldSrc<ONE> src, int color) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_ACT, it) {
-        ITEM_WORLD_C(Bt, it, D, w, wid);
+        ITEM_WORLD_S(Bt, it, D, w, wid);
         if (color < 2 && D.st->viscous == 0u) continue;  // this world's step has no sweeps
         I2 b = w.activeBlock(wid);
         if ((w.statesOf(I2{b.x - 1, b.y - 1}, I2{b.x + 1, b.y + 1}) & HAS_VISCOUS) == 0u) continue;
@@ -1364,9 +1376,10 @@ __global__ void k_viscosity(Batch Bt, int color) {
 }
 
 // divergence (fluid.wgsl:1996-2025)
-__global__ void k_divergence(Batch Bt) {
+template <bool ONE>
+__global__ void k_divergence(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     // once a world: its residual and iteration words cleared
     if (threadIdx.x == 0) {
         FOR_ITEMS(Bt, L_ONE, ot) {
@@ -1377,7 +1390,7 @@ __global__ void k_divergence(Batch Bt) {
         }
     }
     FOR_ITEMS(Bt, L_ACT, it) {
-        ITEM_WORLD_C(Bt, it, D, w, wid);
+        ITEM_WORLD_S(Bt, it, D, w, wid);
         I2 c = lidCell(w, wid);
         if (!w.inWorld(c)) continue;
         uint32_t i = w.cellIndex(c);
@@ -1394,11 +1407,12 @@ __global__ void k_divergence(Batch Bt) {
 // ================================================================ the solve's start
 
 // cgStart (fluid.wgsl:2665-2674)
-__global__ void k_cgStart(Batch Bt) {
+template <bool ONE>
+__global__ void k_cgStart(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_ACT, it) {
-        ITEM_WORLD_C(Bt, it, D, w, wid);
+        ITEM_WORLD_S(Bt, it, D, w, wid);
         I2 c = lidCell(w, wid);
         if (!w.inWorld(c)) continue;
         uint32_t i = w.cellIndex(c);
@@ -1407,11 +1421,12 @@ __global__ void k_cgStart(Batch Bt) {
     }
 }
 // cgJoin (fluid.wgsl:2677-2689)
-__global__ void k_cgJoin(Batch Bt) {
+template <bool ONE>
+__global__ void k_cgJoin(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_ACT, it) {
-        ITEM_WORLD_C(Bt, it, D, w, wid);
+        ITEM_WORLD_S(Bt, it, D, w, wid);
         I2 c = lidCell(w, wid);
         if (!w.inWorld(c) || w.gridAt(c).z <= 0.0f) continue;
         for (int d = 0; d < 2; d++) {
@@ -1431,12 +1446,13 @@ __global__ void k_cgJoin(Batch Bt) {
 // regions, their roots and every ufFind are those of cgJoin's; only the
 // intermediate links, a lock-free union-find's timing in the reference too,
 // differ (cgFinish clears them all).
-__global__ void k_cgStartLocal(Batch Bt) {
+template <bool ONE>
+__global__ void k_cgStartLocal(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     __shared__ uint32_t lab[64];
     FOR_ITEMS(Bt, L_ACT, it) {
-        ITEM_WORLD_C(Bt, it, D, w, wid);
+        ITEM_WORLD_S(Bt, it, D, w, wid);
         const I2 c = lidCell(w, wid);
         const bool in = w.inWorld(c);
         const uint32_t i = in ? w.cellIndex(c) : 0u;
@@ -1468,11 +1484,12 @@ __global__ void k_cgStartLocal(Batch Bt) {
 }
 // cgJoin's edges between blocks (to the right and below, from the block's
 // last column and row), after k_cgStartLocal has linked each block's own.
-__global__ void k_cgJoinAcross(Batch Bt) {
+template <bool ONE>
+__global__ void k_cgJoinAcross(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_ACT, it) {
-        ITEM_WORLD_C(Bt, it, D, w, wid);
+        ITEM_WORLD_S(Bt, it, D, w, wid);
         const int lx = (int)(threadIdx.x & 7u), ly = (int)(threadIdx.x >> 3);
         if (lx != 7 && ly != 7) continue;
         I2 c = lidCell(w, wid);
@@ -1485,11 +1502,12 @@ __global__ void k_cgJoinAcross(Batch Bt) {
     }
 }
 // cgAnchor (fluid.wgsl:2692-2705)
-__global__ void k_cgAnchor(Batch Bt) {
+template <bool ONE>
+__global__ void k_cgAnchor(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_ACT, it) {
-        ITEM_WORLD_C(Bt, it, D, w, wid);
+        ITEM_WORLD_S(Bt, it, D, w, wid);
         I2 c = lidCell(w, wid);
         if (!w.inWorld(c) || w.gridAt(c).z <= 0.0f) continue;
         for (int d = 0; d < 4; d++) {
@@ -2146,9 +2164,10 @@ __global__ void k_cgFinish(Dev D) {
 // ================================================================ projection, extrapolation
 
 // project / projectFace (fluid.wgsl:2897-2942)
-__global__ void k_project(Batch Bt) {
+template <bool ONE>
+__global__ void k_project(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     // once a world: the most iterations any step took
     if (threadIdx.x == 0) {
         FOR_ITEMS(Bt, L_ONE, ot) {
@@ -2159,7 +2178,7 @@ __global__ void k_project(Batch Bt) {
         }
     }
     FOR_ITEMS(Bt, L_ACT, it) {
-        ITEM_WORLD_C(Bt, it, D, w, wid);
+        ITEM_WORLD_S(Bt, it, D, w, wid);
         I2 c = lidCell(w, wid);
         if (!w.inWorld(c)) continue;
         int fs[4][3];
@@ -2197,11 +2216,12 @@ __global__ void k_project(Batch Bt) {
 }
 
 // extrapolate / extrapolateFurther (fluid.wgsl:3226-3275)
-__global__ void k_extrapolate(Batch Bt, uint32_t layer) {
+template <bool ONE>
+__global__ void k_extrapolate(Batch Bt, const __grid_constant__ WorldSrc<ONE> src, uint32_t layer) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_ACT, it) {
-        ITEM_WORLD_C(Bt, it, D, w, wid);
+        ITEM_WORLD_S(Bt, it, D, w, wid);
         I2 c = lidCell(w, wid);
         if (!w.inWorld(c)) continue;
         int fs[4][3];
@@ -2387,11 +2407,12 @@ __device__ __forceinline__ void advectOne(const Dev& D, const W& w, uint32_t chu
     }
     if ((w.elem(wordType(stt.x)).flags & F_IMPACT) != 0u && impact > IMPACT_SPEED) it[D.cap + k].x = wordWith(stt.x, FL_BURN);
 }
-__global__ void k_advect(Batch Bt) {
+template <bool ONE>
+__global__ void k_advect(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_PP, qi) {
-        ITEM_WORLD_C(Bt, qi, D, w, chunk);
+        ITEM_WORLD_S(Bt, qi, D, w, chunk);
         advectOne(D, w, chunk);
     }
 }
@@ -2419,22 +2440,24 @@ __device__ __forceinline__ void sortCountOne(const Dev& D, const W& w, uint32_t 
     base = __shfl_sync(peers, base, leader);
     it[D.cap + k].w = base + (uint32_t)__popc(peers & ((1u << lane) - 1u));
 }
-__global__ void k_sortCount(Batch Bt) {
+template <bool ONE>
+__global__ void k_sortCount(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_PP, qi) {
-        ITEM_WORLD_C(Bt, qi, D, w, chunk);
+        ITEM_WORLD_S(Bt, qi, D, w, chunk);
         sortCountOne(D, w, chunk);
     }
 }
 
 // scanBlocks (fluid.wgsl:3730-3753)
-__global__ void __launch_bounds__(64) k_scanBlocks(Batch Bt) {
+template <bool ONE>
+__global__ void __launch_bounds__(64) k_scanBlocks(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     __shared__ uint32_t tile[64];
     FOR_ITEMS(Bt, L_ACT, it) {
-        ITEM_WORLD_C(Bt, it, D, w, wid);
+        ITEM_WORLD_S(Bt, it, D, w, wid);
         const uint32_t fall0 = 4u << (D.st->P.frame & 1u);
         I2 c = lidCell(w, wid);
         uint32_t n = 0;
@@ -2495,11 +2518,12 @@ __global__ void __launch_bounds__(256) k_scanTotals(Batch Bt) {
 }
 
 // scanFinish (fluid.wgsl:3783-3790)
-__global__ void k_scanFinish(Batch Bt) {
+template <bool ONE>
+__global__ void k_scanFinish(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_ACT, it) {
-        ITEM_WORLD_C(Bt, it, D, w, wid);
+        ITEM_WORLD_S(Bt, it, D, w, wid);
         I2 c = lidCell(w, wid);
         if (!w.inWorld(c)) continue;
         *w.gwp(w.cellIndex(c), G_START) += D.blocks[w.totalSlot(wid)];
@@ -2522,11 +2546,12 @@ __device__ __forceinline__ void scatterOne(const Dev& D, const W& w, uint32_t ch
         so[2u * D.cap + m] = it[2u * D.cap + k];
     }
 }
-__global__ void k_scatter(Batch Bt) {
+template <bool ONE>
+__global__ void k_scatter(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_PP, qi) {
-        ITEM_WORLD_C(Bt, qi, D, w, chunk);
+        ITEM_WORLD_S(Bt, qi, D, w, chunk);
         scatterOne(D, w, chunk);
     }
 }
@@ -2550,11 +2575,12 @@ __device__ uint32_t airTo(const W& w, I2 c, bool gas) {
     return NONE;
 }
 // rasterClaims (fluid.wgsl:3928-3948), no people.
-__global__ void k_rasterClaims(Batch Bt) {
+template <bool ONE>
+__global__ void k_rasterClaims(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_ACT, it) {
-        ITEM_WORLD_C(Bt, it, D, w, wid);
+        ITEM_WORLD_S(Bt, it, D, w, wid);
         I2 c = lidCell(w, wid);
         if (!w.inWorld(c)) continue;
         uint32_t i = w.cellIndex(c);
@@ -2595,11 +2621,12 @@ __device__ __forceinline__ float exact_value(unsigned long long wsum, float scal
 }
 
 // raster (fluid.wgsl:3983-4119), no people, the air source unbound.
-__global__ void k_raster(Batch Bt) {
+template <bool ONE>
+__global__ void k_raster(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_ACT, qi) {
-        ITEM_WORLD_C(Bt, qi, D, w, wid);
+        ITEM_WORLD_S(Bt, qi, D, w, wid);
         I2 c = lidCell(w, wid);
         if (!w.inWorld(c)) continue;
         uint32_t i = w.cellIndex(c);
@@ -2701,11 +2728,12 @@ __global__ void k_raster(Batch Bt) {
 }
 
 // unpaint (fluid.wgsl:4163-4182)
-__global__ void k_unpaint(Batch Bt) {
+template <bool ONE>
+__global__ void k_unpaint(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
-    worldCopyInit(wc_);
+    if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_ACT, it) {
-        ITEM_WORLD_C(Bt, it, D, w, wid);
+        ITEM_WORLD_S(Bt, it, D, w, wid);
         I2 c = lidCell(w, wid);
         if (!w.inWorld(c)) continue;
         uint32_t i = w.cellIndex(c);
@@ -2886,8 +2914,16 @@ unsigned list_grid(const BatchShape& S, uint32_t list, unsigned per_sm) {
     return n < g ? (n ? n : 1u) : g;
 }
 
-int launch_pass(const Batch& Bt, const BatchShape& S, const Dev& D0, int pass, uint32_t level, uint32_t cycle,
-                cudaStream_t s) {
+// Launches kernel K's instance for the batch: the single-world one with the
+// world as a parameter when `one` is given, else the table one.
+#define RUN(K, grid, block, ...)                                                                  \
+    do {                                                                                          \
+        if (one) K<true><<<(grid), (block), 0, s>>>(Bt, WorldSrc<true>{*one}, ##__VA_ARGS__);       \
+        else K<false><<<(grid), (block), 0, s>>>(Bt, WorldSrc<false>{}, ##__VA_ARGS__);             \
+    } while (0)
+
+int launch_pass(const Batch& Bt, const BatchShape& S, const World* one, const Dev& D0, int pass, uint32_t level,
+                uint32_t cycle, cudaStream_t s) {
     // the passes shared by every form: over the batch's work lists
     const unsigned A = list_grid(S, L_ACT, 32), WB = list_grid(S, L_WB, 32);
     const unsigned PS = list_grid(S, L_PS, 8), PP = list_grid(S, L_PP, 8);
@@ -2899,25 +2935,25 @@ int launch_pass(const Batch& Bt, const BatchShape& S, const Dev& D0, int pass, u
     };
     const Dev& D = D0;
     switch (pass) {
-    case WIG_PASS_SYNC: k_sync<<<WB, 64, 0, s>>>(Bt, 1); break;
-    case WIG_PASS_SYNC_MARKS: k_sync<<<WB, 64, 0, s>>>(Bt, 0); break;
-    case WIG_PASS_SYNC_PARTICLES: k_syncParticles<<<PS, 256, 0, s>>>(Bt); break;
-    case WIG_PASS_SYNC_SEED: k_syncSeed<<<WB, 64, 0, s>>>(Bt); break;
-    case WIG_PASS_COMPACT: k_compact<<<ALL, 1024, 0, s>>>(Bt); break;
-    case WIG_PASS_RETIRE: k_retire<<<RET, 64, 0, s>>>(Bt); break;
-    case WIG_PASS_CLEAR: k_clear<<<A, 64, 0, s>>>(Bt); break;
-    case WIG_PASS_GATHER: k_gather<<<PP, 256, 0, s>>>(Bt); break;
-    case WIG_PASS_SEAL_JOIN: k_sealJoin<<<A, 64, 0, s>>>(Bt); break;
-    case WIG_PASS_SEAL_ANCHOR: k_sealAnchor<<<A, 64, 0, s>>>(Bt); break;
-    case WIG_PASS_CLASSIFY: k_classify<<<A, 64, 0, s>>>(Bt); break;
-    case WIG_PASS_SET_FACES: k_setFaces<<<A, 64, 0, s>>>(Bt); break;
-    case WIG_PASS_VISCOSITY_RED: k_viscosity<<<A, 64, 0, s>>>(Bt, 0); break;
-    case WIG_PASS_VISCOSITY_BLACK: k_viscosity<<<A, 64, 0, s>>>(Bt, 1); break;
-    case WIG_PASS_UNPRESS: k_viscosity<<<A, 64, 0, s>>>(Bt, 2); break;
-    case WIG_PASS_DIVERGENCE: k_divergence<<<A, 64, 0, s>>>(Bt); break;
-    case WIG_PASS_CG_START: k_cgStart<<<A, 64, 0, s>>>(Bt); break;
-    case WIG_PASS_CG_JOIN: k_cgJoin<<<A, 64, 0, s>>>(Bt); break;
-    case WIG_PASS_CG_ANCHOR: k_cgAnchor<<<A, 64, 0, s>>>(Bt); break;
+    case WIG_PASS_SYNC: RUN(k_sync, WB, 64, 1); break;
+    case WIG_PASS_SYNC_MARKS: RUN(k_sync, WB, 64, 0); break;
+    case WIG_PASS_SYNC_PARTICLES: RUN(k_syncParticles, PS, 256); break;
+    case WIG_PASS_SYNC_SEED: RUN(k_syncSeed, WB, 64); break;
+    case WIG_PASS_COMPACT: RUN(k_compact, ALL, 1024); break;
+    case WIG_PASS_RETIRE: RUN(k_retire, RET, 64); break;
+    case WIG_PASS_CLEAR: RUN(k_clear, A, 64); break;
+    case WIG_PASS_GATHER: RUN(k_gather, PP, 256); break;
+    case WIG_PASS_SEAL_JOIN: RUN(k_sealJoin, A, 64); break;
+    case WIG_PASS_SEAL_ANCHOR: RUN(k_sealAnchor, A, 64); break;
+    case WIG_PASS_CLASSIFY: RUN(k_classify, A, 64); break;
+    case WIG_PASS_SET_FACES: RUN(k_setFaces, A, 64); break;
+    case WIG_PASS_VISCOSITY_RED: RUN(k_viscosity, A, 64, 0); break;
+    case WIG_PASS_VISCOSITY_BLACK: RUN(k_viscosity, A, 64, 1); break;
+    case WIG_PASS_UNPRESS: RUN(k_viscosity, A, 64, 2); break;
+    case WIG_PASS_DIVERGENCE: RUN(k_divergence, A, 64); break;
+    case WIG_PASS_CG_START: RUN(k_cgStart, A, 64); break;
+    case WIG_PASS_CG_JOIN: RUN(k_cgJoin, A, 64); break;
+    case WIG_PASS_CG_ANCHOR: RUN(k_cgAnchor, A, 64); break;
     case WIG_PASS_CG_RESIDUAL: k_cgResidual<<<G, 64, 0, s>>>(D); break;
     case WIG_PASS_CG_PREPARE: k_cgPrepare<<<G, 64, 0, s>>>(D); break;
     case WIG_PASS_RELAX_RIMS: k_relaxRims<<<G, 64, 0, s>>>(D, cycle); break;
@@ -2936,18 +2972,18 @@ int launch_pass(const Batch& Bt, const BatchShape& S, const Dev& D0, int pass, u
     case WIG_PASS_CG_ALPHA: k_cgAlpha<<<1, 256, 0, s>>>(D, cycle); break;
     case WIG_PASS_CG_UPDATE: k_cgUpdate<<<G, 64, 0, s>>>(D, cycle); break;
     case WIG_PASS_CG_FINISH: k_cgFinish<<<G, 64, 0, s>>>(D); break;
-    case WIG_PASS_PROJECT: k_project<<<A, 64, 0, s>>>(Bt); break;
-    case WIG_PASS_EXTRAPOLATE: k_extrapolate<<<A, 64, 0, s>>>(Bt, 1u); break;
-    case WIG_PASS_EXTRAPOLATE_FURTHER: k_extrapolate<<<A, 64, 0, s>>>(Bt, 2u); break;
-    case WIG_PASS_ADVECT: k_advect<<<PP, 256, 0, s>>>(Bt); break;
-    case WIG_PASS_SORT_COUNT: k_sortCount<<<PP, 256, 0, s>>>(Bt); break;
-    case WIG_PASS_SCAN_BLOCKS: k_scanBlocks<<<A, 64, 0, s>>>(Bt); break;
+    case WIG_PASS_PROJECT: RUN(k_project, A, 64); break;
+    case WIG_PASS_EXTRAPOLATE: RUN(k_extrapolate, A, 64, 1u); break;
+    case WIG_PASS_EXTRAPOLATE_FURTHER: RUN(k_extrapolate, A, 64, 2u); break;
+    case WIG_PASS_ADVECT: RUN(k_advect, PP, 256); break;
+    case WIG_PASS_SORT_COUNT: RUN(k_sortCount, PP, 256); break;
+    case WIG_PASS_SCAN_BLOCKS: RUN(k_scanBlocks, A, 64); break;
     case WIG_PASS_SCAN_TOTALS: k_scanTotals<<<ONE, 256, 0, s>>>(Bt); break;
-    case WIG_PASS_SCAN_FINISH: k_scanFinish<<<A, 64, 0, s>>>(Bt); break;
-    case WIG_PASS_SCATTER: k_scatter<<<PP, 256, 0, s>>>(Bt); break;
-    case WIG_PASS_RASTER_CLAIMS: k_rasterClaims<<<A, 64, 0, s>>>(Bt); break;
-    case WIG_PASS_RASTER: k_raster<<<A, 64, 0, s>>>(Bt); break;
-    case WIG_PASS_UNPAINT: k_unpaint<<<A, 64, 0, s>>>(Bt); break;
+    case WIG_PASS_SCAN_FINISH: RUN(k_scanFinish, A, 64); break;
+    case WIG_PASS_SCATTER: RUN(k_scatter, PP, 256); break;
+    case WIG_PASS_RASTER_CLAIMS: RUN(k_rasterClaims, A, 64); break;
+    case WIG_PASS_RASTER: RUN(k_raster, A, 64); break;
+    case WIG_PASS_UNPAINT: RUN(k_unpaint, A, 64); break;
     default:
         // the bodies' passes: world 0 with its bodies bound (no-ops without)
         if (pass < WIG_PASS_BODY_START || pass > WIG_PASS_BODY_PUSH) return WIG_E_ARG;
@@ -2969,10 +3005,10 @@ int launch_pass(const Batch& Bt, const BatchShape& S, const Dev& D0, int pass, u
     return WIG_OK;
 }
 
-void launch_labels(const Batch& Bt, const BatchShape& S, cudaStream_t s, int part) {
+void launch_labels(const Batch& Bt, const BatchShape& S, const World* one, cudaStream_t s, int part) {
     const unsigned A = list_grid(S, L_ACT, 32);
-    if (part == 0) k_cgStartLocal<<<A, 64, 0, s>>>(Bt);
-    else k_cgJoinAcross<<<A, 64, 0, s>>>(Bt);
+    if (part == 0) RUN(k_cgStartLocal, A, 64);
+    else RUN(k_cgJoinAcross, A, 64);
 }
 
 void launch_norm(const Dev& D, cudaStream_t s) { k_norm<<<1, 256, 0, s>>>(D); }

@@ -27,13 +27,16 @@ constexpr uint32_t CYCLE_LOOP = 0xffffffffu;
 
 // One reference pass (enum wig_pass) at Level (level, cycle), on stream s:
 // over the batch's work lists, or (the plain form's solve passes) over
-// world 0, whose descriptor D0 is.
-int launch_pass(const Batch& Bt, const BatchShape& S, const Dev& D0, int pass, uint32_t level, uint32_t cycle,
-                cudaStream_t s);
+// world 0, whose descriptor D0 is.  `one`: the batch's only world (host
+// copy), passed to the kernels as a parameter, so that no CTA starts by
+// loading the world's entry (33 launches of a step of a small world each
+// spent about 1 us of their 4-5 on it); null for a batch of several.
+int launch_pass(const Batch& Bt, const BatchShape& S, const World* one, const Dev& D0, int pass, uint32_t level,
+                uint32_t cycle, cudaStream_t s);
 // A step's cgStart + cgJoin: part 0 cgStart with each block's own
 // labelling (k_cgStartLocal), part 1 the joins between blocks; the same
 // regions and roots as the two passes.
-void launch_labels(const Batch& Bt, const BatchShape& S, cudaStream_t s, int part);
+void launch_labels(const Batch& Bt, const BatchShape& S, const World* one, cudaStream_t s, int part);
 // The plain form's ||b||^2 of world 0 after cgResidual (the tolerance form).
 void launch_norm(const Dev& D, cudaStream_t s);
 // The end of an iteration of the plain form's loop on world 0, after

@@ -61,6 +61,54 @@ __constant__ uint32_t kPhaseA[] = {L_WB, L_PS, L_ONE_ALL, L_ONE,
 __constant__ uint32_t kPhaseB[] = {L_ACT, L_RET, L_ACT4, L_RELAX, L_PP};
 constexpr uint32_t N_PHASE_A = 20, N_PHASE_B = 5;
 
+// A world's StepState from its head, at the step's start.
+__device__ void startState(StepState* st, const StepHead& h) {
+    st->P = h.P;
+    st->tol_mode = h.tol_mode;
+    st->f64 = h.f64;
+    st->book = h.book;
+    st->viscous = h.viscous;
+    st->shift_first = h.shift_first;
+    st->tol = h.tol;
+    st->err = 0u;
+    st->cycles_run = 0u;
+    st->rel = 1.0;
+    st->bnorm2 = 0.0;
+    st->rz = 0.0; st->pq = 0.0; st->alpha = 0.0; st->beta = 0.0;
+    st->cycle = 0u;
+    st->cont = 0u;
+    for (int f = 0; f < 6; f++) st->fdone[f] = 0u;
+    st->check = 0u;
+    st->drift = 0u;
+    st->rel_true = 0.0;
+    st->rz32 = 0.0f; st->pq32 = 0.0f; st->alpha32 = 0.0f; st->beta32 = 0.0f;
+    st->bar_count = 0u;
+    st->bar_gen = 0u;
+}
+
+// This step's table entry of a pooled world (the lists' units read the
+// entries, not the table).
+__device__ void copyEntry(const SchedCtl& c, uint32_t s, uint32_t k) {
+    const uint4* src = reinterpret_cast<const uint4*>(&c.entries[s]);
+    uint4* dst = reinterpret_cast<uint4*>(&c.table[k]);
+    for (uint32_t i = threadIdx.x; i < sizeof(World) / 16u; i += blockDim.x) dst[i] = src[i];
+}
+
+// A batch of one: item g of any list is unit g of world 0, so only the
+// lists' lengths are written, a thread a list, in one launch where the
+// scan and the fill take two.
+__global__ void __launch_bounds__(64) k_schedOne(Batch Bt, SchedCtl c, int phase) {
+    const uint32_t nl = phase == 0 ? N_PHASE_A : N_PHASE_B;
+    if (threadIdx.x < nl) {
+        const uint32_t L = phase == 0 ? kPhaseA[threadIdx.x] : kPhaseB[threadIdx.x];
+        c.count[L] = unitsOf(Bt, c, 0u, L);
+    }
+    if (phase != 0) return;
+    if (c.entries) copyEntry(c, 0u, 0u);
+    // (the last thread, which has no list)
+    if (c.heads && threadIdx.x == 63u) startState(Bt.worlds[0].D.st, c.heads[0]);
+}
+
 // One CTA of 32 warps: warp w scans list w of the phase over the subset
 // (32 entries at a time), leaving each entry's first item in off and the
 // list's total in count.
@@ -99,38 +147,8 @@ __global__ void __launch_bounds__(256) k_schedFill(Batch Bt, SchedCtl c, int pha
     for (uint32_t g = blockIdx.x; g < n * 4u; g += gridDim.x) {
         const uint32_t s = g >> 2, q = g & 3u;
         const uint32_t k = c.sub[s];
-        if (phase == 0 && c.heads && q == 0u && threadIdx.x == 0) {
-            StepState* st = Bt.worlds[k].D.st;
-            const StepHead& h = c.heads[s];
-            st->P = h.P;
-            st->tol_mode = h.tol_mode;
-            st->f64 = h.f64;
-            st->book = h.book;
-            st->viscous = h.viscous;
-            st->shift_first = h.shift_first;
-            st->tol = h.tol;
-            st->err = 0u;
-            st->cycles_run = 0u;
-            st->rel = 1.0;
-            st->bnorm2 = 0.0;
-            st->rz = 0.0; st->pq = 0.0; st->alpha = 0.0; st->beta = 0.0;
-            st->cycle = 0u;
-            st->cont = 0u;
-            for (int f = 0; f < 6; f++) st->fdone[f] = 0u;
-            st->check = 0u;
-            st->drift = 0u;
-            st->rel_true = 0.0;
-            st->rz32 = 0.0f; st->pq32 = 0.0f; st->alpha32 = 0.0f; st->beta32 = 0.0f;
-            st->bar_count = 0u;
-            st->bar_gen = 0u;
-        }
-        if (phase == 0 && c.entries && q == 0u) {
-            // the world's table entry for this step (the scan above read it
-            // from the entries)
-            const uint4* src = reinterpret_cast<const uint4*>(&c.entries[s]);
-            uint4* dst = reinterpret_cast<uint4*>(&c.table[k]);
-            for (uint32_t i = threadIdx.x; i < sizeof(World) / 16u; i += blockDim.x) dst[i] = src[i];
-        }
+        if (phase == 0 && c.heads && q == 0u && threadIdx.x == 0) startState(Bt.worlds[k].D.st, c.heads[s]);
+        if (phase == 0 && c.entries && q == 0u) copyEntry(c, s, k);
         for (uint32_t li = 0; li < nl; li++) {
             const uint32_t L = phase == 0 ? kPhaseA[li] : kPhaseB[li];
             const uint32_t* off = c.off + (size_t)L * (c.max_worlds + 1u);
@@ -145,6 +163,10 @@ __global__ void __launch_bounds__(256) k_schedFill(Batch Bt, SchedCtl c, int pha
 }  // namespace
 
 void sched_lists(const Batch& Bt, const SchedCtl& c, const BatchShape& S, int phase, cudaStream_t s) {
+    if (Bt.single) {
+        k_schedOne<<<1, 64, 0, s>>>(Bt, c, phase);
+        return;
+    }
     k_schedScan<<<1, 1024, 0, s>>>(Bt, c, phase);
     unsigned g = S.worlds * 4u, cap = 148u * 8u;
     k_schedFill<<<g < cap ? g : cap, 256, 0, s>>>(Bt, c, phase);
