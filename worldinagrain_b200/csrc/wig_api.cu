@@ -149,7 +149,7 @@ struct wig_batch {
     std::vector<int> stepped_lane;
     wig::BatchShape S{};
     uint32_t lbits = 31;
-    uint32_t solve_grid = 0;          // the persistent solve's CTAs (a batch of one world)
+    wig::SolveShape solve{};          // the solve in one launch (a batch of one world)
     Lane lane[WIG_BATCH_LANES];
     size_t up_bytes = 0;              // one upload slot
     size_t entries_at = 0;            // offset of the staged world entries in a slot (pooled batches)
@@ -267,6 +267,7 @@ size_t scratch_bytes(const wig::Dev& D) {
         bytes += align256(5u * (size_t)D.level_w[l] * D.level_h[l] * 2u);  // the binary16 operator
     }
     bytes += align256(2u * (size_t)D.B * 4u) + 3u * align256(2u * (size_t)D.B * 8u);
+    bytes += align256((size_t)D.B * 4u) + align256((size_t)D.B * 8u) + align256(512u * 8u);
     return bytes;
 }
 
@@ -298,12 +299,12 @@ void scratch_take(wig::World& Wd, char* p, uint32_t coarse_cells) {
     F.X = fl(C); F.R = fl(C); F.P = fl(C); F.Q = fl(C); F.P2 = fl(C);
     F.part32 = fl(2u * (size_t)D.B);
     F.part64 = reinterpret_cast<double*>(take(2u * (size_t)D.B * 8u));
+    F.pq32 = fl(D.B);
+    F.pq64 = reinterpret_cast<double*>(take((size_t)D.B * 8u));
+    F.col64 = reinterpret_cast<double*>(take(512u * 8u));
     D.part64 = reinterpret_cast<double*>(take(2u * (size_t)D.B * 8u));
     D.norm64 = reinterpret_cast<double*>(take(2u * (size_t)D.B * 8u));
     F.lc = wig::coarse_level(D, coarse_cells);
-    F.lp = D.levels;
-    for (uint32_t l = 1; l <= D.levels; l++)
-        if ((size_t)D.level_w[l] * D.level_h[l] <= wig::PERSISTENT_CTA_CELLS) { F.lp = l; break; }
 }
 
 uint64_t world_buffers_bytes(const wig_world_layout& L) {
@@ -488,8 +489,8 @@ int make_batch(const wig_world_desc* descs, uint32_t n, const wig_elem* elems, u
     if (items_total > 0xffffffffull) return bail(WIG_E_ARG, "work lists too long");
     level_shape(b);
     for (uint32_t k = 0; k < n; k++) b->blocks_all += b->hw[k].D.B;
-    if (S.coarse_smem > 220u * 1024u) return bail(WIG_E_ARG, "coarse levels too large for one CTA");
-    if (wig::fast_prepare_attributes(S.coarse_smem) != cudaSuccess) return bail(WIG_E_CUDA, "cudaFuncSetAttribute");
+    if (S.coarse_smem > wig::SOLVE_SMEM_MOST) return bail(WIG_E_ARG, "coarse levels too large for one CTA");
+    if (wig::fast_prepare_attributes() != cudaSuccess) return bail(WIG_E_CUDA, "cudaFuncSetAttribute");
 
     // device memory: elements, step states, reports, world table, scratch
     if (cudaMalloc(&b->d_elems, sizeof(wig_elem) * n_elems) != cudaSuccess) return bail(WIG_E_OOM, "cudaMalloc elems");
@@ -546,10 +547,10 @@ int make_batch(const wig_world_desc* descs, uint32_t n, const wig_elem* elems, u
     if (cudaMemcpy(b->d_worlds, b->hw.data(), sizeof(wig::World) * n, cudaMemcpyHostToDevice) != cudaSuccess)
         return bail(WIG_E_CUDA, "cudaMemcpy world table");
     if (n == 1) {
-        wig::Fast F0;
-        static_cast<wig::FastW&>(F0) = b->hw[0].S;
-        F0.D = b->hw[0].D;
-        if (wig::fast_solve_grid(F0, &b->solve_grid) != cudaSuccess) return bail(WIG_E_CUDA, "occupancy of the persistent solve");
+        // (a deferred world's memory moves with each admission: no kernel can
+        // take it as a parameter)
+        if (how == Alloc::Deferred) return bail(WIG_E_CUDA, "a deferred batch holds more than one world");
+        if (wig::fast_solve_shape(b->hw[0].D, &b->solve) != cudaSuccess) return bail(WIG_E_CUDA, "occupancy of the one-launch solve");
     }
 
     // lanes
@@ -940,14 +941,15 @@ int record_step_fast(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags
     }
     wig::fast_setup(ln.Bt, ln.S, one, s, prof ? &mk : nullptr);
     R.launches++;
-    if (flags & WIG_STEP_PERSISTENT) {
-        wig::Fast F0;
-        static_cast<wig::FastW&>(F0) = b->hw[0].S;
-        F0.D = b->hw[0].D;
-        F0.max_cycles = max_cycles;
-        F0.solve_grid = b->solve_grid;
-        if (F0.solve_grid == 0u) return fail(WIG_E_STATE, "no grid for the persistent solve");
-        CUDA_TRY(wig::fast_solve(F0, shifted, s, prof ? &mk : nullptr));
+    // a single world's iterations are one launch: on a cooperative grid for
+    // WIG_STEP_PERSISTENT, else on the group that suits its size; with the
+    // knob that puts its coarse levels on a cluster, and when profiled,
+    // they are the loop's launches
+    const bool by_size = one && ln.S.cluster == 0u && (one->D.B <= wig::CLUSTER_BLOCKS || one->D.B > wig::GRID_BLOCKS);
+    const bool one_launch = (flags & WIG_STEP_PERSISTENT) || by_size;
+    const bool solve = one_launch && (capture || (flags & WIG_STEP_PERSISTENT));
+    if (solve) {
+        CUDA_TRY(wig::fast_solve(ln.Bt, *one, b->solve, (flags & WIG_STEP_PERSISTENT) != 0u, s, prof ? &mk : nullptr));
         R.launches++;
         *body = 0;
     } else if (capture) {
@@ -961,6 +963,7 @@ int record_step_fast(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags
         CUDA_TRY(nest.err);
     } else {
         uint32_t* cont = reinterpret_cast<uint32_t*>(ln.h_rsub);  // a word of pinned scratch
+        const uint32_t before = R.launches;
         for (uint32_t c = 0; c < max_cycles; c++) {
             R.launches += wig::fast_cycle(ln.Bt, ln.S, one, s, prof ? &mk : nullptr);
             CUDA_TRY(cudaMemcpyAsync(cont, ln.d_loop, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
@@ -968,8 +971,10 @@ int record_step_fast(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags
             if (!*cont) break;
         }
         *body = 0;
+        // the kernels reported are a step's, profiled or not
+        if (one_launch) R.launches = before + 1u;
     }
-    wig::fast_finish(ln.Bt, ln.S, one, (flags & WIG_STEP_PERSISTENT) == 0u, s, prof ? &mk : nullptr);
+    wig::fast_finish(ln.Bt, ln.S, one, s, prof ? &mk : nullptr);
     R.launches++;
     record_post(R);
     *outside = R.launches;
@@ -1645,7 +1650,7 @@ int wig_batch_set_launch(wig_batch* b, uint32_t knob, uint32_t value) {
         const uint32_t was = S.coarse_cells;
         S.coarse_cells = value;
         level_shape(b);
-        if (S.coarse_smem > 220u * 1024u || wig::fast_prepare_attributes(S.coarse_smem) != cudaSuccess) {
+        if (S.coarse_smem > wig::SOLVE_SMEM_MOST || wig::fast_prepare_attributes() != cudaSuccess) {
             S.coarse_cells = was;
             level_shape(b);
             return fail(WIG_E_ARG, "coarse levels too large for the coarse kernel");

@@ -58,9 +58,9 @@ constexpr uint32_t COUNT_ACTIVE = 0, COUNT_RETIRED = 1, COUNT_VISCOUS = 2, COUNT
 // kernel records WIG_ERR_LOOP in the step's error word and gives up.
 constexpr uint32_t LOOP_LIMIT = 1u << 22;
 constexpr uint32_t ERR_LOOP = 1u, ERR_CAPACITY = 2u, ERR_BARRIER = 4u;
-// A grid barrier's wait: at most this many polls of ~64 ns (about half a
-// second), past which the kernel records ERR_BARRIER and returns.
-constexpr uint32_t BARRIER_SPIN_LIMIT = 1u << 23;
+// A grid barrier's wait: at most this many polls of about 0.7 us (about
+// 0.7 s), past which the kernel records ERR_BARRIER and returns.
+constexpr uint32_t BARRIER_SPIN_LIMIT = 1u << 20;
 // The bounds in force on a device (the two above unless
 // wig_fluid_set_wait_limits lowered them, which the failure-path tests do to
 // see the error come back); read by the loops at run time.
@@ -112,9 +112,8 @@ struct StepState {
     uint32_t drift;     // the mixed form: the true residual is to be put in for the recursive one
     double rel_true;    // the mixed form: the last check's ||b + A x||2/||b||2
     float rz32, pq32, alpha32, beta32;
-    // the persistent solve's grid barrier: arrivals and generation
-    uint32_t bar_count;
-    uint32_t bar_gen;
+    uint32_t bar_count; // the one-launch solve's grid barrier: arrivals
+    uint32_t pad2_;
 };
 static_assert(sizeof(StepHead) == offsetof(StepState, err), "StepHead is StepState's prefix");
 
@@ -429,8 +428,10 @@ struct FastW {
     float* P2;                 // level 0: p of the fast form's odd iterations (p of the even ones in P)
     float* part32;             // partial sums: component c of block b at c * B + b
     double* part64;            // the same in FP64
+    float* pq32;               // cgApply's partial sums, of block b at b
+    double* pq64;
+    double* col64;             // 512 column sums of a group's block sums
     uint32_t lc;               // first level the one-CTA coarse kernel solves
-    uint32_t lp;               // first level CTA 0 of the persistent solve holds
 };
 
 // An entry of a batch's world table (device memory).
@@ -447,6 +448,8 @@ __device__ __forceinline__ void zeroPartials(const Dev& D, const FastW& F, uint3
         F.part64[c * D.B + n] = 0.0;
         D.norm64[c * D.B + n] = 0.0;
     }
+    F.pq32[n] = 0.0f;
+    F.pq64[n] = 0.0;
 }
 
 // Work lists.  A kernel's CTAs take the items of one list in turn (grid

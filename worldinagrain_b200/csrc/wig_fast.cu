@@ -32,8 +32,6 @@ namespace wig {
 namespace {
 
 __device__ __forceinline__ uint32_t vld(const uint32_t* p) { return *(const volatile uint32_t*)p; }
-__device__ __forceinline__ double vldd(const double* p) { return *(const volatile double*)p; }
-__device__ __forceinline__ float vldf(const float* p) { return *(const volatile float*)p; }
 
 __device__ __forceinline__ I2 lidCell(const W& w, uint32_t wid) {
     I2 b = w.activeBlock(wid);
@@ -76,28 +74,6 @@ __device__ __forceinline__ T tree64x4(T* s, T v) {
     return r;
 }
 
-// The same trees of 64 in two halves, one barrier between them: tilePut,
-// in the upper warp of each tile, leaves its 32 values in s (128 entries);
-// after a barrier, tileSum, in the lower warp, adds them (the tree's first
-// step, lane + 32) and finishes the tree by shuffles (lane + h, h = 16 ..
-// 1): the same additions in the same order.  The tile's sum is in its
-// thread 0.  A kernel alternates two buffers between items, so one item's
-// sums and the next item's puts never share one.
-template <class T>
-__device__ __forceinline__ void tilePut(T* s, T v) {
-    const uint32_t lane = threadIdx.x & 63u;
-    if (lane >= 32u) s[((threadIdx.x >> 6) << 5) + (lane - 32u)] = v;
-}
-template <class T>
-__device__ __forceinline__ T tileSum(const T* s, T v) {
-    if ((threadIdx.x & 32u) == 0u) {  // a whole warp: the tile's lower
-        v = v + s[((threadIdx.x >> 6) << 5) + (threadIdx.x & 31u)];
-#pragma unroll
-        for (int h = 16; h > 0; h >>= 1) v = v + __shfl_down_sync(0xffffffffu, v, h);
-    }
-    return v;
-}
-
 // sumBlocks (fluid.wgsl:2645-2661) by a 256-thread CTA, component comp of 2
 // of the active blocks' partials: thread li adds the partials of blocks li,
 // li + 256, ... in that order (loaded ahead in coalesced batches of 16, the
@@ -137,59 +113,6 @@ __device__ T sumBlocks256(const W& w, const T* part, int comp, T* s) {
     T r = s[0];
     __syncthreads();
     return r;
-}
-
-// sumBlocks of both components of the partials in one pass (each component
-// in sumBlocks256's order).
-template <class T>
-__device__ void sumBlocks256x2(const W& w, const T* part, T* s0, T* s1, T* out0, T* out1) {
-    const uint32_t B = w.D.B;
-    const uint32_t* state = w.D.blocks + B;
-    const uint32_t li = threadIdx.x;
-    T a0 = T(0), a1 = T(0);
-    for (uint32_t k0 = li; k0 < B; k0 += 256u * 16u) {
-        T v0[16], v1[16];
-        uint32_t st[16];
-#pragma unroll
-        for (int u = 0; u < 16; u++) {
-            const uint32_t k = k0 + 256u * (uint32_t)u;
-            st[u] = k < B ? __ldcg(&state[k]) : 0u;
-            v0[u] = k < B ? __ldcg(&part[k]) : T(0);
-            v1[u] = k < B ? __ldcg(&part[B + k]) : T(0);
-        }
-#pragma unroll
-        for (int u = 0; u < 16; u++)
-            if ((st[u] & ACTIVE) != 0u) {
-                a0 = a0 + v0[u];
-                a1 = a1 + v1[u];
-            }
-    }
-    s0[li] = a0;
-    s1[li] = a1;
-    __syncthreads();
-    for (int h = 128; h > 32; h >>= 1) {
-        if ((int)li < h) {
-            s0[li] = s0[li] + s0[li + h];
-            s1[li] = s1[li] + s1[li + h];
-        }
-        __syncthreads();
-    }
-    if (li < 32u) {
-        T v0 = s0[li] + s0[li + 32u], v1 = s1[li] + s1[li + 32u];
-#pragma unroll
-        for (int h = 16; h > 0; h >>= 1) {
-            v0 = v0 + __shfl_down_sync(0xffffffffu, v0, h);
-            v1 = v1 + __shfl_down_sync(0xffffffffu, v1, h);
-        }
-        if (li == 0u) {
-            s0[0] = v0;
-            s1[0] = v1;
-        }
-    }
-    __syncthreads();
-    *out0 = s0[0];
-    *out1 = s1[0];
-    __syncthreads();
 }
 
 // Whether this CTA counted the last of `total` tiles: a threadfence
@@ -512,75 +435,63 @@ __device__ __forceinline__ float mixed1(float a, float b) {
 // `second`: the iteration's relaxation after the V-cycle, on the other
 // tiling from the first (each world's first tiling is its step's).
 constexpr int RXS = RIM + 2;
-template <bool ONE, class T>
-__global__ void __launch_bounds__(128) k_fRelax(Batch Bt, const __grid_constant__ WorldSrc<ONE> src, int second) {
-    __shared__ float2 tp[4][RIM * RXS];
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    float2* sp = tp[warp];
-    const uint32_t n = Bt.n(L_RELAX);
-    const uint32_t warps = gridDim.x * 4u, per = (n + warps - 1u) / warps;
-    const uint32_t first = (blockIdx.x * 4u + warp) * per, last = min(first + per, n);
+template <class T>
+__device__ __forceinline__ void relaxTile(const Dev& D, const FastW& F, const W& w, uint32_t na, uint32_t j, int shift,
+                                          float2* sp) {
+    const uint32_t lane = threadIdx.x & 31u;
     const int ly = (int)(lane >> 2), q = (int)(lane & 3u);
     // the lane's cell around the tile: the left and right columns, the rows
     // above and below, 8 lanes each
     const int side = (int)(lane >> 3), along = (int)(lane & 7u);
     const int rx_ = side == 0 ? -1 : side == 1 ? BLOCK : along, ry_ = side == 2 ? -1 : side == 3 ? BLOCK : along;
-    for (uint32_t g = first; g < last; g++) {
-        const uint32_t it = Bt.item(L_RELAX, g);
-        const World& Wd = src.getG(Bt, it);
-        const Dev& D = Wd.D;
-        const FastW& F = Wd.S;
-        const W w(D);
-        const uint32_t j = Bt.unit(it);
-        if (D.st->cont == 0u) continue;
-        const int shift = ((D.st->shift_first ^ (uint32_t)second) & 1u) ? BLOCK / 2 : 0;
-        const Fine& Z = F.Z;
-        const uint32_t na = w.activeCount();
-        const uint32_t wid = j < na ? j : D.B + (j - na);
-        const I2 b = tileBlockF(w, wid, shift);
-        const int ox = b.x * BLOCK - shift, oy = b.y * BLOCK - shift;
-        if (b.x < 0 || ox >= D.W || oy >= D.H) continue;
-        const uint32_t states = w.statesOf(I2{ox / BLOCK, oy / BLOCK}, I2{(ox + BLOCK - 1) / BLOCK, (oy + BLOCK - 1) / BLOCK});
-        // the lane's two cells and its cell around the tile, all loads
-        // issued together (and before the tile's state is known)
-        const int p0 = (ox + oy + ly) & 1;
-        int t[2];
-        uint32_t idx[2], mk[2];
-        float R[2], ry[2];
-        float4 bb[2];
-        float2 v[2];
+    const Fine& Z = F.Z;
+    const uint32_t wid = j < na ? j : D.B + (j - na);
+    const I2 b = tileBlockF(w, wid, shift);
+    const int ox = b.x * BLOCK - shift, oy = b.y * BLOCK - shift;
+    if (b.x < 0 || ox >= D.W || oy >= D.H) return;
+    const uint32_t states = w.statesOf(I2{ox / BLOCK, oy / BLOCK}, I2{(ox + BLOCK - 1) / BLOCK, (oy + BLOCK - 1) / BLOCK});
+    // the lane's two cells and its cell around the tile, all loads issued
+    // together (and before the tile's state is known)
+    const int p0 = (ox + oy + ly) & 1;
+    int t[2];
+    uint32_t idx[2], mk[2];
+    float R[2], ry[2];
+    float4 bb[2];
+    float2 v[2];
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+        const int lx = 2 * q + (c == 0 ? p0 : 1 - p0);
+        const I2 me{ox + lx, oy + ly};
+        const bool in = w.inWorld(me);
+        t[c] = (ly + 1) * RXS + lx + 1;
+        idx[c] = in ? w.cellIndex(me) : 0u;
+        mk[c] = in ? Z.mask[idx[c]] : 0u;
+        R[c] = F.R[idx[c]];
+        ry[c] = Z.ry[idx[c]];
+        bb[c] = fineCoef(F, idx[c], T());
+        v[c] = in ? Z.rim[idx[c]] : make_float2(0.0f, 0.0f);
+    }
+    const I2 rc{ox + rx_, oy + ry_};
+    const float2 around = w.inWorld(rc) ? Z.rim[w.cellIndex(rc)] : make_float2(0.0f, 0.0f);
+    if ((states & HAS_FLUID) == 0u) return;
+    float dx[2], dy[2];
+    bool solving[2], visc[2];
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+        const float dg = diagOf(bb[c]);
+        dx[c] = dg + ((mk[c] & FM_PIN) != 0u ? PIN : 0.0f);
+        dy[c] = fmaxf(dg, 1e-30f);
+        solving[c] = (mk[c] & FM_LIQUID) != 0u && dx[c] > 0.0f;
+        visc[c] = dg > 0.0f;
+        sp[t[c]] = v[c];
+    }
+    sp[(ry_ + 1) * RXS + rx_ + 1] = around;
+    __syncwarp();
+    // (a loop, not 8 sweeps in a row: its instructions are fetched once)
+#pragma unroll 1
+    for (int pair = 0; pair < SWEEPS; pair++) {
 #pragma unroll
         for (int c = 0; c < 2; c++) {
-            const int lx = 2 * q + (c == 0 ? p0 : 1 - p0);
-            const I2 me{ox + lx, oy + ly};
-            const bool in = w.inWorld(me);
-            t[c] = (ly + 1) * RXS + lx + 1;
-            idx[c] = in ? w.cellIndex(me) : 0u;
-            mk[c] = in ? Z.mask[idx[c]] : 0u;
-            R[c] = F.R[idx[c]];
-            ry[c] = Z.ry[idx[c]];
-            bb[c] = fineCoef(F, idx[c], T());
-            v[c] = in ? Z.rim[idx[c]] : make_float2(0.0f, 0.0f);
-        }
-        const I2 rc{ox + rx_, oy + ry_};
-        const float2 around = w.inWorld(rc) ? Z.rim[w.cellIndex(rc)] : make_float2(0.0f, 0.0f);
-        if ((states & HAS_FLUID) == 0u) continue;
-        float dx[2], dy[2];
-        bool solving[2], visc[2];
-#pragma unroll
-        for (int c = 0; c < 2; c++) {
-            const float dg = diagOf(bb[c]);
-            dx[c] = dg + ((mk[c] & FM_PIN) != 0u ? PIN : 0.0f);
-            dy[c] = fmaxf(dg, 1e-30f);
-            solving[c] = (mk[c] & FM_LIQUID) != 0u && dx[c] > 0.0f;
-            visc[c] = dg > 0.0f;
-            sp[t[c]] = v[c];
-        }
-        sp[(ry_ + 1) * RXS + rx_ + 1] = around;
-        __syncwarp();
-#pragma unroll
-        for (int sw = 0; sw < 2 * SWEEPS; sw++) {
-            const int c = sw & 1;
             if (solving[c]) {
                 const float2* s = sp + t[c];
                 const float2 l = s[-1], r = s[1], u = s[-RXS], d = s[RXS];
@@ -594,9 +505,28 @@ __global__ void __launch_bounds__(128) k_fRelax(Batch Bt, const __grid_constant_
             }
             __syncwarp();
         }
+    }
 #pragma unroll
-        for (int c = 0; c < 2; c++)
-            if (solving[c]) Z.pot[idx[c]] = v[c];
+    for (int c = 0; c < 2; c++)
+        if (solving[c]) Z.pot[idx[c]] = v[c];
+}
+
+template <bool ONE, class T>
+__global__ void __launch_bounds__(128) k_fRelax(Batch Bt, const __grid_constant__ WorldSrc<ONE> src, int second) {
+    __shared__ float2 tp[4][RIM * RXS];
+    const uint32_t warp = threadIdx.x >> 5;
+    const uint32_t n = Bt.n(L_RELAX);
+    const uint32_t warps = gridDim.x * 4u, per = (n + warps - 1u) / warps;
+    const uint32_t first = (blockIdx.x * 4u + warp) * per, last = min(first + per, n);
+#pragma unroll 1
+    for (uint32_t g = first; g < last; g++) {
+        const uint32_t it = Bt.item(L_RELAX, g);
+        const World& Wd = src.getG(Bt, it);
+        const Dev& D = Wd.D;
+        const W w(D);
+        if (D.st->cont == 0u) continue;
+        const int shift = ((D.st->shift_first ^ (uint32_t)second) & 1u) ? BLOCK / 2 : 0;
+        relaxTile<T>(D, Wd.S, w, w.activeCount(), Bt.unit(it), shift, tp[warp]);
     }
 }
 
@@ -716,46 +646,6 @@ __device__ void restrictCell(const Dev& D, const FastW& F, const W& w, uint32_t 
     st(V.rho + j, rho);
 }
 
-// One cell of smoothAt (fluid.wgsl:2318-2334) on level l >= 1, the
-// coefficients worked out on the step's first iteration and kept.
-template <class T = float>
-__device__ void smoothCell(const Dev& D, const FastW& F, uint32_t l, int color, bool first, uint32_t j) {
-    const int lw = (int)D.level_w[l], lh = (int)D.level_h[l];
-    const int cx = (int)(j % (uint32_t)lw), cy = (int)(j / (uint32_t)lw);
-    if (((cx + cy) & 1) != color) return;
-    const LRef<T> V = lref<T>(F, l);
-    const float rho = ld(V.rho + j);
-    if (rho <= 0.0f) return;
-    float b[4];
-    float dg;
-    if (first) {
-        for (int d = 0; d < 4; d++) {
-            b[d] = 0.0f;
-            if (!nbrIn(cx, cy, lw, lh, d)) continue;
-            float r = ld(V.rho + nbr(j, cx, cy, lw, lh, d));
-            if (r < 0.0f) continue;
-            b[d] = faceBeta(rho, r);
-        }
-        st(V.b0 + j, b[0]); st(V.b1 + j, b[1]); st(V.b2 + j, b[2]); st(V.b3 + j, b[3]);
-    }
-    // worked in what is stored, as later iterations read it
-    const float4 bs = V.coef(j);
-    b[0] = bs.x; b[1] = bs.y; b[2] = bs.z; b[3] = bs.w;
-    dg = diagOf(bs);
-    if (dg <= 0.0f) return;
-    float sx = 0.0f, sy = 0.0f;
-#pragma unroll
-    for (int d = 0; d < 4; d++) {
-        uint32_t n = nbr(j, cx, cy, lw, lh, d);
-        sx = sx + b[d] * ld(V.px + n);
-        sy = sy + b[d] * ld(V.py + n);
-    }
-    const float h2 = (float)(1u << (2u * l));
-    const float ex = ld(V.px + j), ey = ld(V.py + j);
-    st(V.px + j, mixf(ex, (sx - h2 * ld(V.rx + j)) / dg, 1.0f));
-    st(V.py + j, mixf(ey, (sy - h2 * ld(V.ry + j)) / dg, 1.0f));
-}
-
 // prolonged (fluid.wgsl:2478-2497) from level l + 1's arrays.  The four
 // coarse cells' words are loaded before any is used (a cell past the
 // level's edge reads a clamped one and is left out), then weighed in the
@@ -791,19 +681,6 @@ __device__ __forceinline__ V2 prolongedFrom(const T* rho, const P* px, const P* 
     }
     const float ww = fmaxf(weight, 1e-6f);
     return V2{ax / ww, ay / ww};
-}
-
-// One cell of prolong (fluid.wgsl:2459-2470), level l from l + 1.
-template <class T = float>
-__device__ void prolongCell(const Dev& D, const FastW& F, uint32_t l, uint32_t j) {
-    const int lw = (int)D.level_w[l];
-    const LRef<T> V = lref<T>(F, l);
-    if (ld(V.rho + j) <= 0.0f) return;
-    const LRef<T> U = lref<T>(F, l + 1u);
-    V2 e = prolongedFrom(U.rho, U.px, U.py, (int)D.level_w[l + 1], (int)D.level_h[l + 1], (int)(j % (uint32_t)lw),
-                         (int)(j / (uint32_t)lw));
-    st(V.px + j, ld(V.px + j) + e.x);
-    st(V.py + j, ld(V.py + j) + e.y);
 }
 
 // ---------------------------------------------------------------- level tiles
@@ -859,16 +736,29 @@ __device__ __forceinline__ void tileSweepCell(LevelTile& t, int ix, int iy, int 
     t.py[i] = mixf(t.py[i], (sy - h2 * t.ry[i]) / dg, SMOOTH_OMEGA);
 }
 
+// The NT threads that work a tile: a CTA, or a part of one under named
+// barrier `bar` (0: the CTA's own).
+template <int NT>
+struct Team {
+    int tid, bar;
+    __device__ __forceinline__ void sync() const {
+        if (bar == 0) __syncthreads();
+        else asm volatile("bar.sync %0, %1;" ::"r"(bar), "n"(NT) : "memory");
+    }
+};
+
 // The red sweep over the tile's ring of 1, the black over the tile itself.
-__device__ __forceinline__ void tileSmooth(LevelTile& t, int x0, int y0, int lw, int lh, float h2) {
-    for (int k = (int)threadIdx.x; k < (LT + 2) * (LT + 2); k += (int)blockDim.x) {
+template <int NT>
+__device__ __forceinline__ void tileSmooth(LevelTile& t, const Team<NT>& tm, int x0, int y0, int lw, int lh, float h2) {
+#pragma unroll 1
+    for (int k = tm.tid; k < (LT + 2) * (LT + 2); k += NT) {
         const int ix = k % (LT + 2) - 1, iy = k / (LT + 2) - 1, cx = x0 + ix, cy = y0 + iy;
         if (cx < 0 || cy < 0 || cx >= lw || cy >= lh || ((cx + cy) & 1) != 0) continue;
         tileSweepCell(t, ix, iy, cx, cy, lw, lh, h2);
     }
-    __syncthreads();
-    if (threadIdx.x >= (unsigned)(LT * LT)) return;  // a wide CTA's threads past the tile's cells
-    const int ix = (int)threadIdx.x % LT, iy = (int)threadIdx.x / LT, cx = x0 + ix, cy = y0 + iy;
+    tm.sync();
+    if (tm.tid >= LT * LT) return;  // a wide team's threads past the tile's cells
+    const int ix = tm.tid % LT, iy = tm.tid / LT, cx = x0 + ix, cy = y0 + iy;
     if (cx < lw && cy < lh && ((cx + cy) & 1) == 1) tileSweepCell(t, ix, iy, cx, cy, lw, lh, h2);
 }
 
@@ -878,77 +768,85 @@ __device__ __forceinline__ void tileSmooth(LevelTile& t, int x0, int y0, int lw,
 // from the densities (as the step's first iteration works and stores them,
 // and later ones read them back), stored by the tile's own cells on the
 // first iteration.
+template <class T, int NT, bool FINE>
+__device__ __forceinline__ void downTile(const Dev& D, const FastW& F, const W& w, uint32_t l, uint32_t tile, bool first,
+                                         LevelTile& t, const Team<NT>& tm) {
+    const int lw = (int)D.level_w[l], lh = (int)D.level_h[l], tw = (lw + LT - 1) / LT;
+    const int x0 = (int)(tile % (uint32_t)tw) * LT, y0 = (int)(tile / (uint32_t)tw) * LT;
+    if (l >= F.lc) {
+        const int cx = x0 + tm.tid % LT, cy = y0 + tm.tid / LT;
+        if (tm.tid < LT * LT && cx < lw && cy < lh)
+            restrictCell<T, FINE>(D, F, w, l, (uint32_t)(cy * lw + cx));
+        return;
+    }
+    const LRef<T> V = lref<T>(F, l);
+#pragma unroll 1
+    for (int k = tm.tid; k < LRR; k += NT) {
+        const int ix = k % LR - 2, iy = k / LR - 2, cx = x0 + ix, cy = y0 + iy;
+        float rho = -1.0f, rx = 0.0f, ry = 0.0f;
+        if (cx >= 0 && cy >= 0 && cx < lw && cy < lh) {
+            const bool res = ix >= -1 && iy >= -1 && ix <= LT && iy <= LT;
+            restrictedAt<T, FINE>(D, F, w, l, cx, cy, res, rho, rx, ry);
+        }
+        t.rho[k] = asStored(rho, T());
+        t.rx[k] = rx;
+        t.ry[k] = ry;
+        t.px[k] = 0.0f;
+        t.py[k] = 0.0f;
+    }
+    tm.sync();
+#pragma unroll 1
+    for (int k = tm.tid; k < (LT + 2) * (LT + 2); k += NT) {
+        const int ix = k % (LT + 2) - 1, iy = k / (LT + 2) - 1, cx = x0 + ix, cy = y0 + iy;
+        if (cx < 0 || cy < 0 || cx >= lw || cy >= lh) continue;
+        const int i = lsi(ix, iy);
+        const float rho = t.rho[i];
+        if (rho <= 0.0f) continue;
+        float b[4];
+#pragma unroll
+        for (int d = 0; d < 4; d++) {
+            b[d] = 0.0f;
+            if (!nbrIn(cx, cy, lw, lh, d)) continue;
+            const float r = t.rho[lsn(ix, iy, cx, cy, lw, lh, d)];
+            if (r < 0.0f) continue;
+            b[d] = faceBeta(rho, r);
+        }
+        const bool own = ix >= 0 && iy >= 0 && ix < LT && iy < LT;
+        if (first && own) {
+            const uint32_t j = (uint32_t)(cy * lw + cx);
+            st(V.b0 + j, b[0]); st(V.b1 + j, b[1]); st(V.b2 + j, b[2]); st(V.b3 + j, b[3]);
+        }
+#pragma unroll
+        for (int d = 0; d < 4; d++) t.b[d][i] = asStored(b[d], T());
+        t.dg[i] = ((t.b[0][i] + t.b[1][i]) + t.b[2][i]) + t.b[3][i];
+    }
+    tm.sync();
+    tileSmooth(t, tm, x0, y0, lw, lh, (float)(1u << (2u * l)));
+    if (tm.tid < LT * LT) {
+        const int ix = tm.tid % LT, iy = tm.tid / LT, cx = x0 + ix, cy = y0 + iy;
+        if (cx < lw && cy < lh) {
+            const uint32_t j = (uint32_t)(cy * lw + cx);
+            const int i = lsi(ix, iy);
+            st(V.px + j, t.px[i]);
+            st(V.py + j, t.py[i]);
+            st(V.rx + j, t.rx[i]);
+            st(V.ry + j, t.ry[i]);
+            st(V.rho + j, t.rho[i]);
+        }
+    }
+    tm.sync();  // the tile's arrays are free for the next tile
+}
+
 template <bool ONE, class T, int NT, bool FINE>
 __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 2) k_fDown(Batch Bt, const __grid_constant__ WorldSrc<ONE> src, uint32_t l) {
     __shared__ WorldCopy wc_;
     if (!ONE) worldCopyInit(wc_);
     __shared__ LevelTile t;
+    const Team<NT> tm{(int)threadIdx.x, 0};
     FOR_ITEMS(Bt, L_RES + l - 1u, it) {
         FAST_ITEM(Bt, it, D, F, w, tile);
         if (D.st->cont == 0u) continue;
-        const int lw = (int)D.level_w[l], lh = (int)D.level_h[l], tw = (lw + LT - 1) / LT;
-        const int x0 = (int)(tile % (uint32_t)tw) * LT, y0 = (int)(tile / (uint32_t)tw) * LT;
-        if (l >= F.lc) {
-            const int cx = x0 + (int)threadIdx.x % LT, cy = y0 + (int)threadIdx.x / LT;
-            if (threadIdx.x < (unsigned)(LT * LT) && cx < lw && cy < lh)
-                restrictCell<T, FINE>(D, F, w, l, (uint32_t)(cy * lw + cx));
-            continue;
-        }
-        const LRef<T> V = lref<T>(F, l);
-        const bool first = D.st->cycle == 0u;
-        for (int k = (int)threadIdx.x; k < LRR; k += (int)blockDim.x) {
-            const int ix = k % LR - 2, iy = k / LR - 2, cx = x0 + ix, cy = y0 + iy;
-            float rho = -1.0f, rx = 0.0f, ry = 0.0f;
-            if (cx >= 0 && cy >= 0 && cx < lw && cy < lh) {
-                const bool res = ix >= -1 && iy >= -1 && ix <= LT && iy <= LT;
-                restrictedAt<T, FINE>(D, F, w, l, cx, cy, res, rho, rx, ry);
-            }
-            t.rho[k] = asStored(rho, T());
-            t.rx[k] = rx;
-            t.ry[k] = ry;
-            t.px[k] = 0.0f;
-            t.py[k] = 0.0f;
-        }
-        __syncthreads();
-        for (int k = (int)threadIdx.x; k < (LT + 2) * (LT + 2); k += (int)blockDim.x) {
-            const int ix = k % (LT + 2) - 1, iy = k / (LT + 2) - 1, cx = x0 + ix, cy = y0 + iy;
-            if (cx < 0 || cy < 0 || cx >= lw || cy >= lh) continue;
-            const int i = lsi(ix, iy);
-            const float rho = t.rho[i];
-            if (rho <= 0.0f) continue;
-            float b[4];
-#pragma unroll
-            for (int d = 0; d < 4; d++) {
-                b[d] = 0.0f;
-                if (!nbrIn(cx, cy, lw, lh, d)) continue;
-                const float r = t.rho[lsn(ix, iy, cx, cy, lw, lh, d)];
-                if (r < 0.0f) continue;
-                b[d] = faceBeta(rho, r);
-            }
-            const bool own = ix >= 0 && iy >= 0 && ix < LT && iy < LT;
-            if (first && own) {
-                const uint32_t j = (uint32_t)(cy * lw + cx);
-                st(V.b0 + j, b[0]); st(V.b1 + j, b[1]); st(V.b2 + j, b[2]); st(V.b3 + j, b[3]);
-            }
-#pragma unroll
-            for (int d = 0; d < 4; d++) t.b[d][i] = asStored(b[d], T());
-            t.dg[i] = ((t.b[0][i] + t.b[1][i]) + t.b[2][i]) + t.b[3][i];
-        }
-        __syncthreads();
-        tileSmooth(t, x0, y0, lw, lh, (float)(1u << (2u * l)));
-        if (threadIdx.x < (unsigned)(LT * LT)) {
-            const int ix = (int)threadIdx.x % LT, iy = (int)threadIdx.x / LT, cx = x0 + ix, cy = y0 + iy;
-            if (cx < lw && cy < lh) {
-                const uint32_t j = (uint32_t)(cy * lw + cx);
-                const int i = lsi(ix, iy);
-                st(V.px + j, t.px[i]);
-                st(V.py + j, t.py[i]);
-                st(V.rx + j, t.rx[i]);
-                st(V.ry + j, t.ry[i]);
-                st(V.rho + j, t.rho[i]);
-            }
-        }
-        __syncthreads();  // the tile's arrays are free for the next item
+        downTile<T, NT, FINE>(D, F, w, l, tile, D.st->cycle == 0u, t, tm);
     }
 }
 
@@ -957,72 +855,81 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 2) k_fDown(Batch Bt, const
 // coefficients.  The way down's potentials are read from px, py (the ring
 // too) and the results go to ux, uy, so no CTA reads a cell that another
 // writes in the same launch; level l + 1's results are its ux, uy.
+template <class T, int NT>
+__device__ __forceinline__ void upTile(const Dev& D, const FastW& F, uint32_t l, uint32_t tile, LevelTile& t,
+                                       const Team<NT>& tm) {
+    const int lw = (int)D.level_w[l], lh = (int)D.level_h[l], tw = (lw + LT - 1) / LT;
+    const int x0 = (int)(tile % (uint32_t)tw) * LT, y0 = (int)(tile / (uint32_t)tw) * LT;
+    const LRef<T> V = lref<T>(F, l);
+    const T* urho = lref<T>(F, l + 1u).rho;
+    const auto* lux = upx<T>(F, l + 1u);
+    const auto* luy = upy<T>(F, l + 1u);
+    const int uw = (int)D.level_w[l + 1], uh = (int)D.level_h[l + 1];
+#pragma unroll 1
+    for (int k = tm.tid; k < LRR; k += NT) {
+        const int ix = k % LR - 2, iy = k / LR - 2, cx = x0 + ix, cy = y0 + iy;
+        float rho = -1.0f, px = 0.0f, py = 0.0f;
+        if (cx >= 0 && cy >= 0 && cx < lw && cy < lh) {
+            // every word the cell may need loaded before any is used (a
+            // cell not liquid drops them)
+            const uint32_t j = (uint32_t)(cy * lw + cx);
+            const bool ring1 = ix >= -1 && iy >= -1 && ix <= LT && iy <= LT;
+            rho = ld(V.rho + j);
+            px = ld(V.px + j);
+            py = ld(V.py + j);
+            const V2 e = prolongedFrom(urho, lux, luy, uw, uh, cx, cy);
+            float rx = 0.0f, ry = 0.0f, b0 = 0.0f, b1 = 0.0f, b2 = 0.0f, b3 = 0.0f;
+            if (ring1) {
+                rx = ld(V.rx + j);
+                ry = ld(V.ry + j);
+                b0 = ld(V.b0 + j);
+                b1 = ld(V.b1 + j);
+                b2 = ld(V.b2 + j);
+                b3 = ld(V.b3 + j);
+            }
+            if (rho > 0.0f) {
+                px = px + e.x;
+                py = py + e.y;
+                if (ring1) {
+                    t.rx[k] = rx;
+                    t.ry[k] = ry;
+                    t.b[0][k] = b0;
+                    t.b[1][k] = b1;
+                    t.b[2][k] = b2;
+                    t.b[3][k] = b3;
+                    t.dg[k] = ((b0 + b1) + b2) + b3;
+                }
+            }
+        }
+        t.rho[k] = rho;
+        t.px[k] = px;
+        t.py[k] = py;
+    }
+    tm.sync();
+    tileSmooth(t, tm, x0, y0, lw, lh, (float)(1u << (2u * l)));
+    if (tm.tid < LT * LT) {
+        const int ix = tm.tid % LT, iy = tm.tid / LT, cx = x0 + ix, cy = y0 + iy;
+        const int i = lsi(ix, iy);
+        if (cx < lw && cy < lh && t.rho[i] > 0.0f) {
+            const uint32_t j = (uint32_t)(cy * lw + cx);
+            st(upx<T>(F, l) + j, t.px[i]);
+            st(upy<T>(F, l) + j, t.py[i]);
+        }
+    }
+    tm.sync();
+}
+
 template <bool ONE, class T, int NT = 256>
 __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 2) k_fUp(Batch Bt, const __grid_constant__ WorldSrc<ONE> src, uint32_t l) {
     __shared__ WorldCopy wc_;
     if (!ONE) worldCopyInit(wc_);
     __shared__ LevelTile t;
+    const Team<NT> tm{(int)threadIdx.x, 0};
     FOR_ITEMS(Bt, L_SM + l - 1u, it) {
         FAST_ITEM(Bt, it, D, F, w, tile);
+        (void)w;
         if (D.st->cont == 0u) continue;
-        const int lw = (int)D.level_w[l], lh = (int)D.level_h[l], tw = (lw + LT - 1) / LT;
-        const int x0 = (int)(tile % (uint32_t)tw) * LT, y0 = (int)(tile / (uint32_t)tw) * LT;
-        const LRef<T> V = lref<T>(F, l);
-        const T* urho = lref<T>(F, l + 1u).rho;
-        const auto* lux = upx<T>(F, l + 1u);
-        const auto* luy = upy<T>(F, l + 1u);
-        const int uw = (int)D.level_w[l + 1], uh = (int)D.level_h[l + 1];
-        for (int k = (int)threadIdx.x; k < LRR; k += (int)blockDim.x) {
-            const int ix = k % LR - 2, iy = k / LR - 2, cx = x0 + ix, cy = y0 + iy;
-            float rho = -1.0f, px = 0.0f, py = 0.0f;
-            if (cx >= 0 && cy >= 0 && cx < lw && cy < lh) {
-                // every word the cell may need loaded before any is used (a
-                // cell not liquid drops them)
-                const uint32_t j = (uint32_t)(cy * lw + cx);
-                const bool ring1 = ix >= -1 && iy >= -1 && ix <= LT && iy <= LT;
-                rho = ld(V.rho + j);
-                px = ld(V.px + j);
-                py = ld(V.py + j);
-                const V2 e = prolongedFrom(urho, lux, luy, uw, uh, cx, cy);
-                float rx = 0.0f, ry = 0.0f, b0 = 0.0f, b1 = 0.0f, b2 = 0.0f, b3 = 0.0f;
-                if (ring1) {
-                    rx = ld(V.rx + j);
-                    ry = ld(V.ry + j);
-                    b0 = ld(V.b0 + j);
-                    b1 = ld(V.b1 + j);
-                    b2 = ld(V.b2 + j);
-                    b3 = ld(V.b3 + j);
-                }
-                if (rho > 0.0f) {
-                    px = px + e.x;
-                    py = py + e.y;
-                    if (ring1) {
-                        t.rx[k] = rx;
-                        t.ry[k] = ry;
-                        t.b[0][k] = b0;
-                        t.b[1][k] = b1;
-                        t.b[2][k] = b2;
-                        t.b[3][k] = b3;
-                        t.dg[k] = ((b0 + b1) + b2) + b3;
-                    }
-                }
-            }
-            t.rho[k] = rho;
-            t.px[k] = px;
-            t.py[k] = py;
-        }
-        __syncthreads();
-        tileSmooth(t, x0, y0, lw, lh, (float)(1u << (2u * l)));
-        if (threadIdx.x < (unsigned)(LT * LT)) {
-            const int ix = (int)threadIdx.x % LT, iy = (int)threadIdx.x / LT, cx = x0 + ix, cy = y0 + iy;
-            const int i = lsi(ix, iy);
-            if (cx < lw && cy < lh && t.rho[i] > 0.0f) {
-                const uint32_t j = (uint32_t)(cy * lw + cx);
-                st(upx<T>(F, l) + j, t.px[i]);
-                st(upy<T>(F, l) + j, t.py[i]);
-            }
-        }
-        __syncthreads();
+        upTile<T, NT>(D, F, l, tile, t, tm);
     }
 }
 
@@ -1057,6 +964,7 @@ __device__ __forceinline__ int slvRow(const SLv& V, int j) {
 // density is not negative, else 0; all 0 for a cell that is not liquid.
 __device__ void slv_coefficients(const SLv& V, int tid, int nt) {
     const int n = V.w * V.h;
+#pragma unroll 1
     for (int j = tid; j < n; j += nt) {
         const int cy = slvRow(V, j), cx = j - cy * V.w;
         const float rho = V.rho[j];
@@ -1096,6 +1004,7 @@ __device__ __forceinline__ void slv_stencil(const SLv& V, int j, int cx, int cy,
 __device__ void slv_sweep(const SLv& V, uint32_t l, int color, float omega, int tid, int nt) {
     const int n = V.w * V.h, pairs = (n + 1) / 2;
     const float h2 = (float)(1u << (2u * l));
+#pragma unroll 1
     for (int k = tid; k < pairs; k += nt) {
         int j = 2 * k, cy = slvRow(V, j), cx = j - cy * V.w;
         if (((cx + cy) & 1) != color) {
@@ -1116,6 +1025,7 @@ __device__ void slv_sweep(const SLv& V, uint32_t l, int color, float omega, int 
 }
 
 __device__ void slv_smooth(const SLv& V, uint32_t l, int tid, int nt) {
+#pragma unroll 1
     for (int color = 0; color < 2; color++) {
         slv_sweep(V, l, color, SMOOTH_OMEGA, tid, nt);
         __syncthreads();
@@ -1181,6 +1091,7 @@ __device__ __forceinline__ void solveUpdate(const SLv& V, const SolveCell& c) {
 __device__ void coarseCore(const Dev& D, const W& w, uint32_t lc, float* sm, const uint32_t* off) {
     const uint32_t L = D.levels;
     const int tid = (int)threadIdx.x, nt = (int)blockDim.x;
+#pragma unroll 1
     for (uint32_t l = lc; l <= L; l++) {
         const SLv V = slv(sm, off, D, l);
         const int n = V.w * V.h;
@@ -1190,6 +1101,7 @@ __device__ void coarseCore(const Dev& D, const W& w, uint32_t lc, float* sm, con
             // 1 / h^2 of level l - 1: a power of two, so the product is the
             // quotient's bits
             const float inv_h2u = 1.0f / (float)(1u << (2u * (l - 1u)));
+#pragma unroll 1
             for (int j = tid; j < n; j += nt) {
                 const int cy = slvRow(V, j), cx = j - cy * V.w;
                 if (span <= BLOCK) {
@@ -1251,6 +1163,7 @@ __device__ void coarseCore(const Dev& D, const W& w, uint32_t lc, float* sm, con
                     c0 = c1;
                     c1 = t;
                 }
+#pragma unroll 1
                 for (int s = 0; s < COARSE_SWEEPS; s++) {
                     solveUpdate(V, c0);
                     barSub(npair);
@@ -1266,10 +1179,12 @@ __device__ void coarseCore(const Dev& D, const W& w, uint32_t lc, float* sm, con
         }
         __syncthreads();
     }
+#pragma unroll 1
     for (int l = (int)L - 1; l >= (int)lc; l--) {
         const SLv V = slv(sm, off, D, (uint32_t)l);
         const SLv U = slv(sm, off, D, (uint32_t)l + 1u);
         const int n = V.w * V.h;
+#pragma unroll 1
         for (int j = tid; j < n; j += nt) {
             if (V.rho[j] <= 0.0f) continue;
             const int cy = slvRow(V, j);
@@ -1287,15 +1202,14 @@ __device__ void coarseCore(const Dev& D, const W& w, uint32_t lc, float* sm, con
 // solve (40 SOR sweep pairs, omega 1.8), prolong (fluid.wgsl:2318-2470).
 // Each level's face coefficients are worked out once, when its densities
 // are in place, and read by its sweeps and by the restriction below it.
-// Level lc's results go to its ux, uy (`up`, the fast form) or back into its
-// px, py (the persistent form).
-template <class T = float>
-__device__ void coarseLevels(const Dev& D, const FastW& F, const W& w, uint32_t lc, float* sm, uint32_t* off,
-                             bool up) {
+// Level lc's results go to its ux, uy.
+template <class T>
+__device__ void coarseLevels(const Dev& D, const FastW& F, const W& w, uint32_t lc, float* sm, uint32_t* off) {
     const uint32_t L = D.levels;
     const int tid = (int)threadIdx.x, nt = (int)blockDim.x;
     if (tid == 0) {
         uint32_t o = 0;
+#pragma unroll 1
         for (uint32_t l = lc; l <= L; l++) {
             off[l] = o;
             o += SLV_ARRAYS * D.level_w[l] * D.level_h[l];
@@ -1306,6 +1220,7 @@ __device__ void coarseLevels(const Dev& D, const FastW& F, const W& w, uint32_t 
         const SLv V = slv(sm, off, D, lc);
         const LRef<T> G = lref<T>(F, lc);
         const int n = V.w * V.h;
+#pragma unroll 1
         for (int j = tid; j < n; j += nt) {
             V.px[j] = ld(G.px + j);
             V.py[j] = ld(G.py + j);
@@ -1318,9 +1233,10 @@ __device__ void coarseLevels(const Dev& D, const FastW& F, const W& w, uint32_t 
     coarseCore(D, w, lc, sm, off);
     {
         const SLv V = slv(sm, off, D, lc);
-        auto* ox = up ? upx<T>(F, lc) : lref<T>(F, lc).px;
-        auto* oy = up ? upy<T>(F, lc) : lref<T>(F, lc).py;
+        auto* ox = upx<T>(F, lc);
+        auto* oy = upy<T>(F, lc);
         const int n = V.w * V.h;
+#pragma unroll 1
         for (int j = tid; j < n; j += nt) {
             st(ox + j, V.px[j]);
             st(oy + j, V.py[j]);
@@ -1338,7 +1254,7 @@ __global__ void __launch_bounds__(1024) k_fCoarse(Batch Bt, const __grid_constan
         FAST_ITEM(Bt, it, D, F, w, unused_);
         (void)unused_;
         if (D.st->cont == 0u) continue;
-        coarseLevels<T>(D, F, w, F.lc, sm, off, true);
+        coarseLevels<T>(D, F, w, F.lc, sm, off);
         __syncthreads();
     }
 }
@@ -1432,6 +1348,7 @@ __device__ __forceinline__ void dl_stencil(const DLv& V, const float* r, int x, 
 // slv_coefficients over this CTA's strip.
 __device__ void dl_coefficients(const DLv& V, unsigned me) {
     const int n = (V.r1 - V.r0) * V.w;
+#pragma unroll 1
     for (int j = (int)threadIdx.x; j < n; j += (int)blockDim.x) {
         int x, y;
         dlCell(V, j, &x, &y);
@@ -1461,6 +1378,7 @@ __device__ void dl_coefficients(const DLv& V, unsigned me) {
 __device__ void dl_sweep(const DLv& V, uint32_t l, int color, float omega, unsigned me) {
     const int n = (V.r1 - V.r0) * V.w, pairs = (n + 1) / 2;
     const float h2 = (float)(1u << (2u * l));
+#pragma unroll 1
     for (int k = (int)threadIdx.x; k < pairs; k += (int)blockDim.x) {
         int j = 2 * k, x, y;
         dlCell(V, j, &x, &y);
@@ -1609,6 +1527,7 @@ __global__ void __launch_bounds__(1024) k_fCoarseCluster(Batch Bt, const __grid_
         const DLv A = dlv(sm, D, lc, lc, me);
         const LRef<T> G = lref<T>(F, lc);
         const int n = (A.r1 - A.r0) * A.w;
+#pragma unroll 1
         for (int j = (int)threadIdx.x; j < n; j += (int)blockDim.x) {
             const int g = A.r0 * A.w + j;
             A.a(A_PX)[j] = ld(G.px + g);
@@ -1625,6 +1544,7 @@ __global__ void __launch_bounds__(1024) k_fCoarseCluster(Batch Bt, const __grid_
         if (l > lc) {
             const DLv U = dlv(sm, D, lc, l - 1u, me);
             const int n = (A.r1 - A.r0) * A.w;
+#pragma unroll 1
             for (int j = (int)threadIdx.x; j < n; j += (int)blockDim.x) {
                 int x, y;
                 dlCell(A, j, &x, &y);
@@ -1646,6 +1566,7 @@ __global__ void __launch_bounds__(1024) k_fCoarseCluster(Batch Bt, const __grid_
         const DLv U = dlv(sm, D, lc, ls - 1u, me);
         const SLv S = slv(sm0, off, D, ls);
         const int n = S.w * S.h;
+#pragma unroll 1
         for (int j = (int)threadIdx.x; j < n; j += (int)blockDim.x) {
             const int cy = slvRow(S, j), cx = j - cy * S.w;
             dl_restricted(D, w, ls, U, cx, cy, me, &S.px[j], &S.py[j], &S.rx[j], &S.ry[j], &S.rho[j]);
@@ -1664,6 +1585,7 @@ __global__ void __launch_bounds__(1024) k_fCoarseCluster(Batch Bt, const __grid_
             const int lw = (int)D.level_w[ls], lh = (int)D.level_h[ls];
             const int nl = lw * lh;
             const float* b0 = cl.map_shared_rank(sm0, 0u);
+#pragma unroll 1
             for (int j = (int)threadIdx.x; j < n; j += (int)blockDim.x) {
                 if (A.a(A_RHO)[j] <= 0.0f) continue;
                 int x, y;
@@ -1674,6 +1596,7 @@ __global__ void __launch_bounds__(1024) k_fCoarseCluster(Batch Bt, const __grid_
             }
         } else {
             const DLv U = dlv(sm, D, lc, (uint32_t)l + 1u, me);
+#pragma unroll 1
             for (int j = (int)threadIdx.x; j < n; j += (int)blockDim.x) {
                 if (A.a(A_RHO)[j] <= 0.0f) continue;
                 int x, y;
@@ -1695,6 +1618,7 @@ __global__ void __launch_bounds__(1024) k_fCoarseCluster(Batch Bt, const __grid_
         const int n = (A.r1 - A.r0) * A.w;
         auto* ox = upx<T>(F, lc);
         auto* oy = upy<T>(F, lc);
+#pragma unroll 1
         for (int j = (int)threadIdx.x; j < n; j += (int)blockDim.x) {
             const int g = A.r0 * A.w + j;
             st(ox + g, A.a(A_PX)[j]);
@@ -1702,33 +1626,6 @@ __global__ void __launch_bounds__(1024) k_fCoarseCluster(Batch Bt, const __grid_
         }
     }
 }
-
-// prolongFine (fluid.wgsl:2500-2512), and the rims for the relaxation after.
-template <bool ONE, class T>
-__global__ void k_fProlongFine(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
-    __shared__ WorldCopy wc_;
-    if (!ONE) worldCopyInit(wc_);
-    FOR_ITEMS(Bt, L_ACT, it) {
-        FAST_ITEM(Bt, it, D, F, w, wid);
-        if (D.st->cont == 0u) continue;
-        const T* urho = lref<T>(F, 1u).rho;
-        I2 c = lidCell(w, wid);
-        if (!w.inWorld(c)) continue;
-        uint32_t i = w.cellIndex(c);
-        // the cell's words and the prolongation's loaded together, then used
-        // for a liquid cell only
-        const uint32_t mk = F.Z.mask[i];
-        const float2 p = F.Z.pot[i];
-        const V2 e = prolongedFrom(urho, upx<T>(F, 1u), upy<T>(F, 1u), (int)D.level_w[1], (int)D.level_h[1], c.x, c.y);
-        if ((mk & FM_LIQUID) != 0u) {
-            const float2 v = make_float2(p.x + e.x, p.y + e.y);
-            F.Z.pot[i] = v;
-            F.Z.rim[i] = v;
-        }
-    }
-}
-
-// ================================================================ conjugate gradients
 
 // The CG kernels: a warp a tile of 8x8 cells, lane l the cells l and l + 32
 // of the tile (rows l / 8 and l / 8 + 4), so a tile's tree of 64 (its first
@@ -1759,6 +1656,37 @@ __device__ __forceinline__ void forTileRuns(const Batch& Bt, const WorldSrc<ONE>
         g += m;
     }
 }
+
+// prolongFine (fluid.wgsl:2500-2512) of cell c, and its rim for the
+// relaxation after: the cell's words and the prolongation's loaded together,
+// then used for a liquid cell only.  (A lane a quad of cells, whose
+// nine coarse cells it loads once, was slower: 32 us a launch against 21 on
+// a 48-world batch, for want of loads in flight.)
+template <class T>
+__device__ __forceinline__ void prolongFineCell(const Dev& D, const FastW& F, const W& w, I2 c) {
+    const uint32_t i = w.cellIndex(c);
+    const uint32_t mk = F.Z.mask[i];
+    const float2 p = F.Z.pot[i];
+    const V2 e = prolongedFrom(lref<T>(F, 1u).rho, upx<T>(F, 1u), upy<T>(F, 1u), (int)D.level_w[1], (int)D.level_h[1], c.x, c.y);
+    if ((mk & FM_LIQUID) == 0u) return;
+    const float2 v = make_float2(p.x + e.x, p.y + e.y);
+    F.Z.pot[i] = v;
+    F.Z.rim[i] = v;
+}
+
+template <bool ONE, class T>
+__global__ void k_fProlongFine(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
+    __shared__ WorldCopy wc_;
+    if (!ONE) worldCopyInit(wc_);
+    FOR_ITEMS(Bt, L_ACT, it) {
+        FAST_ITEM(Bt, it, D, F, w, wid);
+        if (D.st->cont == 0u) continue;
+        const I2 c = lidCell(w, wid);
+        if (w.inWorld(c)) prolongFineCell<T>(D, F, w, c);
+    }
+}
+
+// ================================================================ conjugate gradients
 
 // A lane's two cells of tile wid: their indices and whether they are in the
 // world (a ragged world's last blocks), and the tile's block.
@@ -1792,61 +1720,69 @@ __device__ __forceinline__ T warpTree(T lo, T hi) {
     return v;
 }
 
-// sumBlocks (fluid.wgsl:2645-2661) of the first NC components of a world's
-// B block partials by a CTA of CG_THREADS: column li (of 256) adds blocks
-// li, li + 256, ... in that order, 16 rows' loads in flight a thread.  Two
-// components: a half of the CTA each.  One: the halves take 16 rows each of
-// a column in turn and pass its sum on, so the order of the adds stays.
-// A block not worked on has partials of +0, and a sum that starts from +0 is
-// never -0, so adding them changes no bit: its state is not read.  The sums
-// in thread 0.
+// The tree of 256 of NC components' column sums, a component's at s + 256 c,
+// written by the CTA's threads; the sums in s[256 c], for every thread.
 template <class T, int NC>
-__device__ __noinline__ void sumBlocksCg(uint32_t B, const T* part, T* s, T* out) {
-    constexpr uint32_t ROWS = 16u, HALF = 256u * ROWS;
-    const uint32_t li = threadIdx.x & 255u, half = threadIdx.x >> 8;
-    T* own = s + (NC == 2 ? 256u * half : 0u) + li;
-    const T* at = part + (NC == 2 ? (size_t)B * half : 0u);
-    T acc = T(0);
-    for (uint32_t r0 = 0; r0 < B; r0 += NC == 2 ? HALF : 2u * HALF) {
-        T v[ROWS];
-        const uint32_t k0 = r0 + (NC == 2 ? 0u : half * HALF) + li;
-#pragma unroll
-        for (uint32_t u = 0; u < ROWS; u++) v[u] = k0 + 256u * u < B ? __ldcg(at + k0 + 256u * u) : T(0);
-        if (NC == 2 || half == 0u) {
-#pragma unroll
-            for (uint32_t u = 0; u < ROWS; u++) acc = acc + v[u];
-        }
-        if (NC == 2 || r0 + HALF >= B) continue;  // (uniform: the second half has no row)
-        if (half == 0u) *own = acc;
-        __syncthreads();
-        if (half == 1u) {
-            acc = *own;
-#pragma unroll
-            for (uint32_t u = 0; u < ROWS; u++) acc = acc + v[u];
-            *own = acc;
-        }
-        __syncthreads();
-        if (half == 0u) acc = *own;
-    }
-    const bool adds = NC == 2 || half == 0u;
-    if (adds) *own = acc;
+__device__ __forceinline__ void treeColumns(T* s) {
+    const uint32_t li = threadIdx.x & 255u, c = threadIdx.x >> 8;
+    T* own = s + 256u * c + li;
     __syncthreads();
 #pragma unroll
     for (uint32_t h = 128u; h > 32u; h >>= 1) {
-        if (adds && li < h) *own = *own + own[h];
+        if (c < NC && li < h) *own = *own + own[h];
         __syncthreads();
     }
-    if (adds && li < 32u) {
+    if (c < NC && li < 32u) {
         T v = *own + own[32];
 #pragma unroll
         for (int h = 16; h > 0; h >>= 1) v = v + __shfl_down_sync(0xffffffffu, v, h);
         if (li == 0u) *own = v;
     }
     __syncthreads();
-    if (threadIdx.x == 0u) {
+}
+
+// sumBlocks (fluid.wgsl:2645-2661) of the first NC components of a world's
+// B block partials by a CTA of NT threads: column li (of 256) adds blocks
+// li, li + 256, ... in that order, 16 rows' loads in flight a thread, the
+// CTA's groups of 256 threads sharing the components and, NT / 256 / NC a
+// component, taking 16 rows each of a column in turn and passing its sum on,
+// so the order of the adds stays.  A block not worked on has partials of
+// +0, and a sum that starts from +0 is never -0, so adding them changes no
+// bit: its state is not read.  The sums in s[256 c], for every thread.
+template <class T, int NC, int NT>
+__device__ __noinline__ void sumColumns(uint32_t B, const T* part, T* s) {
+    constexpr uint32_t ROWS = 16u, SPAN = 256u * ROWS, TURNS = NT / 256 / NC;
+    const uint32_t li = threadIdx.x & 255u, group = threadIdx.x >> 8;
+    const uint32_t c = group / TURNS, turn = group % TURNS;
+    T* own = s + 256u * c + li;
+    const T* at = part + (size_t)B * c;
+    T acc = T(0);
+    for (uint32_t r0 = 0; r0 < B; r0 += TURNS * SPAN) {
+        T v[ROWS];
+        const uint32_t k0 = r0 + turn * SPAN + li;
 #pragma unroll
-        for (int c = 0; c < NC; c++) out[c] = s[256 * c];
+        for (uint32_t u = 0; u < ROWS; u++) v[u] = k0 + 256u * u < B ? __ldcg(at + k0 + 256u * u) : T(0);
+#pragma unroll
+        for (uint32_t t = 0; t < TURNS; t++) {
+            if (t > 0u && r0 + t * SPAN >= B) break;  // (uniform: no more rows)
+            if (t > 0u) __syncthreads();
+            if (turn == t) {
+                if (t > 0u || (TURNS > 1u && r0 > 0u)) acc = *own;
+#pragma unroll
+                for (uint32_t u = 0; u < ROWS; u++) acc = acc + v[u];
+                if (TURNS > 1u) *own = acc;
+            }
+        }
+        if (TURNS > 1u) __syncthreads();
     }
+    if (TURNS == 1u) *own = acc;
+}
+template <class T, int NC, int NT>
+__device__ __forceinline__ void sumBlocksCg(uint32_t B, const T* part, T* s, T (&out)[NC]) {
+    sumColumns<T, NC, NT>(B, part, s);
+    treeColumns<T, NC>(s);
+#pragma unroll
+    for (int c = 0; c < NC; c++) out[c] = s[256 * c];
 }
 
 // Counts the CTA's m tiles of a world whose partials its warps' first lanes
@@ -1870,13 +1806,63 @@ __device__ __forceinline__ bool countTiles(uint32_t* counter, uint32_t m, uint32
     return last != 0;
 }
 
+// A world's partial sums as a kernel writes them: component c of block b at
+// c * B + b, in FP64 or f32.
+struct Parts {
+    double* d;
+    float* f;
+};
+
+// cgRho's sums (fluid.wgsl:2736-2750) of tiles j[0] and, when two, j[1].
+__device__ __forceinline__ void rhoTiles(const Dev& D, const FastW& F, const W& w, const uint32_t (&j)[2], bool two, bool f64,
+                                         const Parts& out) {
+    const Fine& Z = F.Z;
+    const uint32_t lane = threadIdx.x & 31u;
+    TileLane t[2];
+    uint32_t mk[2][2];
+    float z[2][2], r[2][2], q[2][2];
+#pragma unroll
+    for (int u = 0; u < 2; u++) t[u] = tileLane(w, j[u], u == 0 || two);
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const uint32_t i = t[u].i[h];
+            mk[u][h] = Z.mask[i];
+            z[u][h] = Z.pot[i].x;
+            r[u][h] = F.R[i];
+            q[u][h] = F.Q[i];
+        }
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        if (u == 1 && !two) break;  // (warp-uniform)
+        const bool f0 = t[u].in[0] && (mk[u][0] & FM_LIQUID) != 0u, f1 = t[u].in[1] && (mk[u][1] & FM_LIQUID) != 0u;
+        // the f32 trees only without FP64 dots, which read none of them
+        if (f64) {
+            const double x = warpTree(f0 ? (double)r[u][0] * (double)z[u][0] : 0.0, f1 ? (double)r[u][1] * (double)z[u][1] : 0.0);
+            const double y = warpTree(f0 ? (double)q[u][0] * (double)z[u][0] : 0.0, f1 ? (double)q[u][1] * (double)z[u][1] : 0.0);
+            if (lane == 0u) {
+                out.d[t[u].n] = x;
+                out.d[D.B + t[u].n] = y;
+            }
+        } else {
+            const float x = warpTree(f0 ? r[u][0] * z[u][0] : 0.0f, f1 ? r[u][1] * z[u][1] : 0.0f);
+            const float y = warpTree(f0 ? q[u][0] * z[u][0] : 0.0f, f1 ? q[u][1] * z[u][1] : 0.0f);
+            if (lane == 0u) {
+                out.f[t[u].n] = x;
+                out.f[D.B + t[u].n] = y;
+            }
+        }
+    }
+}
+
 // cgRho + cgBeta (fluid.wgsl:2736-2764).
 template <bool ONE>
 __global__ void __launch_bounds__(CG_THREADS, 2) k_fRhoBeta(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
     if (!ONE) worldCopyInit(wc_);
     __shared__ double s64[512];
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t warp = threadIdx.x >> 5;
     forTileRuns<ONE>(Bt, src, wc_, [&](const World& Wd, uint32_t na, uint32_t j0, uint32_t m) {
         const Dev& D = Wd.D;
         const FastW& F = Wd.S;
@@ -1884,58 +1870,22 @@ __global__ void __launch_bounds__(CG_THREADS, 2) k_fRhoBeta(Batch Bt, const __gr
         if (D.st->cont == 0u) return;
         const bool f64 = D.st->f64 != 0u;
         const uint32_t cycle = D.st->cycle;
-        const Fine& Z = F.Z;
-        for (uint32_t t0 = warp; t0 < m; t0 += 2u * CG_WARPS) {
-            TileLane t[2];
-            uint32_t mk[2][2];
-            float z[2][2], r[2][2], q[2][2];
-#pragma unroll
-            for (int u = 0; u < 2; u++) t[u] = tileLane(w, j0 + t0 + (uint32_t)u * CG_WARPS, t0 + (uint32_t)u * CG_WARPS < m);
-#pragma unroll
-            for (int u = 0; u < 2; u++)
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const uint32_t i = t[u].i[h];
-                    mk[u][h] = Z.mask[i];
-                    z[u][h] = Z.pot[i].x;
-                    r[u][h] = F.R[i];
-                    q[u][h] = F.Q[i];
-                }
-#pragma unroll
-            for (int u = 0; u < 2; u++) {
-                if (t0 + (uint32_t)u * CG_WARPS >= m) break;  // (warp-uniform)
-                const bool f0 = t[u].in[0] && (mk[u][0] & FM_LIQUID) != 0u, f1 = t[u].in[1] && (mk[u][1] & FM_LIQUID) != 0u;
-                // the f32 trees only without FP64 dots, which read none of them
-                if (f64) {
-                    const double x = warpTree(f0 ? (double)r[u][0] * (double)z[u][0] : 0.0,
-                                              f1 ? (double)r[u][1] * (double)z[u][1] : 0.0);
-                    const double y = warpTree(f0 ? (double)q[u][0] * (double)z[u][0] : 0.0,
-                                              f1 ? (double)q[u][1] * (double)z[u][1] : 0.0);
-                    if (lane == 0u) {
-                        F.part64[t[u].n] = x;
-                        F.part64[D.B + t[u].n] = y;
-                    }
-                } else {
-                    const float x = warpTree(f0 ? r[u][0] * z[u][0] : 0.0f, f1 ? r[u][1] * z[u][1] : 0.0f);
-                    const float y = warpTree(f0 ? q[u][0] * z[u][0] : 0.0f, f1 ? q[u][1] * z[u][1] : 0.0f);
-                    if (lane == 0u) {
-                        F.part32[t[u].n] = x;
-                        F.part32[D.B + t[u].n] = y;
-                    }
-                }
-            }
+#pragma unroll 1
+        for (uint32_t t = warp; t < m; t += 2u * CG_WARPS) {
+            const uint32_t j[2] = {j0 + t, j0 + t + CG_WARPS};
+            rhoTiles(D, F, w, j, t + CG_WARPS < m, f64, Parts{F.part64, F.part32});
         }
         if (!countTiles(&D.st->fdone[1], m, na, [] {})) return;
         if (f64) {
             double v[2];
-            sumBlocksCg<double, 2>(D.B, F.part64, s64, v);
+            sumBlocksCg<double, 2, CG_THREADS>(D.B, F.part64, s64, v);
             if (threadIdx.x == 0) {
                 D.st->rz = v[0];
                 D.st->beta = (cycle == 0u || D.st->pq <= 0.0) ? 0.0 : -v[1] / D.st->pq;
             }
         } else {
             float v[2];
-            sumBlocksCg<float, 2>(D.B, F.part32, reinterpret_cast<float*>(s64), v);
+            sumBlocksCg<float, 2, CG_THREADS>(D.B, F.part32, reinterpret_cast<float*>(s64), v);
             if (threadIdx.x == 0) {
                 D.st->rz32 = v[0];
                 D.st->beta32 = (cycle == 0u || D.st->pq32 <= 0.0f) ? 0.0f : -v[1] / D.st->pq32;
@@ -1944,113 +1894,173 @@ __global__ void __launch_bounds__(CG_THREADS, 2) k_fRhoBeta(Batch Bt, const __gr
     });
 }
 
-// cgDirection + cgApply + cgAlpha (fluid.wgsl:2767-2814): the direction p =
+// cgDirection + cgApply (fluid.wgsl:2767-2795) of tile j: the direction p =
 // z + beta p_old of the tile's cells and of the 32 cells around it, a cell
 // of these a lane (worked again from their z and p_old, the same
-// arithmetic), in the warp's 10x10 of shared memory; q = A p, and the tile
-// trees of p q.  p_old is read from one of the two p arrays and p written
+// arithmetic), in the warp's 10x10 of shared memory; q = A p, and the tile's
+// tree of p q.  p_old is read from one of the two p arrays and p written
 // to the other (by the iteration's parity), so no warp reads a p that
-// another writes in the launch.
+// another writes in the pass.
+__device__ __forceinline__ void applyTile(const Dev& D, const FastW& F, const W& w, uint32_t j, bool odd, bool f64, float beta,
+                                          double beta64, float* sp, const Parts& out) {
+    const Fine& Z = F.Z;
+    const float* Pold = odd ? F.P2 : F.P;
+    float* Pnew = odd ? F.P : F.P2;
+    const uint32_t lane = threadIdx.x & 31u;
+    // the lane's cell around the tile: left and right columns, rows above
+    // and below, 8 lanes each
+    const int side = (int)(lane >> 3), at = (int)(lane & 7u);
+    const int ox = side == 0 ? -1 : side == 1 ? BLOCK : at, oy = side == 2 ? -1 : side == 3 ? BLOCK : at;
+    auto dir = [&](float z, float p) { return f64 ? (float)((double)z + beta64 * (double)p) : z + beta * p; };
+    const TileLane t = tileLane(w, j, true);
+    const I2 b = w.blockAt(t.n);
+    const I2 oc{b.x * BLOCK + ox, b.y * BLOCK + oy};
+    const bool oin = w.inWorld(oc);
+    const uint32_t oi = oin ? w.cellIndex(oc) : 0u;
+    const float oz = Z.pot[oi].x, op = Pold[oi];
+    float4 bb[2];
+    float z[2], po[2];
+    uint32_t mk[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const uint32_t i = t.i[h];
+        mk[h] = Z.mask[i];
+        bb[h] = Z.b[i];
+        z[h] = Z.pot[i].x;
+        po[h] = Pold[i];
+    }
+    float p[2];
+    const int c0 = ((int)(lane >> 3) + 1) * RIM + (int)(lane & 7u) + 1;
+    sp[(oy + 1) * RIM + ox + 1] = dir(oz, op);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        p[h] = dir(z[h], po[h]);
+        sp[c0 + 4 * RIM * h] = p[h];
+    }
+    __syncwarp();
+    float q[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        const int c = c0 + 4 * RIM * h;
+        q[h] = 0.0f;
+        if (t.in[h] && (mk[h] & FM_LIQUID) != 0u) {
+            float sum = 0.0f;
+            if (mk[h] & 1u) sum = sum + bb[h].x * sp[c - 1];
+            if (mk[h] & 2u) sum = sum + bb[h].y * sp[c + 1];
+            if (mk[h] & 4u) sum = sum + bb[h].z * sp[c - RIM];
+            if (mk[h] & 8u) sum = sum + bb[h].w * sp[c + RIM];
+            const float dgp = diagOf(bb[h]) + ((mk[h] & FM_PIN) != 0u ? PIN : 0.0f);
+            q[h] = dgp * p[h] - sum + 0.0f;
+        } else {
+            p[h] = 0.0f;
+        }
+        if (t.in[h]) {
+            Pnew[t.i[h]] = p[h];
+            F.Q[t.i[h]] = q[h];
+        }
+    }
+    if (f64) {
+        const double x = warpTree((double)p[0] * (double)q[0], (double)p[1] * (double)q[1]);
+        if (lane == 0u) out.d[t.n] = x;
+    } else {
+        const float x = warpTree(p[0] * q[0], p[1] * q[1]);
+        if (lane == 0u) out.f[t.n] = x;
+    }
+    __syncwarp();  // the warp's p is free for its next tile
+}
+
+// cgDirection + cgApply + cgAlpha (fluid.wgsl:2767-2814).
 template <bool ONE>
 __global__ void __launch_bounds__(CG_THREADS, 2) k_fApplyAlpha(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
     if (!ONE) worldCopyInit(wc_);
     __shared__ double s64[256];
     __shared__ float tp[CG_WARPS][RIM * RIM];
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    float* sp = tp[warp];
-    // the lane's cell around the tile: left and right columns, rows above
-    // and below, 8 lanes each
-    const int side = (int)(lane >> 3), at = (int)(lane & 7u);
-    const int ox = side == 0 ? -1 : side == 1 ? BLOCK : at, oy = side == 2 ? -1 : side == 3 ? BLOCK : at;
-    const int so = (oy + 1) * RIM + ox + 1;
+    const uint32_t warp = threadIdx.x >> 5;
     forTileRuns<ONE>(Bt, src, wc_, [&](const World& Wd, uint32_t na, uint32_t j0, uint32_t m) {
         const Dev& D = Wd.D;
         const FastW& F = Wd.S;
         const W w(D);
         if (D.st->cont == 0u) return;
-        const bool f64 = D.st->f64 != 0u;
+        const bool f64 = D.st->f64 != 0u, odd = (D.st->cycle & 1u) != 0u;
         const float beta = D.st->beta32;
         const double beta64 = D.st->beta;
-        const bool odd = (D.st->cycle & 1u) != 0u;
-        const float* Pold = odd ? F.P2 : F.P;
-        float* Pnew = odd ? F.P : F.P2;
-        const Fine& Z = F.Z;
-        auto dir = [&](float z, float p) { return f64 ? (float)((double)z + beta64 * (double)p) : z + beta * p; };
-        for (uint32_t t0 = warp; t0 < m; t0 += CG_WARPS) {
-            const TileLane t = tileLane(w, j0 + t0, true);
-            const I2 b = w.blockAt(t.n);
-            const I2 oc{b.x * BLOCK + ox, b.y * BLOCK + oy};
-            const bool oin = w.inWorld(oc);
-            const uint32_t oi = oin ? w.cellIndex(oc) : 0u;
-            const float oz = Z.pot[oi].x, op = Pold[oi];
-            float4 bb[2];
-            float z[2], po[2];
-            uint32_t mk[2];
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const uint32_t i = t.i[h];
-                mk[h] = Z.mask[i];
-                bb[h] = Z.b[i];
-                z[h] = Z.pot[i].x;
-                po[h] = Pold[i];
-            }
-            float p[2];
-            const int c0 = ((int)(lane >> 3) + 1) * RIM + (int)(lane & 7u) + 1;
-            sp[so] = dir(oz, op);
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                p[h] = dir(z[h], po[h]);
-                sp[c0 + 4 * RIM * h] = p[h];
-            }
-            __syncwarp();
-            float q[2];
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int c = c0 + 4 * RIM * h;
-                q[h] = 0.0f;
-                if (t.in[h] && (mk[h] & FM_LIQUID) != 0u) {
-                    float sum = 0.0f;
-                    if (mk[h] & 1u) sum = sum + bb[h].x * sp[c - 1];
-                    if (mk[h] & 2u) sum = sum + bb[h].y * sp[c + 1];
-                    if (mk[h] & 4u) sum = sum + bb[h].z * sp[c - RIM];
-                    if (mk[h] & 8u) sum = sum + bb[h].w * sp[c + RIM];
-                    const float dgp = diagOf(bb[h]) + ((mk[h] & FM_PIN) != 0u ? PIN : 0.0f);
-                    q[h] = dgp * p[h] - sum + 0.0f;
-                } else {
-                    p[h] = 0.0f;
-                }
-                if (t.in[h]) {
-                    Pnew[t.i[h]] = p[h];
-                    F.Q[t.i[h]] = q[h];
-                }
-            }
-            if (f64) {
-                const double x = warpTree((double)p[0] * (double)q[0], (double)p[1] * (double)q[1]);
-                if (lane == 0u) F.part64[t.n] = x;
-            } else {
-                const float x = warpTree(p[0] * q[0], p[1] * q[1]);
-                if (lane == 0u) F.part32[t.n] = x;
-            }
-            __syncwarp();  // the warp's p is free for its next tile
-        }
+#pragma unroll 1
+        for (uint32_t t = warp; t < m; t += CG_WARPS)
+            applyTile(D, F, w, j0 + t, odd, f64, beta, beta64, tp[warp], Parts{F.pq64, F.pq32});
         if (!countTiles(&D.st->fdone[2], m, na, [] {})) return;
         if (f64) {
             double v[1];
-            sumBlocksCg<double, 1>(D.B, F.part64, s64, v);
+            sumBlocksCg<double, 1, CG_THREADS>(D.B, F.pq64, s64, v);
             if (threadIdx.x == 0) {
                 D.st->pq = v[0];
                 D.st->alpha = v[0] <= 0.0 ? 0.0 : D.st->rz / v[0];
             }
         } else {
             float v[1];
-            sumBlocksCg<float, 1>(D.B, F.part32, reinterpret_cast<float*>(s64), v);
+            sumBlocksCg<float, 1, CG_THREADS>(D.B, F.pq32, reinterpret_cast<float*>(s64), v);
             if (threadIdx.x == 0) {
                 D.st->pq32 = v[0];
                 D.st->alpha32 = v[0] <= 0.0f ? 0.0f : D.st->rz32 / v[0];
             }
         }
     });
+}
+
+// cgUpdate's work (fluid.wgsl:2857-2880) on tiles j[0] and, when two, j[1],
+// with each tile's sum of r^2 when tol; the lane's largest |r| (bits of a
+// non-negative float).
+__device__ __forceinline__ uint32_t updateTiles(const Dev& D, const FastW& F, const W& w, const uint32_t (&j)[2], bool two,
+                                                const float* P, bool f64, bool tol, float alpha, double alpha64) {
+    const Fine& Z = F.Z;
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t most = 0u;
+    TileLane t[2];
+    uint32_t mk[2][2];
+    float vx[2][2], vy[2][2], vz[2][2], vw[2][2], py[2][2];
+#pragma unroll
+    for (int u = 0; u < 2; u++) t[u] = tileLane(w, j[u], u == 0 || two);
+#pragma unroll
+    for (int u = 0; u < 2; u++)
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const uint32_t i = t[u].i[h];
+            mk[u][h] = Z.mask[i];
+            vx[u][h] = F.X[i];
+            vy[u][h] = F.R[i];
+            vz[u][h] = P[i];
+            vw[u][h] = F.Q[i];
+            py[u][h] = Z.pot[i].y;
+        }
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+        if (u == 1 && !two) break;  // (warp-uniform)
+        double r2[2] = {0.0, 0.0};
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            if (!t[u].in[h] || (mk[u][h] & FM_LIQUID) == 0u) continue;
+            const uint32_t i = t[u].i[h];
+            float r, x;
+            if (f64) {
+                r = (float)((double)vy[u][h] - alpha64 * (double)vw[u][h]);
+                x = (float)((double)vx[u][h] + alpha64 * (double)vz[u][h]);
+            } else {
+                r = vy[u][h] - alpha * vw[u][h];
+                x = vx[u][h] + alpha * vz[u][h];
+            }
+            F.X[i] = x;
+            F.R[i] = r;
+            Z.pot[i].x = 0.0f;
+            Z.rim[i] = make_float2(0.0f, py[u][h]);
+            most = max(most, __float_as_uint(fabsf(r)));
+            r2[h] = (double)r * (double)r;
+        }
+        if (tol) {
+            const double v = warpTree(r2[0], r2[1]);
+            if (lane == 0u) D.norm64[t[u].n] = v;
+        }
+    }
+    return most;
 }
 
 // cgUpdate (fluid.wgsl:2852-2880), the tolerance form's norm, and the loop's
@@ -2075,55 +2085,12 @@ __global__ void __launch_bounds__(CG_THREADS, 2) k_fUpdate(Batch Bt, const __gri
         const bool f64 = D.st->f64 != 0u, tol = D.st->tol_mode != 0u;
         const float alpha = D.st->alpha32;
         const double alpha64 = D.st->alpha;
-        const Fine& Z = F.Z;
         const float* P = (cycle & 1u) ? F.P : F.P2;
         uint32_t most = 0u;
-        for (uint32_t t0 = warp; t0 < m; t0 += 2u * CG_WARPS) {
-            TileLane t[2];
-            uint32_t mk[2][2];
-            float vx[2][2], vy[2][2], vz[2][2], vw[2][2], py[2][2];
-#pragma unroll
-            for (int u = 0; u < 2; u++) t[u] = tileLane(w, j0 + t0 + (uint32_t)u * CG_WARPS, t0 + (uint32_t)u * CG_WARPS < m);
-#pragma unroll
-            for (int u = 0; u < 2; u++)
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const uint32_t i = t[u].i[h];
-                    mk[u][h] = Z.mask[i];
-                    vx[u][h] = F.X[i];
-                    vy[u][h] = F.R[i];
-                    vz[u][h] = P[i];
-                    vw[u][h] = F.Q[i];
-                    py[u][h] = Z.pot[i].y;
-                }
-#pragma unroll
-            for (int u = 0; u < 2; u++) {
-                if (t0 + (uint32_t)u * CG_WARPS >= m) break;  // (warp-uniform)
-                double r2[2] = {0.0, 0.0};
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    if (!t[u].in[h] || (mk[u][h] & FM_LIQUID) == 0u) continue;
-                    const uint32_t i = t[u].i[h];
-                    float r, x;
-                    if (f64) {
-                        r = (float)((double)vy[u][h] - alpha64 * (double)vw[u][h]);
-                        x = (float)((double)vx[u][h] + alpha64 * (double)vz[u][h]);
-                    } else {
-                        r = vy[u][h] - alpha * vw[u][h];
-                        x = vx[u][h] + alpha * vz[u][h];
-                    }
-                    F.X[i] = x;
-                    F.R[i] = r;
-                    Z.pot[i].x = 0.0f;
-                    Z.rim[i] = make_float2(0.0f, py[u][h]);
-                    most = max(most, __float_as_uint(fabsf(r)));
-                    r2[h] = (double)r * (double)r;
-                }
-                if (tol) {
-                    const double v = warpTree(r2[0], r2[1]);
-                    if (lane == 0u) D.norm64[t[u].n] = v;
-                }
-            }
+#pragma unroll 1
+        for (uint32_t t = warp; t < m; t += 2u * CG_WARPS) {
+            const uint32_t j[2] = {j0 + t, j0 + t + CG_WARPS};
+            most = max(most, updateTiles(D, F, w, j, t + CG_WARPS < m, P, f64, tol, alpha, alpha64));
         }
         // the run's largest |r| into the world's residual slot (a max of
         // maxima: the same word), before its tiles are counted
@@ -2136,7 +2103,7 @@ __global__ void __launch_bounds__(CG_THREADS, 2) k_fUpdate(Batch Bt, const __gri
             }))
             return;
         double rr[1] = {0.0};
-        if (tol) sumBlocksCg<double, 1>(D.B, D.norm64, s64, rr);
+        if (tol) sumBlocksCg<double, 1, CG_THREADS>(D.B, D.norm64, s64, rr);
         if (threadIdx.x == 0) {
             bool conv;
             if (tol) {
@@ -2186,83 +2153,89 @@ __device__ __forceinline__ double trueResidualAt(const Dev& D, const FastW& F, I
     return -((double)D.field[8u * (size_t)i + 1u] + ax);
 }
 
-// The mixed form's guard, over the worlds k_fUpdate flagged: the FP64 norm
-// of the true residual and of the FP32 rounding floor; when the true one
-// has drifted above twice the recursive one plus four floors (the
-// low-precision preconditioner's rounding lost the recursion's accuracy),
-// the world goes on with the true residual put in (k_fTrueFix), else it
-// stops or goes on as k_fUpdate decided.
-template <bool ONE>
-__global__ void __launch_bounds__(256) k_fTrueCheck(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
-    __shared__ WorldCopy wc_;
-    if (!ONE) worldCopyInit(wc_);
-    __shared__ double s64[256], s64b[256];
-    uint32_t pend_ = 0;
-    FOR_ITEMS(Bt, L_ACT4, it) {
-        FAST_ITEM(Bt, it, D, F, w, g);
-        if (D.st->check == 0u) continue;
-        const Fine& Z = F.Z;
-        const uint32_t na = w.activeCount();
-        const uint32_t wid = g * 4u + (threadIdx.x >> 6);
-        const bool valid = wid < na;
-        double r2 = 0.0, f2 = 0.0;
-        if (valid) {
-            I2 c = tileCell(w, wid);
-            if (w.inWorld(c)) {
-                const uint32_t i = w.cellIndex(c);
-                if ((Z.mask[i] & FM_LIQUID) != 0u) {
-                    const double r = trueResidualAt(D, F, c, i, &f2);
-                    r2 = r * r;
-                }
-            }
+// A tile's sums of the squares of its cells' true residuals and floors, of
+// block b at b and B + b of out.
+__device__ __forceinline__ void trueCheckTile(const Dev& D, const FastW& F, const W& w, uint32_t j, double* out) {
+    const TileLane t = tileLane(w, j, true);
+    double r2[2] = {0.0, 0.0}, f2[2] = {0.0, 0.0};
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+        if (t.in[h] && (F.Z.mask[t.i[h]] & FM_LIQUID) != 0u) {
+            const double r = trueResidualAt(D, F, I2{t.x, t.y[h]}, t.i[h], &f2[h]);
+            r2[h] = r * r;
         }
-        const double t2 = tree64x4(s64, r2);
-        const double u2 = tree64x4(s64, f2);
-        if (valid && (threadIdx.x & 63u) == 0u) {
-            const uint32_t b = w.blockIndex(w.activeBlock(wid));
-            D.norm64[b] = t2;
-            D.norm64[D.B + b] = u2;
-        }
-        pend_ += min(4u, na - g * 4u);
-        if (flushTiles(Bt, g_it, e_it, it, pend_, &D.st->fdone[4], na)) {
-            double rr, ff;
-            sumBlocks256x2(w, D.norm64, s64, s64b, &rr, &ff);
-            if (threadIdx.x == 0) {
-                const double bn = D.st->bnorm2;
-                const double rel = bn > 0.0 ? sqrt(rr / bn) : 0.0, flo = bn > 0.0 ? sqrt(ff / bn) : 0.0;
-                D.st->rel_true = rel;
-                D.st->check = 0u;
-                if (rel > 2.0 * D.st->rel + 4.0 * flo) {
-                    D.st->drift = 1u;
-                    if (Bt.cond_drift) cudaGraphSetConditional(Bt.cond_drift, 1u);
-                    const uint32_t cont = D.st->cycle < Bt.max_cycles ? 1u : 0u;
-                    D.st->cont = cont;
-                    if (cont) {
-                        *Bt.loop = 1u;
-                        if (Bt.cond) cudaGraphSetConditional(Bt.cond, 1u);
-                    }
-                }
-            }
-        }
+    const double t2 = warpTree(r2[0], r2[1]), u2 = warpTree(f2[0], f2[1]);
+    if ((threadIdx.x & 31u) == 0u) {
+        out[t.n] = t2;
+        out[D.B + t.n] = u2;
     }
 }
+// The true residual's norm and the floor's, relative to b's; and whether the
+// true one has drifted above twice the recursive one plus four floors (the
+// low-precision preconditioner's rounding lost the recursion's accuracy).
+__device__ __forceinline__ void trueRel(double rr, double ff, double bn, double* rel, double* flo) {
+    *rel = bn > 0.0 ? sqrt(rr / bn) : 0.0;
+    *flo = bn > 0.0 ? sqrt(ff / bn) : 0.0;
+}
+__device__ __forceinline__ bool drifted(double rel_true, double rel, double flo) { return rel_true > 2.0 * rel + 4.0 * flo; }
+// The true residual put in for the recursive one.
+__device__ __forceinline__ void trueFixTile(const Dev& D, const FastW& F, const W& w, uint32_t j) {
+    const TileLane t = tileLane(w, j, true);
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+        if (t.in[h] && (F.Z.mask[t.i[h]] & FM_LIQUID) != 0u) {
+            double f2;
+            F.R[t.i[h]] = (float)trueResidualAt(D, F, I2{t.x, t.y[h]}, t.i[h], &f2);
+        }
+}
 
-// The true residual put in for the recursive one, for the worlds k_fTrueCheck found drifted.
+// The mixed form's guard, over the worlds k_fUpdate flagged: a world whose
+// true residual has drifted goes on with it put in (k_fTrueFix), else it
+// stops or goes on as k_fUpdate decided.
 template <bool ONE>
-__global__ void k_fTrueFix(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
+__global__ void __launch_bounds__(CG_THREADS, 2) k_fTrueCheck(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
     if (!ONE) worldCopyInit(wc_);
-    FOR_ITEMS(Bt, L_ACT, it) {
-        FAST_ITEM(Bt, it, D, F, w, wid);
-        if (D.st->drift == 0u) continue;
-        const Fine& Z = F.Z;
-        I2 c = lidCell(w, wid);
-        if (!w.inWorld(c)) continue;
-        const uint32_t i = w.cellIndex(c);
-        if ((Z.mask[i] & FM_LIQUID) == 0u) continue;
-        double f2;
-        F.R[i] = (float)trueResidualAt(D, F, c, i, &f2);
-    }
+    __shared__ double s64[512];
+    forTileRuns<ONE>(Bt, src, wc_, [&](const World& Wd, uint32_t na, uint32_t j0, uint32_t m) {
+        const Dev& D = Wd.D;
+        const W w(D);
+        if (D.st->check == 0u) return;
+#pragma unroll 1
+        for (uint32_t t = threadIdx.x >> 5; t < m; t += CG_WARPS) trueCheckTile(D, Wd.S, w, j0 + t, Wd.S.part64);
+        if (!countTiles(&D.st->fdone[4], m, na, [] {})) return;
+        double v[2];
+        sumBlocksCg<double, 2, CG_THREADS>(D.B, Wd.S.part64, s64, v);
+        if (threadIdx.x == 0) {
+            double rel, flo;
+            trueRel(v[0], v[1], D.st->bnorm2, &rel, &flo);
+            D.st->rel_true = rel;
+            D.st->check = 0u;
+            if (drifted(rel, D.st->rel, flo)) {
+                D.st->drift = 1u;
+                if (Bt.cond_drift) cudaGraphSetConditional(Bt.cond_drift, 1u);
+                const uint32_t cont = D.st->cycle < Bt.max_cycles ? 1u : 0u;
+                D.st->cont = cont;
+                if (cont) {
+                    *Bt.loop = 1u;
+                    if (Bt.cond) cudaGraphSetConditional(Bt.cond, 1u);
+                }
+            }
+        }
+    });
+}
+
+// The worlds k_fTrueCheck found drifted.
+template <bool ONE>
+__global__ void __launch_bounds__(CG_THREADS, 2) k_fTrueFix(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
+    __shared__ WorldCopy wc_;
+    if (!ONE) worldCopyInit(wc_);
+    forTileRuns<ONE>(Bt, src, wc_, [&](const World& Wd, uint32_t na, uint32_t j0, uint32_t m) {
+        const W w(Wd.D);
+        if (Wd.D.st->drift == 0u) return;
+#pragma unroll 1
+        for (uint32_t t = threadIdx.x >> 5; t < m; t += CG_WARPS) trueFixTile(Wd.D, Wd.S, w, j0 + t);
+    });
 }
 
 // An iteration's start: the loop stops unless a world's k_fUpdate says
@@ -2301,7 +2274,7 @@ __global__ void k_fLoopStart(Batch Bt) {
 // iterations the reference still dispatches would clear (cgUpdate's first
 // lines run whether or not the iteration is skipped).
 template <bool ONE>
-__global__ void k_fFinish(Batch Bt, const __grid_constant__ WorldSrc<ONE> src, int two_p) {
+__global__ void k_fFinish(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
     if (!ONE) worldCopyInit(wc_);
     if (threadIdx.x == 0) {
@@ -2323,162 +2296,156 @@ __global__ void k_fFinish(Batch Bt, const __grid_constant__ WorldSrc<ONE> src, i
         if ((Z.mask[i] & FM_LIQUID) != 0u) f[1] = -F.R[i];
         w.fv(2u * i + 1u)[0] = Z.pot[i].y;
         // the last iteration's p: P2 after an odd number of iterations
-        const float* P = (two_p && (D.st->cycle & 1u)) ? F.P2 : F.P;
+        const float* P = (D.st->cycle & 1u) ? F.P2 : F.P;
         reinterpret_cast<float4*>(D.cg)[i] = make_float4(F.X[i], F.R[i], P[i], F.Q[i]);
         *w.gwp(i, G_REGION) = 0u;
     }
 }
 
 
-// ================================================================ the persistent solve
+// ================================================================ one world's solve in one launch
 //
-// All the iterations of a step's solve in one cooperative launch: each
-// reference pass of an iteration is a phase, every CTA taking its share of
-// the phase's cells or tiles, the phases separated by a grid barrier; the
-// levels of at most 1024 cells are CTA 0's, in its shared memory; the block
-// sums are finished by CTA 0 after the barrier.  Same cells, same values,
-// same order of every sum as the passes.
+// All the iterations of a single world's solve in one kernel, by a group of
+// CTAs: each pass of an iteration is a phase, every warp (or half CTA)
+// taking its share of the phase's tiles, the phases separated by the
+// group's barrier; the coarse levels are CTA 0's, in its shared memory.
+// Same tiles, same values, same order of every sum as the passes' kernels.
+//
+// Why: an iteration is 14 to 16 launches, each of which costs about 2.5 us
+// between kernels in the step's graph and starts by loading what the last
+// one knew (its world's state, its list's length): on small worlds most of
+// the solve, on a 1024x1024 world 50 of its 185 us an iteration.  A barrier
+// among the CTAs of a cluster is under 1 us, among those of a grid about
+// 1.5 us.
+constexpr int SOLVE_THREADS = 1024, SOLVE_WARPS = SOLVE_THREADS / 32, TEAM = SOLVE_THREADS / 2;
 
-// A grid barrier (all CTAs are resident: cooperative launch).  Each wait is
-// bounded: past g_spin_limit polls it records ERR_BARRIER and every CTA
-// returns false from here on.
-__device__ bool gridBarrier(StepState* st, uint32_t nblocks) {
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile uint32_t* gen = &st->bar_gen;
-        const uint32_t g0 = *gen;
-        __threadfence();
-        const uint32_t arrived = atomicAdd(&st->bar_count, 1u) + 1u;
-        int ok = 1;
-        if (arrived == nblocks) {
-            atomicExch(&st->bar_count, 0u);
-            __threadfence();
-            atomicAdd(&st->bar_gen, 1u);
-        } else {
-            uint32_t it = 0;
+// The CTAs of one cluster.
+struct ClusterGroup {
+    uint32_t rank, n;
+    __device__ explicit ClusterGroup(StepState*)
+        : rank(cooperative_groups::this_cluster().block_rank()), n(cooperative_groups::this_cluster().num_blocks()) {}
+    __device__ __forceinline__ bool sync() {
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+        return true;
+    }
+};
+
+// The CTAs of a cooperative launch (all resident): arrivals counted up in
+// the world's StepState, the k-th barrier passed at k n of them.  Each wait
+// is bounded: past g_spin_limit polls a CTA records ERR_BARRIER, raises the
+// count past any barrier's, and every CTA returns false from here on.
+struct GridGroup {
+    StepState* st;
+    uint32_t rank, n, target;
+    __device__ explicit GridGroup(StepState* s) : st(s), rank(blockIdx.x), n(gridDim.x), target(0u) {}
+    __device__ bool sync() {
+        constexpr uint32_t GAVE_UP = 1u << 30;
+        __shared__ int s_ok;
+        target += n;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            uint32_t v, it = 0;
             const uint32_t limit = g_spin_limit;
-            while (*gen == g0) {
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&st->bar_count) : "memory");
+            while (true) {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&st->bar_count) : "memory");
+                if (v >= target) break;
                 if (++it > limit) {
                     atomicOr(&st->err, ERR_BARRIER);
-                    ok = 0;
+                    atomicAdd(&st->bar_count, GAVE_UP);
+                    v = GAVE_UP;
                     break;
                 }
-                __nanosleep(64);
+            }
+            s_ok = v < GAVE_UP ? 1 : 0;
+        }
+        __syncthreads();
+        return s_ok != 0;
+    }
+};
+
+// A world of more blocks has its block sums' columns shared by the group's
+// CTAs (a warp a column) and a barrier more; below, every CTA sums them all
+// itself (a round of loads for 4096 blocks, about 1 us).
+constexpr uint32_t SPLIT_BLOCKS = 8192;
+
+// sumBlocks of NC components of the partials, for every CTA of the group
+// (all its threads): the sums in s[256 c].  col: 512 values of scratch.
+template <class T, int NC, class Group>
+__device__ __forceinline__ bool groupSums(Group& g, uint32_t B, const T* part, T* s, float* sm, double* col64) {
+    if (B <= SPLIT_BLOCKS) {
+        sumColumns<T, NC, SOLVE_THREADS>(B, part, s);
+        treeColumns<T, NC>(s);
+        return true;
+    }
+    T* col = reinterpret_cast<T*>(col64);
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t id = g.rank + g.n * warp;
+    if (id < 256u * NC) {
+        constexpr uint32_t ROWS = 256u;
+        T* rows = reinterpret_cast<T*>(sm) + ROWS * warp;
+        const T* at = part + (size_t)B * (id >> 8);
+        const uint32_t li = id & 255u;
+        T acc = T(0);
+        for (uint32_t r0 = 0; r0 * 256u < B; r0 += ROWS) {
+            T v[ROWS / 32u];
+#pragma unroll
+            for (uint32_t u = 0; u < ROWS / 32u; u++) {
+                const uint32_t k = (r0 + lane + 32u * u) * 256u + li;
+                v[u] = k < B ? __ldcg(at + k) : T(0);
+            }
+            __syncwarp();
+#pragma unroll
+            for (uint32_t u = 0; u < ROWS / 32u; u++) rows[lane + 32u * u] = v[u];
+            __syncwarp();
+            if (lane == 0u) {
+                const uint32_t m = min(ROWS, (B + 255u) / 256u - r0);  // (the rest are +0)
+#pragma unroll 8
+                for (uint32_t k = 0; k < m; k++) acc = acc + rows[k];
             }
         }
-        __threadfence();
-        if ((vld(&st->err) & ERR_BARRIER) != 0u) ok = 0;
-        s_ok = ok;
+        if (lane == 0u) col[id] = acc;
     }
-    __syncthreads();
-    return s_ok != 0;
+    if (!g.sync()) return false;
+    for (uint32_t k = threadIdx.x; k < 256u * NC; k += SOLVE_THREADS) s[k] = __ldcg(col + k);
+    treeColumns<T, NC>(s);
+    return true;
 }
 
-// relaxTile (fluid.wgsl:2109-2182), four tiles a 256-thread CTA.
-__device__ void relaxGroups(const Fast& F, const W& w, int shift, float (*tpx)[RIM * RIM], float (*tpy)[RIM * RIM],
-                            int* s_live, int* s_ox, int* s_oy) {
-    const Dev& D = F.D;
-    const Fine& Z = F.Z;
-    const uint32_t na = w.activeCount();
-    const uint32_t total = na + (shift ? D.edge_tiles : 0u);
-    const int q = (int)(threadIdx.x >> 6), lane = (int)(threadIdx.x & 63u);
-    for (uint32_t g = blockIdx.x; g * 4u < total; g += gridDim.x) {
-        const uint32_t j = g * 4u + (uint32_t)q;
-        if (lane == 0) {
-            int live = 0, ox = 0, oy = 0;
-            if (j < total) {
-                uint32_t wid = j < na ? j : D.B + (j - na);
-                I2 b = tileBlockF(w, wid, shift);
-                ox = b.x * BLOCK - shift;
-                oy = b.y * BLOCK - shift;
-                if (b.x >= 0 && ox < D.W && oy < D.H)
-                    live = (int)(w.statesOf(I2{ox / BLOCK, oy / BLOCK}, I2{(ox + BLOCK - 1) / BLOCK, (oy + BLOCK - 1) / BLOCK}) & HAS_FLUID);
-            }
-            s_live[q] = live;
-            s_ox[q] = ox;
-            s_oy[q] = oy;
-        }
-        __syncthreads();
-        const bool live = s_live[q] != 0;
-        const int ox = s_ox[q], oy = s_oy[q];
-        if (live) {
-            for (int k = lane; k < RIM * RIM; k += 64) {
-                I2 c{ox - 1 + k % RIM, oy - 1 + k / RIM};
-                float px = 0.0f, py = 0.0f;
-                if (w.inWorld(c)) {
-                    uint32_t i = w.cellIndex(c);
-                    const float2 v = __ldcg(&Z.rim[i]);
-                    px = v.x;
-                    py = v.y;
-                }
-                tpx[q][k] = px;
-                tpy[q][k] = py;
-            }
-        }
-        __syncthreads();
-        const int lx = lane & 7, ly = lane >> 3;
-        const I2 me{ox + lx, oy + ly};
-        const int t = (ly + 1) * RIM + lx + 1;
-        float rx = 0.0f, ry = 0.0f, bx = 0.0f, by = 0.0f, bz = 0.0f, bw = 0.0f, diag = 0.0f, pinv = 0.0f;
-        uint32_t idx = 0;
-        bool fluid = false;
-        if (live && w.inWorld(me)) {
-            idx = w.cellIndex(me);
-            fluid = (Z.mask[idx] & FM_LIQUID) != 0u;
-        }
-        if (fluid) {
-            rx = -__ldcg(&F.R[idx]);
-            ry = Z.ry[idx];
-            const float4 b4 = Z.b[idx];
-            bx = b4.x;
-            by = b4.y;
-            bz = b4.z;
-            bw = b4.w;
-            diag = diagOf(b4);
-            pinv = (Z.mask[idx] & FM_PIN) != 0u ? PIN : 0.0f;
-        }
-        const float dx = diag + pinv, dy = fmaxf(diag, 1e-30f);
-        const bool solving = fluid && dx > 0.0f;
-        const int color = (me.x + me.y) & 1;
-        for (int sw = 0; sw < 2 * SWEEPS; sw++) {
-            if (solving && color == (sw & 1)) {
-                float sx = bx * tpx[q][t - 1] + by * tpx[q][t + 1] + bz * tpx[q][t - RIM] + bw * tpx[q][t + RIM];
-                float sy = bx * tpy[q][t - 1] + by * tpy[q][t + 1] + bz * tpy[q][t - RIM] + bw * tpy[q][t + RIM];
-                float nx = mixf(tpx[q][t], (sx - rx) / dx, SMOOTH_OMEGA);
-                float ny = mixf(tpy[q][t], (sy - ry) / dy, SMOOTH_OMEGA);
-                tpx[q][t] = nx;
-                if (diag > 0.0f) tpy[q][t] = ny;
-            }
-            __syncthreads();
-        }
-        if (solving) {
-            Z.pot[idx] = make_float2(tpx[q][t], tpy[q][t]);
-        }
-        __syncthreads();
-    }
-}
+// The columns' warps must be there: 32 a CTA, so 16 CTAs of a group that
+// splits.
+constexpr uint32_t SPLIT_CTAS = 16;
 
-__global__ void __launch_bounds__(256, 4) k_fSolve(Fast F, int shifted) {
-    extern __shared__ float sm_coarse[];
-    __shared__ float tpx[4][RIM * RIM], tpy[4][RIM * RIM];
-    __shared__ int s_live[4], s_ox[4], s_oy[4];
-    __shared__ float sx[256], sy[256];
-    __shared__ double s64[256];
-    __shared__ uint32_t most[4];
+template <class Group, class T>
+__global__ void __launch_bounds__(SOLVE_THREADS, 1) k_fSolve(const __grid_constant__ World Wd, uint32_t max_cycles) {
+    extern __shared__ __align__(16) float sm[];
+    __shared__ double s64[512];
     __shared__ uint32_t s_off[WIG_MG_LEVELS + 1];
-    const Dev& D = F.D;
-    W w(D);
+    __shared__ uint32_t s_most;
+    const Dev& D = Wd.D;
+    const FastW& F = Wd.S;
+    const W w(D);
     StepState* st = D.st;
-    const uint32_t nb = gridDim.x;
-    const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x, gn = gridDim.x * blockDim.x;
+    Group g(st);
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const bool f64 = st->f64 != 0u, tol = st->tol_mode != 0u;
-    const uint32_t na = w.activeCount();
-    const uint32_t lp = F.lp;
-    const Fine& Z = F.Z;
+    const double tolerance = st->tol, bnorm2 = st->bnorm2;
+    const uint32_t shift_first = st->shift_first & 1u;
+    const uint32_t na = w.activeCount(), lc = F.lc;
+    float* s32 = reinterpret_cast<float*>(s64);
+    // the group's first warp of a phase over tiles, and its stride
+    const uint32_t w0 = g.rank * SOLVE_WARPS + warp, wn = g.n * SOLVE_WARPS;
+    const Team<TEAM> tm{(int)(tid % TEAM), 2 + (int)(tid / TEAM)};
+    LevelTile& lt = reinterpret_cast<LevelTile*>(sm)[tid / TEAM];
+    const uint32_t t0 = g.rank + g.n * (tid / TEAM), tn = 2u * g.n;
+    if (tid == 0u) s_most = 0u;
+    double rz = 0.0, pq = 0.0, rel = 1.0, rel_true = 0.0;
+    float rz32 = 0.0f, pq32 = 0.0f;
+    uint32_t cycle = 0;
     if (na == 0u) {
         // nothing to solve: the first iteration counted, as cgUpdate counts it
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (g.rank == 0u && tid == 0u) {
             D.blocks[w.countSlot(COUNT_RESIDUAL + 1u)] = 0u;
             D.blocks[w.countSlot(COUNT_CYCLES)] += 1u;
             st->cycle = 1u;
@@ -2486,263 +2453,136 @@ __global__ void __launch_bounds__(256, 4) k_fSolve(Fast F, int shifted) {
         }
         return;
     }
-    for (uint32_t cycle = 0; cycle < F.max_cycles; cycle++) {
-        // relax (relaxRims's snapshot is the scratch's rims)
-        relaxGroups(F, w, shifted ? BLOCK / 2 : 0, tpx, tpy, s_live, s_ox, s_oy);
-        if (!gridBarrier(st, nb)) return;
-        for (uint32_t l = 1; l < lp; l++) {
-            const uint32_t n = D.level_w[l] * D.level_h[l];
-            for (uint32_t j = gt; j < n; j += gn) {
-                if (l == 1u) restrictCell<float, true>(F.D, F, w, l, j);
-                else restrictCell<float, false>(F.D, F, w, l, j);
-            }
-            if (!gridBarrier(st, nb)) return;
-            for (int color = 0; color < 2; color++) {
-                for (uint32_t j = gt; j < n; j += gn) smoothCell(F.D, F, l, color, cycle == 0u, j);
-                if (!gridBarrier(st, nb)) return;
-            }
-        }
-        {
-            const uint32_t n = D.level_w[lp] * D.level_h[lp];
-            for (uint32_t j = gt; j < n; j += gn) {
-                if (lp == 1u) restrictCell<float, true>(F.D, F, w, lp, j);
-                else restrictCell<float, false>(F.D, F, w, lp, j);
-            }
-            if (!gridBarrier(st, nb)) return;
-        }
-        if (blockIdx.x == 0) coarseLevels(F.D, F, w, lp, sm_coarse, s_off, false);
-        if (!gridBarrier(st, nb)) return;
-        for (uint32_t l = lp - 1; l >= 1; l--) {
-            const uint32_t n = D.level_w[l] * D.level_h[l];
-            for (uint32_t j = gt; j < n; j += gn) prolongCell(F.D, F, l, j);
-            if (!gridBarrier(st, nb)) return;
-            for (int color = 0; color < 2; color++) {
-                for (uint32_t j = gt; j < n; j += gn) smoothCell(F.D, F, l, color, false, j);
-                if (!gridBarrier(st, nb)) return;
-            }
-        }
-        // prolongFine, and the rims of the relaxation after
-        for (uint32_t t = gt; t < na * 64u; t += gn) {
-            const uint32_t wid = t >> 6, lane = t & 63u;
-            I2 b = w.activeBlock(wid);
-            I2 c{b.x * BLOCK + (int)(lane & 7u), b.y * BLOCK + (int)(lane >> 3)};
-            if (!w.inWorld(c)) continue;
-            uint32_t i = w.cellIndex(c);
-            if ((Z.mask[i] & FM_LIQUID) != 0u) {
-                const Lvl& U = F.L[1];
-                V2 e = prolongedFrom(U.rho, U.px, U.py, (int)D.level_w[1], (int)D.level_h[1], c.x, c.y);
-                const float2 p = Z.pot[i], v = make_float2(p.x + e.x, p.y + e.y);
-                Z.pot[i] = v;
-                Z.rim[i] = v;
-            }
-        }
-        if (!gridBarrier(st, nb)) return;
-        relaxGroups(F, w, shifted ? 0 : BLOCK / 2, tpx, tpy, s_live, s_ox, s_oy);
-        if (!gridBarrier(st, nb)) return;
-        // cgRho
-        for (uint32_t g = blockIdx.x; g * 4u < na; g += gridDim.x) {
-            const uint32_t wid = g * 4u + (threadIdx.x >> 6);
-            const bool valid = wid < na;
-            float vx = 0.0f, vy = 0.0f;
-            double ex = 0.0, ey = 0.0;
-            if (valid) {
-                I2 c = tileCell(w, wid);
-                if (w.inWorld(c)) {
-                    uint32_t i = w.cellIndex(c);
-                    if ((Z.mask[i] & FM_LIQUID) != 0u) {
-                        float z = Z.pot[i].x;
-                        float r = F.R[i], q = F.Q[i];
-                        vx = r * z;
-                        vy = q * z;
-                        ex = (double)r * (double)z;
-                        ey = (double)q * (double)z;
-                    }
-                }
-            }
-            float tx = tree64x4(sx, vx);
-            float ty = tree64x4(sy, vy);
-            double dx = 0.0, dy = 0.0;
-            if (f64) {
-                dx = tree64x4(s64, ex);
-                dy = tree64x4(s64, ey);
-            }
-            if (valid && (threadIdx.x & 63u) == 0u) {
-                const uint32_t b = w.blockIndex(w.activeBlock(wid));
-                F.part32[b] = tx;
-                F.part32[D.B + b] = ty;
-                if (f64) {
-                    F.part64[b] = dx;
-                    F.part64[D.B + b] = dy;
-                }
-            }
-        }
-        if (!gridBarrier(st, nb)) return;
-        // cgBeta
-        if (blockIdx.x == 0) {
-            if (f64) {
-                double rz = sumBlocks256(w, F.part64, 0, s64);
-                double zq = sumBlocks256(w, F.part64, 1, s64);
-                if (threadIdx.x == 0) {
-                    double pq = vldd(&st->pq);
-                    st->rz = rz;
-                    st->beta = (cycle == 0u || pq <= 0.0) ? 0.0 : -zq / pq;
-                }
-            } else {
-                float rz = sumBlocks256(w, F.part32, 0, sx);
-                float zq = sumBlocks256(w, F.part32, 1, sx);
-                if (threadIdx.x == 0) {
-                    float pq = vldf(&st->pq32);
-                    st->rz32 = rz;
-                    st->beta32 = (cycle == 0u || pq <= 0.0f) ? 0.0f : -zq / pq;
-                }
-            }
-        }
-        if (!gridBarrier(st, nb)) return;
-        // cgDirection
-        {
-            const float beta = vldf(&st->beta32);
-            const double beta64 = vldd(&st->beta);
-            for (uint32_t t = gt; t < na * 64u; t += gn) {
-                const uint32_t wid = t >> 6, lane = t & 63u;
-                I2 b = w.activeBlock(wid);
-                I2 c{b.x * BLOCK + (int)(lane & 7u), b.y * BLOCK + (int)(lane >> 3)};
-                if (!w.inWorld(c)) continue;
-                uint32_t i = w.cellIndex(c);
-                float p = 0.0f;
-                if ((Z.mask[i] & FM_LIQUID) != 0u) {
-                    float z = Z.pot[i].x;
-                    p = f64 ? (float)((double)z + beta64 * (double)F.P[i]) : z + beta * F.P[i];
-                }
-                F.P[i] = p;
-            }
-        }
-        if (!gridBarrier(st, nb)) return;
-        // cgApply
-        for (uint32_t g = blockIdx.x; g * 4u < na; g += gridDim.x) {
-            const uint32_t wid = g * 4u + (threadIdx.x >> 6);
-            const bool valid = wid < na;
-            float vx = 0.0f;
-            double ex = 0.0;
-            if (valid) {
-                I2 c = tileCell(w, wid);
-                if (w.inWorld(c)) {
-                    uint32_t i = w.cellIndex(c);
-                    float q = 0.0f;
-                    const float p = __ldcg(&F.P[i]);
-                    if ((Z.mask[i] & FM_LIQUID) != 0u) {
-                        const uint32_t m = Z.mask[i];
-                        const float4 b4 = Z.b[i];
-                        const float bb[4] = {b4.x, b4.y, b4.z, b4.w};
-                        float sum = 0.0f;
-#pragma unroll
-                        for (int d = 0; d < 4; d++)
-                            if (m & (1u << d)) sum = sum + bb[d] * __ldcg(&F.P[nbr(i, c.x, c.y, D.W, D.H, d)]);
-                        float dg = diagOf(b4) + ((m & FM_PIN) != 0u ? PIN : 0.0f);
-                        q = dg * p - sum + 0.0f;
-                    }
-                    F.Q[i] = q;
-                    vx = p * q;
-                    ex = (double)p * (double)q;
-                }
-            }
-            float tx = tree64x4(sx, vx);
-            double dx = 0.0;
-            if (f64) dx = tree64x4(s64, ex);
-            if (valid && (threadIdx.x & 63u) == 0u) {
-                const uint32_t b = w.blockIndex(w.activeBlock(wid));
-                F.part32[b] = tx;
-                F.part32[D.B + b] = 0.0f;
-                if (f64) {
-                    F.part64[b] = dx;
-                    F.part64[D.B + b] = 0.0;
-                }
-            }
-        }
-        if (!gridBarrier(st, nb)) return;
-        // cgAlpha
-        if (blockIdx.x == 0) {
-            if (f64) {
-                double pq = sumBlocks256(w, F.part64, 0, s64);
-                if (threadIdx.x == 0) {
-                    st->pq = pq;
-                    st->alpha = pq <= 0.0 ? 0.0 : vldd(&st->rz) / pq;
-                }
-            } else {
-                float pq = sumBlocks256(w, F.part32, 0, sx);
-                if (threadIdx.x == 0) {
-                    st->pq32 = pq;
-                    st->alpha32 = pq <= 0.0f ? 0.0f : vldf(&st->rz32) / pq;
-                }
-            }
-        }
-        if (!gridBarrier(st, nb)) return;
-        // cgUpdate (its first lines: the next slot cleared, the iteration counted)
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
+    for (bool more = true; more;) {
+        if (g.rank == 0u && tid == 0u) {
+            // cgUpdate's first lines: the next slot cleared, the iteration counted
             D.blocks[w.countSlot(COUNT_RESIDUAL + (cycle + 1u) % 3u)] = 0u;
             D.blocks[w.countSlot(COUNT_CYCLES)] += 1u;
         }
-        {
-            const float alpha = vldf(&st->alpha32);
-            const double alpha64 = vldd(&st->alpha);
-            for (uint32_t g = blockIdx.x; g * 4u < na; g += gridDim.x) {
-                const uint32_t wid = g * 4u + (threadIdx.x >> 6);
-                const bool valid = wid < na;
-                if ((threadIdx.x & 63u) == 0u) most[threadIdx.x >> 6] = 0u;
-                __syncthreads();
-                double r2 = 0.0;
-                if (valid) {
-                    I2 c = tileCell(w, wid);
-                    if (w.inWorld(c)) {
-                        uint32_t i = w.cellIndex(c);
-                        if ((Z.mask[i] & FM_LIQUID) != 0u) {
-                            float vx = F.X[i], vy = F.R[i], vz = __ldcg(&F.P[i]), vw = __ldcg(&F.Q[i]);
-                            float r, x;
-                            if (f64) {
-                                r = (float)((double)vy - alpha64 * (double)vw);
-                                x = (float)((double)vx + alpha64 * (double)vz);
-                            } else {
-                                r = vy - alpha * vw;
-                                x = vx + alpha * vz;
-                            }
-                            F.X[i] = x;
-                            F.R[i] = r;
-                            const float py = __ldcg(&Z.pot[i]).y;
-                            Z.pot[i].x = 0.0f;
-                            Z.rim[i] = make_float2(0.0f, py);
-                            atomicMax(&most[threadIdx.x >> 6], __float_as_uint(fabsf(r)));
-                            r2 = (double)r * (double)r;
-                        }
-                    }
+        float2* rim = reinterpret_cast<float2*>(sm) + RIM * RXS * warp;
+#pragma unroll 1
+        for (uint32_t half = 0; half < 2u; half++) {
+            // relax: the active blocks' tiles, and on the shifted tiling the edge tiles
+            const int shift = (shift_first ^ half) ? BLOCK / 2 : 0;
+            const uint32_t total = na + (shift ? D.edge_tiles : 0u);
+#pragma unroll 1
+            for (uint32_t j = w0; j < total; j += wn) relaxTile<T>(D, F, w, na, j, shift, rim);
+            if (!g.sync()) return;
+            if (half) break;
+#pragma unroll 1
+            for (uint32_t l = 1; l <= lc; l++) {
+                const uint32_t tiles = levelTiles(D.level_w[l], D.level_h[l]);
+#pragma unroll 1
+                for (uint32_t t = t0; t < tiles; t += tn) {
+                    if (l == 1u) downTile<T, TEAM, true>(D, F, w, l, t, cycle == 0u, lt, tm);
+                    else downTile<T, TEAM, false>(D, F, w, l, t, cycle == 0u, lt, tm);
                 }
-                double t2 = 0.0;
-                if (tol) t2 = tree64x4(s64, r2);
-                __syncthreads();
-                if (valid && (threadIdx.x & 63u) == 0u) {
-                    if (tol) D.norm64[w.blockIndex(w.activeBlock(wid))] = t2;
-                    atomicMax(&D.blocks[w.countSlot(COUNT_RESIDUAL + cycle % 3u)], most[threadIdx.x >> 6]);
+                if (!g.sync()) return;
+            }
+            if (g.rank == 0u) coarseLevels<T>(D, F, w, lc, sm, s_off);
+            if (!g.sync()) return;
+#pragma unroll 1
+            for (uint32_t l = lc - 1u; l >= 1u; l--) {
+                const uint32_t tiles = levelTiles(D.level_w[l], D.level_h[l]);
+#pragma unroll 1
+                for (uint32_t t = t0; t < tiles; t += tn) upTile<T, TEAM>(D, F, l, t, lt, tm);
+                if (!g.sync()) return;
+            }
+            for (uint32_t j = w0; j < na; j += wn) {
+                const I2 b = w.activeBlock(j);
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    const I2 c{b.x * BLOCK + (int)(lane & 7u), b.y * BLOCK + (int)(lane >> 3) + 4 * h};
+                    if (w.inWorld(c)) prolongFineCell<T>(D, F, w, c);
                 }
-                __syncthreads();
+            }
+            if (!g.sync()) return;
+        }
+        // cgRho, cgBeta
+        double beta = 0.0, alpha = 0.0;
+        float beta32 = 0.0f, alpha32 = 0.0f;
+#pragma unroll 1
+        for (uint32_t j0 = w0; j0 < na; j0 += 2u * wn) {
+            const uint32_t j[2] = {j0, j0 + wn};
+            rhoTiles(D, F, w, j, j0 + wn < na, f64, Parts{F.part64, F.part32});
+        }
+        if (!g.sync()) return;
+        if (f64) {
+            if (!groupSums<double, 2>(g, D.B, F.part64, s64, sm, F.col64)) return;
+            rz = s64[0];
+            beta = (cycle == 0u || pq <= 0.0) ? 0.0 : -s64[256] / pq;
+        } else {
+            if (!groupSums<float, 2>(g, D.B, F.part32, s32, sm, F.col64)) return;
+            rz32 = s32[0];
+            beta32 = (cycle == 0u || pq32 <= 0.0f) ? 0.0f : -s32[256] / pq32;
+        }
+        __syncthreads();  // the sums are read: their memory is free
+        // cgDirection, cgApply, cgAlpha
+        const bool odd = (cycle & 1u) != 0u;
+#pragma unroll 1
+        for (uint32_t j = w0; j < na; j += wn)
+            applyTile(D, F, w, j, odd, f64, beta32, beta, sm + RIM * RIM * warp, Parts{F.pq64, F.pq32});
+        if (!g.sync()) return;
+        if (f64) {
+            if (!groupSums<double, 1>(g, D.B, F.pq64, s64, sm, F.col64)) return;
+            pq = s64[0];
+            alpha = pq <= 0.0 ? 0.0 : rz / pq;
+        } else {
+            if (!groupSums<float, 1>(g, D.B, F.pq32, s32, sm, F.col64)) return;
+            pq32 = s32[0];
+            alpha32 = pq32 <= 0.0f ? 0.0f : rz32 / pq32;
+        }
+        __syncthreads();
+        // cgUpdate
+        uint32_t most = 0u;
+#pragma unroll 1
+        for (uint32_t j0 = w0; j0 < na; j0 += 2u * wn) {
+            const uint32_t j[2] = {j0, j0 + wn};
+            most = max(most, updateTiles(D, F, w, j, j0 + wn < na, odd ? F.P : F.P2, f64, tol, alpha32, alpha));
+        }
+        most = __reduce_max_sync(0xffffffffu, most);
+        if (lane == 0u && most) atomicMax(&s_most, most);
+        __syncthreads();
+        if (tid == 0u) {
+            if (s_most) atomicMax(&D.blocks[w.countSlot(COUNT_RESIDUAL + cycle % 3u)], s_most);
+            s_most = 0u;
+        }
+        if (!g.sync()) return;
+        // converged (fluid.wgsl:2223-2226) for the next iteration: every CTA
+        // decides the same from the same sums
+        bool conv;
+        if (tol) {
+            if (!groupSums<double, 1>(g, D.B, D.norm64, s64, sm, F.col64)) return;
+            rel = bnorm2 > 0.0 ? sqrt(s64[0] / bnorm2) : 0.0;
+            conv = rel <= tolerance;
+        } else {
+            conv = __uint_as_float(__ldcg(&D.blocks[w.countSlot(COUNT_RESIDUAL + cycle % 3u)])) < LIQUID_TOLERANCE;
+        }
+        __syncthreads();
+        cycle++;
+        more = !conv && cycle < max_cycles;
+        if (sizeof(T) == 2 && (conv || cycle % 8u == 0u || cycle >= max_cycles)) {
+            // the mixed form's guard (k_fTrueCheck, k_fTrueFix)
+#pragma unroll 1
+            for (uint32_t j = w0; j < na; j += wn) trueCheckTile(D, F, w, j, F.part64);
+            if (!g.sync()) return;
+            if (!groupSums<double, 2>(g, D.B, F.part64, s64, sm, F.col64)) return;
+            double flo;
+            trueRel(s64[0], s64[256], bnorm2, &rel_true, &flo);
+            __syncthreads();
+            if (drifted(rel_true, rel, flo)) {
+                more = cycle < max_cycles;
+#pragma unroll 1
+                for (uint32_t j = w0; j < na; j += wn) trueFixTile(D, F, w, j);
+                if (!g.sync()) return;
             }
         }
-        if (!gridBarrier(st, nb)) return;
-        // converged (fluid.wgsl:2223-2226) for the next iteration
-        if (blockIdx.x == 0) {
-            bool conv;
-            if (tol) {
-                double rr = sumBlocks256(w, D.norm64, 0, s64);
-                double rel = vldd(&st->bnorm2) > 0.0 ? sqrt(rr / vldd(&st->bnorm2)) : 0.0;
-                if (threadIdx.x == 0) st->rel = rel;
-                conv = rel <= st->tol;
-            } else {
-                conv = __uint_as_float(__ldcg(&D.blocks[w.countSlot(COUNT_RESIDUAL + cycle % 3u)])) < LIQUID_TOLERANCE;
-            }
-            if (threadIdx.x == 0) {
-                st->cycle = cycle + 1u;
-                st->cont = (!conv && cycle + 1u < F.max_cycles) ? 1u : 0u;
-            }
-        }
-        if (!gridBarrier(st, nb)) return;
-        if (vld(&st->cont) == 0u) break;
+    }
+    if (g.rank == 0u && tid == 0u) {
+        st->cycle = cycle;
+        st->cont = 0u;
+        st->rel = rel;
+        st->rel_true = rel_true;
     }
 }
 
@@ -2843,7 +2683,6 @@ uint32_t fast_cycle_t(const Batch& Bt0, const BatchShape& S, const World* one, c
         Bt.cond_check = (unsigned long long)hc;
         Bt.cond_drift = (unsigned long long)hd;
     }
-    const unsigned G = list_grid(S, L_ACT, 32), G4 = list_grid(S, L_ACT4, S.cg_per_sm);
     // the CG kernels: at most a tile a warp
     const unsigned GC = std::max(std::min((S.max_items[L_ACT] + CG_WARPS - 1u) / CG_WARPS, 148u * S.cg_per_sm), 1u);
     const unsigned GR = std::max(std::min((S.max_items[L_RELAX] + 3u) / 4u, 148u * S.relax_per_sm), 1u);
@@ -2908,7 +2747,7 @@ uint32_t fast_cycle_t(const Batch& Bt0, const BatchShape& S, const World* one, c
         mark(WIG_SLOT_F_PROLONG, 1);
     }
     mark(WIG_SLOT_F_PROLONG_FINE, 0);
-    LAUNCH_T(k_fProlongFine, T, G, 64, 0);
+    LAUNCH_T(k_fProlongFine, T, list_grid(S, L_ACT, 32), 64, 0);
     mark(WIG_SLOT_F_PROLONG_FINE, 1);
     mark(WIG_SLOT_F_RELAX, 0);
     LAUNCH_T(k_fRelax, T, GR, 128, 0, 1);
@@ -2926,15 +2765,15 @@ uint32_t fast_cycle_t(const Batch& Bt0, const BatchShape& S, const World* one, c
         // captured: launched only on the iterations that check (not counted
         // among every iteration's launches)
         if (nest->err == cudaSuccess)
-            nest->err = captureIf(s, hc, nest->s, [&](cudaStream_t s) { LAUNCH(k_fTrueCheck, G4, 256, 0); });
+            nest->err = captureIf(s, hc, nest->s, [&](cudaStream_t s) { LAUNCH(k_fTrueCheck, GC, CG_THREADS, 0); });
         if (nest->err == cudaSuccess)
-            nest->err = captureIf(s, hd, nest->s, [&](cudaStream_t s) { LAUNCH(k_fTrueFix, G, 64, 0); });
+            nest->err = captureIf(s, hd, nest->s, [&](cudaStream_t s) { LAUNCH(k_fTrueFix, GC, CG_THREADS, 0); });
     } else if (Bt.mixed) {
         mark(WIG_SLOT_F_UPDATE, 0);
-        LAUNCH(k_fTrueCheck, G4, 256, 0);
+        LAUNCH(k_fTrueCheck, GC, CG_THREADS, 0);
         mark(WIG_SLOT_F_UPDATE, 1);
         mark(WIG_SLOT_F_UPDATE, 0);
-        LAUNCH(k_fTrueFix, G, 64, 0);
+        LAUNCH(k_fTrueFix, GC, CG_THREADS, 0);
         mark(WIG_SLOT_F_UPDATE, 1);
     }
     return launches;
@@ -2945,14 +2784,16 @@ uint32_t fast_cycle(const Batch& Bt, const BatchShape& S, const World* one, cuda
     return Bt.mixed ? fast_cycle_t<__half>(Bt, S, one, s, m, nest) : fast_cycle_t<float>(Bt, S, one, s, m, nest);
 }
 
-void fast_finish(const Batch& Bt, const BatchShape& S, const World* one, bool two_p, cudaStream_t s, const Marker* m) {
+void fast_finish(const Batch& Bt, const BatchShape& S, const World* one, cudaStream_t s, const Marker* m) {
     if (m) m->fn(m->ctx, WIG_SLOT_F_FINISH, 0);
-    LAUNCH(k_fFinish, list_grid(S, L_ACT, 32), 64, 0, two_p ? 1 : 0);
+    LAUNCH(k_fFinish, list_grid(S, L_ACT, 32), 64, 0);
     if (m) m->fn(m->ctx, WIG_SLOT_F_FINISH, 1);
 }
 
-cudaError_t fast_prepare_attributes(size_t smem) {
-    const int b = (int)smem;
+cudaError_t fast_prepare_attributes() {
+    // the limit is the kernel's, not a batch's (another batch's launches
+    // come under it too): room for any
+    const int b = (int)SOLVE_SMEM_MOST;
     cudaError_t e = cudaFuncSetAttribute(k_fCoarse<true, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_fCoarse<false, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(k_fCoarse<true, __half>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
@@ -2962,36 +2803,97 @@ cudaError_t fast_prepare_attributes(size_t smem) {
     return e;
 }
 
-size_t fast_solve_smem(const Fast& F) { return fast_coarse_smem(F.D, F.lp); }
+// A solve's shared memory from level lc: the coarse levels', and at least
+// what the other phases take.
+size_t solve_smem(const Dev& D, uint32_t lc) {
+    const size_t least = std::max({2u * sizeof(LevelTile), (size_t)SOLVE_WARPS * RIM * RXS * sizeof(float2),
+                                   (size_t)SOLVE_WARPS * 256u * sizeof(double)});
+    return std::max(fast_coarse_smem(D, lc), least);
+}
 
-cudaError_t fast_solve_grid(const Fast& F, uint32_t* grid) {
+template <class Group, class T>
+cudaError_t solve_attributes(size_t smem, bool cluster) {
+    cudaError_t e = cudaFuncSetAttribute(k_fSolve<Group, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess && cluster)
+        e = cudaFuncSetAttribute(k_fSolve<Group, T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    return e;
+}
+
+// Launches k_fSolve<Group, T> on n CTAs: one cluster, or a cooperative grid.
+template <class Group, class T>
+cudaError_t solve_launch(const World& Wd, uint32_t max_cycles, uint32_t n, bool cluster, cudaStream_t s) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(n);
+    c.blockDim = dim3(SOLVE_THREADS);
+    c.dynamicSmemBytes = solve_smem(Wd.D, Wd.S.lc);
+    c.stream = s;
+    cudaLaunchAttribute at[1];
+    if (cluster) {
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = n;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+    } else {
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+    }
+    c.attrs = at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, k_fSolve<Group, T>, Wd, max_cycles);
+}
+
+cudaError_t fast_solve_shape(const Dev& D, SolveShape* out) {
     int dev = 0, sms = 0, per = 0;
     cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess) return e;
-    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(k_fSolve, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fast_solve_smem(F));
-    if (e != cudaSuccess) return e;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_fSolve, 256, fast_solve_smem(F));
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // the attributes are the kernels', not this world's: room for any
+    const size_t most = SOLVE_SMEM_MOST;
+    if (e == cudaSuccess) e = solve_attributes<GridGroup, float>(most, false);
+    if (e == cudaSuccess) e = solve_attributes<GridGroup, __half>(most, false);
+    if (e == cudaSuccess) e = solve_attributes<ClusterGroup, float>(most, true);
+    if (e == cudaSuccess) e = solve_attributes<ClusterGroup, __half>(most, true);
+    out->lc = coarse_level(D, COARSE_CTA_CELLS);
+    const size_t smem = solve_smem(D, out->lc);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_fSolve<GridGroup, float>, SOLVE_THREADS, smem);
     if (e != cudaSuccess) return e;
     if (per < 1) return cudaErrorInvalidConfiguration;
-    *grid = (uint32_t)(sms * (per < 4 ? per : 4));
+    out->grid = std::min((uint32_t)sms, std::max(SPLIT_CTAS, (D.B + GRID_TILES - 1u) / GRID_TILES));
+    // the cluster, for a world of few blocks: the most CTAs that fit
+    out->cluster = 0;
+    if (D.B <= CLUSTER_BLOCKS) {
+        for (uint32_t n = SOLVE_CLUSTER; n >= 4u && out->cluster == 0u; n /= 2u) {
+            cudaLaunchConfig_t c = {};
+            c.gridDim = dim3(n);
+            c.blockDim = dim3(SOLVE_THREADS);
+            c.dynamicSmemBytes = smem;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = n;
+            at[0].val.clusterDim.y = 1;
+            at[0].val.clusterDim.z = 1;
+            c.attrs = at;
+            c.numAttrs = 1;
+            int fit = 0;
+            if (cudaOccupancyMaxActiveClusters(&fit, k_fSolve<ClusterGroup, float>, &c) == cudaSuccess && fit > 0) out->cluster = n;
+            else cudaGetLastError();
+        }
+    }
     return cudaSuccess;
 }
 
-cudaError_t fast_solve(const Fast& F, bool shifted, cudaStream_t s, const Marker* m) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(F.solve_grid);
-    cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = fast_solve_smem(F);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+cudaError_t fast_solve(const Batch& Bt, const World& W0, const SolveShape& h, bool grid, cudaStream_t s, const Marker* m) {
+    World Wd = W0;
+    // (a coarse level of the cluster coarse kernel's is too large for one CTA)
+    Wd.S.lc = std::max(Wd.S.lc, h.lc);
     if (m) m->fn(m->ctx, WIG_SLOT_F_SOLVE, 0);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, k_fSolve, F, shifted ? 1 : 0);
+    cudaError_t e;
+    if (!grid && h.cluster) {
+        e = Bt.mixed ? solve_launch<ClusterGroup, __half>(Wd, Bt.max_cycles, h.cluster, true, s)
+                     : solve_launch<ClusterGroup, float>(Wd, Bt.max_cycles, h.cluster, true, s);
+    } else {
+        e = Bt.mixed ? solve_launch<GridGroup, __half>(Wd, Bt.max_cycles, h.grid, false, s)
+                     : solve_launch<GridGroup, float>(Wd, Bt.max_cycles, h.grid, false, s);
+    }
     if (m) m->fn(m->ctx, WIG_SLOT_F_SOLVE, 1);
     return e;
 }

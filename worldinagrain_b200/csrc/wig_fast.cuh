@@ -8,16 +8,8 @@
 
 namespace wig {
 
-// One world's fast form with its step's settings: the persistent solve's
-// argument (a batch of one world).
-struct Fast : FastW {
-    Dev D;
-    uint32_t solve_grid;       // CTAs of the persistent solve (all resident)
-    uint32_t max_cycles;
-};
-
-// The one-CTA coarse kernel holds levels of at most this many cells; CTA 0
-// of the persistent solve, of at most PERSISTENT_CTA_CELLS.
+// The one-CTA coarse kernel (and CTA 0 of a world's solve in one launch)
+// holds levels of at most this many cells.
 constexpr uint32_t COARSE_CTA_CELLS = 4096;
 // A single world's coarse levels from a level of up to this many cells run
 // on a thread-block cluster (k_fCoarseCluster).
@@ -30,7 +22,28 @@ inline uint32_t coarse_level(const Dev& D, uint32_t cells) {
         if ((size_t)D.level_w[l] * D.level_h[l] <= cells) return l;
     return D.levels;
 }
-constexpr uint32_t PERSISTENT_CTA_CELLS = 1024;
+// The most dynamic shared memory a CTA of these kernels takes.
+constexpr size_t SOLVE_SMEM_MOST = 220u * 1024u;
+
+// How a single world's solve in one launch is shaped: the CTAs of a
+// cooperative grid; the CTAs of one cluster (0: the world has too many
+// blocks for one); the first level that fits one CTA.
+struct SolveShape {
+    uint32_t grid, cluster, lc;
+};
+constexpr uint32_t SOLVE_CLUSTER = 16;
+// The sizes, in blocks, a single world's solve is one launch at: up to
+// CLUSTER_BLOCKS on a cluster, whose barrier is the cheapest but whose 16
+// multiprocessors are few (a step of a pond of 75x52 200 us against 218 as
+// the loop's launches, of the dam at 192x192 673 against 724, of two liquids
+// at 224x224 928 against 890); above GRID_BLOCKS on a grid of all of them
+// (the disks at 640x640 2572 us against 2786, at 512x512 1595 against 1554).
+// Between, the loop's launches.
+constexpr uint32_t CLUSTER_BLOCKS = 640, GRID_BLOCKS = 4096;
+// A grid's CTAs: a tile of the fine level for every other warp, at most a
+// CTA a multiprocessor (a tile a warp is 1% slower at 256x256, 4 or 8 tiles
+// a CTA the same).
+constexpr uint32_t GRID_TILES = 16;
 
 // A profiler's hook around each launch: fn(ctx, slot, 0) before, (ctx, slot, 1) after.
 struct Marker {
@@ -56,8 +69,8 @@ struct NestCapture {
 void fast_setup(const Batch& Bt, const BatchShape& S, const World* one, cudaStream_t s, const Marker* m);
 uint32_t fast_cycle(const Batch& Bt, const BatchShape& S, const World* one, cudaStream_t s, const Marker* m,
                     NestCapture* nest = nullptr);
-// cgFinish; `two_p`: the fast form's p is in P or P2 by the iterations' parity.
-void fast_finish(const Batch& Bt, const BatchShape& S, const World* one, bool two_p, cudaStream_t s, const Marker* m);
+// cgFinish.
+void fast_finish(const Batch& Bt, const BatchShape& S, const World* one, cudaStream_t s, const Marker* m);
 // Level 0's arrays and the block partials of one world zeroed (after its buffers are written by the host).
 void fast_zero_level0(const World& Wd, cudaStream_t s);
 // The same for the blocks not worked on, of every world of the step whose
@@ -69,10 +82,10 @@ size_t fast_coarse_smem(const Dev& D, uint32_t lc);
 // from level lc; 0 when that kernel does not apply (level lc fits the one-CTA
 // kernel, or the world's coarsest level does not fit one CTA of the cluster).
 size_t fast_cluster_smem(const Dev& D, uint32_t lc);
-cudaError_t fast_prepare_attributes(size_t smem);
-// The persistent solve of one world: all iterations in one cooperative launch.
-size_t fast_solve_smem(const Fast& F);
-cudaError_t fast_solve_grid(const Fast& F, uint32_t* grid);
-cudaError_t fast_solve(const Fast& F, bool shifted, cudaStream_t s, const Marker* m);
+cudaError_t fast_prepare_attributes();
+// A single world's solve: all its iterations in one launch, on one cluster
+// or (`grid`, or no cluster fits it) a cooperative grid.
+cudaError_t fast_solve_shape(const Dev& D, SolveShape* out);
+cudaError_t fast_solve(const Batch& Bt, const World& W0, const SolveShape& h, bool grid, cudaStream_t s, const Marker* m);
 
 }  // namespace wig

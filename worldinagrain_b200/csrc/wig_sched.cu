@@ -83,7 +83,6 @@ __device__ void startState(StepState* st, const StepHead& h) {
     st->rel_true = 0.0;
     st->rz32 = 0.0f; st->pq32 = 0.0f; st->alpha32 = 0.0f; st->beta32 = 0.0f;
     st->bar_count = 0u;
-    st->bar_gen = 0u;
 }
 
 // This step's table entry of a pooled world (the lists' units read the
