@@ -267,7 +267,7 @@ size_t scratch_bytes(const wig::Dev& D) {
         bytes += align256(5u * (size_t)D.level_w[l] * D.level_h[l] * 2u);  // the binary16 operator
     }
     bytes += align256(2u * (size_t)D.B * 4u) + 3u * align256(2u * (size_t)D.B * 8u);
-    bytes += align256((size_t)D.B * 4u) + align256((size_t)D.B * 8u) + align256(512u * 8u);
+    bytes += 2u * align256((size_t)D.B * 4u) + align256((size_t)D.B * 8u) + align256(512u * 8u);
     return bytes;
 }
 
@@ -302,6 +302,7 @@ void scratch_take(wig::World& Wd, char* p, uint32_t coarse_cells) {
     F.pq32 = fl(D.B);
     F.pq64 = reinterpret_cast<double*>(take((size_t)D.B * 8u));
     F.col64 = reinterpret_cast<double*>(take(512u * 8u));
+    F.base = reinterpret_cast<uint32_t*>(take((size_t)D.B * 4u));
     D.part64 = reinterpret_cast<double*>(take(2u * (size_t)D.B * 8u));
     D.norm64 = reinterpret_cast<double*>(take(2u * (size_t)D.B * 8u));
     F.lc = wig::coarse_level(D, coarse_cells);
@@ -682,6 +683,9 @@ struct Rec {
     void run(int pass, uint32_t level = 0, uint32_t cycle = 0) {
         timed(pass, [&] { wig::launch_pass(ln.Bt, ln.S, one_world(b), b->hw[0].D, pass, level, cycle, s); });
     }
+    void step_pass(int pass) {
+        timed(pass, [&] { wig::launch_step_pass(ln.Bt, ln.S, one_world(b), pass, s); });
+    }
     // cgStart + cgJoin as a step runs them (profiled as the two passes)
     void labels() {
         timed(WIG_PASS_CG_START, [&] { wig::launch_labels(ln.Bt, ln.S, one_world(b), s, 0); });
@@ -774,13 +778,11 @@ void record_post(Rec& R) {
     }
     R.run(WIG_PASS_EXTRAPOLATE);
     R.run(WIG_PASS_EXTRAPOLATE_FURTHER);
-    R.run(WIG_PASS_ADVECT);
-    R.run(WIG_PASS_SORT_COUNT);
+    R.step_pass(WIG_PASS_ADVECT);  // and sortCount
     R.run(WIG_PASS_SCAN_BLOCKS);
     R.run(WIG_PASS_SCAN_TOTALS);
-    R.run(WIG_PASS_SCAN_FINISH);
-    R.run(WIG_PASS_SCATTER);
-    R.run(WIG_PASS_RASTER_CLAIMS);
+    R.step_pass(WIG_PASS_SCATTER);
+    R.step_pass(WIG_PASS_RASTER_CLAIMS);  // and scanFinish
     R.run(WIG_PASS_RASTER);
     R.run(WIG_PASS_UNPAINT);
     R.report();

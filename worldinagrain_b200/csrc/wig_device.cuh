@@ -431,6 +431,7 @@ struct FastW {
     float* pq32;               // cgApply's partial sums, of block b at b
     double* pq64;
     double* col64;             // 512 column sums of a group's block sums
+    uint32_t* base;            // each active block's first place in `sorted`
     uint32_t lc;               // first level the one-CTA coarse kernel solves
 };
 

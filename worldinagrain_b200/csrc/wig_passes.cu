@@ -507,9 +507,8 @@ __device__ V2 pairWay(uint32_t a, uint32_t b) {
     return V2{c * sg, s * sg};
 }
 
-// apart (fluid.wgsl:713-734)
-__device__ V2 apart(const W& w, uint32_t k, uint32_t h, V2 pos, uint32_t id) {
-    uint32_t start = w.gw(h, G_START), n = w.gw(h, G_SORT);
+// apart (fluid.wgsl:713-734) of particle k among its cell's n from start.
+__device__ V2 apart(const W& w, uint32_t k, uint32_t start, uint32_t n, V2 pos, uint32_t id) {
     if (n < 2u) return pos;
     const uint4* it = w.items(w.D.sorted);
     int32_t px = 0, py = 0;
@@ -610,8 +609,9 @@ __global__ void k_syncParticles(Batch Bt, const __grid_constant__ WorldSrc<ONE> 
         aff = make_float4(__uint_as_float(af.x), __uint_as_float(af.y), __uint_as_float(af.z), __uint_as_float(af.w));
         I2 hc = w.cellOf(pos.x, pos.y);
         uint32_t h = w.cellIndex(hc);
-        pos = apart(w, k, h, pos, id);
-        uint32_t d = w.gw(h, G_DEST);
+        // the cell's words in flight together, before any is used
+        const uint32_t g_start = w.gw(h, G_START), g_sort = w.gw(h, G_SORT), d = w.gw(h, G_DEST), drawn = w.gw(h, G_TYPE);
+        pos = apart(w, k, g_start, g_sort, pos, id);
         if (d == DEST_KEEP) {
             keep = true;
             markBlockOf(w, pos.x, pos.y);
@@ -626,11 +626,10 @@ __global__ void k_syncParticles(Batch Bt, const __grid_constant__ WorldSrc<ONE> 
             uint32_t to = claimedCell(d);
             uint4 v = w.cell(to);
             uint32_t n = liquidCount(v.w);
-            if (n == LIQUID_COUNT_MAX || w.gw(h, G_SORT) <= n || rankById(w, h, k, id, word, wordType(v.x)) < n) {
+            if (n == LIQUID_COUNT_MAX || g_sort <= n || rankById(w, h, k, id, word, wordType(v.x)) < n) {
                 if (to != h)
                     pos = V2{(float)(to % (uint32_t)D.W) + (pos.x - floorf(pos.x)), (float)(to / (uint32_t)D.W) + (pos.y - floorf(pos.y))};
                 temp = __uint_as_float(v.y);
-                uint32_t drawn = w.gw(h, G_TYPE);
                 uint32_t pt = wordType(word);
                 if (holdsSolute(pt) && pt == (drawn & 0xffu) && wordType(v.x) == pt &&
                     (wordAux(word) == ((drawn >> 8u) & 0xffu) || wordAux(word) == 0u)) {
@@ -825,7 +824,11 @@ __global__ void k_retire(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     }
 }
 
-// clear (fluid.wgsl:962-985)
+// clear (fluid.wgsl:962-985).  A block's row of counters is 88 words in a
+// run (8 cells of 11), so consecutive threads write consecutive words, 11
+// stores a thread for the block; a thread a cell writing its 11 words 44
+// bytes from its neighbour's touched 8 times the sectors (70 us a step of a
+// 48-world batch, 127 us of the 2048x2048 column).
 template <bool ONE>
 __global__ void k_clear(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
@@ -834,11 +837,19 @@ __global__ void k_clear(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
         ITEM_WORLD_S(Bt, it, D, w, wid);
         I2 b = w.activeBlock(wid);
         if (threadIdx.x == 0) D.blocks[w.blockIndex(b)] = 0u;
+        const int x0 = b.x * BLOCK, y0 = b.y * BLOCK;
+        const uint32_t words = (uint32_t)min(BLOCK, D.W - x0) * CELL_WORDS;
+        const int rows = min(BLOCK, D.H - y0);
+        for (int r = 0; r < rows; r++) {
+            const uint32_t i0 = w.cellIndex(I2{x0, y0 + r});
+            uint32_t* at = w.gwp(i0, 0u);
+            for (uint32_t q = threadIdx.x; q < words; q += 64u) {
+                const uint32_t c = q / CELL_WORDS;
+                at[q] = q - c * CELL_WORDS == G_REGION ? i0 + c : 0u;
+            }
+        }
         I2 c = lidCell(w, wid);
         if (!w.inWorld(c)) continue;
-        uint32_t i = w.cellIndex(c);
-        for (uint32_t g = 0; g < CELL_WORDS; g++) *w.gwp(i, g) = 0u;
-        *w.gwp(i, G_REGION) = i;
         int fs[4][3];
         w.facesOf(c, fs);
         for (int j = 0; j < 4; j++) {
@@ -852,7 +863,11 @@ __global__ void k_clear(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
 
 // ================================================================ splat
 
-// splatAxis (fluid.wgsl:1000-1015)
+__device__ __forceinline__ bool walls(const W& w, I2 c) {
+    if (!w.inWorld(c)) return true;
+    uint32_t k = w.kindOfCell(w.cellIndex(c));
+    return k == WIG_KIND_SOLID || k == WIG_KIND_POWDER;
+}
 // Where the splat's fixed-point adds go.  DirectSink: global atomics, a site
 // at a time.  WinSink: a warp's window in shared memory, summed there and
 // added to the global words once a site (WarpGather); the sums are
@@ -905,11 +920,6 @@ __device__ __forceinline__ void splatAxis(const W& w, const Sink& k, float sx, f
         float there = vel + (gx * ((float)at.x - sx) + gy * ((float)at.y - sy));
         k.face(isU, at, (uint32_t)f2i(rnd_even(there * wgt * FIX)), (uint32_t)f2i(rnd_even(wgt * FIX)));
     }
-}
-__device__ __forceinline__ bool walls(const W& w, I2 c) {
-    if (!w.inWorld(c)) return true;
-    uint32_t k = w.kindOfCell(w.cellIndex(c));
-    return k == WIG_KIND_SOLID || k == WIG_KIND_POWDER;
 }
 // splatDensity (fluid.wgsl:1069-1087)
 template <class Sink>
@@ -989,12 +999,12 @@ __device__ __forceinline__ void gatherWarp(const Dev& D, const W& w, uint32_t k,
         return;
     }
     if (x1 < x0) return;  // no particle in the warp
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t bw = (uint32_t)(x1 - x0 + 1), nbox = bw * (uint32_t)(y1 - y0 + 1);
     if (has) gatherTo(w, WinSink{win, x0, y0}, p);
     __syncwarp();
     // the flush: the sites' box alone (every add fell inside it), a lane a
     // window entry; each nonzero sum added to its global word and cleared
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t bw = (uint32_t)(x1 - x0 + 1), nbox = bw * (uint32_t)(y1 - y0 + 1);
     for (uint32_t q = lane; q < nbox; q += 32u) {
         const uint32_t qy = q / bw, qx = q - qy * bw;
         const uint32_t e = qy * (uint32_t)(GWX + 1) + qx;
@@ -1484,21 +1494,38 @@ __global__ void k_cgStartLocal(Batch Bt, const __grid_constant__ WorldSrc<ONE> s
 }
 // cgJoin's edges between blocks (to the right and below, from the block's
 // last column and row), after k_cgStartLocal has linked each block's own.
+// An edge is left to the one before it along the border (above it, or to
+// its left) when both its cells have their links in common with that one's:
+// then joining that edge joins these two as well, and the first of such a
+// run is never left out.  (A link here is a region's lower cell, so equal
+// links are one region, whatever other joins have done to them meanwhile.)
+// With every edge joined, eight walks to the same two roots and as many
+// atomics on them a border, the pass took 327 us on the 2048x2048 column
+// and 141 us on a 48-world batch.
 template <bool ONE>
 __global__ void k_cgJoinAcross(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
     if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_ACT, it) {
         ITEM_WORLD_S(Bt, it, D, w, wid);
-        const int lx = (int)(threadIdx.x & 7u), ly = (int)(threadIdx.x >> 3);
-        if (lx != 7 && ly != 7) continue;
-        I2 c = lidCell(w, wid);
-        if (!w.inWorld(c) || w.gridAt(c).z <= 0.0f) continue;
-        for (int d = 0; d < 2; d++) {
-            if ((d == 0 && lx != 7) || (d == 1 && ly != 7)) continue;
-            I2 n = d == 0 ? I2{c.x + 1, c.y} : I2{c.x, c.y + 1};
-            if (rhoAt(w, 0, n) > 0.0f) ufJoin(w, w.cellIndex(c), w.cellIndex(n));
-        }
+        // thread k < 8: the edge to the right of row k; < 16: below column k - 8
+        const int k = (int)(threadIdx.x & 7u);
+        if (threadIdx.x >= 16u) continue;
+        const bool right = threadIdx.x < 8u;
+        const I2 b = w.activeBlock(wid);
+        const I2 c = right ? I2{b.x * BLOCK + BLOCK - 1, b.y * BLOCK + k} : I2{b.x * BLOCK + k, b.y * BLOCK + BLOCK - 1};
+        const I2 n = right ? I2{c.x + 1, c.y} : I2{c.x, c.y + 1};
+        if (!w.inWorld(c) || !w.inWorld(n)) continue;
+        const uint32_t i = w.cellIndex(c), j = w.cellIndex(n);
+        const uint32_t back = right ? (uint32_t)D.W : 1u;
+        const uint32_t ib = k > 0 ? i - back : i, jb = k > 0 ? j - back : j;
+        const float zi = w.fv(2u * i)[2], zj = w.fv(2u * j)[2], zib = w.fv(2u * ib)[2], zjb = w.fv(2u * jb)[2];
+        const uint32_t li = vload(w.gwp(i, G_REGION)), lj = vload(w.gwp(j, G_REGION));
+        const uint32_t lib = vload(w.gwp(ib, G_REGION)), ljb = vload(w.gwp(jb, G_REGION));
+        auto joins = [](float zc, float zn) { return !(zc <= 0.0f) && zn > 0.0f; };
+        if (!joins(zi, zj)) continue;
+        if (k > 0 && joins(zib, zjb) && li == lib && lj == ljb) continue;
+        ufJoin(w, i, j);
     }
 }
 // cgAnchor (fluid.wgsl:2692-2705)
@@ -2295,9 +2322,9 @@ __device__ __forceinline__ bool escapesTo(const W& w, I2 q, uint32_t side) {
     const uint32_t cup = cupOf(w, w.cellIndex(q));
     return cup == NONE || cup == side;
 }
-// escape (fluid.wgsl:3552-3594), no bodies, the Earth's down.
+// escape (fluid.wgsl:3552-3594), no bodies, the Earth's down: of a position
+// in an obstacle.
 __device__ V2 escape(const W& w, V2 pos) {
-    if (!isObstacle(w, pos.x, pos.y)) return pos;
     I2 c{f2i(floorf(pos.x)), f2i(floorf(pos.y))};
     const uint32_t side = w.inWorld(c) ? cupBefore(w, w.cellIndex(c)) : NONE;
     V2 best = pos;
@@ -2337,17 +2364,24 @@ __device__ __forceinline__ V2 clampSpeed(V2 v) {
     return v;
 }
 
-// advect (fluid.wgsl:3616-3694)
-__device__ __forceinline__ void advectOne(const Dev& D, const W& w, uint32_t chunk) {
-    uint32_t live = min(D.parts[0], D.cap);
-    uint32_t k = chunk * blockDim.x + threadIdx.x;
-    if (k >= live) return;
+// advect (fluid.wgsl:3616-3694) of particle k; where it ends.
+__device__ __forceinline__ V2 advectOne(const Dev& D, const W& w, uint32_t k) {
     uint4* it = w.items(D.parts);
     uint4 mo = it[k], stt = it[D.cap + k];
     V2 orig{__uint_as_float(mo.x), __uint_as_float(mo.y)};
     V2 qvel{__uint_as_float(mo.z), __uint_as_float(mo.w)};
     float temp = __uint_as_float(stt.y);
-    V2 qpos = escape(w, orig);
+    // the last cell found to be no obstacle: a sub-step that stays in it asks
+    // nothing again (most stay: three lookups a particle become one)
+    I2 open{-0x7fffffff, -0x7fffffff};
+    auto obstacle = [&](float x, float y) {
+        const I2 c{f2i(floorf(x)), f2i(floorf(y))};
+        if (c.x == open.x && c.y == open.y) return false;
+        if (isObstacle(w, x, y)) return true;
+        open = c;
+        return false;
+    };
+    V2 qpos = obstacle(orig.x, orig.y) ? escape(w, orig) : orig;
     Sample u = sampleAxis(w, qpos.x - 0.0f, qpos.y - 0.5f, true);
     Sample v = sampleAxis(w, qpos.x - 0.5f, qpos.y - 0.0f, false);
     V2 flow{u.weight > 0.0f ? u.now : qvel.x, v.weight > 0.0f ? v.now : qvel.y};
@@ -2374,14 +2408,14 @@ __device__ __forceinline__ void advectOne(const Dev& D, const W& w, uint32_t chu
     float impact = 0.0f;
     for (int s = 0; s < steps; s++) {
         float nx = pos.x + dx, nxy = pos.y + 0.0f;
-        if (dx != 0.0f && isObstacle(w, nx, nxy)) {
+        if (dx != 0.0f && obstacle(nx, nxy)) {
             if (vel.x * dx > 0.0f) { impact = fmaxf(impact, fabsf(vel.x)); vel.x = 0.0f; }
             dx = 0.0f;
         } else {
             pos = V2{nx, nxy};
         }
         float nyx = pos.x + 0.0f, ny = pos.y + dy;
-        if (dy != 0.0f && isObstacle(w, nyx, ny)) {
+        if (dy != 0.0f && obstacle(nyx, ny)) {
             if (vel.y * dy > 0.0f) { impact = fmaxf(impact, fabsf(vel.y)); vel.y = 0.0f; }
             dy = 0.0f;
         } else {
@@ -2406,47 +2440,58 @@ __device__ __forceinline__ void advectOne(const Dev& D, const W& w, uint32_t chu
         atomicOr(w.gwp(w.cellIndex(w.cellOf(pos.x, pos.y)), G_CAME), falling ? CAME_FALLING : CAME_PRESSING);
     }
     if ((w.elem(wordType(stt.x)).flags & F_IMPACT) != 0u && impact > IMPACT_SPEED) it[D.cap + k].x = wordWith(stt.x, FL_BURN);
+    return pos;
 }
-template <bool ONE>
-__global__ void k_advect(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
+
+// sortCount (fluid.wgsl:3700-3708) of the warp's particles (a lane one,
+// where `has`), at pos: each particle's slot among its cell's.  The lanes of
+// a warp whose particles share a cell (parts is in cell order from the last
+// sort, so mostly neighbours) take their slots with one atomic add by the
+// lowest of them, each lane its rank among them past the base; the slots
+// within a cell are any order of 0..n-1, as the reference's atomics give
+// them.
+__device__ __forceinline__ void sortCountWarp(const Dev& D, const W& w, uint32_t k, bool has, V2 pos) {
+    const uint32_t act = __ballot_sync(0xffffffffu, has);
+    if (!has) return;
+    const uint32_t i = w.cellIndex(w.cellOf(pos.x, pos.y));
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t peers = __match_any_sync(act, i);
+    const int leader = __ffs(peers) - 1;
+    uint32_t base = 0u;
+    if ((int)lane == leader) base = atomicAdd(w.gwp(i, G_SORT), (uint32_t)__popc(peers));
+    base = __shfl_sync(peers, base, leader);
+    w.items(D.parts)[D.cap + k].w = base + (uint32_t)__popc(peers & ((1u << lane) - 1u));
+}
+
+// advect, and with SORT (a step's) sortCount of each particle where it ends:
+// the pass that reads every particle again for its cell took 86 us of a
+// 48-world batch's step (27 us at 1024x1024, 105 us at 2048x2048).
+template <bool ONE, bool SORT>
+__global__ void __launch_bounds__(256, 5) k_advect(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
     if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_PP, qi) {
         ITEM_WORLD_S(Bt, qi, D, w, chunk);
-        advectOne(D, w, chunk);
+        const uint32_t k = chunk * blockDim.x + threadIdx.x;
+        const bool has = k < min(D.parts[0], D.cap);
+        V2 pos{0.0f, 0.0f};
+        if (has) pos = advectOne(D, w, k);
+        if (SORT) sortCountWarp(D, w, k, has, pos);
     }
 }
 
 // ================================================================ sort
 
-// sortCount (fluid.wgsl:3700-3708): each particle's slot among its cell's.
-// The lanes of a warp whose particles share a cell (parts is in cell order
-// from the last sort, so mostly neighbours) take their slots with one atomic
-// add by the lowest of them, each lane its rank among them past the base;
-// the slots within a cell are any order of 0..n-1, as the reference's
-// atomics give them.
-__device__ __forceinline__ void sortCountOne(const Dev& D, const W& w, uint32_t chunk) {
-    uint32_t live = min(D.parts[0], D.cap);
-    uint32_t k = chunk * blockDim.x + threadIdx.x;
-    if (k >= live) return;
-    uint4* it = w.items(D.parts);
-    uint4 mo = it[k];
-    uint32_t i = w.cellIndex(w.cellOf(__uint_as_float(mo.x), __uint_as_float(mo.y)));
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t peers = __match_any_sync(__activemask(), i);
-    const int leader = __ffs(peers) - 1;
-    uint32_t base = 0u;
-    if ((int)lane == leader) base = atomicAdd(w.gwp(i, G_SORT), (uint32_t)__popc(peers));
-    base = __shfl_sync(peers, base, leader);
-    it[D.cap + k].w = base + (uint32_t)__popc(peers & ((1u << lane) - 1u));
-}
 template <bool ONE>
 __global__ void k_sortCount(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
     if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_PP, qi) {
         ITEM_WORLD_S(Bt, qi, D, w, chunk);
-        sortCountOne(D, w, chunk);
+        const uint32_t k = chunk * blockDim.x + threadIdx.x;
+        const bool has = k < min(D.parts[0], D.cap);
+        const uint4 mo = has ? w.items(D.parts)[k] : make_uint4(0, 0, 0, 0);
+        sortCountWarp(D, w, k, has, V2{__uint_as_float(mo.x), __uint_as_float(mo.y)});
     }
 }
 
@@ -2484,34 +2529,48 @@ __global__ void __launch_bounds__(64) k_scanBlocks(Batch Bt, const __grid_consta
     }
 }
 
-// scanTotals (fluid.wgsl:3757-3780): one CTA of 256.
-__global__ void __launch_bounds__(256) k_scanTotals(Batch Bt) {
-  __shared__ uint32_t tile[256];
+// scanTotals (fluid.wgsl:3757-3780): one CTA of 1024 a world, a thread a run
+// of the active blocks, 8 totals' loads in flight; each block's first place
+// also by the block (FastW::base), for a step's scatter.
+__global__ void __launch_bounds__(1024) k_scanTotals(Batch Bt) {
+  __shared__ uint32_t tile[1024];
   FOR_ITEMS(Bt, L_ONE, ot) {
     ITEM_WORLD(Bt, ot, D, w, unused_);
     (void)unused_;
+    uint32_t* base = Bt.world(ot).S.base;
     const uint32_t n = w.activeCount();
-    const uint32_t per = (n + 255u) / 256u;
+    const uint32_t per = (n + 1023u) / 1024u;
     const uint32_t lo = min(threadIdx.x * per, n), hi = min(lo + per, n);
     uint32_t sum = 0;
+#pragma unroll 8
     for (uint32_t j = lo; j < hi; j++) sum += D.blocks[w.totalSlot(j)];
     tile[threadIdx.x] = sum;
     __syncthreads();
-    for (uint32_t o = 1; o < 256u; o <<= 1) {
+    for (uint32_t o = 1; o < 1024u; o <<= 1) {
         uint32_t add = threadIdx.x >= o ? tile[threadIdx.x - o] : 0u;
         __syncthreads();
         tile[threadIdx.x] += add;
         __syncthreads();
     }
     uint32_t run = tile[threadIdx.x] - sum;
-    for (uint32_t j = lo; j < hi; j++) {
-        uint32_t t = D.blocks[w.totalSlot(j)];
-        D.blocks[w.totalSlot(j)] = run;
-        run += t;
+    for (uint32_t j0 = lo; j0 < hi; j0 += 8u) {
+        uint32_t t[8], n8[8];
+#pragma unroll
+        for (uint32_t u = 0; u < 8u; u++) {
+            t[u] = j0 + u < hi ? D.blocks[w.totalSlot(j0 + u)] : 0u;
+            n8[u] = j0 + u < hi ? D.blocks[w.activeSlot(j0 + u)] : 0u;
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < 8u; u++) {
+            if (j0 + u >= hi) break;
+            D.blocks[w.totalSlot(j0 + u)] = run;
+            base[n8[u]] = run;
+            run += t[u];
+        }
     }
-    if (threadIdx.x == 255u) {
-        D.sorted[0] = tile[255];
-        D.blocks[w.countSlot(COUNT_PARTICLES)] = tile[255];
+    if (threadIdx.x == 1023u) {
+        D.sorted[0] = tile[1023];
+        D.blocks[w.countSlot(COUNT_PARTICLES)] = tile[1023];
     }
     __syncthreads();
   }
@@ -2530,15 +2589,18 @@ __global__ void k_scanFinish(Batch Bt, const __grid_constant__ WorldSrc<ONE> src
     }
 }
 
-// scatter (fluid.wgsl:3793-3808)
-__device__ __forceinline__ void scatterOne(const Dev& D, const W& w, uint32_t chunk) {
+// scatter (fluid.wgsl:3793-3808); base: each block's first place, where
+// scanFinish has not added it to its cells' yet (a step's: rasterClaims
+// does), else null.
+__device__ __forceinline__ void scatterOne(const Dev& D, const W& w, uint32_t chunk, const uint32_t* base) {
     uint32_t live = min(D.parts[0], D.cap);
     uint32_t k = chunk * blockDim.x + threadIdx.x;
     if (k >= live) return;
     const uint4* it = w.items(D.parts);
     uint4 mo = it[k], stt = it[D.cap + k];
-    uint32_t i = w.cellIndex(w.cellOf(__uint_as_float(mo.x), __uint_as_float(mo.y)));
-    uint32_t m = w.gw(i, G_START) + stt.w;
+    const I2 c = w.cellOf(__uint_as_float(mo.x), __uint_as_float(mo.y));
+    uint32_t m = w.gw(w.cellIndex(c), G_START) + stt.w;
+    if (base) m += base[w.blockIndex(I2{c.x / BLOCK, c.y / BLOCK})];
     if (m < D.cap) {
         uint4* so = w.items(D.sorted);
         so[m] = mo;
@@ -2546,13 +2608,13 @@ __device__ __forceinline__ void scatterOne(const Dev& D, const W& w, uint32_t ch
         so[2u * D.cap + m] = it[2u * D.cap + k];
     }
 }
-template <bool ONE>
+template <bool ONE, bool STEP>
 __global__ void k_scatter(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
     if (!ONE) worldCopyInit(wc_);
     FOR_ITEMS(Bt, L_PP, qi) {
         ITEM_WORLD_S(Bt, qi, D, w, chunk);
-        scatterOne(D, w, chunk);
+        scatterOne(D, w, chunk, STEP ? Wd_qi.S.base : nullptr);
     }
 }
 
@@ -2574,8 +2636,9 @@ __device__ uint32_t airTo(const W& w, I2 c, bool gas) {
     }
     return NONE;
 }
-// rasterClaims (fluid.wgsl:3928-3948), no people.
-template <bool ONE>
+// rasterClaims (fluid.wgsl:3928-3948), no people; with STEP, scanFinish of
+// the cell first (scatter has read the block's own places).
+template <bool ONE, bool STEP>
 __global__ void k_rasterClaims(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
     if (!ONE) worldCopyInit(wc_);
@@ -2584,6 +2647,7 @@ __global__ void k_rasterClaims(Batch Bt, const __grid_constant__ WorldSrc<ONE> s
         I2 c = lidCell(w, wid);
         if (!w.inWorld(c)) continue;
         uint32_t i = w.cellIndex(c);
+        if (STEP) *w.gwp(i, G_START) += D.blocks[w.totalSlot(wid)];
         uint32_t to = NONE;
         uint32_t t = w.cellType(i);
         if (w.gw(i, G_SORT) > 0u) {
@@ -2922,6 +2986,13 @@ unsigned list_grid(const BatchShape& S, uint32_t list, unsigned per_sm) {
         else K<false><<<(grid), (block), 0, s>>>(Bt, WorldSrc<false>{}, ##__VA_ARGS__);             \
     } while (0)
 
+// The same for a kernel with a variant.
+#define RUN2(K, V, grid, block)                                                          \
+    do {                                                                                 \
+        if (one) K<true, V><<<(grid), (block), 0, s>>>(Bt, WorldSrc<true>{*one});          \
+        else K<false, V><<<(grid), (block), 0, s>>>(Bt, WorldSrc<false>{});                \
+    } while (0)
+
 int launch_pass(const Batch& Bt, const BatchShape& S, const World* one, const Dev& D0, int pass, uint32_t level,
                 uint32_t cycle, cudaStream_t s) {
     // the passes shared by every form: over the batch's work lists
@@ -2975,13 +3046,13 @@ int launch_pass(const Batch& Bt, const BatchShape& S, const World* one, const De
     case WIG_PASS_PROJECT: RUN(k_project, A, 64); break;
     case WIG_PASS_EXTRAPOLATE: RUN(k_extrapolate, A, 64, 1u); break;
     case WIG_PASS_EXTRAPOLATE_FURTHER: RUN(k_extrapolate, A, 64, 2u); break;
-    case WIG_PASS_ADVECT: RUN(k_advect, PP, 256); break;
+    case WIG_PASS_ADVECT: RUN2(k_advect, false, PP, 256); break;
     case WIG_PASS_SORT_COUNT: RUN(k_sortCount, PP, 256); break;
     case WIG_PASS_SCAN_BLOCKS: RUN(k_scanBlocks, A, 64); break;
-    case WIG_PASS_SCAN_TOTALS: k_scanTotals<<<ONE, 256, 0, s>>>(Bt); break;
+    case WIG_PASS_SCAN_TOTALS: k_scanTotals<<<ONE, 1024, 0, s>>>(Bt); break;
     case WIG_PASS_SCAN_FINISH: RUN(k_scanFinish, A, 64); break;
-    case WIG_PASS_SCATTER: RUN(k_scatter, PP, 256); break;
-    case WIG_PASS_RASTER_CLAIMS: RUN(k_rasterClaims, A, 64); break;
+    case WIG_PASS_SCATTER: RUN2(k_scatter, false, PP, 256); break;
+    case WIG_PASS_RASTER_CLAIMS: RUN2(k_rasterClaims, false, A, 64); break;
     case WIG_PASS_RASTER: RUN(k_raster, A, 64); break;
     case WIG_PASS_UNPAINT: RUN(k_unpaint, A, 64); break;
     default:
@@ -3009,6 +3080,16 @@ void launch_labels(const Batch& Bt, const BatchShape& S, const World* one, cudaS
     const unsigned A = list_grid(S, L_ACT, 32);
     if (part == 0) RUN(k_cgStartLocal, A, 64);
     else RUN(k_cgJoinAcross, A, 64);
+}
+
+void launch_step_pass(const Batch& Bt, const BatchShape& S, const World* one, int pass, cudaStream_t s) {
+    const unsigned A = list_grid(S, L_ACT, 32), PP = list_grid(S, L_PP, 8);
+    switch (pass) {
+    case WIG_PASS_ADVECT: RUN2(k_advect, true, PP, 256); break;
+    case WIG_PASS_SCATTER: RUN2(k_scatter, true, PP, 256); break;
+    case WIG_PASS_RASTER_CLAIMS: RUN2(k_rasterClaims, true, A, 64); break;
+    default: break;
+    }
 }
 
 void launch_norm(const Dev& D, cudaStream_t s) { k_norm<<<1, 256, 0, s>>>(D); }

@@ -33,6 +33,9 @@ constexpr uint32_t CYCLE_LOOP = 0xffffffffu;
 // spent about 1 us of their 4-5 on it); null for a batch of several.
 int launch_pass(const Batch& Bt, const BatchShape& S, const World* one, const Dev& D0, int pass, uint32_t level,
                 uint32_t cycle, cudaStream_t s);
+// A step's own forms of three passes, which take in two others: advect with
+// sortCount, scatter from the blocks' places, rasterClaims with scanFinish.
+void launch_step_pass(const Batch& Bt, const BatchShape& S, const World* one, int pass, cudaStream_t s);
 // A step's cgStart + cgJoin: part 0 cgStart with each block's own
 // labelling (k_cgStartLocal), part 1 the joins between blocks; the same
 // regions and roots as the two passes.
