@@ -930,6 +930,8 @@ int record_step_fast(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags
     record_pre(R, (flags & WIG_STEP_VISCOUS) != 0u);
     R.labels();
     R.run(WIG_PASS_CG_ANCHOR);
+    const bool bodies = has_bodies(b);
+    if (bodies) R.run(WIG_PASS_CG_BODY_X);
     wig::Marker mk{&Rec::mark, &R};
     ln.Bt.max_cycles = max_cycles;
     ln.Bt.cond = 0;
@@ -943,13 +945,14 @@ int record_step_fast(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags
     }
     wig::fast_setup(ln.Bt, ln.S, one, s, prof ? &mk : nullptr);
     R.launches++;
-    // a single world's iterations are one launch: on a cooperative grid for
-    // WIG_STEP_PERSISTENT, else on the group that suits its size; with the
-    // knob that puts its coarse levels on a cluster, and when profiled,
-    // they are the loop's launches
+    // a single world's iterations are one launch: with bodies (which the
+    // loop's launches do not couple in), for WIG_STEP_PERSISTENT (then on a
+    // cooperative grid at any size), and at the sizes where it is the faster
+    // form; with its coarse levels on a cluster, and when profiled, they are
+    // the loop's launches
     const bool by_size = one && ln.S.cluster == 0u && (one->D.B <= wig::CLUSTER_BLOCKS || one->D.B > wig::GRID_BLOCKS);
-    const bool one_launch = (flags & WIG_STEP_PERSISTENT) || by_size;
-    const bool solve = one_launch && (capture || (flags & WIG_STEP_PERSISTENT));
+    const bool one_launch = (flags & WIG_STEP_PERSISTENT) || bodies || by_size;
+    const bool solve = one_launch && (capture || bodies || (flags & WIG_STEP_PERSISTENT));
     if (solve) {
         CUDA_TRY(wig::fast_solve(ln.Bt, *one, b->solve, (flags & WIG_STEP_PERSISTENT) != 0u, s, prof ? &mk : nullptr));
         R.launches++;
@@ -978,6 +981,7 @@ int record_step_fast(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags
     }
     wig::fast_finish(ln.Bt, ln.S, one, s, prof ? &mk : nullptr);
     R.launches++;
+    if (bodies) R.run(WIG_PASS_CG_BODY_F);
     record_post(R);
     *outside = R.launches;
     return WIG_OK;
@@ -1397,11 +1401,11 @@ int wig_fluid_bind_bodies(wig_fluid* h, void* motion, void* pushes, void* stamps
     return upload_world_entry(b, 0);
 }
 
-// A world with its free bodies bound steps in the plain form (the coupled
-// operator is the reference's pass sequence, fluid.wgsl:2819-2845).
+// A world with its free bodies bound steps in the plain form when asked, else
+// in the fast form, in FP32 (the coupling in the solve's one launch).
 uint32_t step_flags_of(const wig_fluid* h, uint32_t flags) {
     if (!has_bodies(h->b)) return flags;
-    return (flags | WIG_STEP_PLAIN) & ~(WIG_STEP_PERSISTENT | WIG_STEP_MIXED);
+    return flags & ~(WIG_STEP_PERSISTENT | WIG_STEP_MIXED);
 }
 
 int wig_fluid_buffers_of(wig_fluid* h, wig_fluid_buffers* out) {

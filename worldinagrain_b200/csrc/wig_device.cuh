@@ -405,7 +405,8 @@ struct Fine {
     float *rho, *ry;
     uint8_t* mask;  // FM_*; bit d < 4 set when neighbour d is liquid
 };
-constexpr uint32_t FM_PIN = 16u, FM_LIQUID = 32u;  // held at PIN; liquid
+// held at PIN; liquid; liquid and beside a free body's cell
+constexpr uint32_t FM_PIN = 16u, FM_LIQUID = 32u, FM_BODY = 64u;
 
 // A level's operator in binary16 (the mixed-precision form), n values an
 // array from base: on a coarse level its density and four stencil

@@ -26,6 +26,7 @@
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
+#include "wig_bodies.cuh"
 #include "wig_fast.cuh"
 
 namespace wig {
@@ -191,7 +192,7 @@ __device__ __forceinline__ void zeroFine(const FastW& F, uint32_t i) {
 // group of four active blocks an item; the CTA that counts a world's last
 // tile sums its ||b||^2), and the blocks that dropped out this step zeroed
 // (the invariant).
-template <bool ONE>
+template <bool ONE, bool BODIES>
 __global__ void __launch_bounds__(256) k_fSetup(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
     if (!ONE) worldCopyInit(wc_);
@@ -241,7 +242,13 @@ __global__ void __launch_bounds__(256) k_fSetup(Batch Bt, const __grid_constant_
                 const float pinv = (vld(w.gwp(i, G_REGION)) == i) ? PIN : 0.0f;
                 if (pinv > 0.0f) mask |= FM_PIN;
                 float res = gc.y - (sx - (dg + pinv) * gc.x) / 1.0f;
-                R = -res - 0.0f;
+                float coupled = 0.0f;
+                if (BODIES) {
+                    coupled = couplingAt(w, c, PUSH_X);
+                    for (int d = 0; d < 4; d++)
+                        if (rigidAt(w, beside(c, d)) != NONE) mask |= FM_BODY;
+                }
+                R = -res - coupled;
                 double bd = (double)gc.y;
                 b2 = bd * bd;
             }
@@ -1197,13 +1204,22 @@ __device__ void coarseCore(const Dev& D, const W& w, uint32_t lc, float* sm, con
     }
 }
 
+// A coarse level's cell as the reference's field holds it.
+__device__ __forceinline__ void keepLevelCell(const Dev& D, uint32_t l, uint32_t j, float px, float py, float rx, float ry,
+                                              float rho) {
+    float4* f = reinterpret_cast<float4*>(D.field) + D.level_start[l] + 2u * j;
+    f[0] = make_float4(px, py, rx, ry);
+    f[1] = make_float4(rho, 0.0f, 0.0f, 0.0f);
+}
+
 // The levels lc (restricted already, in the scratch) down to the coarsest and
 // back up to lc, in one CTA's shared memory: smoothRed/Black, restrictLevel,
 // solve (40 SOR sweep pairs, omega 1.8), prolong (fluid.wgsl:2318-2470).
 // Each level's face coefficients are worked out once, when its densities
 // are in place, and read by its sweeps and by the restriction below it.
-// Level lc's results go to its ux, uy.
-template <class T>
+// Level lc's results go to its ux, uy; with KEEP, every level's words also
+// to field's coarse levels, as the reference's passes leave them.
+template <class T, bool KEEP = false>
 __device__ void coarseLevels(const Dev& D, const FastW& F, const W& w, uint32_t lc, float* sm, uint32_t* off) {
     const uint32_t L = D.levels;
     const int tid = (int)threadIdx.x, nt = (int)blockDim.x;
@@ -1240,6 +1256,14 @@ __device__ void coarseLevels(const Dev& D, const FastW& F, const W& w, uint32_t 
         for (int j = tid; j < n; j += nt) {
             st(ox + j, V.px[j]);
             st(oy + j, V.py[j]);
+        }
+    }
+    if (KEEP) {
+#pragma unroll 1
+        for (uint32_t l = lc; l <= L; l++) {
+            const SLv V = slv(sm, off, D, l);
+            const int n = V.w * V.h;
+            for (int j = tid; j < n; j += nt) keepLevelCell(D, l, (uint32_t)j, V.px[j], V.py[j], V.rx[j], V.ry[j], V.rho[j]);
         }
     }
 }
@@ -1659,10 +1683,11 @@ __device__ __forceinline__ void forTileRuns(const Batch& Bt, const WorldSrc<ONE>
 
 // prolongFine (fluid.wgsl:2500-2512) of cell c, and its rim for the
 // relaxation after: the cell's words and the prolongation's loaded together,
-// then used for a liquid cell only.  (A lane a quad of cells, whose
+// then used for a liquid cell only.  With KEEP the rim also goes where
+// relaxRims leaves it (counters' G_RIM).  (A lane a quad of cells, whose
 // nine coarse cells it loads once, was slower: 32 us a launch against 21 on
 // a 48-world batch, for want of loads in flight.)
-template <class T>
+template <class T, bool KEEP = false>
 __device__ __forceinline__ void prolongFineCell(const Dev& D, const FastW& F, const W& w, I2 c) {
     const uint32_t i = w.cellIndex(c);
     const uint32_t mk = F.Z.mask[i];
@@ -1672,6 +1697,10 @@ __device__ __forceinline__ void prolongFineCell(const Dev& D, const FastW& F, co
     const float2 v = make_float2(p.x + e.x, p.y + e.y);
     F.Z.pot[i] = v;
     F.Z.rim[i] = v;
+    if (KEEP) {
+        *w.gwp(i, G_RIM) = __float_as_uint(v.x);
+        *w.gwp(i, G_RIM + 1u) = __float_as_uint(v.y);
+    }
 }
 
 template <bool ONE, class T>
@@ -1967,6 +1996,58 @@ __device__ __forceinline__ void applyTile(const Dev& D, const FastW& F, const W&
         if (lane == 0u) out.f[t.n] = x;
     }
     __syncwarp();  // the warp's p is free for its next tile
+}
+
+// With free bodies A p needs every body's J p first: cgDirection and
+// cgBodyP (fluid.wgsl:2767-2776, :2828-2836) of tile j.
+__device__ __forceinline__ void directionTile(const Dev& D, const FastW& F, const W& w, uint32_t j, uint32_t cycle, bool f64,
+                                              float beta, double beta64) {
+    const bool odd = (cycle & 1u) != 0u;
+    const float* Pold = odd ? F.P2 : F.P;
+    float* Pnew = odd ? F.P : F.P2;
+    const TileLane t = tileLane(w, j, true);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        if (!t.in[h]) continue;
+        const uint32_t i = t.i[h], mk = F.Z.mask[i];
+        const float z = F.Z.pot[i].x, po = Pold[i];
+        float p = 0.0f;
+        if ((mk & FM_LIQUID) != 0u) p = f64 ? (float)((double)z + beta64 * (double)po) : z + beta * po;
+        Pnew[i] = p;
+        if ((mk & FM_BODY) != 0u) addPressurePush(w, I2{t.x, t.y[h]}, p, PUSH_P0 + cycle % 2u);
+    }
+}
+// ... and cgApply (fluid.wgsl:2779-2795) of tile j from them, its f32 sums
+// also where the reference's cg keeps them.
+__device__ __forceinline__ void applyCoupledTile(const Dev& D, const FastW& F, const W& w, uint32_t j, uint32_t cycle,
+                                                 bool f64, const Parts& out) {
+    const float* P = (cycle & 1u) != 0u ? F.P : F.P2;
+    const TileLane t = tileLane(w, j, true);
+    float p[2] = {0.0f, 0.0f}, q[2] = {0.0f, 0.0f};
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        if (!t.in[h]) continue;
+        const uint32_t i = t.i[h], mk = F.Z.mask[i];
+        if ((mk & FM_LIQUID) != 0u) {
+            const float4 bb = F.Z.b[i];
+            const float b[4] = {bb.x, bb.y, bb.z, bb.w};
+            p[h] = P[i];
+            float sum = 0.0f;
+#pragma unroll
+            for (int d = 0; d < 4; d++)
+                if (mk & (1u << d)) sum = sum + b[d] * P[nbr(i, t.x, t.y[h], D.W, D.H, d)];
+            const float dgp = diagOf(bb) + ((mk & FM_PIN) != 0u ? PIN : 0.0f);
+            q[h] = dgp * p[h] - sum + ((mk & FM_BODY) != 0u ? couplingAt(w, I2{t.x, t.y[h]}, PUSH_P0 + cycle % 2u) : 0.0f);
+        }
+        F.Q[i] = q[h];
+    }
+    const float x32 = warpTree(p[0] * q[0], p[1] * q[1]);
+    const double x = warpTree((double)p[0] * (double)q[0], (double)p[1] * (double)q[1]);
+    if ((threadIdx.x & 31u) == 0u) {
+        if (f64) out.d[t.n] = x;
+        else out.f[t.n] = x32;
+        reinterpret_cast<float4*>(D.cg)[D.C + t.n] = make_float4(x32, 0.0f, 0.0f, 0.0f);
+    }
 }
 
 // cgDirection + cgApply + cgAlpha (fluid.wgsl:2767-2814).
@@ -2417,7 +2498,10 @@ __device__ __forceinline__ bool groupSums(Group& g, uint32_t B, const T* part, T
 // splits.
 constexpr uint32_t SPLIT_CTAS = 16;
 
-template <class Group, class T>
+// BODIES: the world's free bodies coupled in (A = L + J^T M^-1 J: cgBodyP's
+// phase more an iteration), and the solve's scratch words left in the
+// reference's buffers too.
+template <class Group, class T, bool BODIES>
 __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_fSolve(const __grid_constant__ World Wd, uint32_t max_cycles) {
     extern __shared__ __align__(16) float sm[];
     __shared__ double s64[512];
@@ -2479,7 +2563,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_fSolve(const __grid_consta
                 }
                 if (!g.sync()) return;
             }
-            if (g.rank == 0u) coarseLevels<T>(D, F, w, lc, sm, s_off);
+            if (g.rank == 0u) coarseLevels<T, BODIES>(D, F, w, lc, sm, s_off);
             if (!g.sync()) return;
 #pragma unroll 1
             for (uint32_t l = lc - 1u; l >= 1u; l--) {
@@ -2488,12 +2572,13 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_fSolve(const __grid_consta
                 for (uint32_t t = t0; t < tiles; t += tn) upTile<T, TEAM>(D, F, l, t, lt, tm);
                 if (!g.sync()) return;
             }
+#pragma unroll 1
             for (uint32_t j = w0; j < na; j += wn) {
                 const I2 b = w.activeBlock(j);
 #pragma unroll
                 for (int h = 0; h < 2; h++) {
                     const I2 c{b.x * BLOCK + (int)(lane & 7u), b.y * BLOCK + (int)(lane >> 3) + 4 * h};
-                    if (w.inWorld(c)) prolongFineCell<T>(D, F, w, c);
+                    if (w.inWorld(c)) prolongFineCell<T, BODIES>(D, F, w, c);
                 }
             }
             if (!g.sync()) return;
@@ -2519,9 +2604,17 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_fSolve(const __grid_consta
         __syncthreads();  // the sums are read: their memory is free
         // cgDirection, cgApply, cgAlpha
         const bool odd = (cycle & 1u) != 0u;
+        if (BODIES) {
 #pragma unroll 1
-        for (uint32_t j = w0; j < na; j += wn)
-            applyTile(D, F, w, j, odd, f64, beta32, beta, sm + RIM * RIM * warp, Parts{F.pq64, F.pq32});
+            for (uint32_t j = w0; j < na; j += wn) directionTile(D, F, w, j, cycle, f64, beta32, beta);
+            if (!g.sync()) return;
+#pragma unroll 1
+            for (uint32_t j = w0; j < na; j += wn) applyCoupledTile(D, F, w, j, cycle, f64, Parts{F.pq64, F.pq32});
+        } else {
+#pragma unroll 1
+            for (uint32_t j = w0; j < na; j += wn)
+                applyTile(D, F, w, j, odd, f64, beta32, beta, sm + RIM * RIM * warp, Parts{F.pq64, F.pq32});
+        }
         if (!g.sync()) return;
         if (f64) {
             if (!groupSums<double, 1>(g, D.B, F.pq64, s64, sm, F.col64)) return;
@@ -2533,6 +2626,16 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_fSolve(const __grid_consta
             alpha32 = pq32 <= 0.0f ? 0.0f : rz32 / pq32;
         }
         __syncthreads();
+        if (BODIES && g.rank == 0u) {
+            // the bodies' sums of this iteration's direction, done with,
+            // emptied for the iteration after next (fluid.wgsl:2808-2813),
+            // and the scalars where the reference's cg keeps them
+            const uint32_t which = PUSH_P0 + cycle % 2u;
+            for (uint32_t k = tid; k < MAX_BODIES * 6u; k += SOLVE_THREADS) D.pushes[pushSlot(k / 6u, which, 0u) + k % 6u] = 0u;
+            if (tid == 0u)
+                reinterpret_cast<float4*>(D.cg)[D.C + D.B] =
+                    f64 ? make_float4((float)rz, (float)alpha, (float)beta, (float)pq) : make_float4(rz32, alpha32, beta32, pq32);
+        }
         // cgUpdate
         uint32_t most = 0u;
 #pragma unroll 1
@@ -2575,6 +2678,20 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_fSolve(const __grid_consta
 #pragma unroll 1
                 for (uint32_t j = w0; j < na; j += wn) trueFixTile(D, F, w, j);
                 if (!g.sync()) return;
+            }
+        }
+    }
+    if (BODIES) {
+        // the levels above the coarse ones (no CTA writes them any more)
+        for (uint32_t l = 1; l < lc; l++) {
+            const LRef<T> V = lref<T>(F, l);
+            const auto* ux = upx<T>(F, l);
+            const auto* uy = upy<T>(F, l);
+            const uint32_t n = D.level_w[l] * D.level_h[l];
+            for (uint32_t j = g.rank * SOLVE_THREADS + tid; j < n; j += g.n * SOLVE_THREADS) {
+                const float rho = ld(V.rho + j);
+                const float2 h = V.rhs(j);
+                keepLevelCell(D, l, j, rho > 0.0f ? ld(ux + j) : 0.0f, rho > 0.0f ? ld(uy + j) : 0.0f, h.x, h.y, rho);
             }
         }
     }
@@ -2633,7 +2750,10 @@ void fast_zero_idle(const Batch& Bt, const BatchShape& S, cudaStream_t s) {
 
 void fast_setup(const Batch& Bt, const BatchShape& S, const World* one, cudaStream_t s, const Marker* m) {
     if (m) m->fn(m->ctx, WIG_SLOT_F_SETUP, 0);
-    LAUNCH(k_fSetup, list_grid(S, L_ACT4, 8), 256, 0);
+    const unsigned grid = list_grid(S, L_ACT4, 8);
+    if (one && one->D.motion) k_fSetup<true, true><<<grid, 256, 0, s>>>(Bt, WorldSrc<true>{*one});
+    else if (one) k_fSetup<true, false><<<grid, 256, 0, s>>>(Bt, WorldSrc<true>{*one});
+    else k_fSetup<false, false><<<grid, 256, 0, s>>>(Bt, WorldSrc<false>{});
     if (m) m->fn(m->ctx, WIG_SLOT_F_SETUP, 1);
 }
 
@@ -2811,16 +2931,16 @@ size_t solve_smem(const Dev& D, uint32_t lc) {
     return std::max(fast_coarse_smem(D, lc), least);
 }
 
-template <class Group, class T>
+template <class Group, class T, bool BODIES>
 cudaError_t solve_attributes(size_t smem, bool cluster) {
-    cudaError_t e = cudaFuncSetAttribute(k_fSolve<Group, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(k_fSolve<Group, T, BODIES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess && cluster)
-        e = cudaFuncSetAttribute(k_fSolve<Group, T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        e = cudaFuncSetAttribute(k_fSolve<Group, T, BODIES>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return e;
 }
 
-// Launches k_fSolve<Group, T> on n CTAs: one cluster, or a cooperative grid.
-template <class Group, class T>
+// Launches k_fSolve<Group, T, BODIES> on n CTAs: one cluster, or a cooperative grid.
+template <class Group, class T, bool BODIES>
 cudaError_t solve_launch(const World& Wd, uint32_t max_cycles, uint32_t n, bool cluster, cudaStream_t s) {
     cudaLaunchConfig_t c = {};
     c.gridDim = dim3(n);
@@ -2839,7 +2959,7 @@ cudaError_t solve_launch(const World& Wd, uint32_t max_cycles, uint32_t n, bool 
     }
     c.attrs = at;
     c.numAttrs = 1;
-    return cudaLaunchKernelEx(&c, k_fSolve<Group, T>, Wd, max_cycles);
+    return cudaLaunchKernelEx(&c, k_fSolve<Group, T, BODIES>, Wd, max_cycles);
 }
 
 cudaError_t fast_solve_shape(const Dev& D, SolveShape* out) {
@@ -2848,13 +2968,15 @@ cudaError_t fast_solve_shape(const Dev& D, SolveShape* out) {
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     // the attributes are the kernels', not this world's: room for any
     const size_t most = SOLVE_SMEM_MOST;
-    if (e == cudaSuccess) e = solve_attributes<GridGroup, float>(most, false);
-    if (e == cudaSuccess) e = solve_attributes<GridGroup, __half>(most, false);
-    if (e == cudaSuccess) e = solve_attributes<ClusterGroup, float>(most, true);
-    if (e == cudaSuccess) e = solve_attributes<ClusterGroup, __half>(most, true);
+    if (e == cudaSuccess) e = solve_attributes<GridGroup, float, false>(most, false);
+    if (e == cudaSuccess) e = solve_attributes<GridGroup, float, true>(most, false);
+    if (e == cudaSuccess) e = solve_attributes<GridGroup, __half, false>(most, false);
+    if (e == cudaSuccess) e = solve_attributes<ClusterGroup, float, false>(most, true);
+    if (e == cudaSuccess) e = solve_attributes<ClusterGroup, float, true>(most, true);
+    if (e == cudaSuccess) e = solve_attributes<ClusterGroup, __half, false>(most, true);
     out->lc = coarse_level(D, COARSE_CTA_CELLS);
     const size_t smem = solve_smem(D, out->lc);
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_fSolve<GridGroup, float>, SOLVE_THREADS, smem);
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_fSolve<GridGroup, float, true>, SOLVE_THREADS, smem);
     if (e != cudaSuccess) return e;
     if (per < 1) return cudaErrorInvalidConfiguration;
     out->grid = std::min((uint32_t)sms, std::max(SPLIT_CTAS, (D.B + GRID_TILES - 1u) / GRID_TILES));
@@ -2874,7 +2996,7 @@ cudaError_t fast_solve_shape(const Dev& D, SolveShape* out) {
             c.attrs = at;
             c.numAttrs = 1;
             int fit = 0;
-            if (cudaOccupancyMaxActiveClusters(&fit, k_fSolve<ClusterGroup, float>, &c) == cudaSuccess && fit > 0) out->cluster = n;
+            if (cudaOccupancyMaxActiveClusters(&fit, k_fSolve<ClusterGroup, float, true>, &c) == cudaSuccess && fit > 0) out->cluster = n;
             else cudaGetLastError();
         }
     }
@@ -2887,12 +3009,15 @@ cudaError_t fast_solve(const Batch& Bt, const World& W0, const SolveShape& h, bo
     Wd.S.lc = std::max(Wd.S.lc, h.lc);
     if (m) m->fn(m->ctx, WIG_SLOT_F_SOLVE, 0);
     cudaError_t e;
+    const bool bodies = Wd.D.motion != nullptr;
     if (!grid && h.cluster) {
-        e = Bt.mixed ? solve_launch<ClusterGroup, __half>(Wd, Bt.max_cycles, h.cluster, true, s)
-                     : solve_launch<ClusterGroup, float>(Wd, Bt.max_cycles, h.cluster, true, s);
+        e = bodies      ? solve_launch<ClusterGroup, float, true>(Wd, Bt.max_cycles, h.cluster, true, s)
+            : Bt.mixed  ? solve_launch<ClusterGroup, __half, false>(Wd, Bt.max_cycles, h.cluster, true, s)
+                        : solve_launch<ClusterGroup, float, false>(Wd, Bt.max_cycles, h.cluster, true, s);
     } else {
-        e = Bt.mixed ? solve_launch<GridGroup, __half>(Wd, Bt.max_cycles, h.grid, false, s)
-                     : solve_launch<GridGroup, float>(Wd, Bt.max_cycles, h.grid, false, s);
+        e = bodies      ? solve_launch<GridGroup, float, true>(Wd, Bt.max_cycles, h.grid, false, s)
+            : Bt.mixed  ? solve_launch<GridGroup, __half, false>(Wd, Bt.max_cycles, h.grid, false, s)
+                        : solve_launch<GridGroup, float, false>(Wd, Bt.max_cycles, h.grid, false, s);
     }
     if (m) m->fn(m->ctx, WIG_SLOT_F_SOLVE, 1);
     return e;
