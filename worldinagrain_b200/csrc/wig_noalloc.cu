@@ -28,14 +28,17 @@
 #include <string>
 
 #include "wig_device.cuh"
+#include "wig_sums.cuh"
 
 namespace {
 
 constexpr uint32_t MAX_DEVICES = 64;
 
-// One FP64 partial sum per block; only the entries of the blocks worked on
-// are written and read by a call, so nothing in it has to start at zero.
+// One FP64 partial sum per block; a call writes the entries of all its
+// world's blocks before it reads any, so nothing in it has to start at zero.
 static __device__ __align__(256) double g_block_partials[WIG_NOALLOC_MAX_BLOCKS];
+// The CTAs of the call in flight that have written theirs (back to 0 at its end).
+static __device__ uint32_t g_done;
 
 std::mutex g_mutex;
 double* g_partials_of[MAX_DEVICES] = {nullptr};
@@ -45,52 +48,52 @@ int set_error(int code, const std::string& msg) {
     return code;
 }
 
-// Squared residual of the liquid cells of each block worked on (cg's y,
-// the CG residual r, where field's z > 0), a tree of 64 per block, as the
-// step's tolerance form sums it (k_cgUpdate).  The blocks worked on are
-// those whose state word has ACTIVE set, the same set k_sum_partials reads,
-// so no partial left from an earlier call (of this world or another) can
-// enter the sum, whatever the active list holds.
-__global__ void __launch_bounds__(64) k_block_r2(uint32_t W, uint32_t H, uint32_t B, uint32_t BW, const uint32_t* blocks,
-                                                 const float4* field, const float4* cg, double* partials) {
-    __shared__ double s[64];
-    for (uint32_t n = blockIdx.x; n < B; n += gridDim.x) {
-        if ((blocks[B + n] & 1u) == 0u) continue;  // not worked on (uniform in the CTA)
-        const uint32_t bx = n % BW, by = n / BW;
-        const uint32_t x = bx * 8u + (threadIdx.x & 7u), y = by * 8u + (threadIdx.x >> 3);
-        double v = 0.0;
-        if (x < W && y < H) {
-            const uint32_t i = y * W + x;
-            if (field[2u * i].z > 0.0f) {
+// The squared residual of the liquid cells of each block worked on (cg's y,
+// the CG residual r, where field's z > 0), a warp a block: lane l its cells
+// l and l + 32, the block's tree of 64 as the step's tolerance form sums it;
+// +0 for a block not worked on (its state word's ACTIVE not set).  The last
+// CTA to write its blocks' sums adds them in the step's order (sumColumns).
+// One launch: as a launch of 64-thread blocks and one of a single CTA that
+// read each block's state and partial in turn, the call took 16.4 us on a
+// 1024 x 1024 world.
+constexpr int NORM_THREADS = 512, NORM_WARPS = NORM_THREADS / 32;
+__global__ void __launch_bounds__(NORM_THREADS, 2) k_r2(uint32_t W, uint32_t H, uint32_t B, uint32_t BW, const uint32_t* blocks,
+                                                        const float4* field, const float4* cg, double* partials, double* out) {
+    __shared__ double s[256];
+    __shared__ int last;
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t n = blockIdx.x * NORM_WARPS + (threadIdx.x >> 5); n < B; n += gridDim.x * NORM_WARPS) {
+        double v[2] = {0.0, 0.0};
+        if ((blocks[B + n] & 1u) != 0u) {
+            const uint32_t bx = n % BW, by = n / BW;
+            const uint32_t x = bx * 8u + (lane & 7u);
+#pragma unroll
+            for (uint32_t h = 0; h < 2u; h++) {
+                const uint32_t y = by * 8u + (lane >> 3) + 4u * h;
+                if (x >= W || y >= H) continue;
+                const uint32_t i = y * W + x;
+                const float z = field[2u * i].z;
                 const double r = (double)cg[i].y;
-                v = r * r;
+                if (z > 0.0f) v[h] = r * r;
             }
         }
-        s[threadIdx.x] = v;
-        __syncthreads();
-        for (int h = 32; h > 0; h >>= 1) {
-            if ((int)threadIdx.x < h) s[threadIdx.x] = s[threadIdx.x] + s[threadIdx.x + h];
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) partials[n] = s[0];
-        __syncthreads();
+        const double t = wig::warpTree(v[0], v[1]);
+        if (lane == 0u) partials[n] = t;
     }
-}
-
-// One CTA of 256: the active blocks' partials in block-index order, 256
-// strided runs and a tree (the step's k_norm order).
-__global__ void __launch_bounds__(256) k_sum_partials(uint32_t B, const uint32_t* blocks, const double* partials, double* out) {
-    __shared__ double s[256];
-    double acc = 0.0;
-    for (uint32_t k = threadIdx.x; k < B; k += 256u)
-        if ((blocks[B + k] & 1u) != 0u) acc = acc + partials[k];
-    s[threadIdx.x] = acc;
+    if (lane == 0u) __threadfence();
     __syncthreads();
-    for (int h = 128; h > 0; h >>= 1) {
-        if ((int)threadIdx.x < h) s[threadIdx.x] = s[threadIdx.x] + s[threadIdx.x + h];
-        __syncthreads();
+    if (threadIdx.x == 0u) {
+        last = atomicAdd(&g_done, 1u) + 1u == gridDim.x ? 1 : 0;
+        if (last) {
+            g_done = 0u;
+            __threadfence();
+        }
     }
-    if (threadIdx.x == 0) *out = s[0];
+    __syncthreads();
+    if (!last) return;
+    wig::sumColumns<double, 1, NORM_THREADS>(B, partials, s);
+    wig::treeColumns<double, 1>(s);
+    if (threadIdx.x == 0u) *out = s[0];
 }
 
 // The device address of g_block_partials on the current device, looked up
@@ -131,10 +134,9 @@ int wig_fluid_residual_norm2_noalloc(const wig_world_desc* d, const void* field,
     int rc = partials_on_current_device(&partials);
     if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    const unsigned grid = B < 148u * 32u ? (unsigned)B : 148u * 32u;
-    k_block_r2<<<grid, 64, 0, s>>>(d->width, d->height, (uint32_t)B, BW, (const uint32_t*)blocks, (const float4*)field,
-                                   (const float4*)cg, partials);
-    k_sum_partials<<<1, 256, 0, s>>>((uint32_t)B, (const uint32_t*)blocks, partials, out);
+    const unsigned need = (unsigned)((B + NORM_WARPS - 1u) / NORM_WARPS), grid = need < 148u * 2u ? need : 148u * 2u;
+    k_r2<<<grid, NORM_THREADS, 0, s>>>(d->width, d->height, (uint32_t)B, BW, (const uint32_t*)blocks, (const float4*)field,
+                                       (const float4*)cg, partials, out);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return set_error(WIG_E_CUDA, std::string("launch: ") + cudaGetErrorString(e));
     return WIG_OK;

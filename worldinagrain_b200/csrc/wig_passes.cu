@@ -633,6 +633,74 @@ __global__ void __launch_bounds__(1024) k_compact(Batch Bt, const __grid_constan
     }
 }
 
+// compact of a single world of more blocks than a CTA takes in a few rounds
+// (COMPACT_BLOCKS), in two launches: a thread a block finds its flags
+// (FastW::base, which scanTotals writes later) and each 1024 blocks their
+// counts (FastW::col64, which the solve writes later); then each 1024 write
+// their states and their part of the lists, past the counts before them.
+// One CTA of 1024 threads, each block's 9 marks read by one thread of it,
+// took 64 us of a step at 1024x1024 and 404 us at 2048x2048.
+constexpr uint32_t COMPACT_BLOCKS = 4096, COMPACT_CHUNKS = 512;
+__global__ void __launch_bounds__(1024) k_compactFlags(const __grid_constant__ World Wd) {
+    const Dev& D = Wd.D;
+    const W w(D);
+    const uint32_t n = blockIdx.x * 1024u + threadIdx.x;
+    bool liquid = false, was = false;
+    if (n < D.B) {
+        const uint32_t marks = marksAround(w, w.blockAt(n));
+        liquid = (marks & (MARK_LIQUID | MARK_REGION)) != 0u;
+        was = (D.blocks[w.stateSlot(n)] & ACTIVE) != 0u;
+        Wd.S.base[n] = (liquid ? ACTIVE : 0u) | ((marks & MARK_LIQUID) != 0u ? NEAR_LIQUID : 0u) | (was ? 256u : 0u);
+    }
+    const int na = __syncthreads_count(liquid), nr = __syncthreads_count(!liquid && was);
+    if (threadIdx.x == 0u) {
+        uint32_t* counts = reinterpret_cast<uint32_t*>(Wd.S.col64) + 2u * blockIdx.x;
+        counts[0] = (uint32_t)na;
+        counts[1] = (uint32_t)nr;
+    }
+}
+__global__ void __launch_bounds__(1024) k_compactWrite(const __grid_constant__ World Wd) {
+    __shared__ uint32_t before[2], wa[32], wr[32];
+    const Dev& D = Wd.D;
+    const W w(D);
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint32_t* counts = reinterpret_cast<const uint32_t*>(Wd.S.col64);
+    if (threadIdx.x < 2u) before[threadIdx.x] = 0u;
+    __syncthreads();
+    if (warp < 2u) {
+        // the counts of the chunks before this one: warp 0 the active, 1 the retired
+        uint32_t sum = 0;
+        for (uint32_t c = lane; c < blockIdx.x; c += 32u) sum += counts[2u * c + warp];
+        sum = __reduce_add_sync(0xffffffffu, sum);
+        if (lane == 0u) before[warp] = sum;
+    }
+    const uint32_t n = blockIdx.x * 1024u + threadIdx.x;
+    const uint32_t flags = n < D.B ? Wd.S.base[n] : 0u;
+    const bool liquid = (flags & ACTIVE) != 0u, retired = !liquid && (flags & 256u) != 0u;
+    const uint32_t ma = __ballot_sync(0xffffffffu, liquid), mr = __ballot_sync(0xffffffffu, retired);
+    if (lane == 0u) {
+        wa[warp] = (uint32_t)__popc(ma);
+        wr[warp] = (uint32_t)__popc(mr);
+    }
+    __syncthreads();
+    uint32_t ai = before[0], ri = before[1];
+    for (uint32_t k = 0; k < warp; k++) {
+        ai += wa[k];
+        ri += wr[k];
+    }
+    ai += (uint32_t)__popc(ma & ((1u << lane) - 1u));
+    ri += (uint32_t)__popc(mr & ((1u << lane) - 1u));
+    if (n < D.B) {
+        D.blocks[w.stateSlot(n)] = flags & (ACTIVE | NEAR_LIQUID);
+        if (liquid) D.blocks[w.activeSlot(ai)] = n;
+        else if (retired) D.blocks[w.retiredSlot(ri)] = n;
+    }
+    if (n == D.B - 1u) {
+        D.blocks[w.countSlot(COUNT_ACTIVE)] = ai + (liquid ? 1u : 0u);
+        D.blocks[w.countSlot(COUNT_RETIRED)] = ri + (retired ? 1u : 0u);
+    }
+}
+
 // retire (fluid.wgsl:924-951)
 template <bool ONE>
 __global__ void k_retire(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
@@ -2850,7 +2918,15 @@ int launch_pass(const Batch& Bt, const BatchShape& S, const World* one, const De
     case WIG_PASS_SYNC_MARKS: RUN(k_sync, WB, 64, 0); break;
     case WIG_PASS_SYNC_PARTICLES: RUN(k_syncParticles, PS, 256); break;
     case WIG_PASS_SYNC_SEED: RUN(k_syncSeed, WB, 64); break;
-    case WIG_PASS_COMPACT: RUN(k_compact, ALL, 1024); break;
+    case WIG_PASS_COMPACT:
+        if (one && D.B > COMPACT_BLOCKS && D.B <= COMPACT_CHUNKS * 1024u) {
+            const unsigned chunks = (D.B + 1023u) / 1024u;
+            k_compactFlags<<<chunks, 1024, 0, s>>>(*one);
+            k_compactWrite<<<chunks, 1024, 0, s>>>(*one);
+        } else {
+            RUN(k_compact, ALL, 1024);
+        }
+        break;
     case WIG_PASS_RETIRE: RUN(k_retire, RET, 64); break;
     case WIG_PASS_CLEAR: RUN(k_clear, A, 64); break;
     case WIG_PASS_GATHER: RUN(k_gather, PP, 256); break;
