@@ -52,41 +52,7 @@ namespace {
         if (e_ != cudaSuccess) return fail(WIG_E_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     } while (0)
 
-// Device-side report of a world: the FLUID_COUNT words, the particle count
-// and the solve's residuals, gathered by k_report at the end of a step.
-struct Report {
-    uint32_t count[WIG_FLUID_STATS];
-    uint32_t particles;
-    uint32_t err;
-    uint32_t short_of_tol;  // a tolerance-form solve of a nonzero b stopped above its tolerance
-    uint32_t tried;         // particles the step's sync and seeding put into `parts` (past its room: lost)
-    double rel;
-    double bnorm2;
-    double rel_true;
-};
-
-// Each world's report into its slot (by world) and the lane's (by the
-// world's place in the step's list).
-__global__ void k_report(wig::Batch Bt, Report* by_world, Report* by_entry) {
-    if (threadIdx.x != 0) return;
-    FOR_ITEMS(Bt, wig::L_ONE_ALL, it) {
-        const uint32_t k = (uint32_t)((uint64_t)it >> Bt.lbits);
-        const wig::Dev& D = Bt.worlds[k].D;
-        Report r;
-        for (uint32_t c = 0; c < WIG_FLUID_STATS; c++) r.count[c] = D.blocks[4u * D.B + c];
-        r.particles = D.sorted[0];
-        r.tried = D.parts[0];
-        r.err = D.st->err;
-        // a full step of the tolerance form whose solve stopped (max_cycles
-        // run) with the residual still above the tolerance
-        r.short_of_tol = (D.st->tol_mode && !D.st->book && D.st->bnorm2 > 0.0 && D.st->rel > D.st->tol) ? 1u : 0u;
-        r.rel = D.st->rel;
-        r.bnorm2 = D.st->bnorm2;
-        r.rel_true = D.st->rel_true;
-        by_world[k] = r;
-        by_entry[g_it] = r;
-    }
-}
+using wig::Report;
 
 constexpr int RING = 8;
 
@@ -684,12 +650,13 @@ struct Rec {
         timed(pass, [&] { wig::launch_pass(ln.Bt, ln.S, one_world(b), b->hw[0].D, pass, level, cycle, s); });
     }
     void step_pass(int pass) {
-        timed(pass, [&] { wig::launch_step_pass(ln.Bt, ln.S, one_world(b), pass, s); });
+        timed(pass, [&] { wig::launch_step_pass(ln.Bt, ln.S, one_world(b), wig::ReportTo{b->d_report, ln.d_rsub}, pass, s); });
     }
-    // cgStart + cgJoin as a step runs them (profiled as the two passes)
-    void labels() {
-        timed(WIG_PASS_CG_START, [&] { wig::launch_labels(ln.Bt, ln.S, one_world(b), s, 0); });
-        timed(WIG_PASS_CG_JOIN, [&] { wig::launch_labels(ln.Bt, ln.S, one_world(b), s, 1); });
+    // compact, and the lists that follow it (a batch of one's it writes itself)
+    void compact() {
+        run(WIG_PASS_COMPACT);
+        if (wig::compact_split(one_world(b))) launches++;
+        if (!ln.Bt.single) sched(1);
     }
     void norm() {
         timed(WIG_SLOT_NORM, [&] { wig::launch_norm(b->hw[0].D, s); });
@@ -710,11 +677,6 @@ struct Rec {
             cudaEventRecord(e, s);
             prof->marks.push_back({WIG_SLOT_SCHED, {a, e}});
         }
-    }
-    void report() {
-        timed(WIG_SLOT_REPORT, [&] {
-            k_report<<<wig::list_grid(ln.S, wig::L_ONE_ALL, 4), 32, 0, s>>>(ln.Bt, b->d_report, ln.d_rsub);
-        });
     }
     // the fast form's marker hook: events around each of its launches
     static void mark(void* ctx, int slot, int phase) {
@@ -743,10 +705,8 @@ void record_pre(Rec& R, bool viscous) {
     R.run(WIG_PASS_SYNC);
     R.run(WIG_PASS_SYNC_PARTICLES);
     R.run(WIG_PASS_SYNC_SEED);
-    R.run(WIG_PASS_COMPACT);
-    R.sched(1);
-    R.run(WIG_PASS_RETIRE);
-    R.run(WIG_PASS_CLEAR);
+    R.compact();
+    R.step_pass(WIG_PASS_CLEAR);  // and retire
     R.run(WIG_PASS_GATHER);
     R.run(WIG_PASS_SEAL_JOIN);
     R.run(WIG_PASS_SEAL_ANCHOR);
@@ -766,7 +726,7 @@ void record_pre(Rec& R, bool viscous) {
         R.run(WIG_PASS_BODY_DRAG);
         R.run(WIG_PASS_BODY_FACES);
     }
-    R.run(WIG_PASS_DIVERGENCE);
+    R.step_pass(WIG_PASS_DIVERGENCE);  // and cgStart
 }
 
 // encodeFluid's passes after the solve (js/sim.js:2592-2611) and the report.
@@ -784,18 +744,15 @@ void record_post(Rec& R) {
     R.step_pass(WIG_PASS_SCATTER);
     R.step_pass(WIG_PASS_RASTER_CLAIMS);  // and scanFinish
     R.run(WIG_PASS_RASTER);
-    R.run(WIG_PASS_UNPAINT);
-    R.report();
+    R.step_pass(WIG_PASS_UNPAINT);  // and the report
 }
 
 // A single world's bookkeeping-only step (js/sim.js:2480-2485).
 uint32_t record_book(Rec& R) {
     R.sched(0);
     R.run(WIG_PASS_SYNC_MARKS);
-    R.run(WIG_PASS_COMPACT);
-    R.sched(1);
-    R.run(WIG_PASS_RETIRE);
-    R.report();
+    R.compact();
+    R.step_pass(WIG_PASS_RETIRE);  // and the report
     return R.launches;
 }
 
@@ -878,7 +835,7 @@ int record_step(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags, boo
         return WIG_OK;
     }
     record_pre(R, (flags & WIG_STEP_VISCOUS) != 0u);
-    R.labels();
+    R.step_pass(WIG_PASS_CG_JOIN);
     R.run(WIG_PASS_CG_ANCHOR);
     const bool bodies = has_bodies(b);
     if (bodies) R.run(WIG_PASS_CG_BODY_X);
@@ -928,7 +885,7 @@ int record_step_fast(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags
         return WIG_OK;
     }
     record_pre(R, (flags & WIG_STEP_VISCOUS) != 0u);
-    R.labels();
+    R.step_pass(WIG_PASS_CG_JOIN);
     R.run(WIG_PASS_CG_ANCHOR);
     const bool bodies = has_bodies(b);
     if (bodies) R.run(WIG_PASS_CG_BODY_X);

@@ -941,8 +941,10 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 2) k_fUp(Batch Bt, const _
     }
 }
 
-// Named barrier over the first `count` threads (a multiple of 32).
-__device__ __forceinline__ void barSub(uint32_t count) { asm volatile("bar.sync 1, %0;" ::"r"(count) : "memory"); }
+// Named barrier `id` over `count` threads (a multiple of 32).
+__device__ __forceinline__ void barSub(int id, int count) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
+}
 
 // Level l (lc <= l <= levels) of the one-CTA kernel's shared memory: nine
 // arrays of the level's cells from sm + off[l]: the potentials, the
@@ -1079,15 +1081,13 @@ __device__ __forceinline__ SolveCell solveCell(const SLv& V, int j, int n, float
     c.rd = recipOf(c.dg);
     return c;
 }
-// One SOR update (omega 1.8) of a solve cell from its neighbours' potentials.
-__device__ __forceinline__ void solveUpdate(const SLv& V, const SolveCell& c) {
+// One SOR update (omega 1.8) of a solve cell's potential v in P, h^2 times
+// its right-hand side h, from its neighbours' potentials.
+__device__ __forceinline__ void solveUpdate(float* P, const SolveCell& c, float h, float& v) {
     if (!c.mine) return;
-    float* px = V.px;
-    float* py = V.py;
-    float sx = c.b[0] * px[c.nb[0]] + c.b[1] * px[c.nb[1]] + c.b[2] * px[c.nb[2]] + c.b[3] * px[c.nb[3]];
-    float sy = c.b[0] * py[c.nb[0]] + c.b[1] * py[c.nb[1]] + c.b[2] * py[c.nb[2]] + c.b[3] * py[c.nb[3]];
-    px[c.j] = mixf(px[c.j], quotBy(sx - c.hx, c.rd), OMEGA);
-    py[c.j] = mixf(py[c.j], quotBy(sy - c.hy, c.rd), OMEGA);
+    const float s = c.b[0] * P[c.nb[0]] + c.b[1] * P[c.nb[1]] + c.b[2] * P[c.nb[2]] + c.b[3] * P[c.nb[3]];
+    v = mixf(v, quotBy(s - h, c.rd), OMEGA);
+    P[c.j] = v;
 }
 
 // The levels from lc (in sm from offsets off[]: just loaded, or restricted
@@ -1149,40 +1149,40 @@ __device__ void coarseCore(const Dev& D, const W& w, uint32_t lc, float* sm, con
         __syncthreads();
         if (l < L) slv_smooth(V, l, tid, nt);
     }
-    // solve: the coarsest level.  When its cells fit the CTA, thread k of the
-    // first warps holds cells 2k and 2k + 1, one of each colour (in a row, or
-    // across a row's end when the width is odd), their coefficients in
-    // registers across the sweeps: every thread of those warps updates a
-    // cell each sweep, and only they are synchronised (a named barrier over
-    // npair <= blockDim threads); else a thread per cell of the swept
-    // colour, the CTA synchronised.
+    // solve: the coarsest level (at most 512 cells).  The pressure and the
+    // drift are two solves over the same coefficients: each has its own
+    // warps, under its own named barrier.  Thread k of a solve's holds cells
+    // 2k and 2k + 1, one of each colour (in a row, or across a row's end when
+    // the width is odd), their coefficients and potentials in registers
+    // across the sweeps, so every thread updates a cell each sweep.  Bound by
+    // the chain of a sweep (neighbours, sum, quotient, store, barrier) 80
+    // times: 9.9 us on 16x16 cells, 12.6 with both solves in a thread; the
+    // quotient in f32 with two corrections is no shorter (10.6), and a warp a
+    // solve with no barrier but its own spills (77).
     {
         const SLv V = slv(sm, off, D, L);
         const int n = min(V.w * V.h, (int)WIG_MG_COARSEST);
         const float h2 = (float)(1u << (2u * L));
-        const int pairs = (n + 1) / 2;
-        const uint32_t npair = (uint32_t)((pairs + 31) & ~31);
-        if (npair <= (uint32_t)nt) {
-            if (tid < (int)npair) {
-                SolveCell c0 = solveCell(V, 2 * tid, n, h2), c1 = solveCell(V, 2 * tid + 1, n, h2);
-                // c0 the colour-0 cell, c1 the colour-1 one
-                if (c0.color != 0) {
-                    const SolveCell t = c0;
-                    c0 = c1;
-                    c1 = t;
-                }
-#pragma unroll 1
-                for (int s = 0; s < COARSE_SWEEPS; s++) {
-                    solveUpdate(V, c0);
-                    barSub(npair);
-                    solveUpdate(V, c1);
-                    barSub(npair);
-                }
+        const int pairs = (n + 1) / 2, npair = (pairs + 31) & ~31;
+        static_assert(2 * ((WIG_MG_COARSEST / 2 + 31) & ~31) <= 1024, "the two solves' threads fit the CTA");
+        const int which = tid / npair, k = tid - which * npair;
+        if (which < 2) {
+            SolveCell c0 = solveCell(V, 2 * k, n, h2), c1 = solveCell(V, 2 * k + 1, n, h2);
+            // c0 the colour-0 cell, c1 the colour-1 one
+            if (c0.color != 0) {
+                const SolveCell t = c0;
+                c0 = c1;
+                c1 = t;
             }
-        } else {
-            for (int s = 0; s < 2 * COARSE_SWEEPS; s++) {
-                slv_sweep(V, L, s & 1, OMEGA, tid, nt);
-                __syncthreads();
+            float* P = which ? V.py : V.px;
+            const float h0 = which ? c0.hy : c0.hx, h1 = which ? c1.hy : c1.hx;
+            float v0 = c0.mine ? P[c0.j] : 0.0f, v1 = c1.mine ? P[c1.j] : 0.0f;
+#pragma unroll 1
+            for (int s = 0; s < COARSE_SWEEPS; s++) {
+                solveUpdate(P, c0, h0, v0);
+                barSub(1 + which, npair);
+                solveUpdate(P, c1, h1, v1);
+                barSub(1 + which, npair);
             }
         }
         __syncthreads();

@@ -549,6 +549,28 @@ __global__ void k_syncSeed(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) 
   }
 }
 
+// The worlds' reports, a thread of each CTA its share of the worlds.
+__device__ __forceinline__ void writeReports(const Batch& Bt, const ReportTo& to) {
+    if (threadIdx.x != 0) return;
+    FOR_ITEMS(Bt, L_ONE_ALL, it) {
+        const uint32_t k = (uint32_t)((uint64_t)it >> Bt.lbits);
+        const Dev& D = Bt.worlds[k].D;
+        Report r;
+        for (uint32_t c = 0; c < WIG_FLUID_STATS; c++) r.count[c] = D.blocks[4u * D.B + c];
+        r.particles = D.sorted[0];
+        r.tried = D.parts[0];
+        r.err = D.st->err;
+        // a full step of the tolerance form whose solve stopped (max_cycles
+        // run) with the residual still above the tolerance
+        r.short_of_tol = (D.st->tol_mode && !D.st->book && D.st->bnorm2 > 0.0 && D.st->rel > D.st->tol) ? 1u : 0u;
+        r.rel = D.st->rel;
+        r.bnorm2 = D.st->bnorm2;
+        r.rel_true = D.st->rel_true;
+        to.by_world[k] = r;
+        to.by_entry[g_it] = r;
+    }
+}
+
 // The marks of block b's 3x3 neighbourhood (OR of the blocks inside the world).
 __device__ __forceinline__ uint32_t marksAround(const W& w, I2 b) {
     uint32_t m[9];
@@ -561,6 +583,18 @@ __device__ __forceinline__ uint32_t marksAround(const W& w, I2 b) {
 #pragma unroll
     for (int k = 0; k < 9; k++) marks |= m[k];
     return marks;
+}
+
+// The lengths of the lists that follow compact, of a batch of one (its items
+// are their own units: no list to write).
+__device__ __forceinline__ void compactLists(const Batch& Bt, const Dev& D, uint32_t na, uint32_t nr) {
+    uint32_t* count = const_cast<uint32_t*>(Bt.count);
+    const bool book = D.st->book != 0u;
+    count[L_ACT] = book ? 0u : na;
+    count[L_RET] = nr;
+    count[L_ACT4] = book ? 0u : (na + 3u) / 4u;
+    count[L_RELAX] = book ? 0u : na + D.edge_tiles;
+    count[L_PP] = book ? 0u : (min(D.parts[0], D.cap) + 255u) / 256u;
 }
 
 // compact (fluid.wgsl:896-921): one 1024-thread CTA a world, each thread a
@@ -628,6 +662,7 @@ __global__ void __launch_bounds__(1024) k_compact(Batch Bt, const __grid_constan
         if (threadIdx.x == 1023u) {
             D.blocks[w.countSlot(COUNT_ACTIVE)] = sa[1023];
             D.blocks[w.countSlot(COUNT_RETIRED)] = sr[1023];
+            if (Bt.single) compactLists(Bt, D, sa[1023], sr[1023]);
         }
         __syncthreads();
     }
@@ -659,7 +694,7 @@ __global__ void __launch_bounds__(1024) k_compactFlags(const __grid_constant__ W
         counts[1] = (uint32_t)nr;
     }
 }
-__global__ void __launch_bounds__(1024) k_compactWrite(const __grid_constant__ World Wd) {
+__global__ void __launch_bounds__(1024) k_compactWrite(Batch Bt, const __grid_constant__ World Wd) {
     __shared__ uint32_t before[2], wa[32], wr[32];
     const Dev& D = Wd.D;
     const W w(D);
@@ -698,37 +733,43 @@ __global__ void __launch_bounds__(1024) k_compactWrite(const __grid_constant__ W
     if (n == D.B - 1u) {
         D.blocks[w.countSlot(COUNT_ACTIVE)] = ai + (liquid ? 1u : 0u);
         D.blocks[w.countSlot(COUNT_RETIRED)] = ri + (retired ? 1u : 0u);
+        compactLists(Bt, D, ai + (liquid ? 1u : 0u), ri + (retired ? 1u : 0u));
     }
 }
 
-// retire (fluid.wgsl:924-951)
-template <bool ONE>
-__global__ void k_retire(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
+// retire (fluid.wgsl:924-951) of retired block wid.
+__device__ __forceinline__ void retireBlock(const Dev& D, const FastW& F, const W& w, uint32_t wid) {
+    uint32_t n = D.blocks[w.retiredSlot(wid)];
+    // the solve's sums over the world's blocks take its partials for +0
+    if (threadIdx.x == 0) zeroPartials(D, F, n);
+    if (threadIdx.x == 0) D.blocks[n] = 0u;
+    const I2 bq_ = w.blockAt(n);
+    I2 c{bq_.x * BLOCK + (int)(threadIdx.x & 7u), bq_.y * BLOCK + (int)(threadIdx.x >> 3)};
+    if (!w.inWorld(c)) return;
+    uint32_t i = w.cellIndex(c);
+    reinterpret_cast<float4*>(D.field)[2u * i] = make_float4(0, 0, 0, 0);
+    reinterpret_cast<float4*>(D.field)[2u * i + 1u] = make_float4(0, 0, 0, 0);
+    for (uint32_t g = 0; g < CELL_WORDS; g++) *w.gwp(i, g) = 0u;
+    int fs[4][3];
+    w.facesOf(c, fs);
+    for (int j = 0; j < 4; j++) {
+        if (fs[j][2] < 0) continue;
+        uint32_t f = w.faceIndex(I2{fs[j][0], fs[j][1]}, fs[j][2] == 1);
+        reinterpret_cast<float4*>(D.field)[w.faceSlot(f)] = make_float4(0, 0, 0, 0);
+        *w.viscLastP(f) = 0.0f;
+        D.counters[w.sumSlot(f)] = 0u;
+        D.counters[w.sumSlot(f) + 1u] = 0u;
+    }
+}
+// REPORT (a world's bookkeeping-only step's): the worlds' reports too.
+template <bool ONE, bool REPORT>
+__global__ void k_retire(Batch Bt, const __grid_constant__ WorldSrc<ONE> src, ReportTo to) {
     __shared__ WorldCopy wc_;
     if (!ONE) worldCopyInit(wc_);
+    if (REPORT) writeReports(Bt, to);
     FOR_ITEMS(Bt, L_RET, it) {
         ITEM_WORLD_S(Bt, it, D, w, wid);
-        uint32_t n = D.blocks[w.retiredSlot(wid)];
-        // the solve's sums over the world's blocks take its partials for +0
-        if (threadIdx.x == 0) zeroPartials(D, Wd_it.S, n);
-        const I2 bq_ = w.blockAt(n);
-        I2 c{bq_.x * BLOCK + (int)(threadIdx.x & 7u), bq_.y * BLOCK + (int)(threadIdx.x >> 3)};
-        if (!w.inWorld(c)) continue;
-        uint32_t i = w.cellIndex(c);
-        reinterpret_cast<float4*>(D.field)[2u * i] = make_float4(0, 0, 0, 0);
-        reinterpret_cast<float4*>(D.field)[2u * i + 1u] = make_float4(0, 0, 0, 0);
-        for (uint32_t g = 0; g < CELL_WORDS; g++) *w.gwp(i, g) = 0u;
-        int fs[4][3];
-        w.facesOf(c, fs);
-        for (int j = 0; j < 4; j++) {
-            if (fs[j][2] < 0) continue;
-            uint32_t f = w.faceIndex(I2{fs[j][0], fs[j][1]}, fs[j][2] == 1);
-            reinterpret_cast<float4*>(D.field)[w.faceSlot(f)] = make_float4(0, 0, 0, 0);
-            *w.viscLastP(f) = 0.0f;
-            D.counters[w.sumSlot(f)] = 0u;
-            D.counters[w.sumSlot(f) + 1u] = 0u;
-        }
-        if (threadIdx.x == 0) D.blocks[n] = 0u;
+        retireBlock(D, Wd_it.S, w, wid);
     }
 }
 
@@ -737,10 +778,18 @@ __global__ void k_retire(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
 // stores a thread for the block; a thread a cell writing its 11 words 44
 // bytes from its neighbour's touched 8 times the sectors (70 us a step of a
 // 48-world batch, 127 us of the 2048x2048 column).
-template <bool ONE>
+// RETIRE (a step's): the retired blocks first (their words are other cells',
+// but for faces both zero).
+template <bool ONE, bool RETIRE>
 __global__ void k_clear(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
     if (!ONE) worldCopyInit(wc_);
+    if (RETIRE) {
+        FOR_ITEMS(Bt, L_RET, rt) {
+            ITEM_WORLD_S(Bt, rt, D, w, wid);
+            retireBlock(D, Wd_rt.S, w, wid);
+        }
+    }
     FOR_ITEMS(Bt, L_ACT, it) {
         ITEM_WORLD_S(Bt, it, D, w, wid);
         I2 b = w.activeBlock(wid);
@@ -1293,35 +1342,6 @@ __global__ void k_viscosity(Batch Bt, const __grid_constant__ WorldSrc<ONE> src,
     }
 }
 
-// divergence (fluid.wgsl:1996-2025)
-template <bool ONE>
-__global__ void k_divergence(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
-    __shared__ WorldCopy wc_;
-    if (!ONE) worldCopyInit(wc_);
-    // once a world: its residual and iteration words cleared
-    if (threadIdx.x == 0) {
-        FOR_ITEMS(Bt, L_ONE, ot) {
-            ITEM_WORLD(Bt, ot, D, w, unused_);
-            (void)unused_;
-            D.blocks[w.countSlot(COUNT_RESIDUAL)] = 0u;
-            D.blocks[w.countSlot(COUNT_CYCLES)] = 0u;
-        }
-    }
-    FOR_ITEMS(Bt, L_ACT, it) {
-        ITEM_WORLD_S(Bt, it, D, w, wid);
-        I2 c = lidCell(w, wid);
-        if (!w.inWorld(c)) continue;
-        uint32_t i = w.cellIndex(c);
-        if (w.fv(2u * i)[2] <= 0.0f) continue;
-        float out = w.fv(w.faceSlot(w.uFace(c.x + 1, c.y)))[0] - w.fv(w.faceSlot(w.uFace(c.x, c.y)))[0] +
-                    w.fv(w.faceSlot(w.vFace(c.x, c.y + 1)))[0] - w.fv(w.faceSlot(w.vFace(c.x, c.y)))[0];
-        w.fv(2u * i)[1] = out;
-        float n = w.densityAt(c);
-        float room = posedRoom(w, c);
-        w.fv(2u * i + 1u)[1] = w.fv(2u * i + 1u)[2] < 0.0f ? 0.0f : -SPREAD * (n - room);
-    }
-}
-
 // ================================================================ the solve's start
 
 // cgStart (fluid.wgsl:2665-2674)
@@ -1364,42 +1384,70 @@ __global__ void k_cgJoin(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
 // regions, their roots and every ufFind are those of cgJoin's; only the
 // intermediate links, a lock-free union-find's timing in the reference too,
 // differ (cgFinish clears them all).
-template <bool ONE>
-__global__ void k_cgStartLocal(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
+__device__ __forceinline__ void startLocal(const Dev& D, const W& w, I2 c, uint32_t* lab) {
+    const bool in = w.inWorld(c);
+    const uint32_t i = in ? w.cellIndex(c) : 0u;
+    bool fluid = false;
+    if (in) {
+        const float4 g = w.gridAt(c);
+        reinterpret_cast<float4*>(D.cg)[i] = make_float4(g.x, 0.0f, 0.0f, 0.0f);
+        fluid = g.z > 0.0f;
+    }
+    const int t = (int)threadIdx.x, lx = t & 7, ly = t >> 3;
+    lab[t] = fluid ? i : 0xffffffffu;
+    __syncthreads();
+    for (int round = 0; round < 64; round++) {
+        uint32_t m = lab[t];
+        if (fluid) {
+            if (lx > 0) m = min(m, lab[t - 1]);
+            if (lx < 7) m = min(m, lab[t + 1]);
+            if (ly > 0) m = min(m, lab[t - 8]);
+            if (ly < 7) m = min(m, lab[t + 8]);
+        }
+        __syncthreads();
+        const bool changed = m < lab[t];
+        lab[t] = m;
+        if (!__syncthreads_or(changed)) break;
+    }
+    if (in) *w.gwp(i, G_REGION) = fluid ? lab[t] : i;
+    __syncthreads();
+}
+
+// divergence (fluid.wgsl:1996-2025) of cell c.
+__device__ __forceinline__ void divergenceAt(const W& w, I2 c) {
+    uint32_t i = w.cellIndex(c);
+    if (w.fv(2u * i)[2] <= 0.0f) return;
+    float out = w.fv(w.faceSlot(w.uFace(c.x + 1, c.y)))[0] - w.fv(w.faceSlot(w.uFace(c.x, c.y)))[0] +
+                w.fv(w.faceSlot(w.vFace(c.x, c.y + 1)))[0] - w.fv(w.faceSlot(w.vFace(c.x, c.y)))[0];
+    w.fv(2u * i)[1] = out;
+    float n = w.densityAt(c);
+    float room = posedRoom(w, c);
+    w.fv(2u * i + 1u)[1] = w.fv(2u * i + 1u)[2] < 0.0f ? 0.0f : -SPREAD * (n - room);
+}
+// divergence, and with START (a step's) cgStart with the block's own
+// labelling (startLocal: neither reads what the other writes).
+template <bool ONE, bool START>
+__global__ void k_divergence(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
     if (!ONE) worldCopyInit(wc_);
     __shared__ uint32_t lab[64];
+    // once a world: its residual and iteration words cleared
+    if (threadIdx.x == 0) {
+        FOR_ITEMS(Bt, L_ONE, ot) {
+            ITEM_WORLD(Bt, ot, D, w, unused_);
+            (void)unused_;
+            D.blocks[w.countSlot(COUNT_RESIDUAL)] = 0u;
+            D.blocks[w.countSlot(COUNT_CYCLES)] = 0u;
+        }
+    }
     FOR_ITEMS(Bt, L_ACT, it) {
         ITEM_WORLD_S(Bt, it, D, w, wid);
-        const I2 c = lidCell(w, wid);
-        const bool in = w.inWorld(c);
-        const uint32_t i = in ? w.cellIndex(c) : 0u;
-        bool fluid = false;
-        if (in) {
-            const float4 g = w.gridAt(c);
-            reinterpret_cast<float4*>(D.cg)[i] = make_float4(g.x, 0.0f, 0.0f, 0.0f);
-            fluid = g.z > 0.0f;
-        }
-        const int t = (int)threadIdx.x, lx = t & 7, ly = t >> 3;
-        lab[t] = fluid ? i : 0xffffffffu;
-        __syncthreads();
-        for (int round = 0; round < 64; round++) {
-            uint32_t m = lab[t];
-            if (fluid) {
-                if (lx > 0) m = min(m, lab[t - 1]);
-                if (lx < 7) m = min(m, lab[t + 1]);
-                if (ly > 0) m = min(m, lab[t - 8]);
-                if (ly < 7) m = min(m, lab[t + 8]);
-            }
-            __syncthreads();
-            const bool changed = m < lab[t];
-            lab[t] = m;
-            if (!__syncthreads_or(changed)) break;
-        }
-        if (in) *w.gwp(i, G_REGION) = fluid ? lab[t] : i;
-        __syncthreads();
+        I2 c = lidCell(w, wid);
+        if (w.inWorld(c)) divergenceAt(w, c);
+        if (START) startLocal(D, w, c, lab);
     }
 }
+
 // cgJoin's edges between blocks (to the right and below, from the block's
 // last column and row), after k_cgStartLocal has linked each block's own.
 // An edge is left to the one before it along the border (above it, or to
@@ -2699,11 +2747,12 @@ __global__ void k_raster(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     }
 }
 
-// unpaint (fluid.wgsl:4163-4182)
-template <bool ONE>
-__global__ void k_unpaint(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
+// unpaint (fluid.wgsl:4163-4182); with REPORT (a step's) the worlds' reports.
+template <bool ONE, bool REPORT>
+__global__ void k_unpaint(Batch Bt, const __grid_constant__ WorldSrc<ONE> src, ReportTo to) {
     __shared__ WorldCopy wc_;
     if (!ONE) worldCopyInit(wc_);
+    if (REPORT) writeReports(Bt, to);
     FOR_ITEMS(Bt, L_ACT, it) {
         ITEM_WORLD_S(Bt, it, D, w, wid);
         I2 c = lidCell(w, wid);
@@ -2895,10 +2944,10 @@ unsigned list_grid(const BatchShape& S, uint32_t list, unsigned per_sm) {
     } while (0)
 
 // The same for a kernel with a variant.
-#define RUN2(K, V, grid, block)                                                          \
-    do {                                                                                 \
-        if (one) K<true, V><<<(grid), (block), 0, s>>>(Bt, WorldSrc<true>{*one});          \
-        else K<false, V><<<(grid), (block), 0, s>>>(Bt, WorldSrc<false>{});                \
+#define RUN2(K, V, grid, block, ...)                                                                \
+    do {                                                                                            \
+        if (one) K<true, V><<<(grid), (block), 0, s>>>(Bt, WorldSrc<true>{*one}, ##__VA_ARGS__);      \
+        else K<false, V><<<(grid), (block), 0, s>>>(Bt, WorldSrc<false>{}, ##__VA_ARGS__);            \
     } while (0)
 
 int launch_pass(const Batch& Bt, const BatchShape& S, const World* one, const Dev& D0, int pass, uint32_t level,
@@ -2919,16 +2968,16 @@ int launch_pass(const Batch& Bt, const BatchShape& S, const World* one, const De
     case WIG_PASS_SYNC_PARTICLES: RUN(k_syncParticles, PS, 256); break;
     case WIG_PASS_SYNC_SEED: RUN(k_syncSeed, WB, 64); break;
     case WIG_PASS_COMPACT:
-        if (one && D.B > COMPACT_BLOCKS && D.B <= COMPACT_CHUNKS * 1024u) {
+        if (compact_split(one)) {
             const unsigned chunks = (D.B + 1023u) / 1024u;
             k_compactFlags<<<chunks, 1024, 0, s>>>(*one);
-            k_compactWrite<<<chunks, 1024, 0, s>>>(*one);
+            k_compactWrite<<<chunks, 1024, 0, s>>>(Bt, *one);
         } else {
             RUN(k_compact, ALL, 1024);
         }
         break;
-    case WIG_PASS_RETIRE: RUN(k_retire, RET, 64); break;
-    case WIG_PASS_CLEAR: RUN(k_clear, A, 64); break;
+    case WIG_PASS_RETIRE: RUN2(k_retire, false, RET, 64, ReportTo{}); break;
+    case WIG_PASS_CLEAR: RUN2(k_clear, false, A, 64); break;
     case WIG_PASS_GATHER: RUN(k_gather, PP, 256); break;
     case WIG_PASS_SEAL_JOIN: RUN(k_sealJoin, A, 64); break;
     case WIG_PASS_SEAL_ANCHOR: RUN(k_sealAnchor, A, 64); break;
@@ -2937,7 +2986,7 @@ int launch_pass(const Batch& Bt, const BatchShape& S, const World* one, const De
     case WIG_PASS_VISCOSITY_RED: RUN(k_viscosity, A, 64, 0); break;
     case WIG_PASS_VISCOSITY_BLACK: RUN(k_viscosity, A, 64, 1); break;
     case WIG_PASS_UNPRESS: RUN(k_viscosity, A, 64, 2); break;
-    case WIG_PASS_DIVERGENCE: RUN(k_divergence, A, 64); break;
+    case WIG_PASS_DIVERGENCE: RUN2(k_divergence, false, A, 64); break;
     case WIG_PASS_CG_START: RUN(k_cgStart, A, 64); break;
     case WIG_PASS_CG_JOIN: RUN(k_cgJoin, A, 64); break;
     case WIG_PASS_CG_ANCHOR: RUN(k_cgAnchor, A, 64); break;
@@ -2970,7 +3019,7 @@ int launch_pass(const Batch& Bt, const BatchShape& S, const World* one, const De
     case WIG_PASS_SCATTER: RUN2(k_scatter, false, PP, 256); break;
     case WIG_PASS_RASTER_CLAIMS: RUN2(k_rasterClaims, false, A, 64); break;
     case WIG_PASS_RASTER: RUN(k_raster, A, 64); break;
-    case WIG_PASS_UNPAINT: RUN(k_unpaint, A, 64); break;
+    case WIG_PASS_UNPAINT: RUN2(k_unpaint, false, A, 64, ReportTo{}); break;
     default:
         // the bodies' passes: world 0 with its bodies bound (no-ops without)
         if (pass < WIG_PASS_BODY_START || pass > WIG_PASS_BODY_PUSH) return WIG_E_ARG;
@@ -2992,20 +3041,23 @@ int launch_pass(const Batch& Bt, const BatchShape& S, const World* one, const De
     return WIG_OK;
 }
 
-void launch_labels(const Batch& Bt, const BatchShape& S, const World* one, cudaStream_t s, int part) {
-    const unsigned A = list_grid(S, L_ACT, 32);
-    if (part == 0) RUN(k_cgStartLocal, A, 64);
-    else RUN(k_cgJoinAcross, A, 64);
-}
-
-void launch_step_pass(const Batch& Bt, const BatchShape& S, const World* one, int pass, cudaStream_t s) {
-    const unsigned A = list_grid(S, L_ACT, 32), PP = list_grid(S, L_PP, 8);
+void launch_step_pass(const Batch& Bt, const BatchShape& S, const World* one, const ReportTo& to, int pass, cudaStream_t s) {
+    const unsigned A = list_grid(S, L_ACT, 32), RET = list_grid(S, L_RET, 32), PP = list_grid(S, L_PP, 8);
     switch (pass) {
+    case WIG_PASS_RETIRE: RUN2(k_retire, true, RET, 64, to); break;
+    case WIG_PASS_CLEAR: RUN2(k_clear, true, A, 64); break;
+    case WIG_PASS_DIVERGENCE: RUN2(k_divergence, true, A, 64); break;
+    case WIG_PASS_CG_JOIN: RUN(k_cgJoinAcross, A, 64); break;
     case WIG_PASS_ADVECT: RUN2(k_advect, true, PP, 256); break;
     case WIG_PASS_SCATTER: RUN2(k_scatter, true, PP, 256); break;
     case WIG_PASS_RASTER_CLAIMS: RUN2(k_rasterClaims, true, A, 64); break;
+    case WIG_PASS_UNPAINT: RUN2(k_unpaint, true, A, 64, to); break;
     default: break;
     }
+}
+
+bool compact_split(const World* one) {
+    return one && one->D.B > COMPACT_BLOCKS && one->D.B <= COMPACT_CHUNKS * 1024u;
 }
 
 void launch_norm(const Dev& D, cudaStream_t s) { k_norm<<<1, 256, 0, s>>>(D); }

@@ -33,13 +33,33 @@ constexpr uint32_t CYCLE_LOOP = 0xffffffffu;
 // spent about 1 us of their 4-5 on it); null for a batch of several.
 int launch_pass(const Batch& Bt, const BatchShape& S, const World* one, const Dev& D0, int pass, uint32_t level,
                 uint32_t cycle, cudaStream_t s);
-// A step's own forms of three passes, which take in two others: advect with
-// sortCount, scatter from the blocks' places, rasterClaims with scanFinish.
-void launch_step_pass(const Batch& Bt, const BatchShape& S, const World* one, int pass, cudaStream_t s);
-// A step's cgStart + cgJoin: part 0 cgStart with each block's own
-// labelling (k_cgStartLocal), part 1 the joins between blocks; the same
-// regions and roots as the two passes.
-void launch_labels(const Batch& Bt, const BatchShape& S, const World* one, cudaStream_t s, int part);
+// Device-side report of a world: the FLUID_COUNT words, the particle count
+// and the solve's residuals, gathered at the end of a step.
+struct Report {
+    uint32_t count[WIG_FLUID_STATS];
+    uint32_t particles;
+    uint32_t err;
+    uint32_t short_of_tol;  // a tolerance-form solve of a nonzero b stopped above its tolerance
+    uint32_t tried;         // particles the step's sync and seeding put into `parts` (past its room: lost)
+    double rel;
+    double bnorm2;
+    double rel_true;
+};
+// Where a step's reports go: by the world, and by its place in the step's list.
+struct ReportTo {
+    Report* by_world;
+    Report* by_entry;
+};
+// A step's own forms of some passes, which take in others: retire with the
+// reports (a bookkeeping-only step's last pass), clear with retire,
+// divergence with cgStart (its block's own labelling), cgJoin across the
+// blocks (the same regions and roots as cgStart and cgJoin), advect with
+// sortCount, scatter from the blocks' places, rasterClaims with scanFinish,
+// unpaint with the reports.  Each took a launch of 2.5-4 us on a small
+// world, and on a large one a pass over its words.
+void launch_step_pass(const Batch& Bt, const BatchShape& S, const World* one, const ReportTo& to, int pass, cudaStream_t s);
+// Whether a single world's compact is two launches.
+bool compact_split(const World* one);
 // The plain form's ||b||^2 of world 0 after cgResidual (the tolerance form).
 void launch_norm(const Dev& D, cudaStream_t s);
 // The end of an iteration of the plain form's loop on world 0, after
