@@ -39,3 +39,39 @@ def test_fast_steps_with_bodies_equal_plain(size, case):
     assert ca == cb
     diffs = compare_worlds(wa, wb) + [d for n in ("motion", "pushes") if (d := diff_words(getattr(ba, n), getattr(bb, n), n))]
     assert not diffs, "; ".join(diffs)
+
+
+class _Bytes:
+    def __init__(self, ptr, n):
+        self.__cuda_array_interface__ = {"data": (ptr, False), "shape": (n,), "typestr": "|u1", "version": 2}
+
+
+def test_a_host_writing_its_buffers_needs_no_rebinding():
+    """The world taken back by the host's own copies after 30 steps, blocks
+    then worked on idle again; no bind call tells the handle."""
+    import numpy as np
+    import torch
+    from worldinagrain_b200 import fluid
+    world, bodies = W.bodies_world(160, 120, stamps=False)
+    got = []
+    for form in (0, abi.STEP_PLAIN):
+        w, b = world.copy(), bodies.copy()
+        g = fluid.LiquidStep(w, W.body_element_table())
+        g.bind_bodies(b)
+        for s in range(1, 31):
+            g.step(params(w, s), max_cycles=64, flags=TOL | form, tolerance=1e-6)
+        torch.cuda.synchronize()
+        at = g.buffers()
+        for name in abi.BUFFER_NAMES:
+            a = np.ascontiguousarray(getattr(world, name)).view(np.uint8).reshape(-1)
+            torch.as_tensor(_Bytes(getattr(at, name), a.size), device="cuda").copy_(torch.from_numpy(a.copy()))
+        torch.cuda.synchronize()
+        for s in range(1, 4):
+            g.step(params(w, s), max_cycles=64, flags=TOL | form, tolerance=1e-6)
+        g.download()
+        g.download_bodies(b)
+        g.close()
+        got.append((w, b))
+    (wa, ba), (wb, bb) = got
+    diffs = compare_worlds(wa, wb) + [d for n in ("motion", "pushes") if (d := diff_words(getattr(ba, n), getattr(bb, n), n))]
+    assert not diffs, "; ".join(diffs)

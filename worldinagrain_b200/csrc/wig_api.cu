@@ -896,7 +896,10 @@ int record_step_fast(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags
     ln.Bt.cond_drift = 0;
     ln.Bt.mixed = (flags & WIG_STEP_MIXED) ? 1u : 0u;
     const wig::World* one = one_world(b);
-    if (b->pooled) {
+    // the idle blocks' scratch: a pooled step's is lent; and a host that binds
+    // bodies may write its buffers between steps without binding them again
+    // (the plain form, which such a world used to step in, reads no scratch)
+    if (b->pooled || bodies) {
         wig::fast_zero_idle(ln.Bt, ln.S, s);
         R.launches++;
     }
