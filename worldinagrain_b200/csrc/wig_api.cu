@@ -230,6 +230,7 @@ size_t scratch_bytes(const wig::Dev& D) {
     size_t bytes = align256(C) + 3u * align256(C * 8u) + align256(C * 16u) + 7u * align256(C * 4u);
     for (uint32_t l = 1; l <= D.levels; l++) {
         bytes += 11u * align256((size_t)D.level_w[l] * D.level_h[l] * 4u);
+        bytes += align256(wig::levelTiles(D.level_w[l], D.level_h[l]));
         bytes += align256(5u * (size_t)D.level_w[l] * D.level_h[l] * 2u);  // the binary16 operator
     }
     bytes += align256(2u * (size_t)D.B * 4u) + 3u * align256(2u * (size_t)D.B * 8u);
@@ -256,6 +257,7 @@ void scratch_take(wig::World& Wd, char* p, uint32_t coarse_cells) {
         V.px = fl(n); V.py = fl(n); V.rx = fl(n); V.ry = fl(n); V.rho = fl(n);
         V.b0 = fl(n); V.b1 = fl(n); V.b2 = fl(n); V.b3 = fl(n);
         V.ux = fl(n); V.uy = fl(n);
+        V.live = reinterpret_cast<uint8_t*>(take(wig::levelTiles(D.level_w[l], D.level_h[l])));
     }
     F.H[0] = wig::LvlH{reinterpret_cast<__half*>(take(4u * C * 2u)), (uint32_t)C, 0u};
     for (uint32_t l = 1; l <= D.levels; l++) {

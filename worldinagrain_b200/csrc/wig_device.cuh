@@ -393,6 +393,7 @@ struct Lvl {
     float *px, *py, *rx, *ry, *rho;
     float *b0, *b1, *b2, *b3;
     float *ux, *uy;  // the potentials after the V-cycle's way up (the way down's stay in px, py)
+    uint8_t* live;   // whether a 16x16 tile holds liquid (levelTiles of them)
 };
 
 // Level 0, the cells (row-major).  What its kernels read of one cell lies

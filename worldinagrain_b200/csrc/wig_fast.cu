@@ -367,6 +367,10 @@ struct LRef {
     }
     __device__ __forceinline__ float dens(uint32_t k) const { return ld(rho + k); }
     __device__ __forceinline__ float pin(uint32_t) const { return 0.0f; }
+    __device__ __forceinline__ void flags(uint32_t k, bool* liquid, float* pinv) const {
+        *liquid = dens(k) > 0.0f;
+        *pinv = 0.0f;
+    }
 };
 template <class T>
 __device__ __forceinline__ LRef<T> lref(const FastW& F, uint32_t l);
@@ -401,6 +405,11 @@ struct LRef0 {
     __device__ __forceinline__ float4 coef(uint32_t k) const { return fineCoef(F, k, T()); }
     __device__ __forceinline__ float dens(uint32_t k) const { return F.Z.rho[k]; }
     __device__ __forceinline__ float pin(uint32_t k) const { return (F.Z.mask[k] & FM_PIN) != 0u ? PIN : 0.0f; }
+    __device__ __forceinline__ void flags(uint32_t k, bool* liquid, float* pinv) const {
+        const uint32_t m = F.Z.mask[k];
+        *liquid = (m & FM_LIQUID) != 0u;
+        *pinv = (m & FM_PIN) != 0u ? PIN : 0.0f;
+    }
 };
 // Level l's way-up potentials (l >= 1) as a level of operator T stores them.
 template <class T>
@@ -629,6 +638,52 @@ __device__ __forceinline__ void restrictedFrom(const Dev& D, const W& w, uint32_
     ry_o = rho > 0.0f ? ry * 0.25f : 0.0f;
 }
 
+// The restricted residuals alone of a liquid level-l cell (its density, like
+// every level's densities and coefficients, is the step's first
+// iteration's): its finer cells are liquid or obstacles.
+template <class VT>
+__device__ __forceinline__ V2 residualsFrom(const Dev& D, uint32_t l, const VT& U, int cx, int cy) {
+    const int uw = (int)D.level_w[l - 1], uh = (int)D.level_h[l - 1];
+    const int x0 = 2 * cx, y0 = 2 * cy;
+    const bool in_x = x0 + 1 < uw, in_y = y0 + 1 < uh;
+    const uint32_t xs[4] = {(uint32_t)max(x0 - 1, 0), (uint32_t)x0, (uint32_t)min(x0 + 1, uw - 1), (uint32_t)min(x0 + 2, uw - 1)};
+    const uint32_t ys[4] = {(uint32_t)max(y0 - 1, 0) * (uint32_t)uw, (uint32_t)y0 * (uint32_t)uw,
+                            (uint32_t)min(y0 + 1, uh - 1) * (uint32_t)uw, (uint32_t)min(y0 + 2, uh - 1) * (uint32_t)uw};
+    const float inv_h2 = 1.0f / (float)(1u << (2u * (l - 1u)));
+    float2 p[4][4];  // [row][column], corners not read
+    float4 bq[4];
+    float2 hq[4];
+    float pq[4];
+    bool liquid[4];
+#pragma unroll
+    for (int y = 0; y < 4; y++)
+#pragma unroll
+        for (int x = 0; x < 4; x++)
+            if ((x == 1 || x == 2) || (y == 1 || y == 2)) p[y][x] = U.pot(ys[y] + xs[x]);
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        const uint32_t k = ys[1 + (q >> 1)] + xs[1 + (q & 1)];
+        bq[q] = U.coef(k);
+        hq[q] = U.rhs(k);
+        U.flags(k, &liquid[q], &pq[q]);
+    }
+    float rx = 0.0f, ry = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        if ((!in_x && (q & 1)) || (!in_y && (q >> 1)) || !liquid[q]) continue;
+        const int x = 1 + (q & 1), y = 1 + (q >> 1);
+        const V2 e = residualOf(bq[q], p[y][x], p[y][x - 1], p[y][x + 1], p[y - 1][x], p[y + 1][x], hq[q], pq[q], inv_h2);
+        rx = rx + e.x;
+        ry = ry + e.y;
+    }
+    return V2{rx * 0.25f, ry * 0.25f};
+}
+template <class T, bool FINE>
+__device__ __forceinline__ V2 residualsAt(const Dev& D, const FastW& F, uint32_t l, int cx, int cy) {
+    if (FINE) return residualsFrom(D, l, LRef0<T>{F}, cx, cy);
+    return residualsFrom(D, l, lref<T>(F, l - 1u), cx, cy);
+}
+
 // restrictedFrom for level l of a form whose levels store operator T: from
 // level 0 as its smoother reads it (FINE: l is 1), or from level l - 1.
 template <class T, bool FINE>
@@ -641,10 +696,20 @@ __device__ __forceinline__ void restrictedAt(const Dev& D, const FastW& F, const
 // One coarse cell of restrictLevel, level l from l - 1 (FINE: level 1 from
 // level 0) with the levels stored as T: the cell's values, its potentials
 // zeroed.
-template <class T, bool FINE>
-__device__ void restrictCell(const Dev& D, const FastW& F, const W& w, uint32_t l, uint32_t j) {
+template <class T, bool FINE, bool EAGER>
+__device__ void restrictCell(const Dev& D, const FastW& F, const W& w, uint32_t l, uint32_t j, bool first) {
     const int lw = (int)D.level_w[l];
     const LRef<T> V = lref<T>(F, l);
+    if (!first) {
+        // only a liquid cell's right-hand sides have changed
+        const float rho = V.dens(j);
+        if (!EAGER && !(rho > 0.0f)) return;
+        const V2 r = residualsAt<T, FINE>(D, F, l, (int)(j % (uint32_t)lw), (int)(j / (uint32_t)lw));
+        if (EAGER && !(rho > 0.0f)) return;
+        st(V.rx + j, r.x);
+        st(V.ry + j, r.y);
+        return;
+    }
     float rho, rx, ry;
     restrictedAt<T, FINE>(D, F, w, l, (int)(j % (uint32_t)lw), (int)(j / (uint32_t)lw), true, rho, rx, ry);
     st(V.px + j, 0.0f);
@@ -772,74 +837,123 @@ __device__ __forceinline__ void tileSmooth(LevelTile& t, const Team<NT>& tm, int
 
 // Down, level l: restrictLevel, then smoothRed and smoothBlack when the
 // world smooths level l (l < its coarse kernel's first level; else the
-// restriction alone).  The coefficients of each liquid cell of the ring of 1
-// from the densities (as the step's first iteration works and stores them,
-// and later ones read them back), stored by the tile's own cells on the
-// first iteration.
-template <class T, int NT, bool FINE>
+// restriction alone).  The densities and the coefficients of a level are the
+// same in every iteration of a step: the first works the densities out on
+// the ring of 2 and from them the coefficients of each liquid cell of the
+// ring of 1, and the tile's own cells store both and whether the tile holds
+// any liquid; the later ones read them back, work the residuals of liquid
+// cells alone, and leave a tile without liquid as it is.  (With all of it
+// worked again every time, for every tile, the down launches took 37 us of
+// an iteration at 1024x1024 and 72 us on a 48-world batch.)
+//
+// A level of few tiles is bound by the chain of its loads, not by what it
+// loads: its launches (k_fDown with 512 threads) work it all AGAIN every
+// time, a round of loads (the 256x256 dam 788 us a step; reading back, first
+// the tile's flag, then the density, then the rest, 809), and the one-launch
+// solves of small worlds read back EAGER, loading every word a cell may need
+// before the flag or the density says whether it does (a 256x256 tank with
+// bodies 1371 -> 1295; on the 1024x1024 disks, where the skipped tiles and
+// cells count, 4688 -> 5028, so the grid without bodies does not).
+template <class T, int NT, bool FINE, bool AGAIN, bool EAGER>
 __device__ __forceinline__ void downTile(const Dev& D, const FastW& F, const W& w, uint32_t l, uint32_t tile, bool first,
                                          LevelTile& t, const Team<NT>& tm) {
     const int lw = (int)D.level_w[l], lh = (int)D.level_h[l], tw = (lw + LT - 1) / LT;
     const int x0 = (int)(tile % (uint32_t)tw) * LT, y0 = (int)(tile / (uint32_t)tw) * LT;
+    uint8_t* live = F.L[l].live + tile;
+    if (!AGAIN && !EAGER && !first && l < F.lc && *live == 0) return;
     if (l >= F.lc) {
         const int cx = x0 + tm.tid % LT, cy = y0 + tm.tid / LT;
         if (tm.tid < LT * LT && cx < lw && cy < lh)
-            restrictCell<T, FINE>(D, F, w, l, (uint32_t)(cy * lw + cx));
+            restrictCell<T, FINE, EAGER>(D, F, w, l, (uint32_t)(cy * lw + cx), AGAIN || first);
         return;
     }
     const LRef<T> V = lref<T>(F, l);
+    if (AGAIN || first) {
+        if (first && tm.tid == 0) *live = 0;
 #pragma unroll 1
-    for (int k = tm.tid; k < LRR; k += NT) {
-        const int ix = k % LR - 2, iy = k / LR - 2, cx = x0 + ix, cy = y0 + iy;
-        float rho = -1.0f, rx = 0.0f, ry = 0.0f;
-        if (cx >= 0 && cy >= 0 && cx < lw && cy < lh) {
-            const bool res = ix >= -1 && iy >= -1 && ix <= LT && iy <= LT;
-            restrictedAt<T, FINE>(D, F, w, l, cx, cy, res, rho, rx, ry);
+        for (int k = tm.tid; k < LRR; k += NT) {
+            const int ix = k % LR - 2, iy = k / LR - 2, cx = x0 + ix, cy = y0 + iy;
+            float rho = -1.0f, rx = 0.0f, ry = 0.0f;
+            if (cx >= 0 && cy >= 0 && cx < lw && cy < lh) {
+                const bool res = ix >= -1 && iy >= -1 && ix <= LT && iy <= LT;
+                restrictedAt<T, FINE>(D, F, w, l, cx, cy, res, rho, rx, ry);
+            }
+            t.rho[k] = asStored(rho, T());
+            t.rx[k] = rx;
+            t.ry[k] = ry;
+            t.px[k] = 0.0f;
+            t.py[k] = 0.0f;
         }
-        t.rho[k] = asStored(rho, T());
-        t.rx[k] = rx;
-        t.ry[k] = ry;
-        t.px[k] = 0.0f;
-        t.py[k] = 0.0f;
-    }
-    tm.sync();
+        tm.sync();
 #pragma unroll 1
-    for (int k = tm.tid; k < (LT + 2) * (LT + 2); k += NT) {
-        const int ix = k % (LT + 2) - 1, iy = k / (LT + 2) - 1, cx = x0 + ix, cy = y0 + iy;
-        if (cx < 0 || cy < 0 || cx >= lw || cy >= lh) continue;
-        const int i = lsi(ix, iy);
-        const float rho = t.rho[i];
-        if (rho <= 0.0f) continue;
-        float b[4];
+        for (int k = tm.tid; k < (LT + 2) * (LT + 2); k += NT) {
+            const int ix = k % (LT + 2) - 1, iy = k / (LT + 2) - 1, cx = x0 + ix, cy = y0 + iy;
+            if (cx < 0 || cy < 0 || cx >= lw || cy >= lh) continue;
+            const int i = lsi(ix, iy);
+            const float rho = t.rho[i];
+            if (rho <= 0.0f) continue;
+            float b[4];
 #pragma unroll
-        for (int d = 0; d < 4; d++) {
-            b[d] = 0.0f;
-            if (!nbrIn(cx, cy, lw, lh, d)) continue;
-            const float r = t.rho[lsn(ix, iy, cx, cy, lw, lh, d)];
-            if (r < 0.0f) continue;
-            b[d] = faceBeta(rho, r);
-        }
-        const bool own = ix >= 0 && iy >= 0 && ix < LT && iy < LT;
-        if (first && own) {
-            const uint32_t j = (uint32_t)(cy * lw + cx);
-            st(V.b0 + j, b[0]); st(V.b1 + j, b[1]); st(V.b2 + j, b[2]); st(V.b3 + j, b[3]);
-        }
+            for (int d = 0; d < 4; d++) {
+                b[d] = 0.0f;
+                if (!nbrIn(cx, cy, lw, lh, d)) continue;
+                const float r = t.rho[lsn(ix, iy, cx, cy, lw, lh, d)];
+                if (r < 0.0f) continue;
+                b[d] = faceBeta(rho, r);
+            }
+            const bool own = ix >= 0 && iy >= 0 && ix < LT && iy < LT;
+            if (first && own) {
+                const uint32_t j = (uint32_t)(cy * lw + cx);
+                st(V.b0 + j, b[0]); st(V.b1 + j, b[1]); st(V.b2 + j, b[2]); st(V.b3 + j, b[3]);
+            }
 #pragma unroll
-        for (int d = 0; d < 4; d++) t.b[d][i] = asStored(b[d], T());
-        t.dg[i] = ((t.b[0][i] + t.b[1][i]) + t.b[2][i]) + t.b[3][i];
+            for (int d = 0; d < 4; d++) t.b[d][i] = asStored(b[d], T());
+            t.dg[i] = ((t.b[0][i] + t.b[1][i]) + t.b[2][i]) + t.b[3][i];
+        }
+        tm.sync();
+        // (written after the barrier above, which follows the clearing)
+        if (first && tm.tid < LT * LT && t.rho[lsi(tm.tid % LT, tm.tid / LT)] > 0.0f) *live = 1;
+    } else {
+#pragma unroll 1
+        for (int k = tm.tid; k < LRR; k += NT) {
+            const int ix = k % LR - 2, iy = k / LR - 2, cx = x0 + ix, cy = y0 + iy;
+            float rho = -1.0f;
+            if (cx >= 0 && cy >= 0 && cx < lw && cy < lh) {
+                const uint32_t j = (uint32_t)(cy * lw + cx);
+                rho = V.dens(j);
+                if ((EAGER || rho > 0.0f) && ix >= -1 && iy >= -1 && ix <= LT && iy <= LT) {
+                    const float4 b = V.coef(j);
+                    const V2 r = residualsAt<T, FINE>(D, F, l, cx, cy);
+                    if (!EAGER || rho > 0.0f) {
+                        t.rx[k] = r.x;
+                        t.ry[k] = r.y;
+                        t.b[0][k] = b.x;
+                        t.b[1][k] = b.y;
+                        t.b[2][k] = b.z;
+                        t.b[3][k] = b.w;
+                        t.dg[k] = diagOf(b);
+                    }
+                }
+            }
+            t.rho[k] = rho;
+            t.px[k] = 0.0f;
+            t.py[k] = 0.0f;
+        }
+        tm.sync();
     }
-    tm.sync();
     tileSmooth(t, tm, x0, y0, lw, lh, (float)(1u << (2u * l)));
     if (tm.tid < LT * LT) {
         const int ix = tm.tid % LT, iy = tm.tid / LT, cx = x0 + ix, cy = y0 + iy;
         if (cx < lw && cy < lh) {
             const uint32_t j = (uint32_t)(cy * lw + cx);
             const int i = lsi(ix, iy);
-            st(V.px + j, t.px[i]);
-            st(V.py + j, t.py[i]);
-            st(V.rx + j, t.rx[i]);
-            st(V.ry + j, t.ry[i]);
-            st(V.rho + j, t.rho[i]);
+            if (AGAIN || first || t.rho[i] > 0.0f) {
+                st(V.px + j, t.px[i]);
+                st(V.py + j, t.py[i]);
+                st(V.rx + j, t.rx[i]);
+                st(V.ry + j, t.ry[i]);
+            }
+            if (first) st(V.rho + j, t.rho[i]);
         }
     }
     tm.sync();  // the tile's arrays are free for the next tile
@@ -854,7 +968,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 2) k_fDown(Batch Bt, const
     FOR_ITEMS(Bt, L_RES + l - 1u, it) {
         FAST_ITEM(Bt, it, D, F, w, tile);
         if (D.st->cont == 0u) continue;
-        downTile<T, NT, FINE>(D, F, w, l, tile, D.st->cycle == 0u, t, tm);
+        downTile<T, NT, FINE, NT == 512, false>(D, F, w, l, tile, D.st->cycle == 0u, t, tm);
     }
 }
 
@@ -863,9 +977,10 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 2) k_fDown(Batch Bt, const
 // coefficients.  The way down's potentials are read from px, py (the ring
 // too) and the results go to ux, uy, so no CTA reads a cell that another
 // writes in the same launch; level l + 1's results are its ux, uy.
-template <class T, int NT>
+template <class T, int NT, bool EAGER>
 __device__ __forceinline__ void upTile(const Dev& D, const FastW& F, uint32_t l, uint32_t tile, LevelTile& t,
                                        const Team<NT>& tm) {
+    if (!EAGER && F.L[l].live[tile] == 0) return;  // no liquid: nothing to move
     const int lw = (int)D.level_w[l], lh = (int)D.level_h[l], tw = (lw + LT - 1) / LT;
     const int x0 = (int)(tile % (uint32_t)tw) * LT, y0 = (int)(tile / (uint32_t)tw) * LT;
     const LRef<T> V = lref<T>(F, l);
@@ -937,7 +1052,7 @@ __global__ void __launch_bounds__(NT, NT == 256 ? 4 : 2) k_fUp(Batch Bt, const _
         FAST_ITEM(Bt, it, D, F, w, tile);
         (void)w;
         if (D.st->cont == 0u) continue;
-        upTile<T, NT>(D, F, l, tile, t, tm);
+        upTile<T, NT, NT == 512>(D, F, l, tile, t, tm);
     }
 }
 
@@ -2336,6 +2451,7 @@ constexpr int SOLVE_THREADS = 1024, SOLVE_WARPS = SOLVE_THREADS / 32, TEAM = SOL
 
 // The CTAs of one cluster.
 struct ClusterGroup {
+    static constexpr bool EAGER = true;  // (downTile)
     uint32_t rank, n;
     __device__ explicit ClusterGroup(StepState*)
         : rank(cooperative_groups::this_cluster().block_rank()), n(cooperative_groups::this_cluster().num_blocks()) {}
@@ -2351,6 +2467,7 @@ struct ClusterGroup {
 // is bounded: past g_spin_limit polls a CTA records ERR_BARRIER, raises the
 // count past any barrier's, and every CTA returns false from here on.
 struct GridGroup {
+    static constexpr bool EAGER = false;
     StepState* st;
     uint32_t rank, n, target;
     __device__ explicit GridGroup(StepState* s) : st(s), rank(blockIdx.x), n(gridDim.x), target(0u) {}
@@ -2492,8 +2609,8 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_fSolve(const __grid_consta
                 const uint32_t tiles = levelTiles(D.level_w[l], D.level_h[l]);
 #pragma unroll 1
                 for (uint32_t t = t0; t < tiles; t += tn) {
-                    if (l == 1u) downTile<T, TEAM, true>(D, F, w, l, t, cycle == 0u, lt, tm);
-                    else downTile<T, TEAM, false>(D, F, w, l, t, cycle == 0u, lt, tm);
+                    if (l == 1u) downTile<T, TEAM, true, false, Group::EAGER || BODIES>(D, F, w, l, t, cycle == 0u, lt, tm);
+                    else downTile<T, TEAM, false, false, Group::EAGER || BODIES>(D, F, w, l, t, cycle == 0u, lt, tm);
                 }
                 if (!g.sync()) return;
             }
@@ -2503,7 +2620,7 @@ __global__ void __launch_bounds__(SOLVE_THREADS, 1) k_fSolve(const __grid_consta
             for (uint32_t l = lc - 1u; l >= 1u; l--) {
                 const uint32_t tiles = levelTiles(D.level_w[l], D.level_h[l]);
 #pragma unroll 1
-                for (uint32_t t = t0; t < tiles; t += tn) upTile<T, TEAM>(D, F, l, t, lt, tm);
+                for (uint32_t t = t0; t < tiles; t += tn) upTile<T, TEAM, Group::EAGER || BODIES>(D, F, l, t, lt, tm);
                 if (!g.sync()) return;
             }
 #pragma unroll 1
