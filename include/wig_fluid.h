@@ -342,9 +342,10 @@ int wig_fluid_bind(wig_fluid* h, const wig_fluid_buffers* b);
  * swept stamps of last step and the one before, by which a body's seams
  * and cup are found; null: no body has seams or a cup).  With them bound,
  * each step couples the bodies into the solve (A = L + J^T M^-1 J,
- * fluid.wgsl:1181-1470, :2819-2845, :2949-3218) and runs in the plain form
- * (a kernel per reference pass), whatever the form flags ask.  motion and
- * pushes null unbind all three.  Single-world handles only. */
+ * fluid.wgsl:1181-1470, :2819-2845, :2949-3218), in the plain form when
+ * WIG_STEP_PLAIN asks for it, else with all of the solve's iterations in one
+ * launch in FP32 (WIG_STEP_MIXED and WIG_STEP_PERSISTENT are ignored).
+ * motion and pushes null unbind all three.  Single-world handles only. */
 int wig_fluid_bind_bodies(wig_fluid* h, void* motion, void* pushes, void* stamps);
 
 /* The bound (or allocated) device buffers. */
