@@ -411,12 +411,12 @@ int make_batch(const wig_world_desc* descs, uint32_t n, const wig_elem* elems, u
     // Mcells/s against 168.8 from 64x64 and 166.8 from 16x16).  A batch's are
     // the autotuner's starting point.  The CG kernels (a warp a tile) run
     // fastest with few CTAs, each taking more tiles and fewer of them counting
-    // into a world's last-tile counter: a step of a batch of 48 4183 to 4283
-    // us at 4, 4340 to 4435 at 8, 4236 to 4271 at 2; of 128 and 256 worlds the
-    // same at 4 and 8, and up to 4% more at 2.
+    // into a world's last-tile counter: a step of a batch of 48 4224 us at 2,
+    // 4309 at 4, 4340 to 4435 at 8, of 24 small worlds 888 at 2, 927 at 4; of
+    // 128 and 256 worlds the same at 2, 4 and 8 within 2%.
     S.coarse_cells = n == 1 ? 2048u : wig::COARSE_CTA_CELLS;
     S.level_per_sm = n == 1 ? 32u : 8u;
-    S.cg_per_sm = 4u;
+    S.cg_per_sm = n == 1 ? 4u : 2u;
     S.relax_per_sm = n == 1 ? 64u : 16u;
     uint64_t most_units = 1, max_items[wig::L_COUNT] = {0};
     size_t scratch_total = 0;
