@@ -180,8 +180,11 @@ __device__ __forceinline__ I2 tileCell(const W& w, uint32_t wid) {
 
 // ================================================================ set-up
 
-// The level-0 words of cell i that neighbours read, zeroed.
+// The level-0 words of cell i that neighbours read, and its mask, by which a
+// relaxation's tile of four blocks decides whether it solves the cell and a
+// restriction whether it counts it, zeroed.
 __device__ __forceinline__ void zeroFine(const FastW& F, uint32_t i) {
+    F.Z.mask[i] = 0u;
     F.Z.pot[i] = make_float2(0.0f, 0.0f);
     F.Z.rim[i] = make_float2(0.0f, 0.0f);
     F.Z.rho[i] = 0.0f;
