@@ -24,13 +24,13 @@ TOL = abi.STEP_TOLERANCE | abi.STEP_F64_DOTS
 FORMS = {"fast": 0, "persistent": abi.STEP_PERSISTENT, "bodies": 0, "plain": abi.STEP_PLAIN}
 # a cluster's, the loop's and a grid's number of blocks
 SIZES = [(64, 64), (256, 240), (520, 520)]
-CEILING, SURFACE = 15, 24
+CEILING, SURFACE, FLOOR = 15, 24, 47
 
 
 def _box(width, height):
     w = W.World(width, height)
     wall = np.zeros((height, width), dtype=bool)
-    wall[0, :] = wall[-1, :] = True
+    wall[0, :] = wall[FLOOR:, :] = True
     wall[:, 0] = wall[:, -1] = True
     w.paint(wall, abi.WALL)
     w.paint(~wall, abi.WATER)
@@ -190,4 +190,34 @@ def test_a_served_world_beside_another(size, pooled):
     diffs = compare_worlds(w, want, grid=names, particles=("sorted",), scratch=True)
     n = 4 * (2 * want.C + want.L["face_count"] + 2 * ((want.L["face_count"] + 3) // 4))
     diffs += [d] if (d := diff_words(w.field[:n], want.field[:n], "field")) else []
+    assert not diffs, "; ".join(diffs)
+
+
+@pytest.mark.parametrize("between", ["plain", "bookkeeping", "dispatch"])
+@pytest.mark.parametrize("size", SIZES)
+def test_blocks_retired_by_another_form(size, between):
+    """The blocks retire in a plain step, a bookkeeping-only one or passes
+    the host dispatches; the fast steps after it are the plain form's."""
+    got = []
+    for form in (0, abi.STEP_PLAIN):
+        w = _box(*size)
+        g = _handle(w, "fast")
+        _steps(g, w, 1, 3, TOL | form)
+        g.download()
+        _empty_the_top(w)
+        _write_cells(g, w)
+        if between == "plain":
+            _steps(g, w, 4, 4, TOL | abi.STEP_PLAIN)
+        elif between == "bookkeeping":
+            g.step(params(w, 4), max_cycles=64, flags=TOL | form | _parity(4) | abi.STEP_BOOKKEEPING_ONLY, tolerance=1e-6)
+        else:
+            for name in ("SYNC", "SYNC_PARTICLES", "SYNC_SEED", "COMPACT", "RETIRE"):
+                g.dispatch(params(w, 4), name)
+        cycles = _steps(g, w, 5, 7, TOL | form)
+        g.download()
+        g.close()
+        assert _beside_idle(w) > size[0] // 2
+        got.append((w, cycles))
+    assert got[0][1] == got[1][1]
+    diffs = compare_worlds(got[0][0], got[1][0], scratch=True)
     assert not diffs, "; ".join(diffs)

@@ -444,6 +444,17 @@ struct alignas(16) World {
 };
 static_assert(sizeof(World) % 16 == 0, "World copies in 16-byte words");
 
+// The level-0 words of cell i that neighbours read, and its mask, by which a
+// relaxation's tile of four blocks decides whether it solves the cell and a
+// restriction whether it counts it, zeroed.
+__device__ __forceinline__ void zeroFine(const FastW& F, uint32_t i) {
+    F.Z.mask[i] = 0u;
+    F.Z.pot[i] = make_float2(0.0f, 0.0f);
+    F.Z.rim[i] = make_float2(0.0f, 0.0f);
+    F.Z.rho[i] = 0.0f;
+    F.P[i] = 0.0f;
+}
+
 // Block n's partial sums back to +0 (a block not worked on).
 __device__ __forceinline__ void zeroPartials(const Dev& D, const FastW& F, uint32_t n) {
     for (uint32_t c = 0; c < 2u; c++) {

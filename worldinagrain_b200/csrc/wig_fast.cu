@@ -16,10 +16,10 @@
 //     threadfence reduction: the same fixed tree order, one launch fewer);
 //   * the iterations are the body of a CUDA-graph WHILE node: a step runs as
 //     many as it needs, with no launches for the converged ones.
-// The scratch keeps one invariant: level-0 arrays and the blocks' partial
-// sums are zero outside the blocks worked on (zeroed at allocation, when a
-// world is uploaded, and as blocks retire), where the reference's field is
-// zero too.
+// The scratch keeps one invariant: level-0 arrays are zero outside the blocks
+// worked on, and the blocks' partial sums (zeroed at allocation, when a world
+// is uploaded, and by retire, in whichever form's step, which zeroes the
+// reference's field there too).
 
 #include <algorithm>
 
@@ -180,22 +180,10 @@ __device__ __forceinline__ I2 tileCell(const W& w, uint32_t wid) {
 
 // ================================================================ set-up
 
-// The level-0 words of cell i that neighbours read, and its mask, by which a
-// relaxation's tile of four blocks decides whether it solves the cell and a
-// restriction whether it counts it, zeroed.
-__device__ __forceinline__ void zeroFine(const FastW& F, uint32_t i) {
-    F.Z.mask[i] = 0u;
-    F.Z.pot[i] = make_float2(0.0f, 0.0f);
-    F.Z.rim[i] = make_float2(0.0f, 0.0f);
-    F.Z.rho[i] = 0.0f;
-    F.P[i] = 0.0f;
-}
-
 // cgStart, cgResidual, cgPrepare (fluid.wgsl:2665-2732) into the scratch,
 // the cells' coefficients worked out (four tiles a 256-thread CTA, a world's
 // group of four active blocks an item; the CTA that counts a world's last
-// tile sums its ||b||^2), and the blocks that dropped out this step zeroed
-// (the invariant).
+// tile sums its ||b||^2).
 template <bool ONE, bool BODIES>
 __global__ void __launch_bounds__(256) k_fSetup(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
@@ -281,25 +269,11 @@ __global__ void __launch_bounds__(256) k_fSetup(Batch Bt, const __grid_constant_
             }
         }
     }
-    // the blocks that dropped out: their level-0 arrays back to zero (a
-    // retired block a quarter of the CTA)
-    const uint32_t nr = Bt.n(L_RET);
-    for (uint32_t t = blockIdx.x * 4u + (threadIdx.x >> 6); t < nr; t += gridDim.x * 4u) {
-        const uint32_t it = Bt.item(L_RET, t);
-        FAST_ITEM_G(Bt, it, D, F, w, j);
-        uint32_t n = D.blocks[w.retiredSlot(j)];
-        const I2 bq_ = w.blockAt(n);
-        I2 c{bq_.x * BLOCK + (int)(threadIdx.x & 7u), bq_.y * BLOCK + (int)((threadIdx.x >> 3) & 7u)};
-        if (w.inWorld(c)) {
-            uint32_t i = w.cellIndex(c);
-            zeroFine(F, i);
-        }
-    }
 }
 
 // The level-0 arrays neighbours read and the block partials, zeroed in the
-// blocks not worked on (the invariant), for worlds whose scratch is lent by a pool for the step:
-// a CTA per block of the world.
+// blocks not worked on (the invariant), for worlds whose scratch is lent by a pool for the step: a
+// CTA per block of the world.
 __global__ void k_fZeroIdle(Batch Bt) {
     FOR_ITEMS(Bt, L_WB, it) {
         FAST_ITEM_G(Bt, it, D, F, w, n);

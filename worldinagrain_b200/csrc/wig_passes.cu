@@ -737,7 +737,9 @@ __global__ void __launch_bounds__(1024) k_compactWrite(Batch Bt, const __grid_co
     }
 }
 
-// retire (fluid.wgsl:924-951) of retired block wid.
+// retire (fluid.wgsl:924-951) of retired block wid, its words of the fast
+// form's scratch with its field (whichever form the step is of: the next may
+// be a fast one).
 __device__ __forceinline__ void retireBlock(const Dev& D, const FastW& F, const W& w, uint32_t wid) {
     uint32_t n = D.blocks[w.retiredSlot(wid)];
     // the solve's sums over the world's blocks take its partials for +0
@@ -747,6 +749,7 @@ __device__ __forceinline__ void retireBlock(const Dev& D, const FastW& F, const 
     I2 c{bq_.x * BLOCK + (int)(threadIdx.x & 7u), bq_.y * BLOCK + (int)(threadIdx.x >> 3)};
     if (!w.inWorld(c)) return;
     uint32_t i = w.cellIndex(c);
+    zeroFine(F, i);
     reinterpret_cast<float4*>(D.field)[2u * i] = make_float4(0, 0, 0, 0);
     reinterpret_cast<float4*>(D.field)[2u * i + 1u] = make_float4(0, 0, 0, 0);
     for (uint32_t g = 0; g < CELL_WORDS; g++) *w.gwp(i, g) = 0u;
