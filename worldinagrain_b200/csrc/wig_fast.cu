@@ -17,9 +17,9 @@
 //   * the iterations are the body of a CUDA-graph WHILE node: a step runs as
 //     many as it needs, with no launches for the converged ones.
 // The scratch keeps one invariant: level-0 arrays are zero outside the blocks
-// worked on, and the blocks' partial sums (zeroed at allocation, when a world
-// is uploaded, and by retire, in whichever form's step, which zeroes the
-// reference's field there too).
+// worked on (zeroed at allocation, when a world is uploaded, and by retire,
+// in whichever form's step, which zeroes the reference's field there too), and
+// so are the blocks' partial sums (zeroed by each step's set-up).
 
 #include <algorithm>
 
@@ -183,7 +183,9 @@ __device__ __forceinline__ I2 tileCell(const W& w, uint32_t wid) {
 // cgStart, cgResidual, cgPrepare (fluid.wgsl:2665-2732) into the scratch,
 // the cells' coefficients worked out (four tiles a 256-thread CTA, a world's
 // group of four active blocks an item; the CTA that counts a world's last
-// tile sums its ||b||^2).
+// tile sums its ||b||^2), and the partial sums of the blocks not worked on
+// zeroed (the invariant; a block may have dropped out in any way since: as
+// the list of the retired says, or by a host's hand in the blocks' words).
 template <bool ONE, bool BODIES>
 __global__ void __launch_bounds__(256) k_fSetup(Batch Bt, const __grid_constant__ WorldSrc<ONE> src) {
     __shared__ WorldCopy wc_;
@@ -269,16 +271,22 @@ __global__ void __launch_bounds__(256) k_fSetup(Batch Bt, const __grid_constant_
             }
         }
     }
+    const uint32_t nb = Bt.n(L_WB);
+    for (uint32_t t = blockIdx.x * 256u + threadIdx.x; t < nb; t += gridDim.x * 256u) {
+        const uint32_t it = Bt.item(L_WB, t);
+        const World& Wd = src.getG(Bt, it);
+        const uint32_t n = Bt.unit(it);
+        if ((Wd.D.blocks[W(Wd.D).stateSlot(n)] & ACTIVE) == 0u) zeroPartials(Wd.D, Wd.S, n);
+    }
 }
 
-// The level-0 arrays neighbours read and the block partials, zeroed in the
-// blocks not worked on (the invariant), for worlds whose scratch is lent by a pool for the step: a
+// The level-0 arrays neighbours read, zeroed in the blocks not worked on
+// (the invariant), for worlds whose scratch is lent by a pool for the step: a
 // CTA per block of the world.
 __global__ void k_fZeroIdle(Batch Bt) {
     FOR_ITEMS(Bt, L_WB, it) {
         FAST_ITEM_G(Bt, it, D, F, w, n);
         if (D.st->book != 0u || (D.blocks[w.stateSlot(n)] & ACTIVE) != 0u) continue;
-        if (threadIdx.x == 0) zeroPartials(D, F, n);
         for (uint32_t t = threadIdx.x; t < 64u; t += blockDim.x) {
             const I2 bq_ = w.blockAt(n);
             I2 c{bq_.x * BLOCK + (int)(t & 7u), bq_.y * BLOCK + (int)(t >> 3)};
@@ -289,11 +297,9 @@ __global__ void k_fZeroIdle(Batch Bt) {
     }
 }
 
-// Zeroes the level-0 arrays the neighbours read and the block partials
-// (after an upload).
+// Zeroes the level-0 arrays the neighbours read (after an upload).
 __global__ void k_fZero(Dev D, FastW F) {
     const uint32_t C = D.C;
-    for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < D.B; n += gridDim.x * blockDim.x) zeroPartials(D, F, n);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < C; i += gridDim.x * blockDim.x) {
         zeroFine(F, i);
     }

@@ -71,7 +71,7 @@ uint32_t fast_cycle(const Batch& Bt, const BatchShape& S, const World* one, cuda
                     NestCapture* nest = nullptr);
 // cgFinish.
 void fast_finish(const Batch& Bt, const BatchShape& S, const World* one, cudaStream_t s, const Marker* m);
-// Level 0's arrays and the block partials of one world zeroed (after its buffers are written by the host).
+// Level 0's arrays of one world zeroed (after its buffers are written by the host).
 void fast_zero_level0(const World& Wd, cudaStream_t s);
 // The same for the blocks not worked on, of every world of the step whose
 // scratch a pool lends (after compact).

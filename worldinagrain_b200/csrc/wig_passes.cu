@@ -742,8 +742,6 @@ __global__ void __launch_bounds__(1024) k_compactWrite(Batch Bt, const __grid_co
 // be a fast one).
 __device__ __forceinline__ void retireBlock(const Dev& D, const FastW& F, const W& w, uint32_t wid) {
     uint32_t n = D.blocks[w.retiredSlot(wid)];
-    // the solve's sums over the world's blocks take its partials for +0
-    if (threadIdx.x == 0) zeroPartials(D, F, n);
     if (threadIdx.x == 0) D.blocks[n] = 0u;
     const I2 bq_ = w.blockAt(n);
     I2 c{bq_.x * BLOCK + (int)(threadIdx.x & 7u), bq_.y * BLOCK + (int)(threadIdx.x >> 3)};
