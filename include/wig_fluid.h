@@ -439,7 +439,8 @@ void wig_fluid_destroy(wig_fluid* h);
  * loads the library until the process exits), so worlds of more blocks are
  * refused with WIG_E_ARG.  The first call on a device looks up that array's
  * device address; make it before any stream capture.  Calls share the one
- * array: calls whose work overlaps on the GPU race. */
+ * array: calls whose work overlaps on the GPU race, and their results are
+ * worth nothing; those after them are sound. */
 #define WIG_NOALLOC_MAX_BLOCKS 16384u
 int wig_fluid_residual_norm2_noalloc(const wig_world_desc* d, const void* field, const void* blocks, const void* cg,
                                      double* out, void* stream);

@@ -20,8 +20,11 @@
 // cudaGetSymbolAddress (the first call on a device does that set-up) and
 // passes it to the kernels.  That address is kept until
 // wig_fluid_noalloc_forget_device, which a host that resets a device calls.  Every call shares the one array: calls whose
-// work overlaps on the GPU (two streams, or two host threads) race on it.
+// work overlaps on the GPU (two streams, or two host threads) race on it, and
+// their results are worth nothing.  The calls after them are sound: each
+// call's count of finished CTAs is a word of its own.
 
+#include <atomic>
 #include <cstdint>
 #include <cstring>
 #include <mutex>
@@ -37,11 +40,25 @@ constexpr uint32_t MAX_DEVICES = 64;
 // One FP64 partial sum per block; a call writes the entries of all its
 // world's blocks before it reads any, so nothing in it has to start at zero.
 static __device__ __align__(256) double g_block_partials[WIG_NOALLOC_MAX_BLOCKS];
-// The CTAs of the call in flight that have written theirs (back to 0 at its end).
-static __device__ uint32_t g_done;
+// The CTAs of a call that have written theirs: a word a call, 0 before it and
+// put back to 0 by its last CTA, so that a call's count is its own whatever
+// overlaps it.  (One word for all of them, with overlapping calls of other
+// grids counted into it, could be left at any value, and every call after it
+// summed too early or not at all.)  The calls take the first COUNTERS words in
+// turn; a captured call, whose word its graph's replays use for as long as
+// they please, takes one of the others and sets it to 0 itself ahead of the
+// launch (a node of the graph; ahead of every call it would cost about as
+// much as a sixth of it).
+constexpr uint32_t COUNTERS = 1024;
+static __device__ uint32_t g_done[2u * COUNTERS];
 
 std::mutex g_mutex;
-double* g_partials_of[MAX_DEVICES] = {nullptr};
+std::atomic<uint32_t> g_calls{0};
+struct Scratch {
+    double* partials;
+    uint32_t* done;
+};
+Scratch g_scratch_of[MAX_DEVICES] = {};
 
 int set_error(int code, const std::string& msg) {
     wig::set_last_error(msg);
@@ -58,7 +75,8 @@ int set_error(int code, const std::string& msg) {
 // 1024 x 1024 world.
 constexpr int NORM_THREADS = 512, NORM_WARPS = NORM_THREADS / 32;
 __global__ void __launch_bounds__(NORM_THREADS, 2) k_r2(uint32_t W, uint32_t H, uint32_t B, uint32_t BW, const uint32_t* blocks,
-                                                        const float4* field, const float4* cg, double* partials, double* out) {
+                                                        const float4* field, const float4* cg, double* partials, uint32_t* done,
+                                                        double* out) {
     __shared__ double s[256];
     __shared__ int last;
     const uint32_t lane = threadIdx.x & 31u;
@@ -83,9 +101,9 @@ __global__ void __launch_bounds__(NORM_THREADS, 2) k_r2(uint32_t W, uint32_t H, 
     if (lane == 0u) __threadfence();
     __syncthreads();
     if (threadIdx.x == 0u) {
-        last = atomicAdd(&g_done, 1u) + 1u == gridDim.x ? 1 : 0;
+        last = atomicAdd(done, 1u) + 1u == gridDim.x ? 1 : 0;
         if (last) {
-            g_done = 0u;
+            *done = 0u;
             __threadfence();
         }
     }
@@ -96,24 +114,43 @@ __global__ void __launch_bounds__(NORM_THREADS, 2) k_r2(uint32_t W, uint32_t H, 
     if (threadIdx.x == 0u) *out = s[0];
 }
 
-// The device address of g_block_partials on the current device, looked up
-// once per device and kept for the process's life: a host that destroys and
-// recreates a device's primary context (cudaDeviceReset) loads the module
-// anew, so it must call wig_fluid_noalloc_forget_device afterwards.
-int partials_on_current_device(double** out) {
+// The device addresses of g_block_partials and g_done on the current device,
+// looked up once per device and kept for the process's life: a host that
+// destroys and recreates a device's primary context (cudaDeviceReset) loads
+// the module anew, so it must call wig_fluid_noalloc_forget_device afterwards.
+int scratch_on_current_device(Scratch* out) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return set_error(WIG_E_CUDA, std::string("cudaGetDevice: ") + cudaGetErrorString(e));
     if (dev < 0 || (uint32_t)dev >= MAX_DEVICES) return set_error(WIG_E_ARG, "device ordinal past the ones this entry point keeps");
     std::lock_guard<std::mutex> lock(g_mutex);
-    if (!g_partials_of[dev]) {
-        void* p = nullptr;
+    if (!g_scratch_of[dev].partials) {
+        void *p = nullptr, *n = nullptr;
         e = cudaGetSymbolAddress(&p, g_block_partials);
+        if (e == cudaSuccess) e = cudaGetSymbolAddress(&n, g_done);
         if (e != cudaSuccess) return set_error(WIG_E_CUDA, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
-        g_partials_of[dev] = static_cast<double*>(p);
+        g_scratch_of[dev] = Scratch{static_cast<double*>(p), static_cast<uint32_t*>(n)};
     }
-    *out = g_partials_of[dev];
+    *out = g_scratch_of[dev];
     return WIG_OK;
+}
+
+// The word a call on stream s counts its CTAs in, 0 by the time its kernel runs.
+cudaError_t counter_of(cudaStream_t s, uint32_t* done, uint32_t** out) {
+    const uint32_t k = g_calls.fetch_add(1u) % COUNTERS;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    // (the legacy stream cannot be asked while another is captured; nor can
+    // it be launched on, as the launch then says)
+    if (cudaStreamIsCapturing(s, &cs) != cudaSuccess) {
+        cudaGetLastError();
+        cs = cudaStreamCaptureStatusNone;
+    }
+    if (cs == cudaStreamCaptureStatusNone) {
+        *out = done + k;
+        return cudaSuccess;
+    }
+    *out = done + COUNTERS + k;
+    return cudaMemsetAsync(*out, 0, sizeof(uint32_t), s);
 }
 
 }  // namespace
@@ -130,14 +167,17 @@ int wig_fluid_residual_norm2_noalloc(const wig_world_desc* d, const void* field,
     if (B > WIG_NOALLOC_MAX_BLOCKS)
         return set_error(WIG_E_ARG, "world has " + std::to_string(B) + " blocks; the allocation-free entry point holds at most " +
                                         std::to_string(WIG_NOALLOC_MAX_BLOCKS) + " (a 1024 x 1024 world)");
-    double* partials = nullptr;
-    int rc = partials_on_current_device(&partials);
+    Scratch scratch{};
+    int rc = scratch_on_current_device(&scratch);
     if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
+    uint32_t* done = nullptr;
+    cudaError_t e = counter_of(s, scratch.done, &done);
+    if (e != cudaSuccess) return set_error(WIG_E_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
     const unsigned need = (unsigned)((B + NORM_WARPS - 1u) / NORM_WARPS), grid = need < 148u * 2u ? need : 148u * 2u;
     k_r2<<<grid, NORM_THREADS, 0, s>>>(d->width, d->height, (uint32_t)B, BW, (const uint32_t*)blocks, (const float4*)field,
-                                       (const float4*)cg, partials, out);
-    cudaError_t e = cudaGetLastError();
+                                       (const float4*)cg, scratch.partials, done, out);
+    e = cudaGetLastError();
     if (e != cudaSuccess) return set_error(WIG_E_CUDA, std::string("launch: ") + cudaGetErrorString(e));
     return WIG_OK;
 }
@@ -148,7 +188,7 @@ int wig_fluid_noalloc_forget_device(void) {
     if (e != cudaSuccess) return set_error(WIG_E_CUDA, std::string("cudaGetDevice: ") + cudaGetErrorString(e));
     if (dev < 0 || (uint32_t)dev >= MAX_DEVICES) return set_error(WIG_E_ARG, "device ordinal past the ones this entry point keeps");
     std::lock_guard<std::mutex> lock(g_mutex);
-    g_partials_of[dev] = nullptr;
+    g_scratch_of[dev] = Scratch{};
     return WIG_OK;
 }
 
