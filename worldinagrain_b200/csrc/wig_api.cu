@@ -107,6 +107,7 @@ struct wig_batch {
     void* scratch = nullptr;          // the fast form's scratch and FP64 partials of every world
     void* arena = nullptr;            // the worlds' buffers (batches made by wig_batch_create)
     std::vector<void*> wmem;          // each world's allocation (batches made by wig_batch_create_deferred)
+    bool alone = false;               // one world, whose memory stays where it is (not a deferred batch's)
     uint64_t resident = 0;            // bytes of the admitted worlds' allocations
     std::vector<std::array<void*, 7>> own;  // buffers a single-world handle allocated at bind
     std::vector<char> bound, dirty;
@@ -349,7 +350,7 @@ void level_shape(wig_batch* b) {
             if (l < lc) S.max_items[wig::L_SM + l - 1] += ch;
         }
         S.lc_max = std::max(S.lc_max, lc);
-        const size_t c = b->K == 1 ? wig::fast_cluster_smem(D, lc) : 0;
+        const size_t c = b->alone ? wig::fast_cluster_smem(D, lc) : 0;
         if (c) S.cluster = 1;
         S.coarse_smem = std::max(S.coarse_smem, c ? c : wig::fast_coarse_smem(D, lc));
     }
@@ -382,6 +383,7 @@ int make_batch(const wig_world_desc* descs, uint32_t n, const wig_elem* elems, u
         return fail(code, keep);
     };
     b->K = n;
+    b->alone = n == 1 && how != Alloc::Deferred;
     cudaGetDevice(&b->device);
     b->L.resize(n);
     b->hw.assign(n, wig::World{});
@@ -517,10 +519,7 @@ int make_batch(const wig_world_desc* descs, uint32_t n, const wig_elem* elems, u
     }
     if (cudaMemcpy(b->d_worlds, b->hw.data(), sizeof(wig::World) * n, cudaMemcpyHostToDevice) != cudaSuccess)
         return bail(WIG_E_CUDA, "cudaMemcpy world table");
-    if (n == 1) {
-        // (a deferred world's memory moves with each admission: no kernel can
-        // take it as a parameter)
-        if (how == Alloc::Deferred) return bail(WIG_E_CUDA, "a deferred batch holds more than one world");
+    if (b->alone) {
         if (wig::fast_solve_shape(b->hw[0].D, &b->solve) != cudaSuccess) return bail(WIG_E_CUDA, "occupancy of the one-launch solve");
     }
 
@@ -623,9 +622,10 @@ struct Prof {
     std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> marks;
 };
 
-// The batch's only world (whose memory stays where it is: a batch of one is
-// never deferred), for the kernels to take as a parameter.
-const wig::World* one_world(const wig_batch* b) { return b->K == 1 ? &b->hw[0] : nullptr; }
+// The batch's only world, for the kernels to take as a parameter; null for a
+// batch of several, and for a deferred world alone, whose memory moves with
+// each admission and which they take from the world table.
+const wig::World* one_world(const wig_batch* b) { return b->alone ? &b->hw[0] : nullptr; }
 
 // Launch recording with optional per-launch events (Prof).
 struct Rec {
@@ -1610,7 +1610,7 @@ int wig_batch_set_launch(wig_batch* b, uint32_t knob, uint32_t value) {
     if (knob >= WIG_LAUNCH_KNOBS) return fail(WIG_E_ARG, "unknown launch knob");
     // a single world's coarse levels may start higher: on a cluster
     const uint32_t most = knob != WIG_LAUNCH_COARSE_CELLS ? 64u
-                          : b->K == 1                    ? wig::COARSE_CLUSTER_CELLS
+                          : b->alone                     ? wig::COARSE_CLUSTER_CELLS
                                                          : wig::COARSE_CTA_CELLS;
     if (value < 1u || value > most) return fail(WIG_E_ARG, "launch knob value out of range");
     CUDA_TRY(cudaDeviceSynchronize());
