@@ -3008,7 +3008,11 @@ cudaError_t fast_solve_shape(const Dev& D, SolveShape* out) {
     if (e == cudaSuccess) e = solve_attributes<ClusterGroup, float, false>(most, true);
     if (e == cudaSuccess) e = solve_attributes<ClusterGroup, float, true>(most, true);
     if (e == cudaSuccess) e = solve_attributes<ClusterGroup, __half, false>(most, true);
+    // the first level of at most COARSE_CTA_CELLS cells that fits a CTA with
+    // the levels below it (a level a cell or two high only halves, so that
+    // 4096 x 1 cells are 7680 with those below, 276 KB)
     out->lc = coarse_level(D, COARSE_CTA_CELLS);
+    while (out->lc < D.levels && solve_smem(D, out->lc) > most) out->lc++;
     const size_t smem = solve_smem(D, out->lc);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_fSolve<GridGroup, float, true>, SOLVE_THREADS, smem);
     if (e != cudaSuccess) return e;
