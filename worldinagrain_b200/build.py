@@ -15,7 +15,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(LIB_DIR, "libwig_fluid.so")
 SOURCES = ["wig_api.cu", "wig_passes.cu", "wig_fast.cu", "wig_sched.cu", "wig_noalloc.cu"]
-HEADERS = ["wig_bodies.cuh", "wig_device.cuh", "wig_passes.cuh", "wig_fast.cuh", "wig_sched.cuh", "wig_sums.cuh"]
+HEADERS = ["wig_bodies.cuh", "wig_device.cuh", "wig_passes.cuh", "wig_fast.cuh", "wig_sched.cuh", "wig_sums.cuh", "wig_wait.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -29,6 +29,7 @@
 #include "wig_bodies.cuh"
 #include "wig_fast.cuh"
 #include "wig_sums.cuh"
+#include "wig_wait.h"
 
 namespace wig {
 namespace {
@@ -2447,15 +2448,14 @@ struct ClusterGroup {
 
 // The CTAs of a cooperative launch (all resident): arrivals counted up in
 // the world's StepState, the k-th barrier passed at k n of them.  Each wait
-// is bounded: past g_spin_limit polls a CTA records ERR_BARRIER, raises the
-// count past any barrier's, and every CTA returns false from here on.
+// is bounded: past g_spin_limit polls a CTA records ERR_BARRIER and marks the
+// count as given up (wig_wait.h), and every CTA returns false from here on.
 struct GridGroup {
     static constexpr bool EAGER = false;
     StepState* st;
     uint32_t rank, n, target;
     __device__ explicit GridGroup(StepState* s) : st(s), rank(blockIdx.x), n(gridDim.x), target(0u) {}
     __device__ bool sync() {
-        constexpr uint32_t GAVE_UP = 1u << 30;
         __shared__ int s_ok;
         target += n;
         __syncthreads();
@@ -2465,15 +2465,14 @@ struct GridGroup {
             asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&st->bar_count) : "memory");
             while (true) {
                 asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&st->bar_count) : "memory");
-                if (v >= target) break;
+                if (barrierOver(v, target)) break;
                 if (++it > limit) {
                     atomicOr(&st->err, ERR_BARRIER);
-                    atomicAdd(&st->bar_count, GAVE_UP);
-                    v = GAVE_UP;
+                    v = atomicOr(&st->bar_count, BARRIER_GAVE_UP) | BARRIER_GAVE_UP;
                     break;
                 }
             }
-            s_ok = v < GAVE_UP ? 1 : 0;
+            s_ok = barrierGaveUp(v) ? 0 : 1;
         }
         __syncthreads();
         return s_ok != 0;
