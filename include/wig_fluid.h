@@ -456,12 +456,13 @@ int wig_fluid_noalloc_forget_device(void);
  * waits on the current device, for every kernel launched after the call
  * (graphs already captured included): loop_limit bounds each lock-free
  * retry loop (the union-find of sealJoin and cgJoin, label.wgsl:27-55),
- * spin_limit the polls of the persistent form's grid barrier.  0 restores a
- * default (2^22 retries; 2^23 polls of about 64 ns).  A loop that runs out
+ * spin_limit the polls of the one-launch solve's grid barrier.  0 restores a
+ * default (2^22 retries; 2^20 polls of about 0.7 us).  A loop that runs out
  * gives up, and the step's stats read returns WIG_E_STATE; nothing hangs
  * and the device stays usable.  For tests of those failure paths: a host
- * has no other reason to call it.  Limits above the defaults are refused
- * with WIG_E_ARG.  Synchronous (it writes two device words). */
+ * has no other reason to call it.  A spin_limit from the default to 2^23
+ * stands for the default; limits above 2^22 and 2^23 are refused with
+ * WIG_E_ARG.  Synchronous (it writes two device words). */
 int wig_fluid_set_wait_limits(uint32_t loop_limit, uint32_t spin_limit);
 
 /* One-line description of the last error on this thread ("" if none). */

@@ -41,3 +41,15 @@ def test_every_cta_of_a_full_grid_gives_up(limit, lowered_limits):
     assert got[0][1] == got[1][1]
     diffs = compare_worlds(got[0][0], got[1][0], scratch=True)
     assert not diffs, "; ".join(diffs)
+
+
+def test_the_documented_spin_limits_are_taken(lowered_limits):
+    """Up to 2^23 polls are taken, a number from the default up standing for
+    it; more are refused, as are more than 2^22 retries."""
+    from worldinagrain_b200 import fluid
+    for spin in (1, 1 << 20, (1 << 20) + 1, 1 << 22, 1 << 23):
+        lowered_limits(0, spin)
+    lowered_limits(1 << 22, 0)
+    for limits in ((0, (1 << 23) + 1), (0, 0xFFFFFFFF), ((1 << 22) + 1, 0)):
+        with pytest.raises(fluid.WigError, match="WIG_E_ARG"):
+            lowered_limits(*limits)

@@ -1240,7 +1240,7 @@ int batch_read_stats(wig_batch* b, const uint32_t* worlds, uint32_t count, wig_f
         // tolerance
         if (r.err & wig::ERR_BARRIER) {
             if (severity(rc) < severity(WIG_E_STATE))
-                rc = fail(WIG_E_STATE, "the persistent solve's grid barrier waited past its limit");
+                rc = fail(WIG_E_STATE, "the one-launch solve's grid barrier waited past its limit");
         } else if (r.err) {
             if (severity(rc) < severity(WIG_E_STATE))
                 rc = fail(WIG_E_STATE, "a device loop hit its iteration limit (union-find)");
@@ -1290,8 +1290,8 @@ uint32_t wig_fluid_abi_version(void) { return WIG_ABI_VERSION; }
 
 int wig_fluid_set_wait_limits(uint32_t loop_limit, uint32_t spin_limit) {
     const uint32_t lo = loop_limit ? loop_limit : wig::LOOP_LIMIT;
-    const uint32_t sp = spin_limit ? spin_limit : wig::BARRIER_SPIN_LIMIT;
-    if (lo > wig::LOOP_LIMIT || sp > wig::BARRIER_SPIN_LIMIT)
+    const uint32_t sp = spin_limit ? std::min(spin_limit, wig::BARRIER_SPIN_LIMIT) : wig::BARRIER_SPIN_LIMIT;
+    if (lo > wig::LOOP_LIMIT || spin_limit > wig::SPIN_LIMIT_MOST)
         return fail(WIG_E_ARG, "wait limits may only be lowered");
     CUDA_TRY(cudaMemcpyToSymbol(wig::g_loop_limit, &lo, sizeof(lo)));
     CUDA_TRY(cudaMemcpyToSymbol(wig::g_spin_limit, &sp, sizeof(sp)));

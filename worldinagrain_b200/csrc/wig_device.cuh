@@ -61,6 +61,8 @@ constexpr uint32_t ERR_LOOP = 1u, ERR_CAPACITY = 2u, ERR_BARRIER = 4u;
 // A grid barrier's wait: at most this many polls of about 0.7 us (about
 // 0.7 s), past which the kernel records ERR_BARRIER and returns.
 constexpr uint32_t BARRIER_SPIN_LIMIT = 1u << 20;
+// The most polls a host may ask for (then the default holds).
+constexpr uint32_t SPIN_LIMIT_MOST = 1u << 23;
 // The bounds in force on a device (the two above unless
 // wig_fluid_set_wait_limits lowered them, which the failure-path tests do to
 // see the error come back); read by the loops at run time.
