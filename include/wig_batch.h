@@ -119,8 +119,8 @@ int wig_batch_world_bytes_split(const wig_world_desc* d, uint64_t* persistent, u
  * Defaults: COARSE_CELLS 4096, LEVEL_PER_SM 8, CG_PER_SM 2, RELAX_PER_SM 16;
  * for a batch of one world, as every wig_fluid handle is: COARSE_CELLS 2048,
  * LEVEL_PER_SM 32, CG_PER_SM 4, RELAX_PER_SM 64.
- * A single world's solve in one launch (up to 640 blocks, above 4096, with
- * bodies, with WIG_STEP_PERSISTENT) takes of them COARSE_CELLS alone.
+ * A single world's solve in one launch (up to 640 blocks, with bodies, with
+ * WIG_STEP_PERSISTENT) takes of them COARSE_CELLS alone.
  * No step of the batch may be in flight; the lanes' graphs are recaptured
  * at their next step. */
 enum wig_launch_knob {

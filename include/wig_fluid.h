@@ -232,8 +232,10 @@ typedef struct wig_fluid_buffers {
 #define WIG_STEP_F64_DOTS 32u         /* CG dot products in FP64 */
 #define WIG_STEP_SYNC_STATS 64u       /* copy the stats to the host at the end of the step */
 #define WIG_STEP_PLAIN 128u           /* the solve as one kernel per reference pass (else the fast form) */
-#define WIG_STEP_PERSISTENT 256u      /* the fast form's iterations as one cooperative kernel at any size (else so, or on one
-                                         cluster, at the sizes where that is faster than kernels in a graph WHILE loop) */
+#define WIG_STEP_PERSISTENT 256u      /* the fast form's iterations as one cooperative kernel at any size (else in one launch on a
+                                         cluster up to 640 blocks, kernels in a graph WHILE loop above): from about 640x640
+                                         cells up to 6% faster for a world alone on the GPU, but no other work runs beside
+                                         its solve */
 #define WIG_STEP_MIXED 512u           /* mixed precision (fast form, with TOLERANCE and F64_DOTS): the multigrid levels
                                          stored in 16 bits and worked in FP32 (each coarse level's density and stencil
                                          coefficients in binary16, its potentials, right-hand sides and way-up potentials

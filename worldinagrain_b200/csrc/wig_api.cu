@@ -878,8 +878,7 @@ int record_step(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags, boo
 // is captured on the lane's second stream; else the iterations are launched
 // from the host, each decided by reading back the device's verdict (the
 // profiler's path).  *outside gets the kernels outside the loop (all of
-// them when not capturing), *body those of one iteration of the loop.  The
-// persistent form (one world) runs the iterations in one cooperative kernel.
+// them when not capturing), *body those of one iteration of the loop.
 int record_step_fast(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags, bool shifted, cudaStream_t s,
                      Prof* prof, bool capture, uint32_t* outside, uint32_t* body) {
     Rec R{b, ln, s, prof};
@@ -911,10 +910,10 @@ int record_step_fast(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags
     R.launches++;
     // a single world's iterations are one launch: with bodies (which the
     // loop's launches do not couple in), for WIG_STEP_PERSISTENT (then on a
-    // cooperative grid at any size), and at the sizes where it is the faster
-    // form; with its coarse levels on a cluster, and when profiled, they are
-    // the loop's launches
-    const bool by_size = one && ln.S.cluster == 0u && (one->D.B <= wig::CLUSTER_BLOCKS || one->D.B > wig::GRID_BLOCKS);
+    // cooperative grid at any size), and at the sizes where a cluster is the
+    // faster form; with its coarse levels on a cluster, and when profiled,
+    // they are the loop's launches
+    const bool by_size = one && ln.S.cluster == 0u && one->D.B <= wig::CLUSTER_BLOCKS;
     const bool one_launch = (flags & WIG_STEP_PERSISTENT) || bodies || by_size;
     const bool solve = one_launch && (capture || bodies || (flags & WIG_STEP_PERSISTENT));
     if (solve) {
