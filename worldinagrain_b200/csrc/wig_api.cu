@@ -911,9 +911,12 @@ int record_step_fast(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags
     // a single world's iterations are one launch: with bodies (which the
     // loop's launches do not couple in), for WIG_STEP_PERSISTENT (then on a
     // cooperative grid at any size), and at the sizes where a cluster is the
-    // faster form; with its coarse levels on a cluster, and when profiled,
-    // they are the loop's launches
-    const bool by_size = one && ln.S.cluster == 0u && one->D.B <= wig::CLUSTER_BLOCKS;
+    // faster form (whose CTA 0 takes the coarse levels from the first that
+    // fits it, however high the coarse_cells knob starts them; but in the
+    // mixed form the knob says which levels stay FP32, and a level too large
+    // for one CTA does so on the cluster of the loop's coarse kernel); when
+    // profiled, they are the loop's launches
+    const bool by_size = one && one->D.B <= wig::CLUSTER_BLOCKS && !(ln.Bt.mixed && ln.S.cluster);
     const bool one_launch = (flags & WIG_STEP_PERSISTENT) || bodies || by_size;
     const bool solve = one_launch && (capture || bodies || (flags & WIG_STEP_PERSISTENT));
     if (solve) {
