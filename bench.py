@@ -623,7 +623,7 @@ def tuned_summary(shapes, trials):
         k: [[v, None if c is None else round(c, 4)] for v, c in r] for k, r in trials.items()}}),
         file=sys.stderr, flush=True)
     from worldinagrain_b200 import tune
-    return {"shapes": shapes, "steps": tune.steps_needed()}
+    return {"shapes": shapes, "steps": tune.steps_needed() if trials else 0}
 
 
 def launch_overrides(items):

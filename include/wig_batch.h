@@ -130,6 +130,8 @@ enum wig_launch_knob {
     WIG_LAUNCH_RELAX_PER_SM = 3,
     WIG_LAUNCH_KNOBS = 4
 };
+/* As wig_fluid_one_launch, of a batch of one world (0 of several). */
+int wig_batch_one_launch(const wig_batch* b);
 int wig_batch_set_launch(wig_batch* b, uint32_t knob, uint32_t value);
 int wig_batch_get_launch(const wig_batch* b, uint32_t knob, uint32_t* value);
 

@@ -399,9 +399,18 @@ enum wig_profile_slot {
 /* One step as wig_fluid_step, but launched pass by pass with CUDA events
  * around each launch (the reference's per-phase GPU timestamps,
  * js/timer.js:7-98): per slot, the summed milliseconds in ms_out and the
- * launches in calls_out (WIG_PROFILE_SLOTS entries each).  Synchronous. */
+ * launches in calls_out (WIG_PROFILE_SLOTS entries each).  Synchronous.  A
+ * small world's iterations, one launch of its steps (wig_fluid_one_launch),
+ * are profiled as the loop's kernels, a kernel a pass, which say where its
+ * time goes but not how much of it there is; the launches its statistics
+ * then report are a step's. */
 int wig_fluid_step_profile(wig_fluid* h, const wig_params* P, uint32_t max_cycles, uint32_t flags, double tolerance,
                            void* stream, float* ms_out, uint32_t* calls_out);
+
+/* 1 when this world's steps solve in one launch whatever their flags (up to
+ * 640 blocks, or with bodies bound): of the launch shapes below they read
+ * COARSE_CELLS alone, and a profiled step's times speak for none of them. */
+int wig_fluid_one_launch(const wig_fluid* h);
 
 /* The fast form's launch shapes of this world (knob: enum wig_launch_knob of
  * wig_batch.h, the same values and ranges): none changes a result.  No

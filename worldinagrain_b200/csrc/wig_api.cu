@@ -873,6 +873,13 @@ int record_step(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags, boo
     return WIG_OK;
 }
 
+// Whether the batch's steps solve in one launch whatever their flags: a world
+// with bodies, or alone and of a size where that is the faster form.
+bool solves_in_one_launch(const wig_batch* b) {
+    const wig::World* one = one_world(b);
+    return has_bodies(b) || (one && one->D.B <= wig::CLUSTER_BLOCKS);
+}
+
 // Records the fast form's step of the lane's worlds.  With `capture`, s is
 // capturing into a graph and the iterations become a WHILE node whose body
 // is captured on the lane's second stream; else the iterations are launched
@@ -916,8 +923,7 @@ int record_step_fast(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags
     // mixed form the knob says which levels stay FP32, and a level too large
     // for one CTA does so on the cluster of the loop's coarse kernel); when
     // profiled, they are the loop's launches
-    const bool by_size = one && one->D.B <= wig::CLUSTER_BLOCKS && !(ln.Bt.mixed && ln.S.cluster);
-    const bool one_launch = (flags & WIG_STEP_PERSISTENT) || bodies || by_size;
+    const bool one_launch = (flags & WIG_STEP_PERSISTENT) || (solves_in_one_launch(b) && !(ln.Bt.mixed && ln.S.cluster));
     const bool solve = one_launch && (capture || bodies || (flags & WIG_STEP_PERSISTENT));
     if (solve) {
         CUDA_TRY(wig::fast_solve(ln.Bt, *one, b->solve, (flags & WIG_STEP_PERSISTENT) != 0u, s, prof ? &mk : nullptr));
@@ -1454,6 +1460,8 @@ int wig_fluid_get_launch(const wig_fluid* h, uint32_t knob, uint32_t* value) {
     return wig_batch_get_launch(h->b, knob, value);
 }
 
+int wig_fluid_one_launch(const wig_fluid* h) { return h && h->b && solves_in_one_launch(h->b) ? 1 : 0; }
+
 int wig_fluid_read_stats(wig_fluid* h, wig_fluid_stats* out) {
     if (!h || !h->b) return fail(WIG_E_ARG, "null argument");
     const uint32_t w0 = 0;
@@ -1649,6 +1657,8 @@ int wig_batch_get_launch(const wig_batch* b, uint32_t knob, uint32_t* value) {
     }
     return WIG_OK;
 }
+
+int wig_batch_one_launch(const wig_batch* b) { return b && solves_in_one_launch(b) ? 1 : 0; }
 
 int wig_batch_set_lane_pool(wig_batch* b, uint32_t lane, uint64_t bytes) {
     if (!b) return fail(WIG_E_ARG, "null batch");

@@ -51,6 +51,8 @@ FUNCS = {
     "wig_fluid_set_launch": ([C.c_void_p, C.c_uint32, C.c_uint32], C.c_int),
     "wig_fluid_get_launch": ([C.c_void_p, C.c_uint32, C.POINTER(C.c_uint32)], C.c_int),
     "wig_batch_get_launch": ([C.c_void_p, C.c_uint32, C.POINTER(C.c_uint32)], C.c_int),
+    "wig_fluid_one_launch": ([C.c_void_p], C.c_int),
+    "wig_batch_one_launch": ([C.c_void_p], C.c_int),
     "wig_fluid_set_wait_limits": ([C.c_uint32, C.c_uint32], C.c_int),
 }
 
@@ -205,6 +207,11 @@ class LiquidStep:
     def launch_shapes(self):
         return {name: self.get_launch(name) for name in abi.LAUNCH_KNOBS}
 
+    def one_launch(self):
+        """Whether this world's steps solve in one launch, whatever their
+        flags (no profiled step then speaks for a launch shape)."""
+        return bool(lib().wig_fluid_one_launch(self.h))
+
     def dispatch(self, P, name, level=0, cycle=0):
         check(lib().wig_fluid_dispatch(self.h, C.byref(P), abi.PASS[name], level, cycle, self.stream), f"dispatch {name}")
 
@@ -346,3 +353,7 @@ class Batch:
 
     def launch_shapes(self):
         return {name: self.get_launch(name) for name in abi.LAUNCH_KNOBS}
+
+    def one_launch(self):
+        """Whether a batch of one world solves in one launch (LiquidStep.one_launch)."""
+        return bool(lib().wig_batch_one_launch(self.h))

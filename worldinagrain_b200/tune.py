@@ -22,6 +22,10 @@ step's cost per iteration drifts as the worlds move on. The candidates are
 therefore tried in two passes, in order and then in reverse, and each
 candidate's cost is taken over both of its steps: a drift that is linear
 over the knob's steps weighs the same on every candidate.
+
+A world whose steps solve in one launch (LiquidStep.one_launch) is not tuned:
+a profiled step runs the loop's kernels in that launch's place, so what it
+measures is not what the step runs.
 """
 
 from .fluid import WigError
@@ -79,8 +83,12 @@ def autotune(batch, step, knobs=KNOBS, passes=2):
     caller's worlds and returns Batch.step_profile's dict. Each candidate is
     stepped once a pass, the passes alternating in order and in reverse.
     Returns the chosen shapes and, per knob, the (value, cost) of each
-    candidate in the knob's order. The batch keeps the chosen shapes."""
+    candidate in the knob's order. The batch keeps the chosen shapes. A batch
+    whose one world solves in one launch keeps its shapes, with no step and
+    no trial."""
     trials = {}
+    if getattr(batch, "one_launch", bool)():
+        return batch.launch_shapes(), trials
     for name, candidates, slots in knobs:
         keep = batch.get_launch(name)
         ms = {v: 0.0 for v in candidates}
