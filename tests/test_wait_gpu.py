@@ -27,12 +27,12 @@ def test_every_cta_of_a_full_grid_gives_up(limit, lowered_limits):
     g = fluid.LiquidStep(world.copy(), W.element_table())
     lowered_limits(0, limit)
     for s in range(1, 4):
-        g.step(params(world, s), max_cycles=64, flags=TOL, tolerance=1e-6)
+        g.step(params(world, s), max_cycles=64, flags=TOL | abi.STEP_PERSISTENT, tolerance=1e-6)
         with pytest.raises(fluid.WigError, match="WIG_E_STATE.*barrier"):
             g.stats()
     lowered_limits(0, 0)
     got = []
-    for form in (0, abi.STEP_PLAIN):
+    for form in (abi.STEP_PERSISTENT, abi.STEP_PLAIN):
         g.upload(world)
         g.step(params(world, 1), max_cycles=64, flags=TOL | SHIFTED | form, tolerance=1e-6)
         cycles = g.stats().cycles

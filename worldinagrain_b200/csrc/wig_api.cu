@@ -886,8 +886,8 @@ bool solves_in_one_launch(const wig_batch* b) {
 // from the host, each decided by reading back the device's verdict (the
 // profiler's path).  *outside gets the kernels outside the loop (all of
 // them when not capturing), *body those of one iteration of the loop.
-int record_step_fast(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags, bool shifted, cudaStream_t s,
-                     Prof* prof, bool capture, uint32_t* outside, uint32_t* body) {
+int record_step_fast(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags, cudaStream_t s, Prof* prof, bool capture,
+                     uint32_t* outside, uint32_t* body) {
     Rec R{b, ln, s, prof};
     if ((flags & WIG_STEP_BOOKKEEPING_ONLY) && b->K == 1) {
         *outside = record_book(R);
@@ -1114,18 +1114,17 @@ int batch_step(wig_batch* b, const StepArgs& a) {
     uint32_t shape = a.flags & (WIG_STEP_TOLERANCE | WIG_STEP_F64_DOTS | WIG_STEP_PLAIN | WIG_STEP_PERSISTENT | WIG_STEP_MIXED);
     if (viscous) shape |= WIG_STEP_VISCOUS;
     if (book1) shape |= WIG_STEP_BOOKKEEPING_ONLY;
-    const bool parity_keyed = plain || (a.flags & WIG_STEP_PERSISTENT);
     uint32_t bucket = 0;
     ln.S = step_shape(b, a, &bucket);
     const uint64_t key = ((uint64_t)a.max_cycles << 32) | ((uint64_t)bucket << 24) | ((uint64_t)shape << 1) |
-                         ((parity_keyed && sh) ? 1u : 0u);
+                         ((plain && sh) ? 1u : 0u);  // (the plain form's launches know the tiling)
     auto it = ln.graphs.find(key);
     if (it == ln.graphs.end()) {
         Graph G;
         CUDA_TRY(cudaStreamBeginCapture(ln.cap, cudaStreamCaptureModeThreadLocal));
         uint32_t n = 0, nb = 0;
         const int rc2 = plain ? record_step(b, ln, a.max_cycles, shape, sh, ln.cap, nullptr, true, &n, &nb)
-                              : record_step_fast(b, ln, a.max_cycles, shape, sh, ln.cap, nullptr, true, &n, &nb);
+                              : record_step_fast(b, ln, a.max_cycles, shape, ln.cap, nullptr, true, &n, &nb);
         if (rc2) {
             std::string m = g_last_error;
             cudaGraph_t junk = nullptr;
@@ -1179,7 +1178,7 @@ int batch_step_profile(wig_batch* b, const StepArgs& a, float* ms_out, uint32_t*
         rc = record_step(b, ln, a.max_cycles, shape, sh, a.s, &prof, false, &n, &nb);
     } else {
         zero_dirty(b, a);
-        rc = record_step_fast(b, ln, a.max_cycles, shape, sh, a.s, &prof, false, &n, &nb);
+        rc = record_step_fast(b, ln, a.max_cycles, shape, a.s, &prof, false, &n, &nb);
     }
     if (rc) return rc;
     ln.last_launches = n;

@@ -1450,7 +1450,7 @@ __global__ void k_divergence(Batch Bt, const __grid_constant__ WorldSrc<ONE> src
 }
 
 // cgJoin's edges between blocks (to the right and below, from the block's
-// last column and row), after k_cgStartLocal has linked each block's own.
+// last column and row), after startLocal has linked each block's own.
 // An edge is left to the one before it along the border (above it, or to
 // its left) when both its cells have their links in common with that one's:
 // then joining that edge joins these two as well, and the first of such a
