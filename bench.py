@@ -146,6 +146,10 @@ def params(world, step, seed):
 # sides and density read, its way-up potentials written, 28 n in FP32.
 # Averaged over the launches of an iteration (s["levels"]: level_stats'
 # cells of each level's launches; s["mixed"]: the mixed form).
+# This is a dense model, of every cell of a level with all its words: the
+# kernels recompute the diagonal instead of storing it, and past a step's
+# first iteration read no words of tiles and cells without liquid, so they
+# move less than it counts.
 def level_bytes(name, s):
     L = s.get("levels")
     if not L:
@@ -192,18 +196,20 @@ def level_stats(worlds, coarse_cells=4096):
 # algorithmic bytes: the capture's traffic scaled to the launch by the units
 # it processes.
 TRAFFIC_PER_ALG_BYTE = {
-    # k_fDown on level 1 of the disks 1024x1024 world: 23.9 MB read, none
-    # written; 262,144 cells x 180 B
+    # k_fDown on level 1 of the disks 1024x1024 world in a step's first
+    # iteration, which works every tile: 23.9 MB read, none written; 262,144
+    # cells x 180 B.  The later ones read 18.8 MB (tiles and cells without
+    # liquid skipped), so the figure is an upper bound
     ("F_RESTRICT", False): (23.90272e6 / (262144 * 180), "k_fDown, level 1 (512x512) of the disks 1024x1024 world"),
-    # k_fDown on levels 1-3 of one iteration of a 64-world batch, mixed form,
-    # coarse cells 2048: 94.2 MB read and written; 153.3 MB algorithmic
+    # k_fDown on levels 1-3 of an iteration of a 64-world batch, mixed form,
+    # coarse cells 2048: 81.4 MB read and written; 153.3 MB algorithmic
     # (122 B a level-1 cell, 82 below: 1,043,904, 257,952 and 58,312 cells)
-    ("F_RESTRICT", True): (94.191616e6 / 153.289936e6, "k_fDown, levels 1-3 of one iteration of a 64-world mixed batch"),
-    # k_fRelax on the disks 1024x1024 world: 28.0 MB read, 0 written; 24.5 MB
-    # algorithmic (the mixed form reads 12 B a cell less: its coefficients'
-    # binary16 copies, no diagonal)
-    ("F_RELAX", False): (28.0e6 / 24.5e6, "k_fRelax, the disks 1024x1024 world"),
-    ("F_RELAX", True): (28.0e6 / 24.5e6, "k_fRelax, the disks 1024x1024 world"),
+    ("F_RESTRICT", True): (81.429504e6 / 153.289936e6, "k_fDown, levels 1-3 of one iteration of a 64-world mixed batch"),
+    # k_fRelax on the disks 1024x1024 world: 17.6 MB read, 0 written; 24.5 MB
+    # algorithmic (the coefficients and rims of cells not liquid are counted)
+    ("F_RELAX", False): (17.594368e6 / 24.487696e6, "k_fRelax, the disks 1024x1024 world"),
+    # the same on the 64-world mixed batch: 52.8 MB against 100.5 MB
+    ("F_RELAX", True): (52.840704e6 / 100.464392e6, "k_fRelax, a 64-world mixed batch"),
 }
 
 
