@@ -119,7 +119,7 @@ int wig_batch_world_bytes_split(const wig_world_desc* d, uint64_t* persistent, u
  * Defaults: COARSE_CELLS 4096, LEVEL_PER_SM 8, CG_PER_SM 2, RELAX_PER_SM 16;
  * for a batch of one world, as every wig_fluid handle is: COARSE_CELLS 2048,
  * LEVEL_PER_SM 32, CG_PER_SM 4, RELAX_PER_SM 64.
- * A single world's solve in one launch (up to 640 blocks, with bodies, with
+ * A single world's solve in one launch (wig_fluid_one_launch, or with
  * WIG_STEP_PERSISTENT) takes of them COARSE_CELLS alone.
  * No step of the batch may be in flight; the lanes' graphs are recaptured
  * at their next step. */
@@ -131,7 +131,7 @@ enum wig_launch_knob {
     WIG_LAUNCH_KNOBS = 4
 };
 /* As wig_fluid_one_launch, of a batch of one world (0 of several). */
-int wig_batch_one_launch(const wig_batch* b);
+int wig_batch_one_launch(const wig_batch* b, void* stream);
 int wig_batch_set_launch(wig_batch* b, uint32_t knob, uint32_t value);
 int wig_batch_get_launch(const wig_batch* b, uint32_t knob, uint32_t* value);
 

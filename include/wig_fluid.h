@@ -232,10 +232,9 @@ typedef struct wig_fluid_buffers {
 #define WIG_STEP_F64_DOTS 32u         /* CG dot products in FP64 */
 #define WIG_STEP_SYNC_STATS 64u       /* copy the stats to the host at the end of the step */
 #define WIG_STEP_PLAIN 128u           /* the solve as one kernel per reference pass (else the fast form) */
-#define WIG_STEP_PERSISTENT 256u      /* the fast form's iterations as one cooperative kernel at any size (else in one launch on a
-                                         cluster up to 640 blocks, kernels in a graph WHILE loop above): from about 640x640
-                                         cells up to 6% faster for a world alone on the GPU, but no other work runs beside
-                                         its solve */
+#define WIG_STEP_PERSISTENT 256u      /* the fast form's iterations as one cooperative kernel at any size, beside whose solve no other
+                                         work runs (else in one launch on a cluster up to 640 blocks, so too above 4096 on the
+                                         legacy stream, kernels in a graph WHILE loop between and on other streams) */
 #define WIG_STEP_MIXED 512u           /* mixed precision (fast form, with TOLERANCE and F64_DOTS): the multigrid levels
                                          stored in 16 bits and worked in FP32 (each coarse level's density and stencil
                                          coefficients in binary16, its potentials, right-hand sides and way-up potentials
@@ -400,17 +399,21 @@ enum wig_profile_slot {
  * around each launch (the reference's per-phase GPU timestamps,
  * js/timer.js:7-98): per slot, the summed milliseconds in ms_out and the
  * launches in calls_out (WIG_PROFILE_SLOTS entries each).  Synchronous.  A
- * small world's iterations, one launch of its steps (wig_fluid_one_launch),
+ * world's iterations that are one launch of its steps (wig_fluid_one_launch)
  * are profiled as the loop's kernels, a kernel a pass, which say where its
  * time goes but not how much of it there is; the launches its statistics
  * then report are a step's. */
 int wig_fluid_step_profile(wig_fluid* h, const wig_params* P, uint32_t max_cycles, uint32_t flags, double tolerance,
                            void* stream, float* ms_out, uint32_t* calls_out);
 
-/* 1 when this world's steps solve in one launch whatever their flags (up to
- * 640 blocks, or with bodies bound): of the launch shapes below they read
- * COARSE_CELLS alone, and a profiled step's times speak for none of them. */
-int wig_fluid_one_launch(const wig_fluid* h);
+/* 1 when this world's steps on `stream` solve in one launch whatever their
+ * flags: up to 640 blocks, with bodies bound, or (on every multiprocessor, no
+ * other work running beside it) above 4096 blocks on the legacy stream, 0,
+ * which takes turns with a host's blocking streams in any case.  A host that
+ * steps a large world beside other work gives it a stream of its own.  Of the
+ * launch shapes below such steps read COARSE_CELLS alone, and a profiled
+ * step's times speak for none of them. */
+int wig_fluid_one_launch(const wig_fluid* h, void* stream);
 
 /* The fast form's launch shapes of this world (knob: enum wig_launch_knob of
  * wig_batch.h, the same values and ranges): none changes a result.  No

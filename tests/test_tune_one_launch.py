@@ -31,17 +31,23 @@ def test_a_one_launch_world_keeps_its_shapes_without_a_step():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("size,bodies,one", [((200, 200), False, True), ((208, 200), False, False),
-                                             ((520, 520), False, False), ((300, 240), True, True)])
-def test_which_worlds_solve_in_one_launch(size, bodies, one):
-    """The library's word on it against the launches a step reports: the same
-    whatever its iterations, or more with each."""
+@pytest.mark.parametrize("size,bodies,legacy,own", [((200, 200), False, True, True), ((208, 200), False, False, False),
+                                                    ((512, 512), False, False, False), ((520, 512), False, True, False),
+                                                    ((300, 240), True, True, True)])
+@pytest.mark.parametrize("stream", ["legacy", "own"])
+def test_which_worlds_solve_in_one_launch(size, bodies, legacy, own, stream):
+    """The library's word on it against the launches a step reports, on the
+    legacy stream and on one of its own: the same whatever its iterations, or
+    more with each."""
+    import torch
     from worldinagrain_b200 import fluid
+    one = legacy if stream == "legacy" else own
+    s = torch.cuda.Stream()
     if bodies:
         w, table = W.bodies_world(*size, stamps=False)
     else:
         w = W.disks_world(*size, n_disks=8, r_lo=3, r_hi=10, seed=12)
-    g = fluid.LiquidStep(w, W.body_element_table())
+    g = fluid.LiquidStep(w, W.body_element_table(), stream=0 if stream == "legacy" else s.cuda_stream)
     if bodies:
         g.bind_bodies(table)
     assert g.one_launch() is one
@@ -58,8 +64,10 @@ def test_which_worlds_solve_in_one_launch(size, bodies, one):
 @pytest.mark.gpu
 def test_a_batch_says_it_of_one_world_only():
     from worldinagrain_b200 import fluid
-    worlds = [W.dam_break(64, 64, seed=2), W.dam_break(96, 64, seed=3)]
-    for ws, one in ((worlds[:1], True), (worlds, False)):
+    import torch
+    s = torch.cuda.Stream().cuda_stream
+    small, large = [W.dam_break(64, 64, seed=2), W.dam_break(96, 64, seed=3)], [W.dam_break(520, 520, seed=2)]
+    for ws, one in ((small[:1], (True, True)), (small, (False, False)), (large, (True, False))):
         b = fluid.Batch(ws, W.element_table())
-        assert b.one_launch() is one
+        assert (b.one_launch(), b.one_launch(stream=s)) == one
         b.close()

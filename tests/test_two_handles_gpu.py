@@ -1,5 +1,6 @@
-"""Worlds of two handles stepped at once on two streams: each ends as it does
-alone, bit for bit, and large ones run beside one another."""
+"""Worlds of two handles stepped at once on two streams (or the legacy stream
+and one beside it): each ends as it does alone, bit for bit, and large ones
+on streams of their own run beside one another."""
 import pytest
 
 from worldinagrain_b200 import abi
@@ -12,14 +13,14 @@ pytestmark = pytest.mark.gpu
 TOL = abi.STEP_TOLERANCE | abi.STEP_F64_DOTS
 
 
-def _handles(make, n, bodies=False):
+def _handles(make, n, bodies=False, legacy=False):
     import torch
     from worldinagrain_b200 import fluid
     out = []
     for k in range(n):
         s = torch.cuda.Stream()
         w, table = make(k) if bodies else (make(k), None)
-        g = fluid.LiquidStep(w, W.body_element_table(), stream=s.cuda_stream)
+        g = fluid.LiquidStep(w, W.body_element_table(), stream=0 if legacy and k == 0 else s.cuda_stream)
         if bodies:
             g.bind_bodies(table)
         out.append((g, w, s))
@@ -32,7 +33,7 @@ def _step(handles, first, last, flags):
             g.step(params(w, k), max_cycles=64, flags=flags, tolerance=1e-6)
 
 
-@pytest.mark.parametrize("case", ["cluster", "loop", "large", "large_grid", "mixed", "bodies", "bodies_grid"])
+@pytest.mark.parametrize("case", ["cluster", "loop", "large", "large_grid", "large_legacy", "mixed", "bodies", "bodies_grid"])
 def test_two_worlds_at_once_end_as_alone(case):
     flags = TOL | {"large_grid": abi.STEP_PERSISTENT, "mixed": abi.STEP_MIXED}.get(case, 0)
     size = {"cluster": (160, 160), "loop": (256, 256), "bodies": (96, 80), "bodies_grid": (512, 512)}.get(case, (520, 520))
@@ -45,12 +46,12 @@ def test_two_worlds_at_once_end_as_alone(case):
 
     alone = []
     for k in range(2):
-        hs = _handles(lambda _: make(k), 1, bodies)
+        hs = _handles(lambda _: make(k), 1, bodies, case == "large_legacy")
         _step(hs, 1, 4, flags)
         hs[0][0].stats(unconverged_ok=True)
         alone.append(hs[0][0].download())
         hs[0][0].close()
-    hs = _handles(make, 2, bodies)
+    hs = _handles(make, 2, bodies, case == "large_legacy")
     _step(hs, 1, 4, flags)
     for (g, w, _), want in zip(hs, alone):
         g.stats(unconverged_ok=True)

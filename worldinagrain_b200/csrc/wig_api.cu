@@ -873,12 +873,16 @@ int record_step(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags, boo
     return WIG_OK;
 }
 
-// Whether the batch's steps solve in one launch whatever their flags: a world
-// with bodies, or alone and of a size where that is the faster form.
-bool solves_in_one_launch(const wig_batch* b) {
+// Whether the batch's steps on stream s solve in one launch whatever their
+// flags: a world with bodies, or alone and of a size where that is the faster
+// form there.
+bool solves_in_one_launch(const wig_batch* b, cudaStream_t s) {
     const wig::World* one = one_world(b);
-    return has_bodies(b) || (one && one->D.B <= wig::CLUSTER_BLOCKS);
+    const bool legacy = s == nullptr || s == cudaStreamLegacy;
+    return has_bodies(b) || (one && (one->D.B <= wig::CLUSTER_BLOCKS || (legacy && one->D.B > wig::GRID_BLOCKS)));
 }
+// (a step's shape flag, past WIG_STEP_*: it does)
+constexpr uint32_t SHAPE_ONE_LAUNCH = 1u << 12;
 
 // Records the fast form's step of the lane's worlds.  With `capture`, s is
 // capturing into a graph and the iterations become a WHILE node whose body
@@ -917,13 +921,13 @@ int record_step_fast(wig_batch* b, Lane& ln, uint32_t max_cycles, uint32_t flags
     R.launches++;
     // a single world's iterations are one launch: with bodies (which the
     // loop's launches do not couple in), for WIG_STEP_PERSISTENT (then on a
-    // cooperative grid at any size), and at the sizes where a cluster is the
-    // faster form (whose CTA 0 takes the coarse levels from the first that
-    // fits it, however high the coarse_cells knob starts them; but in the
-    // mixed form the knob says which levels stay FP32, and a level too large
-    // for one CTA does so on the cluster of the loop's coarse kernel); when
-    // profiled, they are the loop's launches
-    const bool one_launch = (flags & WIG_STEP_PERSISTENT) || (solves_in_one_launch(b) && !(ln.Bt.mixed && ln.S.cluster));
+    // cooperative grid at any size), and at the sizes and on the stream where
+    // it is the faster form (whose CTA 0 takes the coarse levels from the
+    // first that fits it, however high the coarse_cells knob starts them; but
+    // in the mixed form the knob says which levels stay FP32, and a level too
+    // large for one CTA does so on the cluster of the loop's coarse kernel);
+    // when profiled, they are the loop's launches
+    const bool one_launch = (flags & WIG_STEP_PERSISTENT) || ((flags & SHAPE_ONE_LAUNCH) && !(ln.Bt.mixed && ln.S.cluster));
     const bool solve = one_launch && (capture || bodies || (flags & WIG_STEP_PERSISTENT));
     if (solve) {
         CUDA_TRY(wig::fast_solve(ln.Bt, *one, b->solve, (flags & WIG_STEP_PERSISTENT) != 0u, s, prof ? &mk : nullptr));
@@ -1113,6 +1117,7 @@ int batch_step(wig_batch* b, const StepArgs& a) {
     const bool book1 = b->K == 1 && ((a.world_flags ? a.world_flags[0] : a.flags) & WIG_STEP_BOOKKEEPING_ONLY) != 0u;
     uint32_t shape = a.flags & (WIG_STEP_TOLERANCE | WIG_STEP_F64_DOTS | WIG_STEP_PLAIN | WIG_STEP_PERSISTENT | WIG_STEP_MIXED);
     if (viscous) shape |= WIG_STEP_VISCOUS;
+    if (!plain && solves_in_one_launch(b, a.s)) shape |= SHAPE_ONE_LAUNCH;
     if (book1) shape |= WIG_STEP_BOOKKEEPING_ONLY;
     uint32_t bucket = 0;
     ln.S = step_shape(b, a, &bucket);
@@ -1168,6 +1173,7 @@ int batch_step_profile(wig_batch* b, const StepArgs& a, float* ms_out, uint32_t*
     const bool book1 = b->K == 1 && ((a.world_flags ? a.world_flags[0] : a.flags) & WIG_STEP_BOOKKEEPING_ONLY) != 0u;
     uint32_t shape = a.flags & (WIG_STEP_TOLERANCE | WIG_STEP_F64_DOTS | WIG_STEP_PLAIN | WIG_STEP_PERSISTENT | WIG_STEP_MIXED);
     if (viscous) shape |= WIG_STEP_VISCOUS;
+    if (!plain && solves_in_one_launch(b, a.s)) shape |= SHAPE_ONE_LAUNCH;
     if (book1) shape |= WIG_STEP_BOOKKEEPING_ONLY;
     Prof prof;
     ln.last_body = 0;
@@ -1459,7 +1465,9 @@ int wig_fluid_get_launch(const wig_fluid* h, uint32_t knob, uint32_t* value) {
     return wig_batch_get_launch(h->b, knob, value);
 }
 
-int wig_fluid_one_launch(const wig_fluid* h) { return h && h->b && solves_in_one_launch(h->b) ? 1 : 0; }
+int wig_fluid_one_launch(const wig_fluid* h, void* stream) {
+    return h && h->b && solves_in_one_launch(h->b, (cudaStream_t)stream) ? 1 : 0;
+}
 
 int wig_fluid_read_stats(wig_fluid* h, wig_fluid_stats* out) {
     if (!h || !h->b) return fail(WIG_E_ARG, "null argument");
@@ -1657,7 +1665,9 @@ int wig_batch_get_launch(const wig_batch* b, uint32_t knob, uint32_t* value) {
     return WIG_OK;
 }
 
-int wig_batch_one_launch(const wig_batch* b) { return b && solves_in_one_launch(b) ? 1 : 0; }
+int wig_batch_one_launch(const wig_batch* b, void* stream) {
+    return b && solves_in_one_launch(b, (cudaStream_t)stream) ? 1 : 0;
+}
 
 int wig_batch_set_lane_pool(wig_batch* b, uint32_t lane, uint64_t bytes) {
     if (!b) return fail(WIG_E_ARG, "null batch");

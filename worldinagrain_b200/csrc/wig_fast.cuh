@@ -32,18 +32,20 @@ struct SolveShape {
     uint32_t grid, cluster, lc;
 };
 constexpr uint32_t SOLVE_CLUSTER = 16;
-// A single world of up to this many blocks solves in one launch, on a
+// A single world of up to CLUSTER_BLOCKS blocks solves in one launch, on a
 // cluster, whose barrier is the cheapest but whose 16 multiprocessors are few
 // (a step of a pond of 75x52 200 us against 218 as the loop's launches, of the
 // dam at 192x192 673 against 724, of two liquids at 224x224 928 against 890).
-// Larger ones run the loop's launches.  A grid of all the multiprocessors is
-// 5% faster there for a world alone on the GPU at 640x640 to 1024x1024 (the
-// disks at 1024x1024 4940 us a step against 5220; the dam at 520x520 814
-// against 791, the 2048x2048 column 11330 against 11220), but nothing else
-// runs beside it: two worlds stepped at once on two streams take turns (dams
-// at 520x520 756 us a step each against 489, four 724 against 323, four of
-// the disks at 1024x1024 4660 against 3170).
-constexpr uint32_t CLUSTER_BLOCKS = 640;
+// One of more than GRID_BLOCKS does so on a grid of all the multiprocessors,
+// stepped on the legacy stream: 5-9% faster at 640x640 to 1024x1024 (the disks
+// at 1024x1024 4617 us a step against 5034 as the loop's launches; at 512x512
+// 1595 against 1554, the dam at 520x520 814 against 791, the 2048x2048 column
+// 11330 against 11220).  Nothing else runs beside such a solve, so a world
+// stepped on a stream of its own, as a host gives one that it means to run
+// beside other work, keeps the loop's launches: two dams at 520x520 at once
+// take 489 us a step each so and 756 with grids, four 323 and 724, four of the
+// disks at 1024x1024 3170 and 4660.
+constexpr uint32_t CLUSTER_BLOCKS = 640, GRID_BLOCKS = 4096;
 // A grid's CTAs: a tile of the fine level for every other warp, at most a
 // CTA a multiprocessor (a tile a warp is 1% slower at 256x256, 4 or 8 tiles
 // a CTA the same).

@@ -51,8 +51,8 @@ FUNCS = {
     "wig_fluid_set_launch": ([C.c_void_p, C.c_uint32, C.c_uint32], C.c_int),
     "wig_fluid_get_launch": ([C.c_void_p, C.c_uint32, C.POINTER(C.c_uint32)], C.c_int),
     "wig_batch_get_launch": ([C.c_void_p, C.c_uint32, C.POINTER(C.c_uint32)], C.c_int),
-    "wig_fluid_one_launch": ([C.c_void_p], C.c_int),
-    "wig_batch_one_launch": ([C.c_void_p], C.c_int),
+    "wig_fluid_one_launch": ([C.c_void_p, C.c_void_p], C.c_int),
+    "wig_batch_one_launch": ([C.c_void_p, C.c_void_p], C.c_int),
     "wig_fluid_set_wait_limits": ([C.c_uint32, C.c_uint32], C.c_int),
 }
 
@@ -208,9 +208,10 @@ class LiquidStep:
         return {name: self.get_launch(name) for name in abi.LAUNCH_KNOBS}
 
     def one_launch(self):
-        """Whether this world's steps solve in one launch, whatever their
-        flags (no profiled step then speaks for a launch shape)."""
-        return bool(lib().wig_fluid_one_launch(self.h))
+        """Whether this world's steps on its stream solve in one launch,
+        whatever their flags (no profiled step then speaks for a launch
+        shape)."""
+        return bool(lib().wig_fluid_one_launch(self.h, self.stream))
 
     def dispatch(self, P, name, level=0, cycle=0):
         check(lib().wig_fluid_dispatch(self.h, C.byref(P), abi.PASS[name], level, cycle, self.stream), f"dispatch {name}")
@@ -354,6 +355,6 @@ class Batch:
     def launch_shapes(self):
         return {name: self.get_launch(name) for name in abi.LAUNCH_KNOBS}
 
-    def one_launch(self):
+    def one_launch(self, stream=0):
         """Whether a batch of one world solves in one launch (LiquidStep.one_launch)."""
-        return bool(lib().wig_batch_one_launch(self.h))
+        return bool(lib().wig_batch_one_launch(self.h, C.c_void_p(stream or None)))
