@@ -224,6 +224,9 @@ void dev_shape(wig::Dev& D, const wig_world_layout& L) {
     }
 }
 
+// Bytes of a world's column sums (none of a world whose passes use none).
+size_t col64_bytes(const wig::Dev& D) { return D.B > wig::COMPACT_BLOCKS ? wig::COL64_VALUES * sizeof(double) : 0u; }
+
 // Bytes of a world's fast scratch and FP64 partials.
 size_t scratch_bytes(const wig::Dev& D) {
     const size_t C = D.C;
@@ -235,7 +238,7 @@ size_t scratch_bytes(const wig::Dev& D) {
         bytes += align256(5u * (size_t)D.level_w[l] * D.level_h[l] * 2u);  // the binary16 operator
     }
     bytes += align256(2u * (size_t)D.B * 4u) + 3u * align256(2u * (size_t)D.B * 8u);
-    bytes += 2u * align256((size_t)D.B * 4u) + align256((size_t)D.B * 8u) + align256(512u * 8u);
+    bytes += 2u * align256((size_t)D.B * 4u) + align256((size_t)D.B * 8u) + col64_bytes(D);
     return bytes;
 }
 
@@ -270,7 +273,7 @@ void scratch_take(wig::World& Wd, char* p, uint32_t coarse_cells) {
     F.part64 = reinterpret_cast<double*>(take(2u * (size_t)D.B * 8u));
     F.pq32 = fl(D.B);
     F.pq64 = reinterpret_cast<double*>(take((size_t)D.B * 8u));
-    F.col64 = reinterpret_cast<double*>(take(512u * 8u));
+    F.col64 = reinterpret_cast<double*>(take(col64_bytes(D)));
     F.base = reinterpret_cast<uint32_t*>(take((size_t)D.B * 4u));
     D.part64 = reinterpret_cast<double*>(take(2u * (size_t)D.B * 8u));
     D.norm64 = reinterpret_cast<double*>(take(2u * (size_t)D.B * 8u));

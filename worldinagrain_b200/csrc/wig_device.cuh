@@ -423,6 +423,10 @@ struct LvlH {
     uint32_t pad_;
 };
 
+// A single world of more blocks than this is compacted in two launches; only
+// such worlds use FastW::col64, and have one.
+constexpr uint32_t COMPACT_BLOCKS = 4096, COL64_VALUES = 512;
+
 // A world's fast-form scratch.
 struct FastW {
     Fine Z;                    // level 0
@@ -434,7 +438,7 @@ struct FastW {
     double* part64;            // the same in FP64
     float* pq32;               // cgApply's partial sums, of block b at b
     double* pq64;
-    double* col64;             // 512 column sums of a group's block sums
+    double* col64;             // COL64_VALUES column sums of a group's block sums (worlds of more than COMPACT_BLOCKS blocks)
     uint32_t* base;            // each active block's first place in `sorted`
     uint32_t lc;               // first level the one-CTA coarse kernel solves
 };

@@ -2483,6 +2483,7 @@ struct GridGroup {
 // CTAs (a warp a column) and a barrier more; below, every CTA sums them all
 // itself (a round of loads for 4096 blocks, about 1 us).
 constexpr uint32_t SPLIT_BLOCKS = 8192;
+static_assert(SPLIT_BLOCKS >= COMPACT_BLOCKS && COL64_VALUES >= 2u * 256u, "a splitting world has its columns' memory");
 
 // sumBlocks of NC components of the partials, for every CTA of the group
 // (all its threads): the sums in s[256 c].  col: 512 values of scratch.

@@ -675,7 +675,7 @@ __global__ void __launch_bounds__(1024) k_compact(Batch Bt, const __grid_constan
 // their states and their part of the lists, past the counts before them.
 // One CTA of 1024 threads, each block's 9 marks read by one thread of it,
 // took 64 us of a step at 1024x1024 and 404 us at 2048x2048.
-constexpr uint32_t COMPACT_BLOCKS = 4096, COMPACT_CHUNKS = 512;
+constexpr uint32_t COMPACT_CHUNKS = COL64_VALUES;  // two counts a chunk, in FastW::col64
 __global__ void __launch_bounds__(1024) k_compactFlags(const __grid_constant__ World Wd) {
     const Dev& D = Wd.D;
     const W w(D);
