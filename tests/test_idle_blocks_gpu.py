@@ -247,3 +247,38 @@ def test_blocks_dropped_without_retiring(size):
     assert got[0][1] == got[1][1]
     diffs = compare_worlds(got[0][0], got[1][0], scratch=True)
     assert not diffs, "; ".join(diffs)
+
+
+@pytest.mark.parametrize("size", SIZES)
+def test_a_world_whose_bodies_are_unbound(size):
+    """A host writes all of a world's buffers while bodies are bound (which
+    needs no bind), then unbinds them."""
+    import torch
+    saved = _box(*size)
+    g = _handle(saved, "plain")
+    _steps(g, saved, 1, 3, TOL | abi.STEP_PLAIN)
+    g.download()
+    _empty_the_top(saved)
+    g.upload()
+    _steps(g, saved, 4, 4, TOL | abi.STEP_PLAIN)
+    g.download()
+    g.close()
+    got = []
+    for form in (0, abi.STEP_PLAIN):
+        w = _box(*size)
+        g = _handle(w, "bodies")
+        _steps(g, w, 1, 3, TOL | form)
+        torch.cuda.synchronize()
+        for name in abi.BUFFER_NAMES:
+            a = np.ascontiguousarray(getattr(saved, name)).view(np.uint8).reshape(-1)
+            torch.as_tensor(_Bytes(getattr(g.buffers(), name), a.size), device="cuda").copy_(torch.from_numpy(a.copy()))
+        torch.cuda.synchronize()
+        g.bind_bodies(None)
+        cycles = _steps(g, saved, 5, 6, TOL | form)
+        g.download(w)
+        g.close()
+        assert _beside_idle(w) > size[0] // 2
+        got.append((w, cycles))
+    assert got[0][1] == got[1][1]
+    diffs = compare_worlds(got[0][0], got[1][0], scratch=True)
+    assert not diffs, "; ".join(diffs)

@@ -1378,6 +1378,8 @@ int wig_fluid_bind_bodies(wig_fluid* h, void* motion, void* pushes, void* stamps
     b->hw[0].D.motion = static_cast<uint32_t*>(motion);
     b->hw[0].D.pushes = static_cast<uint32_t*>(pushes);
     b->hw[0].D.stamps = motion ? static_cast<uint32_t*>(stamps) : nullptr;
+    // (with bodies bound the host may have written its buffers with no bind)
+    b->dirty[0] = 1;
     return upload_world_entry(b, 0);
 }
 
